@@ -51,6 +51,7 @@ __global__ void recompute_kernel(CorrArgs a) {
   const long long n = (long long)cnt < a.cand_cap ? (long long)cnt : a.cand_cap;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  unsigned long long n_edge = 0, n_1e6 = 0;  // lane 0's counts, added once per warp
   for (long long c = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); c < n;
        c += nwarps) {
     const uint2 p = a.cand[c];
@@ -66,10 +67,10 @@ __global__ void recompute_kernel(CorrArgs a) {
     if (e) {
       atomicAdd(&a.seg[(size_t)(j / kBlk) * a.n_pad + i], 1);
       atomicAdd(&a.seg[(size_t)(i / kBlk) * a.n_pad + j], 1);
-      atomicAdd(&a.stats[0], 1ull);
+      ++n_edge;
     }
     const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
-    if (fabsf((absm ? fabsf(r) : r) - a.th.tau) <= 1e-6f) atomicAdd(&a.stats[1], 1ull);
+    if (fabsf((absm ? fabsf(r) : r) - a.th.tau) <= 1e-6f) ++n_1e6;
     unsigned long long h = hash64(key) & a.hmask;
     bool stored = false;
     for (unsigned long long probe = 0; probe <= a.hmask; ++probe) {
@@ -84,6 +85,8 @@ __global__ void recompute_kernel(CorrArgs a) {
     }
     if (!stored) atomicOr(a.err, ERR_HASH_FULL);
   }
+  if (n_edge) atomicAdd(&a.stats[0], n_edge);
+  if (n_1e6) atomicAdd(&a.stats[1], n_1e6);
 }
 
 // Gather the candidates flagged in the sub-tiles' edge lists into the

@@ -295,6 +295,7 @@ __global__ void dens_decide_kernel(CorrArgs a, DensState* ds, const uint8_t* cls
   const long long n = c < a.cand_cap ? c : a.cand_cap;
   const float tau = ds->tau;
   const int n_drop = ds->n_drop;
+  unsigned int n_edge = 0, n_1e6 = 0;  // this thread's counts, added once per warp
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const uint8_t k = cls[i];
@@ -307,12 +308,12 @@ __global__ void dens_decide_kernel(CorrArgs a, DensState* ds, const uint8_t* cls
     if (k == 2) {
       r = slot_val[i];
       e = r > tau || (r == tau && !(n_drop > 0 && in_sorted(drop, n_drop, key)));
-      if (fabsf(r - tau) <= 1e-6f) atomicAdd(&a.stats[1], 1ull);
+      if (fabsf(r - tau) <= 1e-6f) ++n_1e6;
     }
     if (e) {
       atomicAdd(&a.seg[(size_t)(pj / kBlk) * a.n_pad + pi], 1);
       atomicAdd(&a.seg[(size_t)(pi / kBlk) * a.n_pad + pj], 1);
-      atomicAdd(&a.stats[0], 1ull);
+      ++n_edge;
     }
     unsigned long long h = hash64(key) & a.hmask;
     bool stored = false;
@@ -327,6 +328,12 @@ __global__ void dens_decide_kernel(CorrArgs a, DensState* ds, const uint8_t* cls
       h = (h + 1) & a.hmask;
     }
     if (!stored) atomicOr(a.err, ERR_HASH_FULL);
+  }
+  n_edge = __reduce_add_sync(0xffffffffu, n_edge);
+  n_1e6 = __reduce_add_sync(0xffffffffu, n_1e6);
+  if ((threadIdx.x & 31) == 0) {
+    if (n_edge) atomicAdd(&a.stats[0], (unsigned long long)n_edge);
+    if (n_1e6) atomicAdd(&a.stats[1], (unsigned long long)n_1e6);
   }
 }
 

@@ -69,10 +69,68 @@ __device__ __forceinline__ bool round_sum_u128(unsigned __int128 acc, unsigned _
   return true;
 }
 
-// The reference value of a pair: float(sum_t double(float(z_it * z_jt))), the
-// double sum in time order (CorMat.cpp:955-964).  A warp evaluates one pair:
-// lanes take t = lane, lane+32, ...; the products are summed exactly in
-// fixed point at the scale of the smallest one.  (1) When every product is
+// The reference value of a pair is float(sum_t double(float(z_it * z_jt))),
+// the double sum in time order (CorMat.cpp:955-964).  A warp evaluates one
+// pair.  First in float-float: lanes take four time steps at a time, sum their
+// products exactly as h + (rounding errors) by TwoSum (Knuth) and the errors c
+// in float, then join by a butterfly of the same.  The rows have unit norm, so
+// sum |p_t| <= 1.01 (Cauchy-Schwarz) bounds every partial sum; with n products
+// per lane c holds n + 5 errors of at most 2^-24 each, added with as many
+// roundings, so |h + c - sum p_t| <= 1.01 (n + 6)^2 2^-48, and the reference's
+// loop lies within 1.01 T 2^-53 of sum p_t.  When no float rounding midpoint
+// lies within both of h + c, the float nearest to h + c is the reference's
+// (all but about 2^-15 of the pairs at T = 240, 2^-11 at T = 1200).
+// Padding columns T .. ldz - 1 of the rows are zero and add nothing.
+// Bound: L2 reads of the two rows.  Of the candidates of a TF32 pass (713,000,
+// T = 355) the fixed-point form alone took 1,118 us.
+__device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
+                                            const float* __restrict__ zj, int T, int lane,
+                                            float* out) {
+  const float4* a4 = reinterpret_cast<const float4*>(zi);
+  const float4* b4 = reinterpret_cast<const float4*>(zj);
+  const int nq = (T + 3) >> 2;
+  float h = 0.0f, c = 0.0f;
+  auto add = [&](float p) {
+    const float s = __fadd_rn(h, p);
+    const float bb = __fsub_rn(s, h);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(p, bb)));
+    h = s;
+  };
+#pragma unroll 2
+  for (int q = lane; q < nq; q += 32) {
+    const float4 a = __ldg(a4 + q), b = __ldg(b4 + q);
+    add(__fmul_rn(a.x, b.x));
+    add(__fmul_rn(a.y, b.y));
+    add(__fmul_rn(a.z, b.z));
+    add(__fmul_rn(a.w, b.w));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, h, o);
+    const float oc = __shfl_xor_sync(0xffffffffu, c, o);
+    c = __fadd_rn(c, oc);
+    add(oh);
+  }
+  // q + l == h + c exactly (TwoSum), q the nearest float
+  const float q = __fadd_rn(h, c);
+  const float bb = __fsub_rn(q, h);
+  const float l = __fadd_rn(__fsub_rn(h, __fsub_rn(q, bb)), __fsub_rn(c, bb));
+  const float n6 = (float)(((nq + 31) >> 5) * 4 + 6);
+  const float bound = 1.02f * (n6 * n6 * 3.5527137e-15f /* 2^-48 */ +
+                               (float)T * 1.1102230e-16f /* 2^-53 */);
+  const uint32_t qb = __float_as_uint(q);
+  const uint32_t e8 = (qb >> 23) & 0xFFu;
+  *out = q;
+  if (e8 < 26u || e8 > 253u) return false;
+  // half the spacing to the neighbouring floats (a quarter below a power of two)
+  const float half = __uint_as_float((e8 - ((qb & 0x7FFFFFu) ? 24u : 25u)) << 23);
+  return __fsub_rn(half, fabsf(l)) > bound;
+}
+
+// The reference value of a pair, raw (NaN for a voxel with a NaN z-score);
+// exact_r_warp_z gives it after post_block's clamp.  Pairs that sum_pair_ff
+// does not decide are summed exactly in fixed point at the scale of the
+// smallest product: lanes take t = lane, lane+32, ....  (1) When every product is
 // normal, the int64 sum cannot overflow and sum |p_t| < 2^53 units of the
 // smallest ulp, every partial sum of the sequential double loop is
 // representable, so that loop equals the exact sum: an int64 reduction.
@@ -80,13 +138,8 @@ __device__ __forceinline__ bool round_sum_u128(unsigned __int128 acc, unsigned _
 // 128-bit fixed point and its float is the reference's unless a rounding
 // midpoint lies within the loop's rounding bound (round_sum_u128).  (3) Only
 // then, or with subnormal or non-finite products, does lane 0 run the
-// sequential double adds.  Returns the raw value (NaN for a voxel with a NaN
-// z-score); exact_r_warp_z gives it after post_block's clamp.
-__device__ __forceinline__ float exact_r_warp_raw(const float* z, const uint8_t* bad, int ldz,
-                                                  int T, int i, int j, int lane) {
-  if (bad[i] | bad[j]) return __int_as_float(0x7fc00000);  // NaN
-  const float* zi = z + (size_t)i * ldz;
-  const float* zj = z + (size_t)j * ldz;
+// sequential double adds.
+static __device__ __noinline__ float exact_r_fixed(const float* zi, const float* zj, int T, int lane) {
   int emin = 1 << 20, emax = -(1 << 20);
   bool special = false;
 #pragma unroll 4
@@ -151,6 +204,16 @@ __device__ __forceinline__ float exact_r_warp_raw(const float* z, const uint8_t*
     r = __double2float_rn(s);
   }
   return __shfl_sync(0xffffffffu, r, 0);
+}
+
+__device__ __forceinline__ float exact_r_warp_raw(const float* z, const uint8_t* bad, int ldz,
+                                                  int T, int i, int j, int lane) {
+  if (bad[i] | bad[j]) return __int_as_float(0x7fc00000);  // NaN
+  const float* zi = z + (size_t)i * ldz;
+  const float* zj = z + (size_t)j * ldz;
+  float r;
+  if (sum_pair_ff(zi, zj, T, lane, &r)) return r;
+  return exact_r_fixed(zi, zj, T, lane);
 }
 
 __device__ __forceinline__ float exact_r_warp_z(const float* z, const uint8_t* bad, int ldz,
