@@ -149,18 +149,22 @@ int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st) {
   ENSURE(S_BLOCKBAD, (size_t)a.nb, bb);
   CK(launch_block_bad(a.bad, a.nb, bb, st));
   ctx->klaunch += 1;
-  if (ctx->tiles_nb != a.nb || ctx->tiles_band != ctx->band_now) {
+  return tc_tiles(ctx, a.nb, st);
+}
+
+int32_t tc_tiles(bna_ctx* ctx, int nb, cudaStream_t st) {
+  if (ctx->tiles_nb != nb || ctx->tiles_band != ctx->band_now) {
     // built on the device in stream order: no host wait for the work ahead
-    const long long nt = tc_tile_count(a.nb);
+    const long long nt = tc_tile_count(nb);
     // every s-th tile: the sample the density histogram may be taken on
     const int s = (int)std::max<long long>(1, nt / kSampleTiles);
     const long long nsmp = (nt + s - 1) / s;
     int2 *d, *ds;
     ENSURE(S_TILES, (size_t)nt * sizeof(int2), d);
     ENSURE(S_TILES_SMP, (size_t)nsmp * sizeof(int2), ds);
-    CK(launch_tile_lists(a.nb, ctx->band_now, d, nsmp, s, ds, st));
+    CK(launch_tile_lists(nb, ctx->band_now, d, nsmp, s, ds, st));
     ctx->klaunch += 2;
-    ctx->tiles_nb = a.nb;
+    ctx->tiles_nb = nb;
     ctx->tiles_band = ctx->band_now;
     ctx->ntiles = (int)nt;
     ctx->ntiles_smp = (int)nsmp;
@@ -217,11 +221,6 @@ void window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, in
 
 int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cudaStream_t st,
                   bool sampled) {
-  if (ctx->avg) {  // the averaged matrix is the source
-    CK(launch_corr_packed(a, pass, st));
-    ctx->klaunch += 1;
-    return BNA_OK;
-  }
   switch (precision) {
     case BNA_PREC_FP32:
       CK(launch_corr_simt(a, pass, st));
@@ -237,10 +236,15 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
       CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
       for (int t0 = 0; t0 < nt; t0 += per, ++ctx->klaunch) {
         if (t0 > 0) gate(ctx, st, BNA_PHASE_CORR, t0);
-        CK(launch_corr_tc(a, pass, precision == BNA_PREC_BF16X3 ? 0 : 1, tiles + t0,
-                          std::min(per, nt - t0),
-                          reinterpret_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]), nullptr, 0,
-                          ctx->sms, sched, st));
+        if (ctx->avg)
+          CK(launch_corr_tc_avg(a, pass, precision == BNA_PREC_BF16X3 ? 0 : 1, ctx->avg->tc,
+                                ctx->avg->S, ctx->avg->fisher, tiles + t0, std::min(per, nt - t0),
+                                nullptr, ctx->sms, sched, st));
+        else
+          CK(launch_corr_tc(a, pass, precision == BNA_PREC_BF16X3 ? 0 : 1, tiles + t0,
+                            std::min(per, nt - t0),
+                            reinterpret_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]), nullptr, 0,
+                            ctx->sms, sched, st));
       }
       return BNA_OK;
     }
@@ -512,8 +516,9 @@ int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
 }
 
 // Everything after the z-scores: count pass(es), candidates, density rule,
-// scan, fill.  With ctx->avg set (multi-subject average) the count pass reads
-// the averaged matrix and candidates get their exact averaged value.
+// scan, fill.  With ctx->avg set (multi-subject average) the count pass takes
+// the averages of the subjects' tiles and candidates get their exact averaged
+// value.
 int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
                            const bna_corr_opts* opts, int prec, double delta, bna_csr* out_dev,
                            bna_corr_stats* stats, cudaStream_t st) {
@@ -544,12 +549,12 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   // ---- threshold of the count pass
   long long k_dens = 0;  // density: exact undirected edge count (CorMat.cpp:327-329)
   if (density) k_dens = bna_density_nnz(N, opts->value) / 2;
-  const bool tc = prec != BNA_PREC_FP32 && !ctx->avg;
+  const bool tc = prec != BNA_PREC_FP32;
   // density with a tensor-core form: the k-th value is selected on the device;
   // its window comes first from a histogram of sampled tiles, and from the
   // full histogram if the sample's window missed
-  bool sampled = density && k_dens > 0 && tc && ctx->ntiles >= 4 * kSampleTiles;
-  bool dev_sel = density && k_dens > 0 && tc;
+  bool sampled = density && k_dens > 0 && tc && !ctx->avg && ctx->ntiles >= 4 * kSampleTiles;
+  bool dev_sel = density && k_dens > 0 && tc && !ctx->avg;
   double winA = 0, winB = 0;
   int passes = 0;
   float* cvals = nullptr;

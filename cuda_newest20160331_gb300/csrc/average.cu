@@ -3,42 +3,39 @@
 // correlation matrix (.cormat) entry point.
 #include "ctx.cuh"
 
-// The multi-subject sums: every subject's z-scores (kept in the arena for the
-// exact recompute; their table goes to subj_dev) and pass 4 over all tiles,
-// into packed / unc (zeroed here), then the division / inverse transform.
-static int32_t avg_accumulate(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev,
-                              int32_t N, const int32_t* T, int fisher, int prec, double delta_opt,
-                              float* packed, uint32_t* unc, void** subj_dev_out, double* dsum,
-                              cudaStream_t st) {
+// Every subject's z-scores (FP32 for the exact values, the form's operands
+// for the tensor-core pass) and the subjects' two tables.
+static int32_t avg_subjects(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev, int32_t N,
+                            const int32_t* T, int fisher, int prec, double delta_opt,
+                            bna_ctx::Avg* out, double* dsum, cudaStream_t st) {
   const int n_pad = round_up(N, kBlk), nb = n_pad / kBlk;
-  const long long M1 = (long long)N * (N - 1) / 2;
-  size_t zoff_total = 0;
-  int ldb_max = 0;
-  std::vector<size_t> zoff(nsub);
+  const bool split = prec == BNA_PREC_BF16X3;
+  size_t zn = 0, bn = 0;
+  std::vector<size_t> zoff(nsub), boff(nsub);
   for (int k = 0; k < nsub; ++k) {
-    zoff[k] = zoff_total;
-    zoff_total += (size_t)n_pad * round_up(T[k], 32);
-    ldb_max = std::max(ldb_max, round_up(T[k], 64));
+    zoff[k] = zn;
+    boff[k] = bn;
+    zn += (size_t)n_pad * round_up(T[k], 32);
+    bn += (size_t)n_pad * round_up(T[k], 64);
   }
   float* zall;
-  uint8_t* badall;
-  void* subj_dev;
-  void* vstat;
+  uint8_t *badall, *bballs;
+  void *subj_dev, *tc_dev, *vstat;
   uint16_t *zhi = nullptr, *zlo = nullptr;
-  ENSURE(S_AVG_Z, zoff_total * sizeof(float), zall);
+  ENSURE(S_AVG_Z, zn * sizeof(float), zall);
   ENSURE(S_AVG_BAD, (size_t)nsub * n_pad, badall);
+  ENSURE(S_BLOCKBAD, (size_t)nsub * nb, bballs);
   ENSURE(S_AVG_SUBJ, (size_t)nsub * avg_subj_bytes(), subj_dev);
+  ENSURE(S_AVG_TC, (size_t)nsub * tc_subj_bytes(), tc_dev);
   ENSURE(S_VSTAT, zscore_scratch_bytes(n_pad), vstat);
-  if (prec == BNA_PREC_BF16X3) {
-    ENSURE(S_ZHI, (size_t)n_pad * ldb_max * 2, zhi);
-    ENSURE(S_ZLO, (size_t)n_pad * ldb_max * 2, zlo);
+  if (split) {
+    ENSURE(S_AVG_ZHI, bn * 2, zhi);
+    ENSURE(S_AVG_ZLO, bn * 2, zlo);
   }
-  CK(cudaMemsetAsync(packed, 0, (size_t)M1 * sizeof(float), st));
-  CK(cudaMemsetAsync(unc, 0, (size_t)((M1 + 31) / 32) * sizeof(uint32_t), st));
   std::vector<char> subj_host((size_t)nsub * avg_subj_bytes());
+  std::vector<char> tc_host((size_t)nsub * tc_subj_bytes());
   *dsum = 0;
   for (int k = 0; k < nsub; ++k) {
-    // subject k: z-scores, then its values added into the sums in file order
     CorrArgs as{};
     as.n = N;
     as.n_pad = n_pad;
@@ -47,37 +44,28 @@ static int32_t avg_accumulate(bna_ctx* ctx, int32_t nsub, const float* const* bo
     as.ldz = round_up(T[k], 32);
     as.ldb = round_up(T[k], 64);
     as.z = zall + zoff[k];
-    as.zhi = zhi;
-    as.zlo = zlo;
+    as.zhi = split ? zhi + boff[k] : nullptr;
+    as.zlo = split ? zlo + boff[k] : nullptr;
     as.bad = badall + (size_t)k * n_pad;
-    CK(launch_zscore(bold_dev[k], N, T[k], n_pad, const_cast<float*>(as.z), as.ldz, zhi, zlo,
-                     as.ldb, const_cast<uint8_t*>(as.bad), vstat, st));
-    ctx->klaunch += 2;
-    int32_t s = tc_prepare(ctx, as, st);
-    if (s) return s;
+    uint8_t* bb = bballs + (size_t)k * nb;
+    CK(launch_zscore(bold_dev[k], N, T[k], n_pad, const_cast<float*>(as.z), as.ldz,
+                     const_cast<uint16_t*>(as.zhi), const_cast<uint16_t*>(as.zlo), as.ldb,
+                     const_cast<uint8_t*>(as.bad), vstat, st));
+    CK(launch_block_bad(as.bad, nb, bb, st));
+    ctx->klaunch += 3;
     const double dk = delta_opt > 0 ? delta_opt : default_delta(prec, T[k]);
     *dsum += dk;
-    as.th.mode = BNA_THR_R_GE;
-    as.th.tau = 2.0f;
-    as.th.delta = (float)dk;
-    AvgPass ap{packed, unc, fisher ? 1 : 0, fisher ? 0.9f : (float)(1.0 - dk)};
-    const int2* tiles = reinterpret_cast<const int2*>(ctx->ptr[S_TILES]);
-    const int per = ctx->tiles_per_launch > 0 ? ctx->tiles_per_launch : ctx->ntiles;
-    unsigned int* sched;
-    ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
-    CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
-    for (int t0 = 0; t0 < ctx->ntiles; t0 += per, ++ctx->klaunch)
-      CK(launch_corr_tc(as, 4, prec == BNA_PREC_BF16X3 ? 0 : 1, tiles + t0,
-                        std::min(per, ctx->ntiles - t0),
-                        reinterpret_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]), nullptr, 0,
-                        ctx->sms, sched, st, &ap));
     avg_subj_fill(subj_host.data(), k, as.z, as.bad, as.ldz, T[k]);
+    if (!tc_subj_fill(tc_host.data(), k, as, bb, split ? 0 : 1,
+                      fisher ? 0.9f : (float)(1.0 - dk)))
+      return fail(ctx, BNA_CUDA_ERROR, "multi-subject call: tensor map encoding failed");
   }
+  const int32_t s = tc_tiles(ctx, nb, st);
+  if (s) return s;
   CK(cudaMemcpyAsync(subj_dev, subj_host.data(), subj_host.size(), cudaMemcpyHostToDevice, st));
-  CK(launch_avg_finalize(packed, M1, nsub, fisher ? 1 : 0, ctx->sms, st));
-  ctx->klaunch += 1;
-  CK(cudaStreamSynchronize(st));  // subj_host is released at return
-  *subj_dev_out = subj_dev;
+  CK(cudaMemcpyAsync(tc_dev, tc_host.data(), tc_host.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaStreamSynchronize(st));  // the host tables are released at return
+  *out = bna_ctx::Avg{subj_dev, tc_dev, nsub, fisher ? 1 : 0};
   return BNA_OK;
 }
 
@@ -118,19 +106,13 @@ int32_t bna_corr_csr_avg(bna_ctx* ctx, int32_t nsub, const float* const* bold_de
   ctx->klaunch = 0;
   ctx->last_ok = false;
   const int n_pad = round_up(N, kBlk), nb = n_pad / kBlk;
-  const long long M1 = (long long)N * (N - 1) / 2;
-  float* packed;
-  uint32_t* unc;
   uint8_t* badz;
-  ENSURE(S_AVG_PACKED, (size_t)M1 * sizeof(float), packed);
-  ENSURE(S_AVG_UNC, (size_t)((M1 + 31) / 32) * sizeof(uint32_t), unc);
   ENSURE(S_AVG_BADZ, (size_t)n_pad, badz);
   CK(cudaMemsetAsync(badz, 0, (size_t)n_pad, st));
   CK(cudaEventRecord(ctx->ev[0], st));
-  void* subj_dev = nullptr;
+  bna_ctx::Avg ac{};
   double dsum = 0;
-  s = avg_accumulate(ctx, nsub, bold_dev, N, T, fisher, prec, opts->delta, packed, unc,
-                     &subj_dev, &dsum, st);
+  s = avg_subjects(ctx, nsub, bold_dev, N, T, fisher, prec, opts->delta, &ac, &dsum, st);
   if (s) return s;
   CK(cudaEventRecord(ctx->ev[1], st));
   // bound of |average~ - average| (per-subject bounds, the float sums and
@@ -147,9 +129,6 @@ int32_t bna_corr_csr_avg(bna_ctx* ctx, int32_t nsub, const float* const* bold_de
   a.T = 1;
   a.ldz = 32;
   a.bad = badz;
-  a.avg_packed = packed;
-  a.avg_unc = unc;
-  const bna_ctx::Avg ac{subj_dev, nsub, fisher ? 1 : 0};
   ctx->avg = &ac;
   s = corr_csr_core(ctx, a, N, 1, opts, prec, davg, out_dev, stats, st);
   ctx->avg = nullptr;
@@ -167,12 +146,32 @@ int32_t bna_corr_packed(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev
   cudaStream_t st = as_stream(stream);
   ctx->klaunch = 0;
   ctx->last_ok = false;
-  const long long M1 = (long long)N * (N - 1) / 2;
-  uint32_t* unc;
-  ENSURE(S_AVG_UNC, (size_t)((M1 + 31) / 32) * sizeof(uint32_t), unc);
-  void* subj_dev = nullptr;
+  bna_ctx::Avg ac{};
   double dsum = 0;
-  return avg_accumulate(ctx, nsub, bold_dev, N, T, fisher, precision, 0.0, packed_dev, unc,
-                        &subj_dev, &dsum, st);
+  s = avg_subjects(ctx, nsub, bold_dev, N, T, fisher, precision, 0.0, &ac, &dsum, st);
+  if (s) return s;
+  CorrArgs a{};
+  a.n = N;
+  a.n_pad = round_up(N, kBlk);
+  a.nb = a.n_pad / kBlk;
+  a.th.mode = BNA_THR_R_GE;
+  a.th.tau = 2.0f;
+  DevStatus* ds;
+  ENSURE(S_STATUS, sizeof(DevStatus), ds);
+  CK(cudaMemsetAsync(ds, 0, sizeof(DevStatus), st));
+  a.err = &ds->err;
+  const int2* tiles = reinterpret_cast<const int2*>(ctx->ptr[S_TILES]);
+  const int per = ctx->tiles_per_launch > 0 ? ctx->tiles_per_launch : ctx->ntiles;
+  unsigned int* sched;
+  ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
+  CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
+  for (int t0 = 0; t0 < ctx->ntiles; t0 += per, ++ctx->klaunch)
+    CK(launch_corr_tc_avg(a, 4, precision == BNA_PREC_BF16X3 ? 0 : 1, ac.tc, nsub, ac.fisher,
+                          tiles + t0, std::min(per, ctx->ntiles - t0), packed_dev, ctx->sms,
+                          sched, st));
+  DevStatus* hs = reinterpret_cast<DevStatus*>(ctx->pinned);
+  CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (hs->err & ERR_TIMEOUT) return fail(ctx, BNA_TIMEOUT, "packed matrix: a bounded wait expired");
+  return BNA_OK;
 }
-

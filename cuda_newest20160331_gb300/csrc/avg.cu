@@ -5,10 +5,9 @@
 // one packed float matrix (post_block with its fishtran flag, :847-883: r is
 // added - or fishertrans(r) - only when -1 <= r <= 1), divides by the number
 // of subjects (and applies inv_fishertrans), then thresholds the result like
-// a single subject's matrix.  Here the accumulation is the tensor-core pass 4
-// (approximate r~ of every pair, corr_tc.cu), these kernels finish the
-// average, and the count pass reads the averaged values instead of a GEMM.
-// Pairs whose average lies near the threshold (or where some subject's r~ is
+// a single subject's matrix.  Here the tensor-core kernel (corr_tc.cu) adds up
+// every subject's approximate r~ tile by tile and thresholds the average in
+// the same pass, without a matrix in memory.  Pairs whose average lies near the threshold (or where some subject's r~ is
 // near +-1, where post_block's rule or the Fisher transform is sensitive) get
 // their exact average: every subject's reference r (float products, time-
 // order double sum), the same float accumulation, division and transforms.
@@ -22,16 +21,6 @@ struct SubjZ {
   const uint8_t* bad;
   int ldz, T;
 };
-
-__global__ void avg_finalize_kernel(float* packed, long long m, int S, int fisher) {
-  const float fs = (float)S;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m;
-       i += (long long)gridDim.x * blockDim.x) {
-    float v = __fdiv_rn(packed[i], fs);
-    if (fisher) v = fisher_r(v);
-    packed[i] = v;
-  }
-}
 
 // Exact averaged value of every candidate slot (warp per candidate).
 __global__ void avg_exact_kernel(CorrArgs a, const SubjZ* __restrict__ subj, int S, int fisher,
@@ -56,12 +45,6 @@ __global__ void avg_exact_kernel(CorrArgs a, const SubjZ* __restrict__ subj, int
     if (fisher) v = fisher_r(v);
     if (lane == 0) out[c] = v;
   }
-}
-
-cudaError_t launch_avg_finalize(float* packed, long long m, int S, int fisher, int sms,
-                                cudaStream_t st) {
-  avg_finalize_kernel<<<sms * 8, 256, 0, st>>>(packed, m, S, fisher);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_avg_exact(const CorrArgs& a, const void* subj, int S, int fisher, float* out,

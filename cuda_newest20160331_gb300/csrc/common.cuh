@@ -68,14 +68,6 @@ __device__ __forceinline__ float fisher_r(float z) {
   return __fdiv_rn(__fsub_rn(e, 1.0f), __fadd_rn(e, 1.0f));
 }
 
-// Multi-subject average pass (tensor-core pass 4) buffers.
-struct AvgPass {
-  float* packed;       // [n(n-1)/2] running sums, upper triangle row-major
-  uint32_t* uncertain; // one bit per pair
-  int fisher;
-  float unc_lim;
-};
-
 // 1 + 1e-6 as the 2mm tools compare it, (double)r <= 1.0 + 1e-6: the largest
 // float not above it is 1 + 8 * 2^-23.
 constexpr float kEpsHi = 1.00000095367431640625f;
@@ -152,16 +144,7 @@ struct CorrArgs {
   unsigned int* hist;         // density histogram pass: kHistBins + 1 counters
   const float* cand_val;      // density: exact values of the candidates (decide pass)
   float* cand_apx;            // density (tensor-core count pass): r~ of every candidate slot
-  // multi-subject average: the averaged values (packed upper triangle) replace
-  // the GEMM as the source of the plain count pass; uncertain pairs are
-  // candidates
-  const float* avg_packed;
-  const uint32_t* avg_unc;
 };
-
-__host__ __device__ __forceinline__ long long packed_index(int i, int j, int n) {
-  return (long long)i * (2LL * n - i - 1) / 2 + (j - i - 1);  // i < j, row-major
-}
 
 // Fill-pass store with a range check (an inconsistent count would otherwise
 // write outside the CSR).

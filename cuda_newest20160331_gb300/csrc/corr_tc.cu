@@ -88,6 +88,7 @@ struct TcSubj {  // 64-byte aligned through its CUtensorMap members
   CorrArgs a;
   const uint8_t* blockbad;
   int nksteps;
+  float unc_lim;  // average: |r~| from which a pair is recomputed exactly (Fisher z: <= 0.9)
 };
 
 constexpr size_t TC_SMEM_BYTES = 1024 + (size_t)TC_RING_BYTES + sizeof(TcSmem);
@@ -95,13 +96,11 @@ static_assert(TC_SMEM_BYTES <= 232448, "shared memory per CTA");
 
 struct TcArgs {
   CorrArgs a;
-  // pass 4 (multi-subject average, post_block with accumulation,
-  // W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:847-883): packed[idx(i, j)] += r~
-  // or its Fisher z; pairs with |r~| >= unc_lim get their uncertain bit
-  float* packed;
-  uint32_t* uncertain;
+  // multi-subject average (AVG): every tile adds up the values of subj[0 ..
+  // nsub); pass 4 writes the averages to packed[idx(i, j)]
+  int nsub;
   int fisher;
-  float unc_lim;
+  float* packed;
   // multi-subject count pass: tiles4 = (I, J-pair, subject), subj the table
   const int4* tiles4;
   const TcSubj* subj;
@@ -144,6 +143,20 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 
+// Fisher z of |r| < 1/2: atanh r = r + r x P(x), x = r^2, P fitted at Chebyshev
+// nodes (error below 4e-8; the logarithm's float form is off by up to 1.1e-7).
+// It keeps the average's epilogue (8 instructions a value instead of about 45)
+// near the tensor-core time of a tile.
+__device__ __forceinline__ float fisher_z_half(float r) {
+  const float x = __fmul_rn(r, r);
+  float q = 0.15813737f;
+  q = __fmaf_rn(q, x, 0.064550176f);
+  q = __fmaf_rn(q, x, 0.11478221f);
+  q = __fmaf_rn(q, x, 0.14263242f);
+  q = __fmaf_rn(q, x, 0.20000497f);
+  q = __fmaf_rn(q, x, 0.33333331f);
+  return __fmaf_rn(r, __fmul_rn(q, x), r);
+}
 // Bounded barrier of the 128 threads of one half (mbarrier based, so a lost
 // peer cannot hang the CTA).
 __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
@@ -159,7 +172,14 @@ __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
 // chunk together with their approximate value (a.cand_apx), which the device
 // selection of the k-th largest value needs.
 // MULTI: the tiles of several subjects in one persistent launch (count pass).
-template <int PASS, bool ABS, int FORM, bool DENS, bool MULTI = false>
+// AVG: the average over subjects (W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:418-670):
+// each tile runs through the subjects in order, and a thread keeps the running
+// sums of its 128 pairs in registers (post_block's accumulation, :847-883: r~
+// or its Fisher z, values outside [-1, 1] skipped), then takes the average
+// through the same epilogue as one subject's values.  No N (N - 1) / 2 matrix
+// is held: adding each subject into one in HBM, 4 bytes per lane in 32
+// different rows, took 4.07 ms per subject at N = 20,000, T = 180-300.
+template <int PASS, bool ABS, int FORM, bool DENS, bool MULTI = false, bool AVG = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     corr_tc_kernel(const __grid_constant__ CUtensorMap tm_hi,
                    const __grid_constant__ CUtensorMap tm_lo, const TcArgs p) {
@@ -197,7 +217,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     ptx::tmem_alloc(ptx::smem_u32(&S.tmem_base), TC_TMEM_COLS);
     ptx::tmem_relinquish();
   }
-  if (!MULTI && warp == 0 && lane == 0) {
+  if (!MULTI && !AVG && warp == 0 && lane == 0) {
     ptx::prefetch_tensormap(&tm_hi);
     if (FORM == FORM_BF16X3) ptx::prefetch_tensormap(&tm_lo);
   }
@@ -206,6 +226,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   ptx::tc_fence_after();
   const uint32_t tmem = S.tmem_base;
   const int nkb = (p.nksteps + 3) / 4;
+  const int nsub = AVG ? p.nsub : 1;  // accumulations per tile
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -234,43 +255,46 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         t_next = (int)atomicAdd(p.sched, 1u);
         int2 tile;
-        const CUtensorMap* mh = &tm_hi;
-        const CUtensorMap* ml = &tm_lo;
-        int nkb_t = nkb;
-        if (MULTI) {
-          const int4 t4 = p.tiles4[t];
-          tile = make_int2(t4.x, t4.y);
-          mh = &p.subj[t4.z].hi;
-          ml = &p.subj[t4.z].lo;
-          nkb_t = (p.subj[t4.z].nksteps + 3) / 4;
-        } else {
+        if (MULTI)
+          tile = make_int2(p.tiles4[t].x, p.tiles4[t].y);
+        else
           tile = p.tiles[t];
-        }
-        for (int kb = 0; kb < nkb_t; ++kb, ++f) {
-          const int s = f % TC_STAGES;
-          const uint32_t round = f / TC_STAGES;
-          const uint32_t empty = ptx::smem_u32(&S.empty[s]);
-          if (!ptx::mbar_wait(empty, (round & 1u) ^ 1u, kWaitNs)) {
-            atomicOr(a.err, ERR_TIMEOUT);
-            S.abort = 1;
-            break;
+        for (int sub = 0; sub < nsub && !S.abort; ++sub) {
+          const CUtensorMap* mh = &tm_hi;
+          const CUtensorMap* ml = &tm_lo;
+          int nkb_t = nkb;
+          if (MULTI || AVG) {
+            const TcSubj& e = p.subj[MULTI ? p.tiles4[t].z : sub];
+            mh = &e.hi;
+            ml = &e.lo;
+            nkb_t = (e.nksteps + 3) / 4;
           }
-          const uint32_t full = ptx::smem_u32(&S.full[s]);
-          const uint32_t base = ptx::smem_u32(smem + (size_t)s * TC_STAGE_BYTES);
-          ptx::mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
-          const int k0 = kb * F::kElemsPerBlock;
-          const int ra = tile.x * TC_BM, rb = tile.y * TC_BN;
-          // stage layout: A parts, then B parts (B = two 128-row boxes each)
-          ptx::tma_load_2d(base, mh, full, k0, ra);
-          if (FORM == FORM_BF16X3) ptx::tma_load_2d(base + TC_A_BYTES, ml, full, k0, ra);
-          const uint32_t bb = base + F::kParts * TC_A_BYTES;
-          ptx::tma_load_2d(bb, mh, full, k0, rb);
-          ptx::tma_load_2d(bb + TC_B_BYTES / 2, mh, full, k0, rb + 128);
-          if (FORM == FORM_BF16X3) {
-            ptx::tma_load_2d(bb + TC_B_BYTES, ml, full, k0, rb);
-            ptx::tma_load_2d(bb + TC_B_BYTES + TC_B_BYTES / 2, ml, full, k0, rb + 128);
+          for (int kb = 0; kb < nkb_t; ++kb, ++f) {
+            const int s = f % TC_STAGES;
+            const uint32_t round = f / TC_STAGES;
+            const uint32_t empty = ptx::smem_u32(&S.empty[s]);
+            if (!ptx::mbar_wait(empty, (round & 1u) ^ 1u, kWaitNs)) {
+              atomicOr(a.err, ERR_TIMEOUT);
+              S.abort = 1;
+              break;
+            }
+            const uint32_t full = ptx::smem_u32(&S.full[s]);
+            const uint32_t base = ptx::smem_u32(smem + (size_t)s * TC_STAGE_BYTES);
+            ptx::mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
+            const int k0 = kb * F::kElemsPerBlock;
+            const int ra = tile.x * TC_BM, rb = tile.y * TC_BN;
+            // stage layout: A parts, then B parts (B = two 128-row boxes each)
+            ptx::tma_load_2d(base, mh, full, k0, ra);
+            if (FORM == FORM_BF16X3) ptx::tma_load_2d(base + TC_A_BYTES, ml, full, k0, ra);
+            const uint32_t bb = base + F::kParts * TC_A_BYTES;
+            ptx::tma_load_2d(bb, mh, full, k0, rb);
+            ptx::tma_load_2d(bb + TC_B_BYTES / 2, mh, full, k0, rb + 128);
+            if (FORM == FORM_BF16X3) {
+              ptx::tma_load_2d(bb + TC_B_BYTES, ml, full, k0, rb);
+              ptx::tma_load_2d(bb + TC_B_BYTES + TC_B_BYTES / 2, ml, full, k0, rb + 128);
+            }
+            last_round[s] = (int)round;
           }
-          last_round[s] = (int)round;
         }
       }
       publish(-1);  // the end (on a timeout the readers' own bounded waits end)
@@ -286,6 +310,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       constexpr uint32_t idesc = FORM == FORM_BF16X3 ? ptx::make_idesc(1, 1, TC_BM, TC_BN)
                                                      : ptx::make_idesc(2, 2, TC_BM, TC_BN);
       uint32_t f = 0;
+      int u = 0;  // accumulations issued
       bool ok = true;
       for (int m = 0; !S.abort; ++m) {
         const int qs = m % kTileQ;
@@ -296,47 +321,51 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int t = S.tq[qs];
         ptx::mbar_arrive(ptx::smem_u32(&S.qempty[qs]));
         if (t < 0) break;
-        const int acc = m & 1;
-        const uint32_t ar = (uint32_t)(m >> 1);
-        if (!ptx::mbar_wait(ptx::smem_u32(&S.tempty[acc]), (ar & 1u) ^ 1u, kWaitNs)) {
-          ok = false;
-          break;
-        }
-        ptx::tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(acc * TC_BN);
-        const int nkb_t = MULTI ? (p.subj[p.tiles4[t].z].nksteps + 3) / 4 : nkb;
-        const int nks_t = MULTI ? p.subj[p.tiles4[t].z].nksteps : p.nksteps;
-        for (int kb = 0; kb < nkb_t; ++kb, ++f) {
-          const int s = f % TC_STAGES;
-          const uint32_t round = f / TC_STAGES;
-          if (!ptx::mbar_wait(ptx::smem_u32(&S.full[s]), round & 1u, kWaitNs)) {
+        for (int sub = 0; sub < nsub && ok; ++sub, ++u) {
+          const int acc = u & 1;
+          const uint32_t ar = (uint32_t)(u >> 1);
+          if (!ptx::mbar_wait(ptx::smem_u32(&S.tempty[acc]), (ar & 1u) ^ 1u, kWaitNs)) {
             ok = false;
             break;
           }
           ptx::tc_fence_after();
-          const uint32_t base = ptx::smem_u32(smem + (size_t)s * TC_STAGE_BYTES);
-          const int steps = min(4, nks_t - kb * 4);
-          if (FORM == FORM_BF16X3) {
-            for (int kk = 0; kk < steps; ++kk) {
-              const uint64_t ahi = ptx::sw128_desc(base + kk * 32);
-              const uint64_t alo = ptx::sw128_desc(base + TC_A_BYTES + kk * 32);
-              const uint64_t bhi = ptx::sw128_desc(base + 2 * TC_A_BYTES + kk * 32);
-              const uint64_t blo = ptx::sw128_desc(base + 2 * TC_A_BYTES + TC_B_BYTES + kk * 32);
-              ptx::mma_bf16(d, ahi, bhi, idesc, (kb | kk) != 0);
-              ptx::mma_bf16(d, ahi, blo, idesc, 1);
-              ptx::mma_bf16(d, alo, bhi, idesc, 1);
+          const uint32_t d = tmem + (uint32_t)(acc * TC_BN);
+          int nks_t = p.nksteps;
+          if (MULTI || AVG) nks_t = p.subj[MULTI ? p.tiles4[t].z : sub].nksteps;
+          const int nkb_t = (nks_t + 3) / 4;
+          for (int kb = 0; kb < nkb_t; ++kb, ++f) {
+            const int s = f % TC_STAGES;
+            const uint32_t round = f / TC_STAGES;
+            if (!ptx::mbar_wait(ptx::smem_u32(&S.full[s]), round & 1u, kWaitNs)) {
+              ok = false;
+              break;
             }
-          } else {
-            for (int kk = 0; kk < steps; ++kk) {
-              const uint64_t ad = ptx::sw128_desc(base + kk * 32);
-              const uint64_t bd = ptx::sw128_desc(base + TC_A_BYTES + kk * 32);
-              ptx::mma_tf32(d, ad, bd, idesc, (kb | kk) != 0);
+            ptx::tc_fence_after();
+            const uint32_t base = ptx::smem_u32(smem + (size_t)s * TC_STAGE_BYTES);
+            const int steps = min(4, nks_t - kb * 4);
+            if (FORM == FORM_BF16X3) {
+              for (int kk = 0; kk < steps; ++kk) {
+                const uint64_t ahi = ptx::sw128_desc(base + kk * 32);
+                const uint64_t alo = ptx::sw128_desc(base + TC_A_BYTES + kk * 32);
+                const uint64_t bhi = ptx::sw128_desc(base + 2 * TC_A_BYTES + kk * 32);
+                const uint64_t blo =
+                    ptx::sw128_desc(base + 2 * TC_A_BYTES + TC_B_BYTES + kk * 32);
+                ptx::mma_bf16(d, ahi, bhi, idesc, (kb | kk) != 0);
+                ptx::mma_bf16(d, ahi, blo, idesc, 1);
+                ptx::mma_bf16(d, alo, bhi, idesc, 1);
+              }
+            } else {
+              for (int kk = 0; kk < steps; ++kk) {
+                const uint64_t ad = ptx::sw128_desc(base + kk * 32);
+                const uint64_t bd = ptx::sw128_desc(base + TC_A_BYTES + kk * 32);
+                ptx::mma_tf32(d, ad, bd, idesc, (kb | kk) != 0);
+              }
             }
+            ptx::mma_commit(ptx::smem_u32(&S.empty[s]));
           }
-          ptx::mma_commit(ptx::smem_u32(&S.empty[s]));
+          if (ok) ptx::mma_commit(ptx::smem_u32(&S.tfull[acc]));
         }
         if (!ok) break;
-        ptx::mma_commit(ptx::smem_u32(&S.tfull[acc]));
       }
       if (!ok) {
         atomicOr(a.err, ERR_TIMEOUT);
@@ -354,6 +383,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // this warp's copy of the current subject's arguments (shared memory)
     CorrArgs& a = S.eargs[warp - 2];
     float tau = 0, delta = 0, lim = 0, lo_thr = 0;
+    float zlo = 0;  // AVG: an average Fisher z below it is no edge and no candidate
     bool simple = false, zero_int = false;
     uint32_t hphase = 0;
     // this warp's current edge-list chunk [wcur, wend) and candidate chunk
@@ -391,6 +421,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       simple = (tau < lim) && (ABS || lo_thr > 0.0f);
       // a pair with a NaN voxel has the exact value 0 (post_block); in the 2mm
       // tools' rule it stays NaN and is never an edge
+      // zlo with a margin for the transforms' errors
+      if (AVG)
+        zlo = PASS == 0 && simple && lo_thr > 0.0f ? fisher_z(lo_thr) * 0.99999f - 1e-5f
+                                                   : -INFINITY;
       zero_int = a.th.mode != BNA_THR_R_EPS && ((0.0f >= lo_thr) || (0.0f >= lim));
       if (PASS == 0) {
         long long x = 0;
@@ -437,6 +471,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       const int jj = 2 * tl.y + h;
       fj = jj < nbs ? bbad[jj] : 0;
     };
+    int u = 0;  // accumulations read (AVG)
     for (int m = 0;; ++m) {
       if (S.abort) break;
       const int qs = m % kTileQ;
@@ -453,15 +488,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       int tile_s;
       uint8_t nbi, nbj;
       tile_at(t, tile, tile_s);
-      flags_of(tile, tile_s, nbi, nbj);
+      if (AVG)
+        nbi = nbj = 0;  // the subjects' own flags apply
+      else
+        flags_of(tile, tile_s, nbi, nbj);
       const bool bad_i = nbi != 0, bad_j = nbj != 0;
       if (tile_s != cur_s) {  // the first tile, or another subject's
         leave();
         enter(tile_s);
       }
       const int I = tile.x, J = 2 * tile.y + h;
-      const int acc = m & 1;
-      const uint32_t ar = (uint32_t)(m >> 1);
       const bool active = (PASS == 2) ? (J < s_nb) : ((J >= I) && (J < s_nb));
       const bool listing = (PASS == 0);
       const int gi = I * 128 + il;
@@ -484,32 +520,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         S.abort = 1;
         break;
       }
-      if (!ptx::mbar_wait(ptx::smem_u32(&S.tfull[acc]), ar & 1u, kWaitNs)) {
-        atomicOr(a.err, ERR_TIMEOUT);
-        S.abort = 1;
-        break;
-      }
-      ptx::tc_fence_after();
-      const uint32_t taddr =
-          tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * TC_BN + h * 128);
       const bool diag = (I == J);
-      const bool slow = active && (bad_i || bad_j);
-      const bool rowbad = slow && s_bad[gi];
       int rowcount = 0;
       uint32_t cmk4[4] = {0u, 0u, 0u, 0u};
-      if (active) {
-        uint32_t vb[2][32];
-        ptx::tmem_ld32_async(taddr, vb[0]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t(&v)[32] = vb[c & 1];
-          ptx::tmem_wait32(v);
-          if (c + 1 < 4) ptx::tmem_ld32_async(taddr + (c + 1) * 32, vb[(c + 1) & 1]);
-          if (PASS == 2) {
-            if (h == p.dump_half)
-              for (int k = 0; k < 32; ++k) p.dump[il * 128 + c * 32 + k] = __uint_as_float(v[k]);
-            continue;
-          }
+      // chunk c of this warp's values: columns c * 32 .. + 31 of the half-tile,
+      // v[k] of row il; unc: columns whose pair is recomputed whatever its value
+      // (AVG); bad: the half-tile has a voxel with NaN z-scores
+      auto chunk = [&](uint32_t(&v)[32], int c, uint32_t unc, bool slow, bool rowbad) {
           const int jb = J * 128 + c * 32;
           uint32_t valid = (jb + 32 <= s_n) ? 0xffffffffu
                                             : (jb >= s_n ? 0u : ((1u << (s_n - jb)) - 1u));
@@ -518,27 +535,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             valid &= (lo <= 0) ? 0xffffffffu : (lo >= 32 ? 0u : (0xffffffffu << lo));
           }
           if (PASS == 4) {
-            uint32_t badm4 = 0;
-            if (slow)
-              for (int k = 0; k < 32; ++k)
-                if (rowbad || (jb + k < s_npad && s_bad[jb + k])) badm4 |= 1u << k;
             if (gi < s_n) {
               // packed upper-triangle index of (gi, j): gi (2n - gi - 1) / 2 + j - gi - 1
               const long long rowbase = (long long)gi * (2LL * s_n - gi - 1) / 2 - gi - 1;
 #pragma unroll
-              for (int k = 0; k < 32; ++k) {
-                if (!((valid >> k) & 1u)) continue;
-                const bool badk = (badm4 >> k) & 1u;
-                const float r = badk ? 0.0f : __uint_as_float(v[k]);
-                const long long idx = rowbase + jb + k;
-                if (!badk && !(fabsf(r) < p.unc_lim))
-                  atomicOr(&p.uncertain[idx >> 5], 1u << (idx & 31));
-                float add = 0.0f;
-                if (r >= -1.0f && r <= 1.0f) add = p.fisher ? fisher_z(r) : r;
-                p.packed[idx] = __fadd_rn(p.packed[idx], add);
-              }
+              for (int k = 0; k < 32; ++k)
+                if ((valid >> k) & 1u) p.packed[rowbase + jb + k] = __uint_as_float(v[k]);
             }
-            continue;
+            return;
           }
           if (PASS == 3) {
             // density histogram of the approximate values (exact 0 for NaN voxels)
@@ -554,7 +558,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 atomicAdd(&S.hist[(!badk && !(fabsf(r) < lim)) ? kHistBins : hist_bin(r)], 1u);
               }
             }
-            continue;
+            return;
           }
           // "interesting" = an edge or a candidate: x >= tau - delta, or
           // |r| >= 1 - delta; 8 partial masks so no long dependency chain forms
@@ -579,6 +583,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
               if (rowbad || (jb + k < s_npad && s_bad[jb + k])) badm |= 1u << k;
             it = (it & ~badm) | (zero_int ? badm : 0u);
           }
+          if (AVG) it |= unc;
           it &= valid;
           // slots in the warp's edge-list chunk: warp prefix scan of the counts
           const int ne = __popc(it);
@@ -602,7 +607,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const float r = __uint_as_float(val);
             const float x = ABS ? fabsf(r) : r;
             uint32_t cf = 0;
-            if (!((x - tau > delta) && (fabsf(r) < lim))) {
+            if (!((x - tau > delta) && (fabsf(r) < lim)) || (AVG && ((unc >> k) & 1u))) {
               cf = 1u;  // candidate: collected for the exact recompute after the pass
               val = 0u;
             }
@@ -614,7 +619,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           S.colmask[h][c * 32 + lane][q] = transpose32(eb, lane);
           wcur += total;
           if (!DENS) {
-            cmk4[c] = it & ~eb;  // candidates of this chunk (listed after the tile)
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4)  // candidates of this chunk (listed after the tile)
+              if (q4 == c) cmk4[q4] = it & ~eb;
           } else if (__any_sync(0xffffffffu, (it & ~eb) != 0u)) {
             // candidates with their approximate values, listed now (v[] is live)
             const uint32_t cmk = it & ~eb;
@@ -653,11 +660,165 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             ccur += ctot;
             n_cand += nc;
           }
+      };
+      if (AVG) {
+        // running sums in registers, rotated so that the loop over the four
+        // chunks keeps one copy of its code: after four turns chunk 0 leads again
+        uint32_t sm[128], un[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int k = 0; k < 128; ++k) sm[k] = 0u;
+        bool expired = false;
+        for (int sub = 0; sub < nsub; ++sub, ++u) {
+          const int acc = u & 1;
+          if (!ptx::mbar_wait(ptx::smem_u32(&S.tfull[acc]), (uint32_t)(u >> 1) & 1u, kWaitNs)) {
+            expired = true;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t taddr =
+              tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * TC_BN + h * 128);
+          if (active) {
+            const TcSubj& e = p.subj[sub];
+            const bool slow = e.blockbad[I] != 0 || e.blockbad[J] != 0;
+            const bool rowbad = slow && e.a.bad[gi];
+            const float unc_lim = e.unc_lim;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              uint32_t um = 0;
+#pragma unroll
+              for (int g = 0; g < 32; g += 16) {  // 16 values at a time fit the registers
+                uint32_t v[16];
+                ptx::tmem_ld16(taddr + c * 32 + g, v);
+                if (slow) {  // a pair with a NaN voxel adds nothing
+                  const uint8_t* eb = e.a.bad + J * 128 + c * 32 + g;
+#pragma unroll
+                  for (int k = 0; k < 16; ++k)
+                    if (rowbad || eb[k]) v[k] = 0u;
+                }
+                // |r| >= 1/2 (and NaN) are rare: the logarithm's form, and
+                // post_block's range, for the columns where some lane has one
+                uint32_t big = 0;
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                  big |= fabsf(__uint_as_float(v[k])) < 0.5f ? 0u : 1u << k;
+                // (one copy of that code in a loop: sixteen in line made the
+                // kernel wait for instructions, 6.3 ms instead of 2.3)
+                for (uint32_t w = __reduce_or_sync(0xffffffffu, big); w; w &= w - 1) {
+                  const int kk = __ffs(w) - 1;
+                  uint32_t x = 0u;
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) x = k == kk ? v[k] : x;
+                  if ((big >> kk) & 1u) {
+                    const float r = __uint_as_float(x);
+                    um |= !(fabsf(r) < unc_lim) ? 1u << (g + kk) : 0u;
+                    const float add = p.fisher ? fisher_z(r) : r;
+                    x = r >= -1.0f && r <= 1.0f ? __float_as_uint(add) : 0u;
+                  }
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) v[k] = k == kk ? x : v[k];
+                }
+                if (p.fisher) {
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) {
+                    const float z = fisher_z_half(__uint_as_float(v[k]));
+                    if (!((big >> k) & 1u)) v[k] = __float_as_uint(z);
+                  }
+                }
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                  sm[g + k] = __float_as_uint(
+                      __fadd_rn(__uint_as_float(sm[g + k]), __uint_as_float(v[k])));
+              }
+              const uint32_t u0 = un[0] | um;
+              uint32_t lead[32];
+#pragma unroll
+              for (int k = 0; k < 32; ++k) lead[k] = sm[k];
+#pragma unroll
+              for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
+#pragma unroll
+              for (int k = 0; k < 32; ++k) sm[96 + k] = lead[k];
+              un[0] = un[1];
+              un[1] = un[2];
+              un[2] = un[3];
+              un[3] = u0;
+            }
+          }
+          ptx::tc_fence_before();
+          ptx::mbar_arrive(ptx::smem_u32(&S.tempty[acc]));
         }
+        if (expired) {
+          atomicOr(a.err, ERR_TIMEOUT);
+          S.abort = 1;
+          break;
+        }
+        if (active) {
+          const float fs = (float)nsub;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[32];  // takes sm[0 .. 31]'s place
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+              v[k] = __float_as_uint(__fdiv_rn(__uint_as_float(sm[k]), fs));
+            }
+            if (p.fisher) {  // back from z, in the columns where some lane's average counts
+              uint32_t need = un[0];
+#pragma unroll
+              for (int k = 0; k < 32; ++k) {
+                const float z = __uint_as_float(v[k]);
+                need |= (ABS ? fabsf(z) : z) < zlo ? 0u : 1u << k;
+              }
+              const uint32_t cols = __reduce_or_sync(0xffffffffu, need);
+              for (uint32_t w = cols; w; w &= w - 1) {
+                const int kk = __ffs(w) - 1;
+                const uint32_t x =
+                    __float_as_uint(fisher_r(__uint_as_float(pick32(v, kk))));
+#pragma unroll
+                for (int k = 0; k < 32; ++k) v[k] = k == kk ? x : v[k];
+              }
+#pragma unroll
+              for (int k = 0; k < 32; ++k)  // 0: below lo_thr
+                if (!((cols >> k) & 1u)) v[k] = 0u;
+            }
+            chunk(v, c, un[0], false, false);
+#pragma unroll
+            for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
+            un[0] = un[1];
+            un[1] = un[2];
+            un[2] = un[3];
+          }
+        }
+      } else {
+        const int acc = m & 1;
+        if (!ptx::mbar_wait(ptx::smem_u32(&S.tfull[acc]), (uint32_t)(m >> 1) & 1u, kWaitNs)) {
+          atomicOr(a.err, ERR_TIMEOUT);
+          S.abort = 1;
+          break;
+        }
+        ptx::tc_fence_after();
+        const uint32_t taddr =
+            tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * TC_BN + h * 128);
+        const bool slow = active && (bad_i || bad_j);
+        const bool rowbad = slow && s_bad[gi];
+        if (active) {
+          uint32_t vb[2][32];
+          ptx::tmem_ld32_async(taddr, vb[0]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t(&v)[32] = vb[c & 1];
+            ptx::tmem_wait32(v);
+            if (c + 1 < 4) ptx::tmem_ld32_async(taddr + (c + 1) * 32, vb[(c + 1) & 1]);
+            if (PASS == 2) {
+              if (h == p.dump_half)
+                for (int k = 0; k < 32; ++k) p.dump[il * 128 + c * 32 + k] = __uint_as_float(v[k]);
+            } else {
+              chunk(v, c, 0u, slow, rowbad);
+            }
+          }
+        }
+        // the accumulator has been read: hand it back to the MMA warp
+        ptx::tc_fence_before();
+        ptx::mbar_arrive(ptx::smem_u32(&S.tempty[acc]));
       }
-      // the accumulator has been read: hand it back to the MMA warp
-      ptx::tc_fence_before();
-      ptx::mbar_arrive(ptx::smem_u32(&S.tempty[acc]));
       if (PASS == 2 || PASS == 3 || PASS == 4) continue;
       // candidates (rare): warp prefix scan into the warp's candidate chunk
       if (!DENS && active &&
@@ -868,7 +1029,8 @@ size_t tc_subj_bytes() { return sizeof(TcSubj); }
 
 // Table entry s (host memory, tc_subj_bytes() per entry) of a multi-subject
 // count pass: the subject's operand maps, arguments and NaN-block flags.
-bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form) {
+bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form,
+                  float unc_lim) {
   TcSubj* e = static_cast<TcSubj*>(host) + s;
   std::memset(e, 0, sizeof *e);
   if (form == FORM_BF16X3) {
@@ -885,6 +1047,7 @@ bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad,
   }
   e->a = a;
   e->blockbad = blockbad;
+  e->unc_lim = unc_lim;
   return true;
 }
 
@@ -934,11 +1097,50 @@ cudaError_t launch_seal_candidates(const CorrArgs& a, int nwarps, cudaStream_t s
   return cudaGetLastError();
 }
 
+// The average over the subjects of a table (tc_subj_fill): pass 0 count (+ edge
+// lists), 3 density histogram, 4 the packed averages.  a: the average's own
+// sizes, rule and lists.
+cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
+                               int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
+                               int grid, unsigned int* sched, cudaStream_t st) {
+  if (!sched || nsub < 1 || (pass == 4 && !packed) || a.cand_apx) return cudaErrorInvalidValue;
+  TcArgs p{};
+  p.a = a;
+  p.sched = sched;
+  p.tiles = tiles;
+  p.ntiles = ntiles;
+  p.subj = static_cast<const TcSubj*>(subj_dev);
+  p.nsub = nsub;
+  p.fisher = fisher;
+  p.packed = packed;
+  const int g = grid < ntiles ? grid : ntiles;
+  if (g <= 0) return cudaSuccess;
+  const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
+  void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
+  if (form == FORM_BF16X3)
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_BF16X3, false, false, true>
+                               : corr_tc_kernel<0, false, FORM_BF16X3, false, false, true>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false, false, true>
+                       : corr_tc_kernel<4, false, FORM_BF16X3, false, false, true>;
+  else
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_TF32, false, false, true>
+                               : corr_tc_kernel<0, false, FORM_TF32, false, false, true>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false, false, true>
+                       : corr_tc_kernel<4, false, FORM_TF32, false, false, true>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)TC_SMEM_BYTES);
+  if (e != cudaSuccess) return e;
+  CUtensorMap dummy;
+  std::memset(&dummy, 0, sizeof dummy);
+  kern<<<g, TC_THREADS, TC_SMEM_BYTES, st>>>(dummy, dummy, p);
+  return cudaGetLastError();
+}
+
 // pass 0 count (+ edge lists), 2 dump (tiles must then hold the one tile to dump),
 // 3 density histogram; form FORM_BF16X3 or FORM_TF32
 cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* tiles, int ntiles,
                            const uint8_t* blockbad, float* dump, int dump_half, int grid,
-                           unsigned int* sched, cudaStream_t st, const AvgPass* avg) {
+                           unsigned int* sched, cudaStream_t st) {
   if (!sched) return cudaErrorInvalidValue;
   CUtensorMap mh, ml;
   if (form == FORM_BF16X3) {
@@ -962,11 +1164,6 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
   p.blockbad = blockbad;
   p.dump = dump;
   p.dump_half = dump_half;
-  p.packed = avg ? avg->packed : nullptr;
-  p.uncertain = avg ? avg->uncertain : nullptr;
-  p.fisher = avg ? avg->fisher : 0;
-  p.unc_lim = avg ? avg->unc_lim : 1.0f;
-  if (pass == 4 && !avg) return cudaErrorInvalidValue;
   const int g = grid < ntiles ? grid : ntiles;
   if (g <= 0) return cudaSuccess;
   const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
@@ -978,14 +1175,12 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
                           : absm ? corr_tc_kernel<0, true, FORM_BF16X3, false>
                                  : corr_tc_kernel<0, false, FORM_BF16X3, false>)
            : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false>
-           : pass == 4 ? corr_tc_kernel<4, false, FORM_BF16X3, false>
                        : corr_tc_kernel<2, false, FORM_BF16X3, false>;
   else
     kern = pass == 0   ? (dens   ? corr_tc_kernel<0, false, FORM_TF32, true>
                           : absm ? corr_tc_kernel<0, true, FORM_TF32, false>
                                  : corr_tc_kernel<0, false, FORM_TF32, false>)
            : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false>
-           : pass == 4 ? corr_tc_kernel<4, false, FORM_TF32, false>
                        : corr_tc_kernel<2, false, FORM_TF32, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)TC_SMEM_BYTES);

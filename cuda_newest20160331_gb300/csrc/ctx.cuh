@@ -98,10 +98,14 @@ cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cuda
 // sched: the launch's tile counters (two, zero; the launch leaves them zero)
 cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* tiles, int ntiles,
                            const uint8_t* blockbad, float* dump, int dump_half, int grid,
-                           unsigned int* sched, cudaStream_t st, const AvgPass* avg = nullptr);
+                           unsigned int* sched, cudaStream_t st);
+cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
+                               int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
+                               int grid, unsigned int* sched, cudaStream_t st);
 cudaError_t launch_seal_candidates(const CorrArgs& a, int nwarps, cudaStream_t st);
 size_t tc_subj_bytes();
-bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form);
+bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form,
+                  float unc_lim = 1.0f);
 cudaError_t prepare_corr_tc_multi(int form, bool dens, bool absm);
 cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, const int4* tiles4,
                                  int ntiles, int form, bool dens, bool absm, int grid,
@@ -116,9 +120,6 @@ cudaError_t launch_rethr_count(const CorrArgs& a, const int32_t* rp, const int32
 cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* valx,
                               const uint8_t* keep, const int32_t* rp2, int32_t* ci2, float* val2,
                               long long nnz2, uint32_t* err, int sms, cudaStream_t st);
-cudaError_t launch_corr_packed(const CorrArgs& a, int pass, cudaStream_t stream);
-cudaError_t launch_avg_finalize(float* packed, long long m, int S, int fisher, int sms,
-                                cudaStream_t st);
 cudaError_t launch_avg_exact(const CorrArgs& a, const void* subj, int S, int fisher, float* out,
                              int sms, cudaStream_t st);
 size_t avg_subj_bytes();
@@ -151,7 +152,7 @@ enum Slot {
   S_DENSE, S_WSTATE, S_VSTAT,
   S_TILES_SMP, S_DSTATE, S_DHIST, S_DCLS, S_DEIDX, S_DEXACT, S_CANDAPX, S_DTIES,
   S_RT_KEEP, S_RT_VALX, S_RT_ROWPTR, S_RT_COL, S_RT_VAL,
-  S_AVG_Z, S_AVG_BAD, S_AVG_PACKED, S_AVG_UNC, S_AVG_BADZ, S_AVG_SUBJ,
+  S_AVG_Z, S_AVG_ZHI, S_AVG_ZLO, S_AVG_BAD, S_AVG_BADZ, S_AVG_SUBJ, S_AVG_TC,
   S_BATCH_SUBJ, S_BATCH_TILES,
   S_MOD_LABEL, S_MOD_ROWS, S_MOD_LOC, S_MOD_CNT, S_MOD_LRP, S_MOD_LCI, S_MOD_VD, S_MOD_VF,
   S_MOD_RS, S_MOD_Y, S_MOD_PARTS, S_MOD_GROUPS, S_MOD_BLKGRP, S_MOD_ASSIGN, S_MOD_KMOD,
@@ -231,10 +232,11 @@ struct bna_ctx {
   // what bna_csr_rethreshold recomputes exact values from
   CorrArgs last{};
   bool last_ok = false;
-  // multi-subject average in progress (bna_corr_csr_avg): subject table on the
-  // device, count, Fisher flag
+  // multi-subject average in progress (bna_corr_csr_avg): the subjects' tables
+  // on the device (exact values; tensor-core pass), count, Fisher flag
   struct Avg {
     const void* subj;
+    const void* tc;
     int S;
     int fisher;
   };
@@ -287,6 +289,8 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
                    cudaStream_t st);
 // Tensor-core preparation: per-block NaN flags and the upper-triangle tile list.
 int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st);
+// The tile list alone, for nb blocks (kept until nb or the band changes).
+int32_t tc_tiles(bna_ctx* ctx, int nb, cudaStream_t st);
 long long elist_chunk(const bna_ctx* ctx, const CorrArgs& a);
 void window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, int N,
                       double delta, double* winA, double* winB, Threshold* th);

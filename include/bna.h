@@ -255,8 +255,9 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
  * :36-42) is added in subject order into one matrix, divided by nsub (then
  * inv_fishertrans :44-50), and thresholded like one subject's matrix (opts:
  * any rule, a tensor-core form).  bold_dev[k] is subject k's time-major
- * [T[k]][N] series (same voxels for all subjects).  Device memory: the packed
- * averaged matrix (N(N-1)/2 floats) and every subject's z-scores. */
+ * [T[k]][N] series (same voxels for all subjects).  Device memory: every
+ * subject's z-scores (and their operand form); the average is taken tile by
+ * tile, without an N x N matrix. */
 int32_t bna_corr_csr_avg(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev, int32_t N,
                          const int32_t* T, int32_t fisher, const bna_corr_opts* opts,
                          bna_csr* out_dev, bna_corr_stats* stats, void* stream);
