@@ -116,7 +116,7 @@ int32_t set_device(bna_ctx* ctx, cudaStream_t st) {
 
 // Z-score into the arena; fills layout fields of `a`.
 int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16, CorrArgs& a,
-                   cudaStream_t st) {
+                   cudaStream_t st, bool need_q8) {
   a.n = N;
   a.T = T;
   a.n_pad = round_up(N, kBlk);
@@ -134,8 +134,20 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
   }
   void* vstat;
   ENSURE(S_VSTAT, zscore_scratch_bytes(a.n_pad), vstat);
-  CK(launch_zscore(bold, N, T, a.n_pad, z, a.ldz, zhi, zlo, a.ldb, bad, vstat, st));
+  uint8_t* zq = nullptr;
+  float* e2 = nullptr;
+  a.ldq = need_q8 ? round_up(T, 128) : 0;
+  if (need_q8) {
+    float* eblk;
+    ENSURE(S_ZQ, (size_t)a.n_pad * a.ldq, zq);
+    ENSURE(S_E2, (size_t)a.n_pad * sizeof(float), e2);
+    ENSURE(S_EBLK, (size_t)a.nb * sizeof(float), eblk);
+    a.eblk = eblk;
+  }
+  CK(launch_zscore(bold, N, T, a.n_pad, z, a.ldz, zhi, zlo, a.ldb, bad, vstat, st, zq, a.ldq,
+                   e2));
   ctx->klaunch += 2;
+  a.zq = zq;
   a.z = z;
   a.zhi = zhi;
   a.zlo = zlo;
@@ -147,9 +159,27 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
 int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st) {
   uint8_t* bb;
   ENSURE(S_BLOCKBAD, (size_t)a.nb, bb);
-  CK(launch_block_bad(a.bad, a.nb, bb, st));
+  CK(launch_block_bad(a.bad, a.nb, bb, st,
+                      a.zq ? static_cast<const float*>(ctx->ptr[S_E2]) : nullptr,
+                      const_cast<float*>(a.eblk)));
   ctx->klaunch += 1;
   return tc_tiles(ctx, a.nb, st);
+}
+
+// Whether a count pass may gain from the tile screen (corr_screen.cu): the
+// rule's limit has to clear the 8-bit operands' error (about kScreenErr for
+// ordinary series) by kScreenSigma standard deviations of a chance correlation
+// of T samples - below that nearly every tile of 32,768 unrelated pairs
+// reaches it - and the pass has to be long against the screen's own launches:
+// series from kScreenMinT steps on, kScreenTiles tiles per SM.  Measured (rule,
+// count pass without -> with): 180,000 x 1,200 in 60 networks, r >= 0.4,
+// 60.4 -> 15.7 ms; every tile with edges (unrelated loadings), 60,000 x 1,000,
+// 5.50 -> 5.60 ms, 15,000 x 600, 0.245 -> 0.271 ms.
+constexpr int kScreenMinT = 512, kScreenTiles = 16;
+constexpr double kScreenErr = 0.06, kScreenSigma = 4.5;
+static bool screen_pays(const bna_ctx* ctx, int nb, int T, float limit) {
+  return T >= kScreenMinT && tc_tile_count(nb) >= (long long)kScreenTiles * ctx->sms &&
+         (double)limit - kScreenErr > kScreenSigma / std::sqrt((double)T);
 }
 
 int32_t tc_tiles(bna_ctx* ctx, int nb, cudaStream_t st) {
@@ -215,6 +245,56 @@ void window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, in
   th->delta = (float)((0.5 * (*winB - *winA) + delta) * (1.0 + 1e-6) + 1e-7);
 }
 
+// The count pass behind the tile screen: the tiles that the screen leaves, in
+// one launch that reads their number on the device, or - where launches are
+// bounded (BNA_OPT_TILES_PER_LAUNCH) - in several; a screen launch of half as
+// many tiles again takes about as long as one of the count pass.
+static int32_t screened_pass(bna_ctx* ctx, const CorrArgs& a, int precision, float limit,
+                             unsigned int* sched, cudaStream_t st) {
+  const long long nsup = sc_tile_count(a.nb);
+  int2 *sup, *out;
+  uint8_t* keep;
+  unsigned int* n_out;
+  const size_t nkeep = ((size_t)nsup + 15) / 16 * 16;
+  ENSURE(S_SC_TILES, (size_t)nsup * sizeof(int2), sup);
+  ENSURE(S_SC_KEEP, nkeep, keep);
+  ENSURE(S_SC_OUT, (size_t)tc_tile_count(a.nb) * sizeof(int2), out);
+  ENSURE(S_SC_COUNT, sizeof(unsigned int), n_out);
+  if (ctx->sc_nb != a.nb || ctx->sc_band != ctx->band_now) {
+    CK(launch_screen_list(a.nb, ctx->band_now, sup, st));
+    ctx->klaunch += 1;
+    ctx->sc_nb = a.nb;
+    ctx->sc_band = ctx->band_now;
+  }
+  CK(cudaMemsetAsync(keep, 0, nkeep, st));
+  const int form = precision == BNA_PREC_BF16X3 ? 0 : 1;
+  const uint8_t* bb = reinterpret_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]);
+  const long long per = ctx->tiles_per_launch;
+  const long long per_sup = per > 0 ? per + (per + 1) / 2 : nsup;
+  for (long long t0 = 0; t0 < nsup; t0 += per_sup, ++ctx->klaunch) {
+    if (t0 > 0) gate(ctx, st, BNA_PHASE_CORR, t0);
+    CK(launch_corr_screen(a, limit, sup + t0, (int)std::min(per_sup, nsup - t0), keep + t0,
+                          t0 + per_sup >= nsup, ctx->sms, sched, st));
+  }
+  CK(launch_screen_compact(keep, sup, (int)nsup, out, n_out, ctx->sms, st));
+  ctx->klaunch += 1;
+  if (per == 0) {
+    CK(launch_corr_tc(a, 0, form, out, ctx->ntiles, bb, nullptr, 0, ctx->sms, sched, st, n_out));
+    ctx->klaunch += 1;
+    return BNA_OK;
+  }
+  unsigned int* left = reinterpret_cast<unsigned int*>(static_cast<char*>(ctx->pinned) + 4000);
+  CK(cudaMemcpyAsync(left, n_out, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  const long long n = *left;
+  for (long long t0 = 0; t0 < n; t0 += per, ++ctx->klaunch) {
+    gate(ctx, st, BNA_PHASE_CORR, t0);
+    CK(launch_corr_tc(a, 0, form, out + t0, (int)std::min(per, n - t0), bb, nullptr, 0, ctx->sms,
+                      sched, st));
+  }
+  return BNA_OK;
+}
+
 // pass 0: count (+ edge lists); pass 3: density histogram (sampled: on the
 // sampled tile list, tensor-core forms)
 
@@ -234,6 +314,11 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
       unsigned int* sched;
       ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
       CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
+      if (pass == 0 && a.zq) {
+        const float limit = screen_limit(a.th, default_delta(precision, a.T));
+        if (screen_pays(ctx, a.nb, a.T, limit))
+          return screened_pass(ctx, a, precision, limit, sched, st);
+      }
       for (int t0 = 0; t0 < nt; t0 += per, ++ctx->klaunch) {
         if (t0 > 0) gate(ctx, st, BNA_PHASE_CORR, t0);
         if (ctx->avg)
@@ -335,6 +420,8 @@ int64_t bna_request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64
   if (opts->precision == BNA_PREC_BF16X3 || opts->precision == BNA_PREC_AUTO)
     b += n_pad * ldb * 4;  // z hi / lo
   b += nb * n_pad * 4 + 2 * n_pad * 8 + 4096 * 8;              // seg, row lengths, block sums
+  if (T >= kScreenMinT && opts->precision != BNA_PREC_FP32)    // tile screen
+    b += n_pad * round_up(T, 128) + n_pad * 4 + ntiles * 13;
   b += nst * 64 + nst * 4 + ntiles * 8 + nb;                   // etab, dense list, tiles, flags
   b += elist * 8;                                              // edge lists
   b += cand * 8 + 2 * cand * 13 + (density ? cand * 4 : 0);    // candidates, hash, values
@@ -384,7 +471,8 @@ void bna::arena_release(bna_ctx* ctx, cudaStream_t st, bool to_driver) {
   cudaStreamSynchronize(st);
   if (to_driver)
     if (cudaMemPool_t pool = lib_pool(ctx->device)) cudaMemPoolTrimTo(pool, 0);
-  ctx->tiles_nb = -1;  // the tile list lived in the arena
+  ctx->tiles_nb = -1;  // the tile lists lived in the arena
+  ctx->sc_nb = -1;
   ctx->last_ok = false;
   if (ctx->ecg.exec) cudaGraphExecDestroy(ctx->ecg.exec);
   ctx->ecg = EcGraph();
@@ -452,9 +540,10 @@ int32_t bna_zscore(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T, fl
   ENSURE(S_BAD, (size_t)n_pad, bad);
   void* vstat;
   ENSURE(S_VSTAT, zscore_scratch_bytes(n_pad), vstat);
-  // The kernel writes n_pad rows; the caller's buffer holds N rows, so stage
-  // through the arena when N is not a multiple of the block.
-  if (n_pad == N) {
+  // The kernel writes n_pad rows, two values per store; the caller's buffer
+  // holds N rows, so stage through the arena when N is not a multiple of the
+  // block or the buffer starts on an odd float.
+  if (n_pad == N && (reinterpret_cast<uintptr_t>(z_dev) & 7u) == 0) {
     CK(launch_zscore(bold_dev, N, T, n_pad, z_dev, ldz, nullptr, nullptr, 0, bad, vstat,
                      as_stream(stream)));
   } else {
@@ -504,14 +593,20 @@ int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
   ctx->last_ok = false;  // the arena is about to be rewritten
   CorrArgs a{};
   CK(cudaEventRecord(ctx->ev[0], st));
-  s = run_zscore(ctx, bold_dev, N, T, prec == BNA_PREC_BF16X3, a, st);
+  const double delta = opts->delta > 0 ? opts->delta : default_delta(prec, T);
+  bool q8 = false;  // operands for the tile screen (a density's limit is not known yet)
+  if (prec != BNA_PREC_FP32) {
+    const Threshold th{opts->mode, rule_tau(opts), (float)delta};
+    q8 = screen_pays(ctx, round_up(N, kBlk) / kBlk, T,
+                     density ? 1.0f : screen_limit(th, default_delta(prec, T)));
+  }
+  s = run_zscore(ctx, bold_dev, N, T, prec == BNA_PREC_BF16X3, a, st, q8);
   if (s) return s;
   if (prec != BNA_PREC_FP32) {
     s = tc_prepare(ctx, a, st);
     if (s) return s;
   }
   CK(cudaEventRecord(ctx->ev[1], st));
-  const double delta = opts->delta > 0 ? opts->delta : default_delta(prec, T);
   return corr_csr_core(ctx, a, N, T, opts, prec, delta, out_dev, stats, st);
 }
 

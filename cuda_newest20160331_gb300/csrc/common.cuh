@@ -109,6 +109,9 @@ struct CorrArgs {
   const float* z;            // voxel-major [n_pad][ldz], FP32 z-scores (exact recompute source)
   const uint16_t* zhi;       // voxel-major [n_pad][ldb] BF16 hi parts (tensor-core forms)
   const uint16_t* zlo;       // BF16 lo parts
+  const uint8_t* zq;         // voxel-major [n_pad][ldq] E4M3 of 256 z (tile screen), or null
+  int ldq;
+  const float* eblk;         // [nb] largest |z_i - q_i| of each 128-block (tile screen)
   const uint8_t* bad;        // [n_pad] 1 = voxel has a NaN z (every r of it is NaN -> 0)
   int n, n_pad, T, ldz, ldb, nb;
   Threshold th;

@@ -104,6 +104,7 @@ struct TcArgs {
   // multi-subject count pass: tiles4 = (I, J-pair, subject), subj the table
   const int4* tiles4;
   const TcSubj* subj;
+  const unsigned int* ntiles_dev;  // non-null: the tile count (the screen's list)
   const int2* tiles;        // (I, Jp): rows of block I x columns of blocks 2Jp, 2Jp+1
   int ntiles;
   // [0]: next tile to claim, [1]: CTAs finished; zero at launch, reset to
@@ -245,9 +246,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         ++m;
         return true;
       };
+      const int ntiles = p.ntiles_dev ? (int)*p.ntiles_dev : p.ntiles;
       // the next tile is claimed while this one's copies are issued
       int t = (int)atomicAdd(p.sched, 1u);
-      for (int t_next; t < p.ntiles && !S.abort; t = t_next) {
+      for (int t_next; t < ntiles && !S.abort; t = t_next) {
         if (!publish(t)) {
           atomicOr(a.err, ERR_TIMEOUT);
           S.abort = 1;
@@ -907,10 +909,21 @@ __global__ void seal_candidates_kernel(CorrArgs a, int nwarps) {
   }
 }
 
-__global__ void block_bad_kernel(const uint8_t* bad, int nb, uint8_t* blockbad) {
+// Per block of 128 voxels: whether one has a NaN z-score, and (e2 given) the
+// largest e_i = sqrt(e2[i]) rounded up (the tile screen's bound).
+__global__ void block_bad_kernel(const uint8_t* bad, int nb, uint8_t* blockbad, const float* e2,
+                                 float* eblk) {
+  __shared__ unsigned int mx[4];
   const int b = blockIdx.x;
   const int any = __syncthreads_or(bad[b * 128 + threadIdx.x] != 0);
   if (threadIdx.x == 0 && b < nb) blockbad[b] = any ? 1 : 0;
+  if (!e2) return;
+  const float e = sqrtf(e2[b * 128 + threadIdx.x]) * 1.001f + 1e-6f;  // non-negative: bits order it
+  const unsigned int w = __reduce_max_sync(0xffffffffu, __float_as_uint(e));
+  if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0 && b < nb)
+    eblk[b] = __uint_as_float(max(max(mx[0], mx[1]), max(mx[2], mx[3])));
 }
 
 // ---------------------------------------------------------------- host side
@@ -948,6 +961,19 @@ bool make_map(CUtensorMap* m, const void* base, int ld, int rows, bool fp32) {
 }
 
 }  // namespace
+
+// 2-D map over [rows][ld] bytes with a 128-byte x 128-row box, 128-byte swizzle.
+bool tc_map_bytes(CUtensorMap* m, const void* base, int ld, int rows) {
+  auto fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld};
+  cuuint32_t box[2] = {128, TC_BM};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box,
+            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Tile list (I, Jp) of the upper triangle in 128 x 256 tiles (rows of block
 // I, columns of blocks 2Jp and 2Jp+1, Jp >= I/2), in bands of `band` row
@@ -1020,8 +1046,9 @@ cudaError_t launch_tile_lists(int nb, int band, int2* tiles, long long n_smp, in
 
 size_t tc_smem_bytes() { return TC_SMEM_BYTES; }
 
-cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cudaStream_t st) {
-  block_bad_kernel<<<nb, 128, 0, st>>>(bad, nb, blockbad);
+cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cudaStream_t st,
+                             const float* e2, float* eblk) {
+  block_bad_kernel<<<nb, 128, 0, st>>>(bad, nb, blockbad, e2, eblk);
   return cudaGetLastError();
 }
 
@@ -1140,7 +1167,8 @@ cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void
 // 3 density histogram; form FORM_BF16X3 or FORM_TF32
 cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* tiles, int ntiles,
                            const uint8_t* blockbad, float* dump, int dump_half, int grid,
-                           unsigned int* sched, cudaStream_t st) {
+                           unsigned int* sched, cudaStream_t st,
+                           const unsigned int* ntiles_dev) {
   if (!sched) return cudaErrorInvalidValue;
   CUtensorMap mh, ml;
   if (form == FORM_BF16X3) {
@@ -1158,6 +1186,7 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
   p.sched = sched;
   p.tiles = tiles;
   p.ntiles = ntiles;
+  p.ntiles_dev = ntiles_dev;
   const int per_step = form == FORM_BF16X3 ? Form<FORM_BF16X3>::kElemsPerStep
                                            : Form<FORM_TF32>::kElemsPerStep;
   p.nksteps = (a.T + per_step - 1) / per_step;

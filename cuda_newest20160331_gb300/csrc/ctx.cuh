@@ -23,9 +23,11 @@
 
 namespace bna {
 size_t zscore_scratch_bytes(int n_pad);
+// zq / ldq / e2: the tile screen's operands and squared errors (optional)
 cudaError_t launch_zscore(const float* bold, int N, int T, int n_pad, float* z, int ldz,
                           uint16_t* zhi, uint16_t* zlo, int ldb, uint8_t* bad, void* scratch,
-                          cudaStream_t stream);
+                          cudaStream_t stream, uint8_t* zq = nullptr, int ldq = 0,
+                          float* e2 = nullptr);
 cudaError_t launch_corr_simt(const CorrArgs& a, int pass, cudaStream_t stream);
 cudaError_t launch_corr_simt_dump(const CorrArgs& a, int I, int J, float* out,
                                   cudaStream_t stream);
@@ -94,11 +96,21 @@ void tc_tile_list(int nb, int band, std::vector<int2>& out);
 long long tc_tile_count(int nb);
 cudaError_t launch_tile_lists(int nb, int band, int2* tiles, long long n_smp, int s, int2* smp,
                               cudaStream_t st);
-cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cudaStream_t st);
+cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cudaStream_t st,
+                             const float* e2 = nullptr, float* eblk = nullptr);
+long long sc_tile_count(int nb);
+cudaError_t launch_screen_list(int nb, int band, int2* out, cudaStream_t st);
+float screen_limit(const Threshold& th, double form_delta);
+cudaError_t launch_corr_screen(const CorrArgs& a, float limit, const int2* sup, int nsup,
+                               uint8_t* keep, bool ends, int grid, unsigned int* sched,
+                               cudaStream_t st);
+cudaError_t launch_screen_compact(const uint8_t* keep, const int2* sup, int nsup, int2* out,
+                                  unsigned int* n_out, int sms, cudaStream_t st);
 // sched: the launch's tile counters (two, zero; the launch leaves them zero)
 cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* tiles, int ntiles,
                            const uint8_t* blockbad, float* dump, int dump_half, int grid,
-                           unsigned int* sched, cudaStream_t st);
+                           unsigned int* sched, cudaStream_t st,
+                           const unsigned int* ntiles_dev = nullptr);
 cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
                                int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
                                int grid, unsigned int* sched, cudaStream_t st);
@@ -156,7 +168,8 @@ enum Slot {
   S_BATCH_SUBJ, S_BATCH_TILES,
   S_MOD_LABEL, S_MOD_ROWS, S_MOD_LOC, S_MOD_CNT, S_MOD_LRP, S_MOD_LCI, S_MOD_VD, S_MOD_VF,
   S_MOD_RS, S_MOD_Y, S_MOD_PARTS, S_MOD_GROUPS, S_MOD_BLKGRP, S_MOD_ASSIGN, S_MOD_KMOD,
-  S_MOD_ADJ, S_EC_SPLIT, S_EC_PART, S_EC_ROWS, S_EC_FLAG, S_TCSCHED, S_COUNT
+  S_MOD_ADJ, S_EC_SPLIT, S_EC_PART, S_EC_ROWS, S_EC_FLAG, S_TCSCHED,
+  S_ZQ, S_E2, S_EBLK, S_SC_TILES, S_SC_KEEP, S_SC_OUT, S_SC_COUNT, S_COUNT
 };
 
 // Small device block the host reads once per pass.
@@ -224,6 +237,8 @@ struct bna_ctx {
   int tiles_band = 0; // and its band height (row blocks listed column by column together)
   int band = kDefaultBand;  // BNA_OPT_TILE_BAND
   int band_now = kDefaultBand;  // the band of the current call (the autotuner's for AUTO)
+  int sc_nb = -1;     // the screen's tile list: block count and band it was built for
+  int sc_band = 0;
   int ntiles = 0;
   int ntiles_smp = 0;  // sampled tile list (density histogram), same block count
   int tiles_per_launch = 0;  // BNA_OPT_TILES_PER_LAUNCH
@@ -286,7 +301,7 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 int32_t set_device(bna_ctx* ctx, cudaStream_t st = nullptr);
 // Z-score into the arena; fills layout fields of `a`.
 int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16, CorrArgs& a,
-                   cudaStream_t st);
+                   cudaStream_t st, bool need_q8 = false);
 // Tensor-core preparation: per-block NaN flags and the upper-triangle tile list.
 int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st);
 // The tile list alone, for nb blocks (kept until nb or the band changes).

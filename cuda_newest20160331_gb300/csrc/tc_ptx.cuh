@@ -122,6 +122,17 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint6
       : "memory");
 }
 
+// D[tmem] (+)= A * B^T, kind::f8f6f4 (8-bit inputs as the instruction descriptor
+// says, FP32 accumulate), K = 32.
+__device__ __forceinline__ void mma_e4m3(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                         uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Arrive on an mbarrier once all previously issued tcgen05 ops of this thread complete.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile(
@@ -205,7 +216,7 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
 }
 
 // Instruction descriptor: dense, FP32 accumulator, A/B K-major, shape M x N.
-// atype/btype: kind::f16 -> 0 F16, 1 BF16; kind::tf32 -> 2 TF32.
+// atype/btype: kind::f16 -> 0 F16, 1 BF16; kind::tf32 -> 2 TF32; kind::f8f6f4 -> 0 E4M3.
 __host__ __device__ constexpr uint32_t make_idesc(uint32_t atype, uint32_t btype, uint32_t M,
                                                   uint32_t N) {
   return (1u << 4)               // D format: F32

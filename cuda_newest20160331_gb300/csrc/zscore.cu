@@ -48,12 +48,14 @@
 //                        With one thread per voxel and a sequential FP64 s2 both
 //                        kernels took 96 us at 4,096 x 240, 215 us at 45,000 x 240
 //                        and 3.55 ms at 180,000 x 1,200; now 40, 135 and 2.1.
-//   zscore_emit_kernel   one element per thread-step over 32 voxels x 32
-//                        steps tiles: reads coalesced along voxels, computes
-//                        z, and writes the voxel-major rows (z FP32, BF16
-//                        hi = bf16(z), lo = bf16(z - hi)) through a shared-
-//                        memory transpose.  bad[i] = 1 when z has a NaN.
+//   zscore_emit_kernel   32 voxels x 64 steps tiles: reads coalesced along
+//                        voxels, computes z, and writes the voxel-major rows
+//                        (z FP32, BF16 hi = bf16(z), lo = bf16(z - hi)) through
+//                        a shared-memory transpose, two steps per lane and
+//                        store.  bad[i] = 1 when z has a NaN.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
 
 #include "common.cuh"
 
@@ -181,7 +183,7 @@ static __device__ __noinline__ double zs_centred_sum(const float* bold, int N, i
 
 __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
     const float* __restrict__ bold, int N, int T, VoxStat* __restrict__ vs,
-    uint8_t* __restrict__ bad) {
+    uint8_t* __restrict__ bad, float* __restrict__ e2) {
   __shared__ uint32_t pmax[kZStatWarps][32], pmin[kZStatWarps][32];
   __shared__ long long pacc[kZStatWarps][32], pmag[kZStatWarps][32];
   __shared__ ulonglong2 pq[kZStatWarps][32];
@@ -318,6 +320,7 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
       vs[gv] = o;
     }
     bad[gv] = 0;
+    if (e2) e2[gv] = 0.0f;  // the emit kernel adds to it
   }
   __syncthreads();
   // voxels outside the integer form: the reference's sums, a warp per voxel
@@ -393,31 +396,36 @@ static __device__ __noinline__ float z_exact_warp(const float* bold, int N, int 
   return zdiv(__dsub_rn(f2d_exact(x), mean), nrm, __drcp_rn(nrm));
 }
 
+// Q8: also the tile screen's operands (corr_screen.cu), zq = E4M3(256 z) (0 for
+// NaN), and e2[i] += the squared error (z - zq / 256)^2 of the block's steps.
+template <bool Q8>
 __global__ __launch_bounds__(256) void zscore_emit_kernel(
     const float* __restrict__ bold, int N, int T, const VoxStat* __restrict__ vs,
     float* __restrict__ z, int ldz, uint16_t* __restrict__ zhi, uint16_t* __restrict__ zlo,
-    int ldb, uint8_t* __restrict__ bad) {
+    int ldb, uint8_t* __restrict__ bad, uint8_t* __restrict__ zq, int ldq,
+    float* __restrict__ e2) {
   // z_near's relative bound: 2^-44, and half of s2's relative distance from S
   // (twice the (T + 16) 2^-53 above, for the conversions and the split)
   const float rel = 5.6843419e-14f + (float)(T + 16) * 1.1102230e-16f;
-  __shared__ float tile[32][33];  // tile[tt][v]: z of voxel v0+v at time t0+tt
+  __shared__ float tile[2][32][33];  // tile[t & 1][t / 2][v]: z of voxel v0+v at time t0+t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int v0 = blockIdx.x * 32;
   const int gv = v0 + lane;
   const bool live = gv < N;
   const VoxStat st = vs[gv];  // gv < n_pad: the grid covers n_pad / 32 groups
-  const int tmax = ldz > ldb ? ldz : ldb;
+  const int tmax = max(max(ldz, ldb), Q8 ? ldq : 0);
   const int tb = blockIdx.y * kZEmitT;
   bool nan_seen = false;
-  for (int t0 = tb; t0 < tb + kZEmitT && t0 < tmax; t0 += 32) {
-    float xs[4];
+  float err[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int t0 = tb; t0 < tb + kZEmitT && t0 < tmax; t0 += 64) {
+    float xs[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 8; ++k) {
       const int t = t0 + warp + 8 * k;
       xs[k] = (live && t < T) ? __ldg(bold + (size_t)t * N + gv) : 0.0f;
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 8; ++k) {
       const int tt = warp + 8 * k, t = t0 + tt;
       float zz = 0.0f;
       bool ok = true;
@@ -432,25 +440,42 @@ __global__ __launch_bounds__(256) void zscore_emit_kernel(
         if (lane == src) zz = ze;
       }
       nan_seen |= (zz != zz);
-      tile[tt][lane] = zz;
+      tile[tt & 1][tt >> 1][lane] = zz;
     }
     __syncthreads();
-    // warp w writes voxels w, w+8, w+16, w+24; lane = time step in the chunk
+    // warp w writes voxels w, w+8, w+16, w+24; a lane two time steps
+    const int t = t0 + 2 * lane;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int vv = warp + 8 * k;
       const size_t gi = (size_t)v0 + vv;
-      const int t = t0 + lane;
-      const float zz = tile[lane][vv];
-      if (t < ldz) z[gi * ldz + t] = zz;
+      const float za = tile[0][lane][vv], zb = tile[1][lane][vv];
+      if (t < ldz) *reinterpret_cast<float2*>(z + gi * ldz + t) = make_float2(za, zb);
       if (zhi != nullptr && t < ldb) {
-        const __nv_bfloat16 hh = __float2bfloat16_rn(zz);
-        const __nv_bfloat16 ll = __float2bfloat16_rn(zz - __bfloat162float(hh));
-        zhi[gi * ldb + t] = __bfloat16_as_ushort(hh);
-        zlo[gi * ldb + t] = __bfloat16_as_ushort(ll);
+        const __nv_bfloat162 hh = __floats2bfloat162_rn(za, zb);
+        const __nv_bfloat162 ll = __floats2bfloat162_rn(za - __low2float(hh), zb - __high2float(hh));
+        *reinterpret_cast<__nv_bfloat162*>(zhi + gi * ldb + t) = hh;
+        *reinterpret_cast<__nv_bfloat162*>(zlo + gi * ldb + t) = ll;
+      }
+      if (Q8 && t < ldq) {
+        const float2 f = make_float2(za == za ? 256.0f * za : 0.0f, zb == zb ? 256.0f * zb : 0.0f);
+        const __nv_fp8x2_storage_t q = __nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E4M3);
+        const __half2 b = __nv_cvt_fp8x2_to_halfraw2(q, __NV_E4M3);
+        const float da = (f.x - __low2float(b)) * 0.00390625f;
+        const float db = (f.y - __high2float(b)) * 0.00390625f;
+        err[k] += da * da + db * db;
+        *reinterpret_cast<__nv_fp8x2_storage_t*>(zq + gi * ldq + t) = q;
       }
     }
     __syncthreads();
+  }
+  if (Q8) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) err[k] += __shfl_xor_sync(0xffffffffu, err[k], o);
+      if (lane == 0) atomicAdd(e2 + v0 + warp + 8 * k, err[k]);
+    }
   }
   if (nan_seen) bad[gv] = 1;
 }
@@ -460,15 +485,21 @@ size_t zscore_scratch_bytes(int n_pad) { return (size_t)n_pad * sizeof(VoxStat);
 // scratch: zscore_scratch_bytes(n_pad) bytes of device memory.
 cudaError_t launch_zscore(const float* bold, int N, int T, int n_pad, float* z, int ldz,
                           uint16_t* zhi, uint16_t* zlo, int ldb, uint8_t* bad, void* scratch,
-                          cudaStream_t stream) {
-  if (n_pad % 128 != 0 || ldz % 32 != 0 || (zhi && ldb % 32 != 0) || !scratch)
+                          cudaStream_t stream, uint8_t* zq, int ldq, float* e2) {
+  if (n_pad % 128 != 0 || ldz % 32 != 0 || (zhi && ldb % 64 != 0) || !scratch ||
+      (zq && (ldq % 128 != 0 || !e2)))
     return cudaErrorInvalidValue;
   VoxStat* vs = static_cast<VoxStat*>(scratch);
-  zscore_stats_kernel<<<n_pad / 32, kZStatWarps * 32, 0, stream>>>(bold, N, T, vs, bad);
+  zscore_stats_kernel<<<n_pad / 32, kZStatWarps * 32, 0, stream>>>(bold, N, T, vs, bad, e2);
   const int ldbv = zhi ? ldb : 0;
-  const int tmax = ldz > ldbv ? ldz : ldbv;
+  const int tmax = max(max(ldz, ldbv), zq ? ldq : 0);
   const dim3 grid(n_pad / 32, (tmax + kZEmitT - 1) / kZEmitT);
-  zscore_emit_kernel<<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv, bad);
+  if (zq)
+    zscore_emit_kernel<true><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
+                                                       bad, zq, ldq, e2);
+  else
+    zscore_emit_kernel<false><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
+                                                        bad, nullptr, 0, nullptr);
   return cudaGetLastError();
 }
 
