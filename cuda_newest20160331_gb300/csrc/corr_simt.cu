@@ -22,6 +22,18 @@ constexpr int SB = 128;  // tile edge
 constexpr int SK = 16;   // K (time) chunk per stage
 constexpr int SPAD = 4;
 
+// d = a * b + d on both floats of a pair.
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a,
+                                     unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ unsigned long long pair_of(float x) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+  return d;
+}
+
 // PASS 0 = count (+ edge list), 2 = dump approximate values of one tile,
 // 3 = density histogram.
 template <int PASS>
@@ -46,11 +58,15 @@ __global__ __launch_bounds__(256, 2) void corr_simt_kernel(CorrArgs a, int nt, i
   const float* Bg = a.z + (size_t)J * SB * a.ldz;
   const int lr = tid >> 2, lk = (tid & 3) * 4;
 
-  float acc[8][8];
+  // two columns' sums per register pair: fma.rn.f32x2 rounds each like fmaf
+  // and takes half the issue slots (the scalar form issued 346 M warp
+  // instructions at N = 10,001, T = 150 and kept the FMA pipe half busy:
+  // 442 us; this 365)
+  unsigned long long acc2[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc2[i][j] = 0ull;
 
   const int kt = (a.T + SK - 1) / SK;
   float4 ra0, ra1, rb0, rb1;
@@ -81,18 +97,29 @@ __global__ __launch_bounds__(256, 2) void corr_simt_kernel(CorrArgs a, int nt, i
     for (int k = 0; k < SK; ++k) {
       const float4 a0 = *reinterpret_cast<const float4*>(&As[b][k][ty * 4]);
       const float4 a1 = *reinterpret_cast<const float4*>(&As[b][k][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[b][k][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[b][k][64 + tx * 4]);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[b][k][tx * 4]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[b][k][64 + tx * 4]);
       const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < 8; ++i) {
+        const unsigned long long ai = pair_of(av[i]);
+        fma2(acc2[i][0], ai, b0.x);
+        fma2(acc2[i][1], ai, b0.y);
+        fma2(acc2[i][2], ai, b1.x);
+        fma2(acc2[i][3], ai, b1.y);
+      }
     }
     if (kk + 1 < kt) sstore(b ^ 1);
     __syncthreads();
   }
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[i][2 * j] = __uint_as_float((uint32_t)acc2[i][j]);
+      acc[i][2 * j + 1] = __uint_as_float((uint32_t)(acc2[i][j] >> 32));
+    }
 
   if (PASS == 2) {
 #pragma unroll
@@ -109,6 +136,7 @@ __global__ __launch_bounds__(256, 2) void corr_simt_kernel(CorrArgs a, int nt, i
     // density histogram of the approximate values in shared memory (the
     // operand tiles are free now), merged into the global one
     unsigned int* h = reinterpret_cast<unsigned int*>(&As[0][0][0]);
+    static_assert(sizeof(As) >= (kHistBins + 1) * sizeof(unsigned int), "histogram fits");
     for (int b = tid; b <= kHistBins; b += 256) h[b] = 0u;
     __syncthreads();
     const bool diag = (I == J);
