@@ -32,6 +32,7 @@
 // double for the sign rule and the division.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -53,15 +54,15 @@ struct ModGroup {
   long long subp, subn;
   int fbuf;      // buffer (0/1) of the final eigenvector iterate
   unsigned int bar_count, bar_gen;
-  unsigned int arrive;  // blocks' arrivals at the summing barriers of this launch
 };
 
 constexpr int kModThreads = 1024;
 constexpr int kModWarps = kModThreads / 32;
-// Partial sums per block: slots 0-3 and 4-7 hold the sums of the summing
-// barriers (start vector; a power step's |y|^2, y.k and the two norms) of
-// even and odd barrier number, 8-11 the eigenvalue sign and side sizes.
-constexpr int kModParts = 12;
+// Words of 8 bytes per block: 0-7 and 8-15 publish the sums of the summing
+// barriers (start vector; a power step's |y|^2, y.k and the two norms) of even
+// and odd barrier number - value w as word 2 w = (hi, barrier number) and 2 w +
+// 1 = (lo, barrier number) - and 16-19 hold the eigenvalue sign and side sizes.
+constexpr int kModParts = 20;
 // Groups of at most this many nodes keep their iterate ((hi, lo) floats) in
 // shared memory during the gathers: 96 KB.
 constexpr int kModStageMax = 12288;
@@ -139,39 +140,44 @@ __device__ __forceinline__ float2 ff_shfl_xor(float2 a, int o) {
   return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
 }
 
-// Block sum of W float-float values per thread (warp butterflies, then a
-// butterfly over the warps' sums: a fixed order) into partial slots
-// k0 .. k0 + W - 1 of this block and into tot for every thread.  Only the
-// first `aw` warps can hold non-zero values; with one such warp the second
-// butterfly is skipped.
+// Warp sum of W = 1 or 4 float-float values.  For four, each of the first two
+// exchanges halves the values a lane carries on (6 additions and 12 shuffles
+// instead of 20 and 40): value w ends in lane 8 w.  A fixed order.
 template <int W>
-__device__ __forceinline__ void block_partials_ff(float2 (&a)[W], float2* parts, int k0, int aw,
-                                                  float2 (&tot)[W]) {
+__device__ __forceinline__ float2 warp_sum_ff(const float2 (&a)[W], int lane) {
+  float2 v = a[0];
+  int o = 16;
+  if (W == 4) {
+    const bool hi = lane & 16, up = lane & 8;
+    const float2 k0 = hi ? a[2] : a[0], k1 = hi ? a[3] : a[1];
+    const float2 s0 = hi ? a[0] : a[2], s1 = hi ? a[1] : a[3];
+    const float2 b0 = ff_add(k0, ff_shfl_xor(s0, 16)), b1 = ff_add(k1, ff_shfl_xor(s1, 16));
+    v = ff_add(up ? b1 : b0, ff_shfl_xor(up ? b0 : b1, 8));
+    o = 4;
+  }
+  for (; o > 0; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
+  return v;
+}
+
+// Block sum of W float-float values per thread (warp sums, then a sum over the
+// warps: a fixed order) into tot for every thread.  Only the first `aw` warps
+// can hold non-zero values.
+template <int W>
+__device__ __forceinline__ void block_sums_ff(float2 (&a)[W], int aw, float2 (&tot)[W]) {
   __shared__ float2 wsf[kModWarps][W];
   __shared__ float2 btf[W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < aw) {
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a[w] = ff_add(a[w], ff_shfl_xor(a[w], o));
-    if (lane == 0)
-#pragma unroll
-      for (int w = 0; w < W; ++w) wsf[warp][w] = a[w];
+    const float2 v = warp_sum_ff<W>(a, lane);
+    if ((lane & 7) == 0 && (lane >> 3) < W) wsf[warp][lane >> 3] = v;
   }
   __syncthreads();
   if (warp == 0) {
+    float2 t[W];
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      float2 t = lane < aw ? wsf[lane][w] : make_float2(0.0f, 0.0f);
-      if (aw > 1)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
-      if (lane == 0) {
-        parts[(size_t)blockIdx.x * kModParts + k0 + w] = t;
-        btf[w] = t;
-      }
-    }
+    for (int w = 0; w < W; ++w) t[w] = lane < aw ? wsf[lane][w] : make_float2(0.0f, 0.0f);
+    const float2 v = warp_sum_ff<W>(t, lane);
+    if ((lane & 7) == 0 && (lane >> 3) < W) btf[lane >> 3] = v;
   }
   __syncthreads();
 #pragma unroll
@@ -218,49 +224,6 @@ __device__ __forceinline__ bool group_barrier(ModGroup* g, int nb, uint64_t limi
 __device__ __forceinline__ int active_warps(int cnt) {
   const int w = (cnt + 31) >> 5;
   return w < kModWarps ? w : kModWarps;
-}
-
-// Sum over the group's blocks [b0, b0 + nb) of float-float partial
-// k0 .. k0 + W - 1 in a fixed order (thread-strided sums, warp butterflies, a
-// butterfly over the warps' sums when more than one warp holds values), so
-// the result does not depend on timing.  Every thread gets the totals.
-template <int W>
-__device__ __forceinline__ void group_reduce(const float2* parts, int b0, int nb, int k0,
-                                             float2 (&out)[W]) {
-  __shared__ float2 ws[kModWarps][W];
-  __shared__ float2 tot[W];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float2 s[W];
-#pragma unroll
-  for (int w = 0; w < W; ++w) s[w] = make_float2(0.0f, 0.0f);
-  for (int b = threadIdx.x; b < nb; b += kModThreads)
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-      s[w] = ff_add(s[w], __ldcg(parts + (size_t)(b0 + b) * kModParts + k0 + w));
-  const int aw = active_warps(nb);
-  if (warp < aw) {
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s[w] = ff_add(s[w], ff_shfl_xor(s[w], o));
-    if (lane == 0)
-#pragma unroll
-      for (int w = 0; w < W; ++w) ws[warp][w] = s[w];
-  }
-  __syncthreads();
-  if (warp == 0)
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      float2 t = lane < aw ? ws[lane][w] : make_float2(0.0f, 0.0f);
-      if (aw > 1)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
-      if (lane == 0) tot[w] = t;
-    }
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < W; ++w) out[w] = tot[w];
-  __syncthreads();
 }
 
 // Induced subgraph of a tree level, built before its launch: positions p of
@@ -337,48 +300,88 @@ __global__ void mod_fill_kernel(int nrows, const int32_t* __restrict__ rows,
 }
 
 // Summing barrier number `epoch` (1, 2, ... in every block of the group, in
-// the same sequence): the block's W float-float values go to its partial
-// slots of the barrier's parity, the block counts its arrival, waits for the
-// group's nb * epoch arrivals (bounded: a longer wait than limit_ns raises
-// g->err and returns false) and then sums every block's partials itself in
-// the group's fixed order, so all blocks hold the same totals.  Two slot sets
-// suffice: a block can rewrite a set only after every block has arrived at
-// the barrier in between, that is, after every block has read the set.
+// the same sequence): the block publishes its W = 1 or 4 float-float sums, each
+// 8-byte word with the barrier's number beside its float, and its threads read
+// every block's words until they carry that number (bounded: a longer wait
+// than limit_ns raises g->err and returns false), then add them in the group's
+// fixed order, so all blocks hold the same totals.  The words are their own
+// flags: one store and one read between the blocks, where an arrival counter,
+// its polling and a second read of the sums took 5,000 cycles of a step.  The
+// fences order the iterates that the blocks exchange around it.  Two word sets
+// suffice: a block rewrites a set only after every block has published the
+// barrier in between, that is, after every block has read the set.
 template <int W>
 __device__ __forceinline__ bool group_sums(float2 (&a)[W], ModGroup* g, int nb, int b0, int aw,
-                                           float2* parts, unsigned int& epoch, uint64_t limit_ns,
-                                           float2 (&out)[W]) {
-  __shared__ int ok_s;
+                                           unsigned long long* parts, unsigned int& epoch,
+                                           uint64_t limit_ns, float2 (&out)[W]) {
+  __shared__ float2 ws[kModWarps][4];
+  __shared__ float2 tot[4];
+  __shared__ int bad_s;
   ++epoch;
-  const int k0 = (int)(epoch & 1u) * 4;
-  block_partials_ff<W>(a, parts, k0, aw, out);  // ends with __syncthreads
-  if (nb == 1) return true;  // a group of one block takes its own totals
-  if (threadIdx.x == 0) {
-    const unsigned int target = (unsigned int)nb * epoch;
-    __threadfence();  // the block's partials before its arrival
-    int ok = 1;
-    if (atomicAdd(&g->arrive, 1u) + 1u < target) {
-      volatile unsigned int* c = &g->arrive;
-      uint64_t t0;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-      while (*c < target) {
+  block_sums_ff<W>(a, aw, out);  // ends with __syncthreads: the block's iterate is written
+  if (nb == 1) return true;      // a group of one block takes its own totals
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k0 = (int)(epoch & 1u) * 8;
+  const unsigned long long tag = (unsigned long long)epoch << 32;
+  if (threadIdx.x == 0) bad_s = 0;
+  if (warp == 0) {
+    if (lane < 2 * W) {
+      __threadfence();  // the iterate before the words that announce it
+      const float2 v = W == 4 ? ((lane >> 1) == 0   ? out[0]
+                                 : (lane >> 1) == 1 ? out[W > 1 ? 1 : 0]
+                                 : (lane >> 1) == 2 ? out[W > 2 ? 2 : 0]
+                                                    : out[W > 3 ? 3 : 0])
+                              : out[0];
+      volatile unsigned long long* w = parts + (size_t)blockIdx.x * kModParts + k0 + lane;
+      *w = tag | __float_as_uint((lane & 1) ? v.y : v.x);
+    }
+  }
+  // thread 4 b + w takes value w of blocks b, b + 256, ...
+  float2 v = make_float2(0.0f, 0.0f);
+  const int w = threadIdx.x & 3;
+  bool ok = true;
+  if (w < W)
+    for (int b = (int)threadIdx.x >> 2; b < nb && ok; b += kModThreads / 4) {
+      const volatile unsigned long long* q = parts + (size_t)(b0 + b) * kModParts + k0 + 2 * w;
+      unsigned long long h = q[0], l = q[1];
+      uint64_t t0 = 0;
+      for (unsigned int spin = 1; (h >> 32) != epoch || (l >> 32) != epoch; ++spin) {
+        h = q[0];
+        l = q[1];
+        if ((spin & 255u) != 0) continue;  // the timer is slow to read
         uint64_t t1;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        if (t0 == 0) t0 = t1;
         if (t1 - t0 > limit_ns) {
-          ok = 0;
-          atomicExch(&g->err, 1);
+          ok = false;
           break;
         }
-        __nanosleep(32);
       }
+      v = ff_add(v, make_float2(__uint_as_float((uint32_t)h), __uint_as_float((uint32_t)l)));
     }
-    __threadfence();
-    ok_s = ok;
+  const int nw = min(kModWarps, (4 * nb + 31) / 32);  // warps that read words
+  if (warp < nw) {
+    __threadfence();  // the other blocks' iterates are read after their words
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v = ff_add(v, ff_shfl_xor(v, o));
+    if (lane < 4) ws[warp][lane] = v;
   }
   __syncthreads();
-  if (!ok_s) return false;
-  group_reduce<W>(parts, b0, nb, k0, out);
-  return true;
+  if (!ok) {
+    bad_s = 1;
+    atomicExch(&g->err, 1);
+  }
+  if (warp == 0) {
+    float2 t[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t[k] = lane < nw ? ws[lane][k] : make_float2(0.0f, 0.0f);
+    const float2 r = warp_sum_ff<4>(t, lane);
+    if ((lane & 7) == 0) tot[lane >> 3] = r;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < W; ++k) out[k] = tot[k];
+  return bad_s == 0;
 }
 
 struct ModArgs {
@@ -392,11 +395,11 @@ struct ModArgs {
   ModGroup* groups;
   const int32_t* blk_grp;  // group index of every block
   double* vd;              // [2][nrows] by position: the final and previous iterates in double;
-                           // during the steps, the iterate of nodes without edges
+                           // during the steps, deep iterates of nodes without edges
   float2* vf;              // [2][nrows] iterate (hi, lo), by position
   float2* rs;              // [nrows] float-float row sums of a step
   double* y;               // [2][nrows] unnormalised iterates (hi, lo floats)
-  double* parts;           // [grid][kModParts]
+  double* parts;           // [grid][kModParts], zero at launch (the words' barrier numbers)
   int nrows;
   int stage_max;           // groups of at most this many nodes gather from shared memory
   int stage_bytes;         // offset of the column slice in dynamic shared memory
@@ -412,6 +415,63 @@ struct ModArgs {
 __device__ __forceinline__ int edge_col(const ModArgs& a, const uint16_t* s16, const int32_t* s32,
                                         int eb0, int e) {
   return s16 ? (int)s16[e - eb0] : s32 ? s32[e - eb0] : __ldg(a.lci + e);
+}
+
+// A_G y over the in-group edges of the block's positions (:342-343),
+// float-float: L lanes per position, four entries per lane in flight.  The
+// sums of the float-float additions are what a step's instructions go to
+// (a warp per position: 190 instructions a row whatever its length, 23,000 to
+// 48,000 cycles a step for groups of 500 to 1,000 nodes with 15 to 25 entries
+// per row), so L follows the group's mean row length.  FAST: iterate and 16-bit
+// columns are both in shared memory (without a branch per entry the four
+// entries' loads overlap: 292 instead of 349 ms for 10,001 nodes).
+template <int L, bool FAST>
+__device__ __forceinline__ void mod_spmv(const ModArgs& a, const float2* stage,
+                                         const float2* ypc, const uint16_t* s16,
+                                         const int32_t* s32, int eb0, int p0, int p1, float2* rs) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int R = 32 / L;
+  for (int pb = p0 + warp * R; pb < p1; pb += kModWarps * R) {
+    const int p = pb + lane / L;
+    int eb = 0, ee = 0;
+    if (p < p1) {
+      eb = __ldg(a.lrp + p);
+      ee = __ldg(a.lrp + p + 1);
+    }
+    float sh = 0.0f, sl = 0.0f;
+    for (int e0 = eb; e0 < ee; e0 += 4 * L) {
+      float2 x[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int e = e0 + lane % L + L * m;
+        x[m] = make_float2(0.0f, 0.0f);
+        if (FAST) {
+          if (e < ee) x[m] = stage[s16[e - eb0]];
+        } else if (e < ee) {
+          const int q = edge_col(a, s16, s32, eb0, e);
+          x[m] = stage ? stage[q] : __ldcg(ypc + q);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float t, e;
+        mod_two_sum(sh, x[m].x, t, e);
+        sh = t;
+        sl = __fadd_rn(sl, __fadd_rn(e, x[m].y));
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
+      const float ol = __shfl_xor_sync(0xffffffffu, sl, o);
+      float t, e;
+      mod_two_sum(sh, oh, t, e);
+      sh = t;
+      sl = __fadd_rn(sl, __fadd_rn(ol, e));
+    }
+    if (lane % L == 0 && p < p1) rs[p] = make_float2(sh, sl);
+  }
 }
 
 // One Lead_Vector call (Modularity_CPU.cpp:315-377) of group g with the
@@ -437,7 +497,7 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
     const int i = a.rows[p];
     const float2 x = ff_from_ll(i);
     a.vf[p] = x;
-    a.vd[p] = (double)i;  // the double iterate of a node without edges
+    a.vd[p] = (double)i;
     yb[p] = x;  // y_0 = x_0 with 1 / |y_0| taken as 1
     if (self_stage) stage[p - off] = x;
     p1s[0] = ff_add(p1s[0], ff_mulf(ff_from_ll(i), (float)(a.rp[i + 1] - a.rp[i])));
@@ -452,10 +512,10 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
   // square root per step)
   const float2 half_inv_m = mod_split(0.5 / Md);
   const float2 eps2 = mod_split(a.eps * a.eps);
-  float2* parts2 = reinterpret_cast<float2*>(a.parts);
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(a.parts);
   // a group of one block takes its own totals: no global barrier, no L2 round trip
   float2 t1[1];
-  if (!group_sums<1>(p1s, g, nb, b0, aw, parts2, epoch, a.limit_ns, t1)) return false;
+  if (!group_sums<1>(p1s, g, nb, b0, aw, words, epoch, a.limit_ns, t1)) return false;
   // Power steps (:327-366) with one group barrier each.  Step s gathers the
   // unnormalised y_{s-1} (published before the previous barrier) and scales
   // the row sums by 1 / |y_{s-1}|, since A (y / |y|) = (A y) / |y|; it forms
@@ -463,6 +523,61 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
   // |y_s|^2, y_s.k, |x_{s-1} -+ x_{s-2}|^2 in one reduction.  So the stop test
   // of iteration s - 1 (:358-361: the norms computed directly, as there) is
   // read one step later, and the step that revealed it is discarded.
+  // A position's degree and sumBG - beta, sumBG = |adj(i) ∩ G| - k K_G / 2 / M
+  // in integers (:258-266).  A thread with one position keeps them, and its
+  // iterate, in registers through the steps (the two divisions and the chain
+  // of loads behind them took as long as the rest of its step).
+  struct Node {
+    float k;
+    float2 sbg;
+  };
+  auto node = [&](int p) {
+    const int i = a.rows[p];
+    const long long k = a.rp[i + 1] - a.rp[i];
+    const float2 sbg = ff_from_ll((long long)(a.lrp[p + 1] - a.lrp[p]) - k * kg / 2 / a.M);
+    return Node{(float)k, ff_add(sbg, nbeta)};
+  };
+  const bool one = p1 - p0 <= kModThreads;
+  const int mine = p0 + (int)threadIdx.x;
+  Node own{0.0f, make_float2(0.0f, 0.0f)};
+  float2 yf = make_float2(0.0f, 0.0f), xf = yf, xfo = yf;  // y_{s-1}, x_{s-2}, x_{s-3} at step s
+  double xd = 0.0, xdo = 0.0;  // the same of a node without edges, once `deep`
+  if (one && mine < p1) {
+    own = node(mine);
+    yf = ff_from_ll(a.rows[mine]);
+  }
+  // Nodes without edges: y = beta x (no gather term, sumBG = 0), so all their
+  // entries are i F, F_0 = 1, F_s = beta F_{s-1} / |y_s|: one thread of the
+  // block keeps F and adds their part of the sums, F^2 times the sum of i^2 (in
+  // doubles each such node took about 35 instructions of the FP64 pipe a step,
+  // 10,000 cycles in a block of 800 nodes).  Under beta > 0 the factor shrinks
+  // step by step; below 2^-1000 (`deep`) every node goes on in its own double,
+  // so that entries reach the subnormal range and stay positive there as the
+  // reference's do (and are counted on the positive side).
+  __shared__ double fac_s[2];      // F of x_{s-1}, x_{s-2} after step s
+  __shared__ int deep_s;
+  __shared__ double iso_s[kModWarps];
+  constexpr double kDeep = 0x1p-1000;
+  double iso = 0.0;  // sum of i^2 of the block's nodes without edges
+  for (int p = p0 + (int)threadIdx.x; p < p1; p += kModThreads) {
+    const int i = a.rows[p];
+    if (a.rp[i + 1] == a.rp[i]) iso += (double)i * (double)i;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) iso += __shfl_xor_sync(0xffffffffu, iso, o);
+  if (lane == 0) iso_s[warp] = iso;
+  if (threadIdx.x == 0) {
+    fac_s[0] = fac_s[1] = 1.0;
+    deep_s = 0;
+  }
+  __syncthreads();
+  iso = 0.0;
+  for (int w = 0; w < kModWarps; ++w) iso += iso_s[w];
+  bool deep = false;
+  // row sums: in shared memory when every position has its thread
+  __shared__ float2 rs_s[kModThreads];
+  float2* const rs = one ? rs_s - p0 : a.rs;
+  const int len = (__ldg(a.lrp + off + nr) - __ldg(a.lrp + off)) / nr;  // mean in-group row
   float2 inv = make_float2(1.0f, 0.0f);            // 1 / |y_{s-1}|
   float2 c = ff_mul(t1[0], half_inv_m);            // v_k / 2 / M of x_{s-1}
   float2 vn = make_float2(0.0f, 0.0f);             // |y_{s-1}|: the eigenvalue estimate
@@ -476,88 +591,90 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
       for (int q = threadIdx.x; q < nr; q += kModThreads) stage[q] = __ldcg(ypc + q);
       __syncthreads();
     }
-    // A_G y_{s-1} over the in-group edges (:342-343), float-float: warp per position
-    for (int p = p0 + warp; p < p1; p += kModWarps) {
-      const int eb = __ldg(a.lrp + p), ee = __ldg(a.lrp + p + 1);
-      float sh = 0.0f, sl = 0.0f;
-      for (int e0 = eb; e0 < ee; e0 += 128) {
-        float2 x[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int e = e0 + lane + 32 * m;
-          const int q = e < ee ? edge_col(a, s16, s32, eb0, e) : -1;
-          x[m] = q < 0 ? make_float2(0.0f, 0.0f) : (staged ? stage[q] : __ldcg(ypc + q));
-        }
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          float t, e;
-          mod_two_sum(sh, x[m].x, t, e);
-          sh = t;
-          sl = __fadd_rn(sl, __fadd_rn(e, x[m].y));
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
-        const float ol = __shfl_xor_sync(0xffffffffu, sl, o);
-        float t, e;
-        mod_two_sum(sh, oh, t, e);
-        sh = t;
-        sl = __fadd_rn(sl, __fadd_rn(ol, e));
-      }
-      if (lane == 0) a.rs[p] = make_float2(sh, sl);
-    }
+    auto spmv = [&](auto fast) {
+      constexpr bool kFast = decltype(fast)::value;
+      const float2* st = staged ? stage : nullptr;
+      if (len <= 6)
+        mod_spmv<2, kFast>(a, st, ypc, s16, s32, eb0, p0, p1, rs);
+      else if (len <= 12)
+        mod_spmv<4, kFast>(a, st, ypc, s16, s32, eb0, p0, p1, rs);
+      else if (len <= 40)
+        mod_spmv<8, kFast>(a, st, ypc, s16, s32, eb0, p0, p1, rs);
+      else if (len <= 80)
+        mod_spmv<16, kFast>(a, st, ypc, s16, s32, eb0, p0, p1, rs);
+      else
+        mod_spmv<32, kFast>(a, st, ypc, s16, s32, eb0, p0, p1, rs);
+    };
+    if (staged && s16)
+      spmv(std::true_type());
+    else
+      spmv(std::false_type());
     __syncthreads();
     // thread per position: x_{s-1} = y_{s-1} / |y_{s-1}| (:349-351), its
     // distances to x_{s-2} (:352-357), and y_s = A_G x_{s-1} - (v_k / 2 / M k
-    // + (sumBG - beta) x_{s-1}) (:344); sumBG = |adj(i) ∩ G| - k K_G / 2 / M
-    // in integers (:258-266)
+    // + (sumBG - beta) x_{s-1}) (:344)
     float2 pe[4] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f),
                     make_float2(0.0f, 0.0f)};
+    const bool go_deep = !deep && deep_s != 0;  // set in the previous step, the same in all threads
     for (int p = p0 + (int)threadIdx.x; p < p1; p += kModThreads) {
-      const int i = a.rows[p];
-      const long long k = a.rp[i + 1] - a.rp[i];
-      if (k == 0) {
-        // A node without edges: y = beta x (no gather term, sumBG = 0), so
-        // under beta > 0 its entry shrinks by a factor per step and can fall
-        // far below float's range while staying positive in the reference's
-        // doubles (and so counted on the positive side).  Its iterate stays
-        // in double (vd, by the parity of the float-float buffers).
-        double xd = a.vd[p];  // x_0 = i
-        if (s > 1) {
-          const double xo = a.vd[xold + p];
-          xd = __dmul_rn(__dmul_rn(beta, xo), ff_to_d(inv));
-          a.vd[xcur + p] = xd;
-          const double d = __dsub_rn(xd, xo), u = __dadd_rn(xd, xo);
+      if (!one) own = node(p);
+      if (own.k == 0.0f) {
+        if (!go_deep && !deep) continue;  // kept as a factor
+        const double xo = go_deep ? (double)a.rows[p] * fac_s[0] : one ? xd : a.vd[xold + p];
+        const double x = __dmul_rn(__dmul_rn(beta, xo), ff_to_d(inv));
+        if (!one) {
+          if (go_deep) a.vd[xold + p] = xo;
+          a.vd[xcur + p] = x;
+        }
+        xdo = xo;
+        xd = x;
+        // squares below 2^-1074 are 0: nothing to add while the entries stay
+        // below 2^-560 (checked on the bits; beta is below 2^20)
+        const int ex = max(__double2hiint(x) & 0x7ff00000, __double2hiint(xo) & 0x7ff00000);
+        if (ex >= (1023 - 560) << 20) {
+          const double d = __dsub_rn(x, xo), u = __dadd_rn(x, xo);
           pe[2] = ff_add(pe[2], mod_split(__dmul_rn(d, d)));
           pe[3] = ff_add(pe[3], mod_split(__dmul_rn(u, u)));
+          const double yd = __dmul_rn(beta, x);
+          pe[0] = ff_add(pe[0], mod_split(__dmul_rn(yd, yd)));
         }
-        const double yd = __dmul_rn(beta, xd);
-        const float2 y = mod_split(yd);
-        yb[ycur + p] = y;
-        if (self_stage) stage[p - off] = y;
-        pe[0] = ff_add(pe[0], mod_split(__dmul_rn(yd, yd)));
         continue;
       }
-      const float2 x = s == 1 ? a.vf[p] : ff_mul(yb[yprv + p], inv);
+      const float2 x = s == 1 ? (one ? yf : a.vf[p]) : ff_mul(one ? yf : yb[yprv + p], inv);
       if (s > 1) {
-        const float2 old = a.vf[xold + p];
-        a.vf[xcur + p] = x;
+        const float2 old = one ? xf : a.vf[xold + p];
+        if (!one) a.vf[xcur + p] = x;
+        xfo = old;
         const float2 d = ff_add(x, ff_neg(old)), u = ff_add(x, old);
         pe[2] = ff_add(pe[2], ff_mul(d, d));
         pe[3] = ff_add(pe[3], ff_mul(u, u));
       }
-      const float2 sbg =
-          ff_from_ll((long long)(a.lrp[p + 1] - a.lrp[p]) - k * kg / 2 / a.M);
-      const float2 corr = ff_add(ff_mulf(c, (float)k), ff_mul(ff_add(sbg, nbeta), x));
-      const float2 y = ff_add(ff_mul(a.rs[p], inv), ff_neg(corr));
+      xf = x;
+      const float2 corr = ff_add(ff_mulf(c, own.k), ff_mul(own.sbg, x));
+      const float2 y = ff_add(ff_mul(rs[p], inv), ff_neg(corr));
+      yf = y;
       yb[ycur + p] = y;
       if (self_stage) stage[p - off] = y;  // the gathers of this step are over
       pe[0] = ff_add(pe[0], ff_mul(y, y));
-      pe[1] = ff_add(pe[1], ff_mulf(y, (float)k));
+      pe[1] = ff_add(pe[1], ff_mulf(y, own.k));
+    }
+    deep = deep || go_deep;
+    if (!deep && iso != 0.0 && threadIdx.x == kModThreads - 1) {
+      const double fo = fac_s[0];
+      const double fx = s > 1 ? __dmul_rn(__dmul_rn(beta, fo), ff_to_d(inv)) : fo;
+      fac_s[1] = fo;
+      fac_s[0] = fx;
+      const double yd = __dmul_rn(beta, fx);
+      pe[0] = ff_add(pe[0], mod_split(__dmul_rn(__dmul_rn(yd, yd), iso)));
+      if (s > 1) {
+        const double d = __dsub_rn(fx, fo), u = __dadd_rn(fx, fo);
+        pe[2] = ff_add(pe[2], mod_split(__dmul_rn(__dmul_rn(d, d), iso)));
+        pe[3] = ff_add(pe[3], mod_split(__dmul_rn(__dmul_rn(u, u), iso)));
+      }
+      if (fx != 0.0 && fabs(fx) < kDeep) deep_s = 1;
     }
     float2 te[4];
-    if (!group_sums<4>(pe, g, nb, b0, aw, parts2, epoch, a.limit_ns, te)) return false;
+    if (!group_sums<4>(pe, g, nb, b0, kModWarps, words, epoch, a.limit_ns, te)) return false;
     it = s - 1;
     if (s > 1) {
       err1 = te[2];
@@ -581,9 +698,18 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
   const size_t fin = (size_t)(it & 1) * a.nrows, prv = (size_t)((it + 1) & 1) * a.nrows;
   for (int p = p0 + (int)threadIdx.x; p < p1; p += kModThreads) {
     const int i = a.rows[p];
-    if (a.rp[i + 1] == a.rp[i]) continue;  // kept in double during the steps
-    a.vd[fin + p] = ff_to_d(a.vf[fin + p]);
-    a.vd[prv + p] = ff_to_d(a.vf[prv + p]);
+    const bool none = a.rp[i + 1] == a.rp[i];
+    if (it == 0) continue;  // no step: vd holds x_0
+    if (none && !deep) {
+      a.vd[fin + p] = (double)i * fac_s[0];
+      a.vd[prv + p] = (double)i * fac_s[1];
+    } else if (one) {
+      a.vd[fin + p] = none ? xd : ff_to_d(xf);
+      a.vd[prv + p] = none ? xdo : ff_to_d(xfo);
+    } else if (!none) {  // those without edges were kept in double during the steps
+      a.vd[fin + p] = ff_to_d(a.vf[fin + p]);
+      a.vd[prv + p] = ff_to_d(a.vf[prv + p]);
+    }
   }
   double best = 0.0;
   int bq = 0x7fffffff;  // position of the maximum (positions ascend with node index)
@@ -630,10 +756,10 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
       sns[0] += sns[w];
     }
     double* pp = a.parts + (size_t)blockIdx.x * kModParts;
-    pp[8] = sb[0];
-    pp[9] = (double)si[0];
-    pp[10] = (double)sps[0];  // counts < 2^53: exact in a double
-    pp[11] = (double)sns[0];
+    pp[16] = sb[0];
+    pp[17] = (double)si[0];
+    pp[18] = (double)sps[0];  // counts < 2^53: exact in a double
+    pp[19] = (double)sns[0];
   }
   if (!group_barrier(g, nb, a.limit_ns)) return false;
   double gb = 0.0;
@@ -641,14 +767,14 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
   long long gp = 0, gn = 0;
   for (int b = 0; b < nb; ++b) {  // fixed order, every block alike
     const double* pp = a.parts + (size_t)(b0 + b) * kModParts;
-    const double ob = __ldcg(pp + 8);
-    const int oi = (int)__ldcg(pp + 9);
+    const double ob = __ldcg(pp + 16);
+    const int oi = (int)__ldcg(pp + 17);
     if (ob > gb || (ob == gb && oi < gq)) {
       gb = ob;
       gq = oi;
     }
-    gp += (long long)__ldcg(pp + 10);
-    gn += (long long)__ldcg(pp + 11);
+    gp += (long long)__ldcg(pp + 18);
+    gn += (long long)__ldcg(pp + 19);
   }
   double prod = 0.0;
   if (gb > 0.0) {
