@@ -426,7 +426,10 @@ int64_t bna_request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64
   b += elist * 8;                                              // edge lists
   b += cand * 8 + 2 * cand * 13 + (density ? cand * 4 : 0);    // candidates, hash, values
   b += (long long)(N + 1) * 4 + nnz * (opts->weighted ? 8 : 4);  // CSR
-  if (with_ec) b += (long long)N * (2 * 16 + 8) + 64 * 1024;     // iterates, output, partials
+  if (with_ec) {  // iterates, output, partials; the streamed form's copy and row ends
+    b += (long long)N * (2 * 16 + 8) + 64 * 1024;
+    if (flow_chunks(N) <= kFlowChunkMax) b += nnz * 6 + (long long)N * (kFlowChunkMax * 8 + 8);
+  }
   return b;
 }
 

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "ec_df.cuh"
 
 namespace bna {
 size_t zscore_scratch_bytes(int n_pad);
@@ -66,11 +67,7 @@ cudaError_t launch_mod_map(int n, const int32_t* label, const int32_t* adj, int3
                            int sms, cudaStream_t s);
 cudaError_t launch_ec_init(int n, double* u, float2* uf, double* parts, void* st, int grid,
                            int max_iter, cudaStream_t stream);
-cudaError_t launch_ec_iter(int n, const int32_t* rp, const int32_t* ci, const float* val,
-                           const double* vald, long long nnz_used, const double* u,
-                           const float2* uf, double* un, float2* unf, double* parts, void* st,
-                           int grid, int max_iter, double eps, cudaStream_t stream);
-cudaError_t launch_ec_iter_sparse(int n, const int32_t* rp, const int32_t* ci, const float* val,
+cudaError_t launch_ec_sparse(int n, const int32_t* rp, const int32_t* ci, const float* val,
                            const double* vald, long long nnz_used, const double* u,
                            const float2* uf, double* un, float2* unf, double* parts, void* st,
                            int grid, int max_iter, double eps, cudaStream_t stream);
@@ -78,16 +75,26 @@ void ec_state_read(const void* host_copy, double* lam2, double* lambda_used, dou
                    double* e2, int* iter, int* done);
 int ec_state_err(const void* host_copy);
 int ec_coop_grid(int n, int sms);
-int ec_chunk_count(int n);
-cudaError_t launch_ec_chunk_prep(int n, const int32_t* rp, const int32_t* ci, long long nnz_used,
-                                 unsigned long long* info, int* csplit, int grid, int* rowsplit,
-                                 cudaStream_t stream);
-cudaError_t prepare_ec_chunk();
-cudaError_t launch_ec_chunk(int n, const int32_t* rp, const int32_t* ci, const float* val,
+constexpr int kFlowChunkMax = 4;  // column chunks of the streamed centrality (graph.cu)
+int flow_chunks(int n);
+int flow_warps_per_block();
+int flow_pad();
+cudaError_t launch_ec_sorted(int n, const int32_t* rp, const int32_t* ci, long long nnz_used,
+                             unsigned long long* info, cudaStream_t stream);
+cudaError_t launch_flow_split(int n, const int32_t* rp, long long nnz_used, int W, int weight,
+                              int* wrow, cudaStream_t stream);
+int ec_range_grid(int sms);
+cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const float* val,
                             const double* vald, long long nnz_used, const double* u,
                             const float2* uf, double* un, float2* unf, double* parts, void* st,
-                            int grid, int max_iter, double eps, const int* rowsplit,
-                            const int* csplit, float2* part, cudaStream_t stream);
+                            int sms, int max_iter, double eps, const int* split, float2* part,
+                            cudaStream_t stream);
+cudaError_t launch_flow_layout(int n, const int32_t* rp, const int32_t* ci, const float* val,
+                               const double* vald, long long nnz_used, const EcFlow& f, int sms,
+                               cudaStream_t stream);
+cudaError_t launch_ec_flow(int n, const int32_t* rp, long long nnz_used, const EcFlow& f,
+                           const double* u, const float2* uf, double* un, float2* unf,
+                           double* parts, void* st, int max_iter, double eps, cudaStream_t stream);
 cudaError_t launch_ec_coop(int n, const int32_t* rp, const int32_t* ci, const float* val,
                            const double* vald, long long nnz_used, double* u, float2* uf,
                            double* parts, void* st, int grid, int it_end, int max_iter,
@@ -168,7 +175,8 @@ enum Slot {
   S_BATCH_SUBJ, S_BATCH_TILES,
   S_MOD_LABEL, S_MOD_ROWS, S_MOD_LOC, S_MOD_CNT, S_MOD_LRP, S_MOD_LCI, S_MOD_VD, S_MOD_VF,
   S_MOD_RS, S_MOD_Y, S_MOD_PARTS, S_MOD_GROUPS, S_MOD_BLKGRP, S_MOD_ASSIGN, S_MOD_KMOD,
-  S_MOD_ADJ, S_EC_SPLIT, S_EC_PART, S_EC_ROWS, S_EC_FLAG, S_TCSCHED,
+  S_MOD_ADJ, S_EC_SPLIT, S_EC_PART, S_EC_ROWS, S_EC_FLAG, S_EC_C16, S_EC_VAL,
+  S_EC_REND, S_EC_WST, S_TCSCHED,
   S_ZQ, S_E2, S_EBLK, S_SC_TILES, S_SC_KEEP, S_SC_OUT, S_SC_COUNT, S_COUNT
 };
 
@@ -185,9 +193,9 @@ struct DevStatus {
 struct EcGraph {
   cudaGraphExec_t exec = nullptr;
   int iters = 0;  // iterations per replay
-  bool chunked = false;  // the column-chunked kernel
-  // the CSR, the iterate, the state block, and the chunked kernel's buffers
-  const void* key[9] = {};
+  int form = 0;  // 0 ranged, 1 a thread per row, 2 streamed
+  // the CSR, the iterate, the state block, and the streamed form's buffers
+  const void* key[12] = {};
   int n = -1, grid = 0, max_iter = 0;
   long long nnz_used = -1;
   double eps = 0;

@@ -31,21 +31,9 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "ec_df.cuh"
 
 namespace bna {
-
-struct EcState {
-  double lam2;        // sum of squares of the current iterate
-  double lambda_used; // lambda of the last completed iteration (the returned eigenvalue)
-  double e1, e2;
-  int iter;           // completed iterations
-  int done;
-  unsigned int counter;
-  int err;                // bounded grid barrier expired (persistent kernel)
-  unsigned int bar_count, bar_gen;  // grid barrier of the persistent kernel
-  double tot[5];          // persistent kernel: lam2, e1, e2, lambda, 1/lambda published by
-                          // the last block to reach the barrier
-};
 
 constexpr int kEcThreads = 256;
 
@@ -56,8 +44,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Fixed-order reduction of `parts` (nparts x 3) by one block; results to out[3].
+template <int T = kEcThreads>
 __device__ __forceinline__ void reduce_partials(const double* parts, int nparts, double* out) {
-  __shared__ double red[kEcThreads][3];
+  __shared__ double red[T][3];
   double s0 = 0, s1 = 0, s2 = 0;
   for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
     s0 += parts[b * 3 + 0];
@@ -91,19 +80,6 @@ __device__ __forceinline__ bool last_block_arrives(EcState* st) {
   __syncthreads();
   if (last) __threadfence();
   return last;
-}
-
-// (hi, lo) float pair of a double: hi = RN(x), lo = RN(x - hi).
-__device__ __forceinline__ float2 split_df(double x) {
-  const float hi = __double2float_rn(x);
-  return make_float2(hi, __double2float_rn(x - (double)hi));
-}
-
-// Knuth's TwoSum: s + e == a + b exactly.
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
 __global__ __launch_bounds__(kEcThreads) void ec_init_kernel(int n, double* u, float2* uf,
@@ -142,58 +118,69 @@ __global__ __launch_bounds__(kEcThreads) void ec_init_kernel(int n, double* u, f
   }
 }
 
-// One nonzero: (sh, sl) += v * (x.hi + x.lo), v given as (vh, vl) (vl = 0 for float values).
-template <int VK>
-__device__ __forceinline__ void df_accum(float& sh, float& sl, float vh, float vl, float2 x) {
-  float p, pe;
-  if (VK == 0) {  // binary graph: v = 1
-    p = x.x;
-    pe = x.y;
-  } else {
-    p = __fmul_rn(vh, x.x);
-    pe = __fmaf_rn(vh, x.x, -p);  // exact low part of vh * x.hi
-    pe = __fmaf_rn(vh, x.y, pe);
-    if (VK == 2) pe = __fmaf_rn(vl, x.x, pe);
-  }
-  float s, e;
-  two_sum(sh, p, s, e);
-  sh = s;
-  sl = __fadd_rn(sl, __fadd_rn(e, pe));
-}
-
 // One warp, one row: (sh, sl) += sum over entries [b, e) of val * x[col], eight
-// entries per lane in flight per round (predicated, so a row costs
-// ceil((e - b) / 256) memory round trips).  l2_only: read x through L2 only
-// (the persistent kernel, whose iterate other blocks rewrite in the same launch).
+// entries per lane in flight per round, the last round predicated with only the
+// arithmetic that it needs (so a row costs ceil((e - b) / 256) memory round
+// trips).  l2_only: read x through L2 only (the persistent kernel, whose iterate
+// other blocks rewrite in the same launch).
 template <int VK>
 __device__ __forceinline__ void ec_row_accum(const int32_t* __restrict__ ci,
                                              const float* __restrict__ val,
                                              const double* __restrict__ vald,
                                              const float2* uf, long long b, long long e,
                                              int lane, float& sh, float& sl, bool l2_only) {
-  for (long long k0 = b; k0 < e; k0 += 256) {
+  if (e <= b) return;
+  const int32_t* cp = ci + b + lane;
+  const float* vp = VK == 1 ? val + b + lane : nullptr;
+  const double* dp = VK == 2 ? vald + b + lane : nullptr;
+  int len = (int)(e - b);  // a row has at most n entries
+  for (; len >= 256; len -= 256) {
     int c[8];
     float vh[8], vl[8];
+    float2 x[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-      const long long k = k0 + lane + 32 * m;
-      const bool ok = k < e;
-      c[m] = ok ? __ldg(ci + k) : -1;
+      c[m] = __ldg(cp + 32 * m);
       vh[m] = 1.0f;
       vl[m] = 0.0f;
-      if (VK == 1) vh[m] = ok ? __ldg(val + k) : 0.0f;
+      if (VK == 1) vh[m] = __ldg(vp + 32 * m);
       if (VK == 2) {
-        const float2 d = split_df(ok ? __ldg(vald + k) : 0.0);
+        const float2 d = split_df(__ldg(dp + 32 * m));
         vh[m] = d.x;
         vl[m] = d.y;
       }
     }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) x[m] = l2_only ? __ldcg(uf + c[m]) : uf[c[m]];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
+    cp += 256;
+    if (VK == 1) vp += 256;
+    if (VK == 2) dp += 256;
+  }
+  if (len > 0) {
+    int c[8];
+    float vh[8], vl[8];
     float2 x[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const bool ok = lane + 32 * m < len;
+      c[m] = ok ? __ldg(cp + 32 * m) : -1;
+      vh[m] = 1.0f;
+      vl[m] = 0.0f;
+      if (VK == 1) vh[m] = ok ? __ldg(vp + 32 * m) : 0.0f;
+      if (VK == 2) {
+        const float2 d = split_df(ok ? __ldg(dp + 32 * m) : 0.0);
+        vh[m] = d.x;
+        vl[m] = d.y;
+      }
+    }
 #pragma unroll
     for (int m = 0; m < 8; ++m)
       x[m] = c[m] < 0 ? make_float2(0.0f, 0.0f) : (l2_only ? __ldcg(uf + c[m]) : uf[c[m]]);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
+    for (int m = 0; m < 8; ++m)
+      if (32 * m < len) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
   }
 }
 
@@ -349,7 +336,7 @@ __device__ __forceinline__ void ec_block_rows_sparse(int n, const int32_t* __res
 // then a butterfly over the warps' sums in warp 0) into parts[blockIdx.x * 3 ..].
 __device__ __forceinline__ void ec_block_partials(double a0, double a1, double a2, int aw,
                                                   double* parts) {
-  __shared__ double ws[kEcThreads / 32][3];
+  __shared__ double ws[32][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < aw) {
 #pragma unroll
@@ -384,9 +371,9 @@ __device__ __forceinline__ void ec_block_partials(double a0, double a1, double a
 }
 
 // VK: 0 binary (val NULL), 1 float values, 2 double values (split into a float pair).
-// SPARSE: rows by ec_block_rows_sparse.
-template <int VK, bool SPARSE = false>
-__global__ __launch_bounds__(kEcThreads, 4) void ec_iter_kernel(
+// The per-iteration kernel of sparse graphs.
+template <int VK>
+__global__ __launch_bounds__(kEcThreads, 4) void ec_sparse_kernel(
     int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, const double* __restrict__ vald, long long nnz_used,
     const double* __restrict__ u, const float2* __restrict__ uf, double* __restrict__ un,
@@ -404,10 +391,7 @@ __global__ __launch_bounds__(kEcThreads, 4) void ec_iter_kernel(
   const double lam = lam_s[0];
   const double inv = lam_s[1];
   double a0 = 0, a1 = 0, a2 = 0;
-  if (SPARSE)
-    ec_block_rows_sparse<VK>(n, rp, ci, val, vald, nnz_used, u, uf, un, unf, inv, a0, a1, a2);
-  else
-    ec_block_rows<VK>(n, rp, ci, val, vald, nnz_used, u, uf, un, unf, inv, false, a0, a1, a2);
+  ec_block_rows_sparse<VK>(n, rp, ci, val, vald, nnz_used, u, uf, un, unf, inv, a0, a1, a2);
   ec_block_partials(a0, a1, a2, kEcThreads / 32, parts);
   if (last_block_arrives(st)) {
     __shared__ double tot[3];
@@ -424,128 +408,86 @@ __global__ __launch_bounds__(kEcThreads, 4) void ec_iter_kernel(
   }
 }
 
-// ---- column-chunked form -------------------------------------------------------
+// ---- ranged form ------------------------------------------------------------
 //
-// For graphs whose iterate does not stay in L1 (random graphs of tens of
-// thousands of vertices), the (hi, lo) iterate gathers of ec_iter_kernel miss
-// L1 and pull a 32-byte L2 sector per 8-byte entry.  Here one 1024-thread block
-// per SM stages the iterate in shared memory a chunk of kEcChunkCols columns
-// at a time and gathers from there; each row's entries are split at the chunk
-// boundaries once per CSR (columns ascending within a row), and a row's
-// partial sum is carried from chunk to chunk in float-float.  Rows go to blocks
-// in contiguous ranges balanced by entries (plus a per-row weight); the FP64
-// epilogue, the block partials and the last-block reduction follow
-// ec_iter_kernel's, in a fixed order.
-constexpr int kEcChunkThreads = 1024;
-constexpr int kEcChunkCols = 24576;  // 192 KB of (hi, lo) pairs
-constexpr int kEcChunkRowsSmem = 3072;  // 24 KB of row sums beside them
-constexpr int kEcRowWeight = 32;     // entries a row costs in the block split
-
-// One warp, one row: eight entries per lane in flight per round of 256.
-template <int VK>
-__device__ __forceinline__ void ec_row_accum_smem(const int32_t* __restrict__ ci,
-                                                  const float* __restrict__ val,
-                                                  const double* __restrict__ vald,
-                                                  const float2* xs, int c0, long long b,
-                                                  long long e, int lane, float& sh, float& sl) {
-  for (long long k0 = b; k0 < e; k0 += 256) {
-    int c[8];
-    float vh[8], vl[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const long long k = k0 + lane + 32 * m;
-      const bool ok = k < e;
-      c[m] = ok ? __ldg(ci + k) - c0 : -1;
-      vh[m] = 1.0f;
-      vl[m] = 0.0f;
-      if (VK == 1) vh[m] = ok ? __ldg(val + k) : 0.0f;
-      if (VK == 2) {
-        const float2 d = split_df(ok ? __ldg(vald + k) : 0.0);
-        vh[m] = d.x;
-        vl[m] = d.y;
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const float2 x = c[m] < 0 ? make_float2(0.0f, 0.0f) : xs[c[m]];
-      df_accum<VK>(sh, sl, vh[m], vl[m], x);
-    }
-  }
-}
+// The per-iteration kernel for large graphs: each block has a contiguous range
+// of rows with about the same cost (entries + kEcRangeWeight per row), its warps
+// take the range's rows from a counter, one at a time, with the next row's ends
+// in flight.  Rows dealt out in turn to all warps of the grid leave the slowest
+// warp with far more than the mean where lengths vary: 120,000 vertices in
+// contiguous networks, rows of 0 to 1,999 entries, 77 M in all, took 153 us per
+// iteration, 137 in ranges, and 121 once the entries that a row has past a
+// multiple of 256 no longer ran the arithmetic of all 256 (5.1 TB/s of column
+// and value; 60,000 vertices, 19 M: 53, 51, 46).  Bound: issue (~30 instructions
+// per 32 entries) and the latency at the end of each row.  Two blocks of 512
+// measured as one of 1,024 or four of 256 (121, 121, 124 us); more warps with
+// fewer registers were slower (126 to 149 us).
+constexpr int kRangeThreads = 512;  // two blocks per SM
+constexpr int kEcRangeRows = 2048;  // row sums of a block kept in shared memory
 
 template <int VK>
-__global__ __launch_bounds__(kEcChunkThreads, 1) void ec_chunk_kernel(
+__global__ __launch_bounds__(kRangeThreads, 4 * kEcThreads / kRangeThreads) void ec_range_kernel(
     int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, const double* __restrict__ vald, long long nnz_used,
     const double* __restrict__ u, const float2* __restrict__ uf, double* __restrict__ un,
     float2* __restrict__ unf, double* parts, EcState* st, int max_iter, double eps,
-    const int* __restrict__ rowsplit, const int* __restrict__ csplit, int nch,
-    float2* __restrict__ part) {
-  extern __shared__ __align__(16) float2 xs[];
+    const int* __restrict__ split, float2* __restrict__ part) {
   if (st->done || st->iter >= max_iter) return;
   __shared__ double lam_s[2];
+  __shared__ float2 rs[kEcRangeRows];
+  __shared__ int next;
+  const int lane = threadIdx.x & 31;
+  const int R0 = split[blockIdx.x], R1 = split[blockIdx.x + 1];
+  const bool in_smem = R1 - R0 <= kEcRangeRows;
   if (threadIdx.x == 0) {
     const double l2 = st->lam2;
     lam_s[1] = rsqrt(l2);
     lam_s[0] = l2 == 0.0 ? 0.0 : l2 * lam_s[1];
+    next = R0;
   }
-  constexpr int kW = kEcChunkThreads / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r0 = rowsplit[blockIdx.x], r1 = rowsplit[blockIdx.x + 1];
-  // the block's row sums between chunks: shared memory when they fit
-  float2* ps = xs + kEcChunkCols;
-  const bool in_smem = r1 - r0 <= kEcChunkRowsSmem;
-  for (int c = 0; c < nch; ++c) {
-    const int c0 = c * kEcChunkCols;
-    const int cn = min(kEcChunkCols, n - c0);
-    __syncthreads();  // the previous chunk's readers are done
-    // two pairs per 16-byte load when the chunk starts on a 16-byte boundary
-    // (the second iterate buffer starts at uf + n: 8-byte aligned for odd n)
-    if ((reinterpret_cast<uintptr_t>(uf + c0) & 15u) == 0) {
-      const float4* src4 = reinterpret_cast<const float4*>(uf + c0);
-      float4* dst4 = reinterpret_cast<float4*>(xs);
-      for (int k = threadIdx.x; k < cn / 2; k += kEcChunkThreads) dst4[k] = src4[k];
-      if ((cn & 1) && threadIdx.x == 0) xs[cn - 1] = uf[c0 + cn - 1];
-    } else {
-      for (int k = threadIdx.x; k < cn; k += kEcChunkThreads) xs[k] = uf[c0 + k];
+  __syncthreads();
+  // the next row's ends are in flight while a row is summed
+  int nrow = 0, nb = 0, ne = 0;
+  auto claim = [&]() {
+    if (lane == 0) nrow = atomicAdd(&next, 1);
+    nrow = __shfl_sync(0xffffffffu, nrow, 0);
+    if (nrow < R1) {
+      nb = __ldg(rp + nrow);
+      ne = __ldg(rp + nrow + 1);
     }
-    __syncthreads();
-    for (int row = r0 + warp; row < r1; row += kW) {
-      long long b = c == 0 ? __ldg(rp + row) : __ldg(csplit + (size_t)(c - 1) * n + row);
-      long long e = c == nch - 1 ? __ldg(rp + row + 1) : __ldg(csplit + (size_t)c * n + row);
-      if (e > nnz_used) e = nnz_used;
-      if (b >= e && c > 0) continue;  // nothing of this row in this chunk
-      float sh = 0.0f, sl = 0.0f;
-      if (b < e) ec_row_accum_smem<VK>(ci, val, vald, xs, c0, b, e, lane, sh, sl);
+  };
+  claim();
+  while (nrow < R1) {
+    const int row = nrow;
+    const long long b = nb;
+    long long e = ne;
+    claim();
+    if (e > nnz_used) e = nnz_used;
+    float sh = 0.0f, sl = 0.0f;
+    ec_row_accum<VK>(ci, val, vald, uf, b, e, lane, sh, sl, false);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
-        const float ol = __shfl_xor_sync(0xffffffffu, sl, o);
-        float s2, e2;
-        two_sum(sh, oh, s2, e2);
-        sh = s2;
-        sl = __fadd_rn(sl, __fadd_rn(ol, e2));
-      }
-      if (lane == 0) {
-        float2* pr = in_smem ? &ps[row - r0] : &part[row];
-        if (c > 0) {  // add to the row's sum of the earlier chunks
-          const float2 p = *pr;
-          float s2, e2;
-          two_sum(p.x, sh, s2, e2);
-          sh = s2;
-          sl = __fadd_rn(__fadd_rn(p.y, sl), e2);
-        }
-        *pr = make_float2(sh, sl);
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
+      const float ol = __shfl_xor_sync(0xffffffffu, sl, o);
+      float s2, e2;
+      two_sum(sh, oh, s2, e2);
+      sh = s2;
+      sl = __fadd_rn(sl, __fadd_rn(ol, e2));
+    }
+    if (lane == 0) {
+      if (in_smem)
+        rs[row - R0] = make_float2(sh, sl);
+      else
+        part[row] = make_float2(sh, sl);
     }
   }
-  __syncthreads();  // every row's sum is in ps[] / part[]
+  __syncthreads();
   const double lam = lam_s[0], inv = lam_s[1];
   double a0 = 0, a1 = 0, a2 = 0;
-  for (int row = r0 + (int)threadIdx.x; row < r1; row += kEcChunkThreads) {
+  for (int row = R0 + (int)threadIdx.x; row < R1; row += kRangeThreads) {
     long long b = __ldg(rp + row), e = __ldg(rp + row + 1);
     if (e > nnz_used) e = nnz_used;
-    const float2 sm = in_smem ? ps[row - r0] : part[row];
+    const float2 sm = in_smem ? rs[row - R0] : part[row];
     // a row without entries gives 0 even when 1 / lambda is infinite
     const double y = e <= b ? 0.0 : ((double)sm.x + (double)sm.y) * inv;
     const double old = u[row];
@@ -556,61 +498,15 @@ __global__ __launch_bounds__(kEcChunkThreads, 1) void ec_chunk_kernel(
     a1 += d * d;
     a2 += p * p;
   }
-  // block partials: warp butterflies, then the warps' sums by warp 0
-  __shared__ double ws[kW][3];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-  }
-  if (lane == 0) {
-    ws[warp][0] = a0;
-    ws[warp][1] = a1;
-    ws[warp][2] = a2;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    double t0 = ws[lane][0], t1 = ws[lane][1], t2 = ws[lane][2];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      t0 += __shfl_xor_sync(0xffffffffu, t0, o);
-      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
-      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
-    }
-    if (lane == 0) {
-      parts[blockIdx.x * 3 + 0] = t0;
-      parts[blockIdx.x * 3 + 1] = t1;
-      parts[blockIdx.x * 3 + 2] = t2;
-    }
-  }
-  // the last block to finish reduces the blocks' partials (warp 0: strided
-  // sums per lane, then a butterfly; a fixed order)
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(&st->counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (warp == 0) {
-    double t0 = 0, t1 = 0, t2 = 0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) {
-      t0 += __ldcg(parts + b * 3 + 0);
-      t1 += __ldcg(parts + b * 3 + 1);
-      t2 += __ldcg(parts + b * 3 + 2);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      t0 += __shfl_xor_sync(0xffffffffu, t0, o);
-      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
-      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
-    }
-    if (lane == 0) {
+  ec_block_partials(a0, a1, a2, kRangeThreads / 32, parts);
+  if (last_block_arrives(st)) {
+    __shared__ double tot[3];
+    reduce_partials<kRangeThreads>(parts, gridDim.x, tot);
+    if (threadIdx.x == 0) {
       st->lambda_used = lam;
-      st->lam2 = t0;
-      st->e1 = sqrt(t1);
-      st->e2 = sqrt(t2);
+      st->lam2 = tot[0];
+      st->e1 = sqrt(tot[1]);
+      st->e2 = sqrt(tot[2]);
       st->iter += 1;
       if (st->e1 <= eps || st->e2 <= eps) st->done = 1;
       st->counter = 0;
@@ -618,73 +514,18 @@ __global__ __launch_bounds__(kEcChunkThreads, 1) void ec_chunk_kernel(
   }
 }
 
-// Columns ascending within every row and inside [0, n) (the chunked form
-// needs both: its gathers index the staged chunk): info[0] = 1 if some row
-// breaks either; and the gathers' locality: info[1] = the
-// entries whose iterate pair lies in another 32-byte sector than the row's
-// previous entry's (about every entry for a graph without column locality).
-// Warp per row.
-__global__ void ec_sorted_kernel(int n, const int32_t* __restrict__ rp,
-                                 const int32_t* __restrict__ ci, long long nnz_used,
-                                 unsigned long long* info) {
-  const int lane = threadIdx.x & 31;
-  const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long fresh = 0;
-  bool bad = false;
-  for (long long row = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); row < n;
-       row += nw) {
-    long long b = rp[row], e = rp[row + 1];
-    if (e > nnz_used) e = nnz_used;
-    for (long long k = b + lane; k < e; k += 32) {
-      const int cur = ci[k];
-      const int prev = k > b ? ci[k - 1] : -8;
-      bad |= (k > b && cur <= prev) || cur < 0 || cur >= n;
-      fresh += (cur >> 2) != (prev >> 2);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) fresh += __shfl_xor_sync(0xffffffffu, fresh, o);
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) {
-    if (bad) atomicOr(info, 1ull);
-    if (fresh) atomicAdd(info + 1, fresh);
-  }
-}
+// Blocks (and ranges) of launch_ec_range.
+int ec_range_grid(int sms) { return sms * (4 * kEcThreads / kRangeThreads); }
 
-// Chunk boundaries of every row: csplit[(c - 1) * n + row] = the first entry
-// of the row with a column >= c * kEcChunkCols (binary search), c = 1..nch-1;
-// and the block ranges: rowsplit[b] = the first row r with rp[r] + w r >=
-// b (nnz_used + w n) / G.
-__global__ void ec_split_kernel(int n, const int32_t* __restrict__ rp,
-                                const int32_t* __restrict__ ci, long long nnz_used, int nch,
-                                int* csplit, int G, int* rowsplit) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) {
-    const int row = (int)t;
-    long long b = rp[row], e = rp[row + 1];
-    if (e > nnz_used) e = nnz_used;
-    if (b > e) b = e;
-    for (int c = 1; c < nch; ++c) {
-      const int col = c * kEcChunkCols;
-      long long lo = b, hi = e;
-      while (lo < hi) {
-        const long long mid = (lo + hi) >> 1;
-        if (ci[mid] < col) lo = mid + 1; else hi = mid;
-      }
-      csplit[(size_t)(c - 1) * n + row] = (int)lo;
-    }
-  }
-  if (t <= G) {
-    const double total = (double)nnz_used + (double)kEcRowWeight * n;
-    const double want = total * (double)t / (double)G;
-    int lo = 0, hi = n;
-    while (lo < hi) {  // first r with min(rp[r], nnz_used) + w r >= want
-      const int mid = (lo + hi) >> 1;
-      const double f = (double)min((long long)rp[mid], nnz_used) + (double)kEcRowWeight * mid;
-      if (f < want) lo = mid + 1; else hi = mid;
-    }
-    rowsplit[t] = t == G ? n : lo;
-  }
+cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const float* val,
+                            const double* vald, long long nnz_used, const double* u,
+                            const float2* uf, double* un, float2* unf, double* parts, void* st,
+                            int sms, int max_iter, double eps, const int* split, float2* part,
+                            cudaStream_t stream) {
+  auto fn = val ? ec_range_kernel<1> : vald ? ec_range_kernel<2> : ec_range_kernel<0>;
+  fn<<<ec_range_grid(sms), kRangeThreads, 0, stream>>>(n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts,
+                                      (EcState*)st, max_iter, eps, split, part);
+  return cudaGetLastError();
 }
 
 // ---- persistent form ----------------------------------------------------------
@@ -880,97 +721,21 @@ cudaError_t launch_ec_coop(int n, const int32_t* rp, const int32_t* ci, const fl
 
 size_t ec_state_bytes() { return sizeof(EcState); }
 
-int ec_chunk_count(int n) { return (n + kEcChunkCols - 1) / kEcChunkCols; }
-
-// The chunked form's preparation: rows sorted and gather locality (info, read
-// by the caller), chunk splits and block ranges.  csplit: (nch - 1) x n ints; rowsplit:
-// grid + 1 ints.
-cudaError_t launch_ec_chunk_prep(int n, const int32_t* rp, const int32_t* ci, long long nnz_used,
-                                 unsigned long long* info, int* csplit, int grid, int* rowsplit,
-                                 cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(info, 0, 2 * sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
-  const int blocks = (n + 7) / 8 < 4096 ? (n + 7) / 8 : 4096;
-  ec_sorted_kernel<<<blocks > 0 ? blocks : 1, 256, 0, stream>>>(n, rp, ci, nnz_used, info);
-  const long long cnt = (long long)n > grid + 1 ? n : grid + 1;
-  ec_split_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(
-      n, rp, ci, nnz_used, ec_chunk_count(n), csplit, grid, rowsplit);
-  return cudaGetLastError();
-}
-
-// Shared-memory limit of the chunked kernels (set outside any capture).
-cudaError_t prepare_ec_chunk() {
-  const int smem = (kEcChunkCols + kEcChunkRowsSmem) * (int)sizeof(float2);
-  cudaError_t e = cudaFuncSetAttribute(ec_chunk_kernel<0>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ec_chunk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ec_chunk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-  return e;
-}
-
-cudaError_t launch_ec_chunk(int n, const int32_t* rp, const int32_t* ci, const float* val,
-                            const double* vald, long long nnz_used, const double* u,
-                            const float2* uf, double* un, float2* unf, double* parts, void* st,
-                            int grid, int max_iter, double eps, const int* rowsplit,
-                            const int* csplit, float2* part, cudaStream_t stream) {
-  const int nch = ec_chunk_count(n);
-  const size_t smem = (size_t)(kEcChunkCols + kEcChunkRowsSmem) * sizeof(float2);
-  if (val)
-    ec_chunk_kernel<1><<<grid, kEcChunkThreads, smem, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps,
-        rowsplit, csplit, nch, part);
-  else if (vald)
-    ec_chunk_kernel<2><<<grid, kEcChunkThreads, smem, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps,
-        rowsplit, csplit, nch, part);
-  else
-    ec_chunk_kernel<0><<<grid, kEcChunkThreads, smem, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps,
-        rowsplit, csplit, nch, part);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_ec_init(int n, double* u, float2* uf, double* parts, void* st, int grid,
                            int max_iter, cudaStream_t stream) {
   ec_init_kernel<<<grid, kEcThreads, 0, stream>>>(n, u, uf, parts, (EcState*)st, max_iter);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ec_iter(int n, const int32_t* rp, const int32_t* ci, const float* val,
-                           const double* vald, long long nnz_used, const double* u,
-                           const float2* uf, double* un, float2* unf, double* parts, void* st,
-                           int grid, int max_iter, double eps, cudaStream_t stream) {
-  if (val)
-    ec_iter_kernel<1><<<grid, kEcThreads, 0, stream>>>(n, rp, ci, val, vald, nnz_used, u, uf, un,
-                                                       unf, parts, (EcState*)st, max_iter, eps);
-  else if (vald)
-    ec_iter_kernel<2><<<grid, kEcThreads, 0, stream>>>(n, rp, ci, val, vald, nnz_used, u, uf, un,
-                                                       unf, parts, (EcState*)st, max_iter, eps);
-  else
-    ec_iter_kernel<0><<<grid, kEcThreads, 0, stream>>>(n, rp, ci, val, vald, nnz_used, u, uf, un,
-                                                       unf, parts, (EcState*)st, max_iter, eps);
-  return cudaGetLastError();
-}
-
-// launch_ec_iter for a graph of average degree <= 2 (rows by thread).
-cudaError_t launch_ec_iter_sparse(int n, const int32_t* rp, const int32_t* ci, const float* val,
+// One iteration of a graph of average degree <= 2 (rows by thread).
+cudaError_t launch_ec_sparse(int n, const int32_t* rp, const int32_t* ci, const float* val,
                                   const double* vald, long long nnz_used, const double* u,
                                   const float2* uf, double* un, float2* unf, double* parts,
                                   void* st, int grid, int max_iter, double eps,
                                   cudaStream_t stream) {
-  if (val)
-    ec_iter_kernel<1, true><<<grid, kEcThreads, 0, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps);
-  else if (vald)
-    ec_iter_kernel<2, true><<<grid, kEcThreads, 0, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps);
-  else
-    ec_iter_kernel<0, true><<<grid, kEcThreads, 0, stream>>>(
-        n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts, (EcState*)st, max_iter, eps);
+  auto fn = val ? ec_sparse_kernel<1> : vald ? ec_sparse_kernel<2> : ec_sparse_kernel<0>;
+  fn<<<grid, kEcThreads, 0, stream>>>(n, rp, ci, val, vald, nnz_used, u, uf, un, unf, parts,
+                                      (EcState*)st, max_iter, eps);
   return cudaGetLastError();
 }
 

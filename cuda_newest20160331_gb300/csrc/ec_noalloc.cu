@@ -33,15 +33,20 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "ec_df.cuh"
 
 namespace bna {
 size_t ec_state_bytes();
 cudaError_t launch_ec_init(int n, double* u, float2* uf, double* parts, void* st, int grid,
                            int max_iter, cudaStream_t stream);
-cudaError_t launch_ec_iter(int n, const int32_t* rp, const int32_t* ci, const float* val,
-                           const double* vald, long long nnz_used, const double* u,
-                           const float2* uf, double* un, float2* unf, double* parts, void* st,
-                           int grid, int max_iter, double eps, cudaStream_t stream);
+int ec_range_grid(int sms);
+cudaError_t launch_flow_split(int n, const int32_t* rp, long long nnz_used, int W, int weight,
+                              int* wrow, cudaStream_t stream);
+cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const float* val,
+                            const double* vald, long long nnz_used, const double* u,
+                            const float2* uf, double* un, float2* unf, double* parts, void* st,
+                            int sms, int max_iter, double eps, const int* split, float2* part,
+                            cudaStream_t stream);
 void ec_state_read(const void* host_copy, double* lam2, double* lambda_used, double* e1,
                    double* e2, int* iter, int* done);
 int ec_state_err(const void* host_copy);
@@ -57,9 +62,10 @@ namespace {
 constexpr int kNoAllocMaxN = 1 << 18;
 constexpr int kNoAllocMaxGrid = 1024;
 constexpr size_t kStateDoubles = 16;  // >= sizeof(EcState) / 8
-// two double iterates, their two (hi, lo) float copies, block partials, state
-constexpr size_t kScratchDoubles =
-    4 * (size_t)kNoAllocMaxN + 3 * (size_t)kNoAllocMaxGrid + kStateDoubles;
+// two double iterates, their two (hi, lo) float copies, block partials, state,
+// row sums, row ranges
+constexpr size_t kScratchDoubles = 5 * (size_t)kNoAllocMaxN + 3 * (size_t)kNoAllocMaxGrid +
+                                   kStateDoubles + kNoAllocMaxGrid / 2 + 1;
 
 // The scratch.  Host code must not take its address directly (that is a host
 // stand-in); the device address comes from cudaGetSymbolAddress below.
@@ -142,6 +148,8 @@ extern "C" int32_t bna_ec_noalloc(const bna_csr* csr_dev, int32_t max_iter, doub
   float2* uf = reinterpret_cast<float2*>(scratch + 2 * (size_t)kNoAllocMaxN);  // 2 * kNoAllocMaxN
   double* parts = scratch + 4 * (size_t)kNoAllocMaxN;                   // 3 * kNoAllocMaxGrid
   void* state = parts + 3 * (size_t)kNoAllocMaxGrid;    // kStateDoubles
+  float2* part = reinterpret_cast<float2*>(parts + 3 * (size_t)kNoAllocMaxGrid + kStateDoubles);
+  int* split = reinterpret_cast<int*>(part + kNoAllocMaxN);  // kNoAllocMaxGrid + 1
   const long long nnz_used = 2 * (csr_dev->nnz / 2);
   // The array keeps the previous call's contents: the state block (with the
   // last-block counter) must start at zero; u and the partials are fully
@@ -167,13 +175,19 @@ extern "C" int32_t bna_ec_noalloc(const bna_csr* csr_dev, int32_t max_iter, doub
     done = 1;
   }
   const int chunk = 32;
+  const int ranges = ec_range_grid(sms);
+  if (!done && max_iter > 0) {
+    if (ranges > kNoAllocMaxGrid) return BNA_INTERNAL;
+    e = launch_flow_split(n, csr_dev->row_ptr, nnz_used, ranges, kEcRangeWeight, split, st);
+    if (e != cudaSuccess) return BNA_CUDA_ERROR;
+  }
   for (int launched = 0; launched < max_iter && !done; launched += chunk) {
     for (int k = 0; k < chunk; ++k) {
       const int gi = launched + k;
       const size_t cur = (size_t)(gi & 1) * n, nxt = (size_t)((gi + 1) & 1) * n;
-      e = launch_ec_iter(n, csr_dev->row_ptr, csr_dev->col_idx, csr_dev->val, nullptr, nnz_used,
-                         u + cur, uf + cur, u + nxt, uf + nxt, parts, state, grid, max_iter, eps,
-                         st);
+      e = launch_ec_range(n, csr_dev->row_ptr, csr_dev->col_idx, csr_dev->val, nullptr, nnz_used,
+                         u + cur, uf + cur, u + nxt, uf + nxt, parts, state, sms, max_iter, eps,
+                          split, part, st);
       if (e != cudaSuccess) return BNA_CUDA_ERROR;
     }
     // pageable stack buffer: the copy is synchronous with respect to the host

@@ -63,18 +63,20 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
 
 // ---------------------------------------------------------------- centrality
 
-// The column-chunked kernel serves graphs of at most kEcChunkMax chunks whose
-// gathers fall in a sector of their own for at least kEcChunkFresh of the
-// entries (measured: a random-like 45k graph, 98 % such entries, 93 -> 73 us
-// per iteration; a block-network 40k graph, 43 %, 33 us with the
-// per-iteration kernel and 93 us chunked).
-constexpr int kEcChunkMax = 4;
-constexpr double kEcChunkFresh = 0.6;
-// ... and at least this many entries per row on average: every block stages
-// the whole iterate each iteration, which a sparse graph's few gathers do not
-// repay (graphs of a few hundred edges on 50,665 and 94,939 vertices took 33
-// and 55 us per iteration chunked, one on 168,220 vertices 33 us unchunked)
-constexpr long long kEcChunkMinDeg = 8;
+// The streamed form (ec_flow.cu) copies the graph once per call, about two
+// iterations' traffic, so it takes calls of at least kFlowMinIters allowed
+// iterations, on graphs whose rows have ascending columns, of up to
+// kFlowChunkMax chunks with at least kFlowMinDeg entries per row and chunk on
+// average (a block stages every chunk and walks every row in it: one chunk,
+// 20,000 vertices, 60 and 100 entries per row: 19.6 and 20.0 us against 19.4 and
+// 22.4 ranged; two, 45,000, 100 and 150: 37.2 and 38.5 against 31.7 and 40.8;
+// four, 90,000, 200 and 300: 99 and 104 against 85 and 113), whose gathers fall in a sector of their own for at
+// least kFlowFresh of the entries (45,000 vertices, 98 % such entries: 93 us
+// per iteration with a warp per row, 56 streamed; 120,000 in contiguous
+// networks, 43 %: 121 us ranged, 334 in streams, L1 serves the gathers).
+constexpr int kFlowMinIters = 16;
+constexpr double kFlowFresh = 0.6;
+constexpr long long kFlowMinDeg = 65;
 // Graphs of at most this many entries per row on average (those whose
 // centrality converges slowly or never) sum their rows a thread per row.
 constexpr long long kEcSparseDeg = 2;
@@ -138,37 +140,47 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
     // must end on the buffer the next one starts from
     giters = std::max(2, giters & ~1);
   }
-  // the column-chunked kernel (iterate staged in shared memory) for graphs
-  // of up to kEcChunkMax chunks whose rows have ascending columns and whose
-  // gathers have little locality (most entries in a sector of their own:
-  // clustered graphs hit L1 with the per-iteration kernel and run faster there)
-  const int nch = ec_chunk_count(n);
-  bool chunked = nch >= 1 && nch <= kEcChunkMax && nnz_used > 0 &&
-                 nnz_used >= kEcChunkMinDeg * (long long)n;
   const bool sparse = nnz_used <= kEcSparseDeg * (long long)n;
-  int* csplit = nullptr;
-  int* rowsplit = nullptr;
-  float2* part = nullptr;
-  const int cgrid_rows = ctx->sms;
-  if (chunked) {
+  EcFlow fl{};
+  bool flow = nnz_used >= kFlowMinDeg * flow_chunks(n) * (long long)n && max_iter >= kFlowMinIters &&
+              flow_chunks(n) <= kFlowChunkMax && nnz_used + flow_pad() < 0x7fffffffLL;
+  if (flow) {
     unsigned long long* info;
-    ENSURE(S_EC_SPLIT, (size_t)std::max(nch - 1, 1) * n * sizeof(int), csplit);
-    ENSURE(S_EC_PART, (size_t)n * sizeof(float2), part);
-    ENSURE(S_EC_ROWS, (size_t)(cgrid_rows + 1) * sizeof(int), rowsplit);
     ENSURE(S_EC_FLAG, 2 * sizeof(unsigned long long), info);
-    CK(launch_ec_chunk_prep(n, rp, ci, nnz_used, info, csplit, cgrid_rows, rowsplit, st));
+    CK(launch_ec_sorted(n, rp, ci, nnz_used, info, st));
     CK(cudaMemcpyAsync(ctx->pinned, info, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                        st));
     CK(cudaStreamSynchronize(st));
     const unsigned long long* h = static_cast<const unsigned long long*>(ctx->pinned);
-    chunked = h[0] == 0 && (double)h[1] >= kEcChunkFresh * (double)nnz_used;
-    if (chunked) CK(prepare_ec_chunk());
+    flow = h[0] == 0 && (double)h[1] >= kFlowFresh * (double)nnz_used;
+    if (flow) {
+      fl.vk = vald ? 2 : val ? 1 : 0;
+      fl.nch = flow_chunks(n);
+      fl.W = ctx->sms * flow_warps_per_block();
+      const size_t ne = (size_t)nnz_used + flow_pad();
+      ENSURE(S_EC_SPLIT, (size_t)std::max(fl.nch - 1, 1) * n * sizeof(int), fl.csplit);
+      ENSURE(S_EC_PART, (size_t)n * sizeof(float2), fl.part);
+      ENSURE(S_EC_ROWS, (size_t)(fl.W + 1) * sizeof(int), fl.wrow);
+      ENSURE(S_EC_C16, ne * sizeof(uint16_t), fl.c16);
+      ENSURE(S_EC_VAL, ne * 4 * (size_t)fl.vk, fl.val);
+      ENSURE(S_EC_REND, (size_t)fl.nch * n * sizeof(int), fl.rend);
+      ENSURE(S_EC_WST, (size_t)fl.nch * fl.W * sizeof(int), fl.wst);
+      CK(launch_flow_layout(n, rp, ci, val, vald, nnz_used, fl, ctx->sms, st));
+    }
+  }
+  const int rgrid = ec_range_grid(ctx->sms);
+  const int form = flow ? 2 : sparse ? 1 : 0;
+  if (form == 0) {  // equal shares of the entries for the blocks
+    ENSURE(S_EC_ROWS, (size_t)(rgrid + 1) * sizeof(int), fl.wrow);
+    ENSURE(S_EC_PART, (size_t)n * sizeof(float2), fl.part);
+    CK(launch_flow_split(n, rp, nnz_used, rgrid, kEcRangeWeight, fl.wrow, st));
   }
   EcGraph& g = ctx->ecg;
-  const void* key[9] = {rp, ci, val, vald, u, state, csplit, rowsplit, part};
+  const void* key[12] = {rp,     ci,      val,    vald,    u,      state,
+                         fl.c16, fl.val,  fl.rend, fl.wst, fl.wrow, fl.part};
   bool same = g.exec && g.n == n && g.grid == grid && g.max_iter == max_iter && g.eps == eps &&
-              g.nnz_used == nnz_used && g.iters == giters && g.chunked == chunked;
-  for (int k = 0; k < 9 && same; ++k) same = (g.key[k] == key[k]);
+              g.nnz_used == nnz_used && g.iters == giters && g.form == form;
+  for (int k = 0; k < 12 && same; ++k) same = (g.key[k] == key[k]);
   if (!same) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g = EcGraph();
@@ -177,15 +189,15 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
     CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
     for (int it = 0; it < giters; ++it) {
       const size_t cur = (size_t)(it & 1) * n, nxt = (size_t)((it + 1) & 1) * n;
-      if (chunked)
-        launch_ec_chunk(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt, uf + nxt,
-                        parts, state, cgrid_rows, max_iter, eps, rowsplit, csplit, part, cap);
+      if (flow)
+        launch_ec_flow(n, rp, nnz_used, fl, u + cur, uf + cur, u + nxt, uf + nxt, parts, state,
+                       max_iter, eps, cap);
       else if (sparse)
-        launch_ec_iter_sparse(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt,
+        launch_ec_sparse(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt,
                               uf + nxt, parts, state, grid, max_iter, eps, cap);
       else
-        launch_ec_iter(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt, uf + nxt,
-                       parts, state, grid, max_iter, eps, cap);
+        launch_ec_range(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt, uf + nxt,
+                        parts, state, ctx->sms, max_iter, eps, fl.wrow, fl.part, cap);
     }
     cudaGraph_t graph;
     cudaError_t ce = cudaStreamEndCapture(cap, &graph);
@@ -194,14 +206,14 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
     ce = cudaGraphInstantiate(&g.exec, graph, 0);
     cudaGraphDestroy(graph);
     CK(ce);
-    for (int k = 0; k < 9; ++k) g.key[k] = key[k];
+    for (int k = 0; k < 12; ++k) g.key[k] = key[k];
     g.n = n;
     g.grid = grid;
     g.max_iter = max_iter;
     g.eps = eps;
     g.nnz_used = nnz_used;
     g.iters = giters;
-    g.chunked = chunked;
+    g.form = form;
   }
   double lam2 = 0, lam = 0, e1 = 0, e2 = 0;
   int it = 0, done = 0;
