@@ -89,6 +89,28 @@ int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
 
 
 
+// Workspaces of a faster form that another form can do without (the tile
+// screen, the streamed centrality): all of them, or none where memory does not
+// reach or the context is to keep to the smaller forms.
+bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want) {
+  if (ctx->lean) return false;
+  bool ok = true;
+  for (const SlotSize& w : want) {
+    void* p;
+    ok = ok && ensure(ctx, w.slot, w.bytes, &p) == BNA_OK;
+  }
+  if (ok) return true;
+  for (const SlotSize& w : want) {
+    if (ctx->ptr[w.slot]) cudaFreeAsync(ctx->ptr[w.slot], ctx->cur);
+    ctx->ptr[w.slot] = nullptr;
+    ctx->cap[w.slot] = 0;
+  }
+  ctx->sc_nb = -1;  // the screen's tile list may have been among them
+  return false;
+}
+
+void ctx_set_lean(bna_ctx* ctx, bool lean) { ctx->lean = lean; }
+
 double default_delta(int precision, int T) {
   const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23);
   switch (precision) {
@@ -136,13 +158,19 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
   ENSURE(S_VSTAT, zscore_scratch_bytes(a.n_pad), vstat);
   uint8_t* zq = nullptr;
   float* e2 = nullptr;
-  a.ldq = need_q8 ? round_up(T, 128) : 0;
-  if (need_q8) {
-    float* eblk;
-    ENSURE(S_ZQ, (size_t)a.n_pad * a.ldq, zq);
-    ENSURE(S_E2, (size_t)a.n_pad * sizeof(float), e2);
-    ENSURE(S_EBLK, (size_t)a.nb * sizeof(float), eblk);
-    a.eblk = eblk;
+  a.ldq = round_up(T, 128);
+  const size_t nsup = (size_t)sc_tile_count(a.nb);
+  if (need_q8 &&
+      ensure_optional(ctx, {{S_ZQ, (size_t)a.n_pad * a.ldq},
+                            {S_E2, (size_t)a.n_pad * sizeof(float)},
+                            {S_EBLK, (size_t)a.nb * sizeof(float)},
+                            {S_SC_TILES, nsup * sizeof(int2)},
+                            {S_SC_KEEP, (nsup + 15) / 16 * 16},
+                            {S_SC_OUT, (size_t)tc_tile_count(a.nb) * sizeof(int2)},
+                            {S_SC_COUNT, sizeof(unsigned int)}})) {
+    zq = static_cast<uint8_t*>(ctx->ptr[S_ZQ]);
+    e2 = static_cast<float*>(ctx->ptr[S_E2]);
+    a.eblk = static_cast<float*>(ctx->ptr[S_EBLK]);
   }
   CK(launch_zscore(bold, N, T, a.n_pad, z, a.ldz, zhi, zlo, a.ldb, bad, vstat, st, zq, a.ldq,
                    e2));
@@ -252,14 +280,11 @@ void window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, in
 static int32_t screened_pass(bna_ctx* ctx, const CorrArgs& a, int precision, float limit,
                              unsigned int* sched, cudaStream_t st) {
   const long long nsup = sc_tile_count(a.nb);
-  int2 *sup, *out;
-  uint8_t* keep;
-  unsigned int* n_out;
+  int2* sup = static_cast<int2*>(ctx->ptr[S_SC_TILES]);  // all by run_zscore
+  int2* out = static_cast<int2*>(ctx->ptr[S_SC_OUT]);
+  uint8_t* keep = static_cast<uint8_t*>(ctx->ptr[S_SC_KEEP]);
+  unsigned int* n_out = static_cast<unsigned int*>(ctx->ptr[S_SC_COUNT]);
   const size_t nkeep = ((size_t)nsup + 15) / 16 * 16;
-  ENSURE(S_SC_TILES, (size_t)nsup * sizeof(int2), sup);
-  ENSURE(S_SC_KEEP, nkeep, keep);
-  ENSURE(S_SC_OUT, (size_t)tc_tile_count(a.nb) * sizeof(int2), out);
-  ENSURE(S_SC_COUNT, sizeof(unsigned int), n_out);
   if (ctx->sc_nb != a.nb || ctx->sc_band != ctx->band_now) {
     CK(launch_screen_list(a.nb, ctx->band_now, sup, st));
     ctx->klaunch += 1;
@@ -400,6 +425,12 @@ int64_t bna_density_nnz(int32_t N, double percent) {
 
 int64_t bna_request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t cap,
                           int32_t with_ec) {
+  return request_bytes(N, T, opts, cap, with_ec != 0, false);
+}
+
+// lean: without the workspaces of ensure_optional.
+int64_t bna::request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t cap,
+                           bool with_ec, bool lean) {
   if (N < 1 || T < 1 || !opts || cap < 0) return -1;
   // the arena slots bna_corr_csr / bna_ec size (run_zscore, the count pass
   // buffers, the CSR), plus the request's own BOLD and centrality buffers
@@ -420,16 +451,14 @@ int64_t bna_request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64
   if (opts->precision == BNA_PREC_BF16X3 || opts->precision == BNA_PREC_AUTO)
     b += n_pad * ldb * 4;  // z hi / lo
   b += nb * n_pad * 4 + 2 * n_pad * 8 + 4096 * 8;              // seg, row lengths, block sums
-  if (T >= kScreenMinT && opts->precision != BNA_PREC_FP32)    // tile screen
+  if (!lean && T >= kScreenMinT && opts->precision != BNA_PREC_FP32)    // tile screen
     b += n_pad * round_up(T, 128) + n_pad * 4 + ntiles * 13;
   b += nst * 64 + nst * 4 + ntiles * 8 + nb;                   // etab, dense list, tiles, flags
   b += elist * 8;                                              // edge lists
   b += cand * 8 + 2 * cand * 13 + (density ? cand * 4 : 0);    // candidates, hash, values
   b += (long long)(N + 1) * 4 + nnz * (opts->weighted ? 8 : 4);  // CSR
-  if (with_ec) {  // iterates, output, partials; the streamed form's copy and row ends
-    b += (long long)N * (2 * 16 + 8) + 64 * 1024;
-    if (flow_chunks(N) <= kFlowChunkMax) b += nnz * 6 + (long long)N * (kFlowChunkMax * 8 + 8);
-  }
+  if (with_ec) b += (long long)N * (2 * 16 + 8) + 64 * 1024;     // iterates, output, partials
+  if (with_ec && !lean) b += ec_optional_bytes(N, nnz);          // the streamed form
   return b;
 }
 

@@ -17,6 +17,7 @@
 #include <string>
 #include <map>
 #include <mutex>
+#include <initializer_list>
 #include <vector>
 
 #include "common.cuh"
@@ -245,6 +246,7 @@ struct bna_ctx {
   int tiles_band = 0; // and its band height (row blocks listed column by column together)
   int band = kDefaultBand;  // BNA_OPT_TILE_BAND
   int band_now = kDefaultBand;  // the band of the current call (the autotuner's for AUTO)
+  bool lean = false;  // leave out the workspaces that only save time (ensure_optional)
   int sc_nb = -1;     // the screen's tile list: block count and band it was built for
   int sc_band = 0;
   int ntiles = 0;
@@ -300,6 +302,15 @@ namespace bna {
 int32_t fail(bna_ctx* c, int32_t st, const char* fmt, ...);
 cudaMemPool_t lib_pool(int device);
 int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out);
+struct SlotSize {
+  Slot slot;
+  size_t bytes;
+};
+bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want);
+void ctx_set_lean(bna_ctx* ctx, bool lean);
+int64_t ec_optional_bytes(int n, long long nnz);
+int64_t request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t cap, bool with_ec,
+                      bool lean);
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 double default_delta(int precision, int T);
 unsigned long long next_pow2(unsigned long long x);

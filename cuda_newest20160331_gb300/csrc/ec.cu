@@ -690,7 +690,6 @@ __global__ __launch_bounds__(kEcThreads, 4) void ec_coop_kernel(
 // stop test runs 10,000 of them) occupies a small share of the GPU.  Larger
 // graphs use per-iteration launches: their gathers then hit in L1, which the
 // persistent kernel must bypass.  Returns 0 for "use per-iteration launches".
-constexpr int kEcCoopMaxN = 16384;
 int ec_coop_grid(int n, int sms) {
   if (n > kEcCoopMaxN) return 0;
   int per_sm = 0;

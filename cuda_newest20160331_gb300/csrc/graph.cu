@@ -81,6 +81,17 @@ constexpr long long kFlowMinDeg = 65;
 // centrality converges slowly or never) sum their rows a thread per row.
 constexpr long long kEcSparseDeg = 2;
 
+// Whether a graph of this size may take the streamed form, and its workspace.
+static bool flow_sized(int n, long long nnz_used) {
+  return n > kEcCoopMaxN && flow_chunks(n) <= kFlowChunkMax &&
+         nnz_used >= kFlowMinDeg * flow_chunks(n) * (long long)n &&
+         nnz_used + flow_pad() < 0x7fffffffLL;
+}
+
+int64_t bna::ec_optional_bytes(int n, long long nnz) {
+  return flow_sized(n, nnz) ? nnz * 6 + (long long)n * (kFlowChunkMax * 8 + 8) : 0;
+}
+
 static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci, const float* val,
                       const double* vald, long long nnz, int max_iter, double eps, double* ec_dev,
                       double* lambda, int32_t* iters, cudaStream_t st) {
@@ -142,8 +153,7 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
   }
   const bool sparse = nnz_used <= kEcSparseDeg * (long long)n;
   EcFlow fl{};
-  bool flow = nnz_used >= kFlowMinDeg * flow_chunks(n) * (long long)n && max_iter >= kFlowMinIters &&
-              flow_chunks(n) <= kFlowChunkMax && nnz_used + flow_pad() < 0x7fffffffLL;
+  bool flow = max_iter >= kFlowMinIters && flow_sized(n, nnz_used) && !ctx->lean;
   if (flow) {
     unsigned long long* info;
     ENSURE(S_EC_FLAG, 2 * sizeof(unsigned long long), info);
@@ -153,18 +163,23 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
     CK(cudaStreamSynchronize(st));
     const unsigned long long* h = static_cast<const unsigned long long*>(ctx->pinned);
     flow = h[0] == 0 && (double)h[1] >= kFlowFresh * (double)nnz_used;
+    fl.vk = vald ? 2 : val ? 1 : 0;
+    fl.nch = flow_chunks(n);
+    fl.W = ctx->sms * flow_warps_per_block();
+    const size_t ne = (size_t)nnz_used + flow_pad();
+    flow = flow && ensure_optional(ctx, {{S_EC_VAL, ne * 4 * (size_t)fl.vk},
+                                         {S_EC_C16, ne * sizeof(uint16_t)},
+                                         {S_EC_SPLIT, (size_t)std::max(fl.nch - 1, 1) * n * 4},
+                                         {S_EC_REND, (size_t)fl.nch * n * sizeof(int)},
+                                         {S_EC_WST, (size_t)fl.nch * fl.W * sizeof(int)}});
     if (flow) {
-      fl.vk = vald ? 2 : val ? 1 : 0;
-      fl.nch = flow_chunks(n);
-      fl.W = ctx->sms * flow_warps_per_block();
-      const size_t ne = (size_t)nnz_used + flow_pad();
-      ENSURE(S_EC_SPLIT, (size_t)std::max(fl.nch - 1, 1) * n * sizeof(int), fl.csplit);
       ENSURE(S_EC_PART, (size_t)n * sizeof(float2), fl.part);
       ENSURE(S_EC_ROWS, (size_t)(fl.W + 1) * sizeof(int), fl.wrow);
-      ENSURE(S_EC_C16, ne * sizeof(uint16_t), fl.c16);
-      ENSURE(S_EC_VAL, ne * 4 * (size_t)fl.vk, fl.val);
-      ENSURE(S_EC_REND, (size_t)fl.nch * n * sizeof(int), fl.rend);
-      ENSURE(S_EC_WST, (size_t)fl.nch * fl.W * sizeof(int), fl.wst);
+      fl.csplit = static_cast<int*>(ctx->ptr[S_EC_SPLIT]);
+      fl.c16 = static_cast<uint16_t*>(ctx->ptr[S_EC_C16]);
+      fl.val = ctx->ptr[S_EC_VAL];
+      fl.rend = static_cast<int*>(ctx->ptr[S_EC_REND]);
+      fl.wst = static_cast<int*>(ctx->ptr[S_EC_WST]);
       CK(launch_flow_layout(n, rp, ci, val, vald, nnz_used, fl, ctx->sms, st));
     }
   }

@@ -49,6 +49,9 @@ cudaMemPool_t lib_pool(int device);
 cudaError_t copy_from_host(const void* src, void* dst, size_t bytes, int sms, cudaStream_t stream,
                            unsigned long long* blocks, int* grid_out);
 int upload_max_blocks();
+void ctx_set_lean(bna_ctx* ctx, bool lean);
+int64_t request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t cap, bool with_ec,
+                      bool lean);
 }
 int32_t bna_ctx_trim_idle(bna_ctx* ctx);
 
@@ -61,6 +64,7 @@ struct Job {
   bna_request req{};
   bna_reply reply{};
   int64_t est = 0;
+  bool lean = false;  // the budget holds only the forms without optional workspaces
   double work = 0;  // N^2 T: selects the stream priority
   bool done = false;
 };
@@ -315,6 +319,7 @@ void run_job(bna_server* srv, Slot* s, Job* j) {
     // only the empty graph)
     bna_ctx_set_option(s->ctx, BNA_OPT_MAX_NNZ, r.cap > 0 ? r.cap : 1);
     bna_ctx_set_option(s->ctx, BNA_OPT_TILES_PER_LAUNCH, tiles_per_launch(r.T));
+    bna::ctx_set_lean(s->ctx, j->lean);
     const int64_t arena0 = bna_ctx_arena_bytes(s->ctx);
     rc = bna_corr_csr(s->ctx, s->bold, r.N, r.T, &r.opts, &csr, &out.stats, st);
     out.t_corr = srv->now();
@@ -527,13 +532,18 @@ int32_t bna_server_submit(bna_server* srv, const bna_request* req, int64_t* tick
   if (!srv || !req || !ticket || !req->bold_host || req->N < 2 || req->T < 1 || req->cap < 0 ||
       (req->row_ptr_host && req->cap > 0 && !req->col_idx_host))
     return BNA_BAD_ARG;
-  const int64_t est = bna_request_bytes(req->N, req->T, &req->opts, req->cap,
-                                        req->ec_max_iter > 0 ? 1 : 0);
+  int64_t est = bna_request_bytes(req->N, req->T, &req->opts, req->cap,
+                                  req->ec_max_iter > 0 ? 1 : 0);
+  // beyond the budget with the workspaces that only save time: without them
+  const bool lean = est > srv->budget;
+  if (lean)
+    est = bna::request_bytes(req->N, req->T, &req->opts, req->cap, req->ec_max_iter > 0, true);
   if (est < 0) return BNA_BAD_ARG;
   if (est > srv->budget) return BNA_OVER_BUDGET;
   Job* j = new Job();
   j->req = *req;
   j->est = est;
+  j->lean = lean;
   j->work = (double)req->N * req->N * req->T;
   std::lock_guard<std::mutex> lk(srv->mu);
   if (srv->stop) {

@@ -59,3 +59,23 @@ def test_screened_graph_matches_oracle(kind, precision, mode, value):
     for g in (res.numpy(), cut.numpy()):
         assert np.array_equal(g.row_ptr, R) and np.array_equal(g.col_idx, C)
         assert len(V) == 0 or np.max(np.abs(g.val - V)) <= delta
+
+
+def test_budget_without_room_for_optional_workspaces():
+    """A server whose budget holds a request only without the tile screen's and
+    the streamed centrality's workspaces still takes it: the same graph, the
+    same centrality within the two forms' rounding (float-float row sums of
+    2^-38)."""
+    n, t = 17000, 520
+    x = bna.synth_bold(n, t, 12, 5)
+    need = bna.request_bytes(n, t, mode="density", value=1.0,
+                             cap=bna.density_nnz(n, 1.0))
+    got = []
+    for budget in (2 * need, need - 1):
+        with bna.Server(0, slots=1, hbm_budget=budget) as s:
+            got.append(s.wait(s.submit(x, mode="density", value=1.0, precision="bf16x3")))
+    a, b = got
+    assert a.status == b.status == 0 and a.nnz == b.nnz >= 65 * n
+    assert np.array_equal(a.row_ptr, b.row_ptr) and np.array_equal(a.col_idx, b.col_idx)
+    assert np.array_equal(a.val, b.val) and a.ec_iters == b.ec_iters
+    assert np.max(np.abs(a.ec - b.ec)) <= 1e-9 * np.max(np.abs(a.ec))
