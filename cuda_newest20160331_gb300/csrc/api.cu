@@ -120,14 +120,6 @@ double default_delta(int precision, int T) {
   }
 }
 
-unsigned long long next_pow2(unsigned long long x) {
-  unsigned long long p = 1;
-  while (p < x) p <<= 1;
-  return p;
-}
-
-
-
 // Every entry point starts here: device current, and the call's stream
 // recorded for stream-ordered arena growth.
 int32_t set_device(bna_ctx* ctx, cudaStream_t st) {
@@ -455,7 +447,7 @@ int64_t bna::request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int6
     b += n_pad * round_up(T, 128) + n_pad * 4 + ntiles * 13;
   b += nst * 64 + nst * 4 + ntiles * 8 + nb;                   // etab, dense list, tiles, flags
   b += elist * 8;                                              // edge lists
-  b += cand * 8 + 2 * cand * 13 + (density ? cand * 4 : 0);    // candidates, hash, values
+  b += cand * 16 + (density ? cand * 4 : 0);                   // candidates, values
   b += (long long)(N + 1) * 4 + nnz * (opts->weighted ? 8 : 4);  // CSR
   if (with_ec) b += (long long)N * (2 * 16 + 8) + 64 * 1024;     // iterates, output, partials
   if (with_ec && !lean) b += ec_optional_bytes(N, nnz);          // the streamed form
@@ -724,31 +716,24 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
       const long long min_pool = (long long)ctx->sms * 8 * 2 * a.echunk;
       if (ctx->elist_cap < min_pool) ctx->elist_cap = min_pool;
       a.ecap = ctx->elist_cap;
-      const unsigned long long hcap = next_pow2((unsigned long long)a.cand_cap * 2);
-      a.hmask = hcap - 1;
       ENSURE(S_CAND, (size_t)a.cand_cap * sizeof(uint2), a.cand);
-      ENSURE(S_HKEYS, hcap * 8, a.hkeys);
-      ENSURE(S_HVAL, hcap * 4, a.hval);
-      ENSURE(S_HEDGE, hcap, a.hedge);
+      ENSURE(S_CANDPOS, (size_t)a.cand_cap * sizeof(long long), a.cand_pos);
       ENSURE(S_ELIST, (size_t)a.ecap * sizeof(uint2), a.elist);
       if ((density && k_dens > 0) || ctx->avg)
         ENSURE(S_CANDVAL, (size_t)a.cand_cap * sizeof(float), cvals);
       a.cand_apx = nullptr;
       if (dev_sel) ENSURE(S_CANDAPX, (size_t)a.cand_cap * sizeof(float), a.cand_apx);
       CK(cudaMemsetAsync(ds, 0, sizeof(DevStatus), st));
-      CK(cudaMemsetAsync(a.hkeys, 0xff, hcap * 8, st));
       const int nwarps = ctx->sms * 8;  // epilogue warps of the tensor-core pass
-      ENSURE(S_WSTATE, (size_t)nwarps * 4 * sizeof(long long), a.wstate);
-      CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 4 * sizeof(long long), st));
+      ENSURE(S_WSTATE, (size_t)nwarps * 2 * sizeof(long long), a.wstate);
+      CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 2 * sizeof(long long), st));
       a.th = count_th;
       s = corr_pass(ctx, a, prec, 0, st);
       if (s) return s;
-      if (tc) CK(launch_seal_candidates(a, nwarps, st));
-      ctx->klaunch += 1;  // seal or collect
       ++passes;
       CK(cudaEventRecord(ctx->ev[2], st));
-      // the tensor-core count pass lists its candidates itself
-      if (!tc) CK(launch_collect_candidates(a, ctx->sms, st));
+      CK(launch_collect_candidates(a, ctx->sms, st));
+      ctx->klaunch += 1;
       if (dev_sel) {
         void* dstate;
         unsigned int* dhist;
@@ -799,7 +784,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
       CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       bool again = false;
-      if ((hs->err & (ERR_BAND_OVERFLOW | ERR_HASH_FULL)) && attempt < 3) {
+      if ((hs->err & ERR_BAND_OVERFLOW) && attempt < 3) {
         ctx->cand_cap = (long long)(hs->cand_count * 3 / 2) + 1024;
         again = true;
       }
@@ -814,7 +799,6 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
       return fail(ctx, BNA_INTERNAL, "candidate list overflow (%llu candidates)", hs->cand_count);
     if (hs->err & ERR_ELIST)
       return fail(ctx, BNA_INTERNAL, "edge-list pool overflow (%llu entries)", hs->epool);
-    if (hs->err & ERR_HASH_FULL) return fail(ctx, BNA_INTERNAL, "candidate hash full");
     if (dev_sel) {
       float tau_d = 0;
       long long n_exact = 0, n_ties = 0;
@@ -846,23 +830,13 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     // larger pair is an edge; of the pairs equal to tau*, the first ones in
     // row-major (i < j) order are kept up to k edges.  Every pair that can be
     // tau* or a tie is a candidate with its exact value here.
-    // candidate slots (the tensor-core pass leaves unused slots marked kCandNone)
-    const long long slots = std::min<long long>((long long)hs->cand_count, a.cand_cap);
+    const long long n = std::min<long long>((long long)hs->cand_count, a.cand_cap);
     const long long definite = (long long)hs->stats[2];
-    std::vector<float> v(slots);
-    std::vector<uint2> keys(slots);
-    CK(cudaMemcpyAsync(v.data(), cvals, slots * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(keys.data(), a.cand, slots * sizeof(uint2), cudaMemcpyDeviceToHost, st));
+    std::vector<float> v(n);
+    std::vector<uint2> keys(n);
+    CK(cudaMemcpyAsync(v.data(), cvals, n * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(keys.data(), a.cand, n * sizeof(uint2), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    long long n = 0;
-    for (long long c = 0; c < slots; ++c)
-      if (keys[c].x != kCandNone) {
-        v[n] = v[c];
-        keys[n] = keys[c];
-        ++n;
-      }
-    v.resize(n);
-    keys.resize(n);
     const long long need = k_dens - definite;
     if (need < 1 || need > n)
       return fail(ctx, BNA_INTERNAL, "density window missed the k-th value (k %lld, definite %lld, "
@@ -905,7 +879,6 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
                          cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (hs->err & ERR_HASH_FULL) return fail(ctx, BNA_INTERNAL, "candidate hash full");
     if (hs->total != 2 * k_dens)
       return fail(ctx, BNA_INTERNAL, "density: %lld entries instead of %lld", hs->total,
                   2 * k_dens);
@@ -922,7 +895,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     }
     return fail(ctx, BNA_CAPACITY, "CSR needs %lld entries, limit %lld", nnz, ctx->max_nnz);
   }
-  const unsigned long long cand_count = hs->stats[3];  // candidates (not slots)
+  const unsigned long long cand_count = hs->stats[3];
   const unsigned long long band_edges = hs->stats[0], band_1e6 = hs->stats[1];
   int32_t* col;
   ENSURE(S_COL, (size_t)std::max(nnz, 1LL) * 4, col);
@@ -979,7 +952,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   CK(cudaEventRecord(ctx->ev[5], st));
   CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if (hs->err & ERR_HASH_MISS) return fail(ctx, BNA_INTERNAL, "fill pass missed a candidate");
+  if (hs->err & ERR_UNRESOLVED) return fail(ctx, BNA_INTERNAL, "fill pass missed a candidate");
   if (hs->err & ERR_RANGE) return fail(ctx, BNA_INTERNAL, "fill pass position out of range");
   out_dev->n = N;
   out_dev->nnz = nnz;

@@ -32,7 +32,6 @@ __global__ void avg_exact_kernel(CorrArgs a, const SubjZ* __restrict__ subj, int
   for (long long c = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); c < n;
        c += nw) {
     const uint2 p = a.cand[c];
-    if (p.x == kCandNone) continue;
     float acc = 0.0f;
     for (int s = 0; s < S; ++s) {
       // post_block'd reference value: outside [-1, 1] (or NaN) it is 0, which
@@ -49,8 +48,7 @@ __global__ void avg_exact_kernel(CorrArgs a, const SubjZ* __restrict__ subj, int
 
 cudaError_t launch_avg_exact(const CorrArgs& a, const void* subj, int S, int fisher, float* out,
                              int sms, cudaStream_t st) {
-  // an odd grid: candidate slots come in 256-slot chunks filled from the front
-  avg_exact_kernel<<<sms * 8 - 1, 256, 0, st>>>(a, static_cast<const SubjZ*>(subj), S, fisher,
+  avg_exact_kernel<<<sms * 8, 256, 0, st>>>(a, static_cast<const SubjZ*>(subj), S, fisher,
                                                  out);
   return cudaGetLastError();
 }

@@ -90,12 +90,8 @@ int32_t batch_buffers(bna_ctx* ctx, BatchSubj& b, bool dev_sel, cudaStream_t st)
   const long long min_pool = (long long)ctx->sms * 8 * 2 * a.echunk;
   if (ctx->elist_cap < min_pool) ctx->elist_cap = min_pool;
   a.ecap = ctx->elist_cap;
-  const unsigned long long hcap = next_pow2((unsigned long long)a.cand_cap * 2);
-  a.hmask = hcap - 1;
   ENSURE(S_CAND, (size_t)a.cand_cap * sizeof(uint2), a.cand);
-  ENSURE(S_HKEYS, hcap * 8, a.hkeys);
-  ENSURE(S_HVAL, hcap * 4, a.hval);
-  ENSURE(S_HEDGE, hcap, a.hedge);
+  ENSURE(S_CANDPOS, (size_t)a.cand_cap * sizeof(long long), a.cand_pos);
   ENSURE(S_ELIST, (size_t)a.ecap * sizeof(uint2), a.elist);
   ENSURE(S_CANDVAL, (size_t)a.cand_cap * sizeof(float), b.cvals);
   a.cand_apx = nullptr;
@@ -109,17 +105,16 @@ int32_t batch_buffers(bna_ctx* ctx, BatchSubj& b, bool dev_sel, cudaStream_t st)
     ENSURE(S_DTIES, 2 * dens_ties_cap() * sizeof(unsigned long long), b.dties);
   }
   const int nwarps = ctx->sms * 8;
-  ENSURE(S_WSTATE, (size_t)nwarps * 4 * sizeof(long long), a.wstate);
+  ENSURE(S_WSTATE, (size_t)nwarps * 2 * sizeof(long long), a.wstate);
   CK(cudaMemsetAsync(b.ds, 0, sizeof(DevStatus), st));
-  CK(cudaMemsetAsync(a.hkeys, 0xff, hcap * 8, st));
-  CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 4 * sizeof(long long), st));
+  CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 2 * sizeof(long long), st));
   return BNA_OK;
 }
 
 // After the count pass: candidates, density selection or recompute, scan.
 int32_t batch_after(bna_ctx* ctx, BatchSubj& b, bool dev_sel, cudaStream_t st) {
   CorrArgs& a = b.a;
-  CK(launch_seal_candidates(a, ctx->sms * 8, st));
+  CK(launch_collect_candidates(a, ctx->sms, st));
   if (dev_sel) {
     CK(dens_set(b.dstate, b.k_dens, (float)b.delta, b.winA, b.winB, st));
     CK(cudaMemsetAsync(b.dhist, 0, 2048 * sizeof(unsigned int), st));
@@ -233,7 +228,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
   std::vector<char> table((size_t)nsub * tc_subj_bytes());
   for (int k = 0; k < nsub; ++k) {
     bna_ctx* kid = ctx->kids[k];
-    s = batch_buffers(kid, bs[k], dev_sel, st);  // the density count pass lists r~ for all
+    s = batch_buffers(kid, bs[k], dev_sel, st);
     if (s) return fail(ctx, s, "subject %d: %s", k, kid->last_error.c_str());
     if (!tc_subj_fill(table.data(), k, bs[k].a,
                       reinterpret_cast<const uint8_t*>(kid->ptr[S_BLOCKBAD]),
@@ -271,7 +266,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
   int launches = 0;
   // the persistent count pass over every subject's tiles, replayed from a
   // captured CUDA graph (one launch, or the chunks a launch gate asks for)
-  CK(prepare_corr_tc_multi(form, dev_sel, absm));  // its attributes: outside the capture
+  CK(prepare_corr_tc_multi(form, absm));  // its attributes: outside the capture
   struct ExecGuard {  // released once its launch is over, on every return path
     cudaGraphExec_t e = nullptr;
     cudaStream_t s = nullptr;
@@ -294,7 +289,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
     cudaError_t ce = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     for (int t0 = 0; ce == cudaSuccess && t0 < ctx->batch_ntiles; t0 += per, ++launches)
       ce = launch_corr_tc_multi(batch, table_dev, tiles4 + t0,
-                                std::min(per, ctx->batch_ntiles - t0), form, dev_sel, absm,
+                                std::min(per, ctx->batch_ntiles - t0), form, absm,
                                 ctx->sms, sched, cap);
     cudaGraph_t graph = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(cap, &graph);
@@ -322,8 +317,8 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
     bna_ctx* kid = ctx->kids[k];
     const DevStatus* hs = reinterpret_cast<const DevStatus*>(kid->pinned);
     BatchSubj& b = bs[k];
-    bool bad = (hs->err & (ERR_BAND_OVERFLOW | ERR_HASH_FULL | ERR_ELIST | ERR_TIMEOUT)) != 0;
-    if (hs->err & (ERR_BAND_OVERFLOW | ERR_HASH_FULL))
+    bool bad = (hs->err & (ERR_BAND_OVERFLOW | ERR_ELIST | ERR_TIMEOUT)) != 0;
+    if (hs->err & (ERR_BAND_OVERFLOW))
       kid->cand_cap = (long long)(hs->cand_count * 3 / 2) + 1024;
     if (hs->err & ERR_ELIST)
       kid->elist_cap = (long long)(hs->epool + hs->epool / 4) + b.a.echunk;
@@ -369,7 +364,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
     BatchSubj& b = bs[k];
     if (!b.fallback) {
       const DevStatus* hs = reinterpret_cast<const DevStatus*>(ctx->kids[k]->pinned);
-      if (hs->err & (ERR_HASH_MISS | ERR_RANGE)) b.fallback = true;
+      if (hs->err & (ERR_UNRESOLVED | ERR_RANGE)) b.fallback = true;
     }
     if (b.fallback) {
       if ((s = single(k))) return s;

@@ -15,8 +15,7 @@ constexpr int kBlk = 128;
 // Error bits raised by kernels into CorrArgs::err (host reads them once per call).
 enum : uint32_t {
   ERR_BAND_OVERFLOW = 1u,   // candidate list full
-  ERR_HASH_MISS = 2u,       // fill pass met a candidate the recompute pass never stored
-  ERR_HASH_FULL = 4u,
+  ERR_UNRESOLVED = 2u,      // fill pass met a candidate the recompute pass never resolved
   ERR_NNZ_INT32 = 8u,
   ERR_TIES = 16u,           // density: tie bookkeeping inconsistent
   ERR_TIMEOUT = 32u,        // a bounded wait in a tensor-core kernel expired
@@ -30,11 +29,6 @@ enum : uint32_t {
 // hold a warp's worst case for one tile (32 rows x 128 columns).
 constexpr long long kElistChunk = 16384;
 constexpr long long kElistChunkMin = 4096;
-// Candidate list: the tensor-core count pass writes its near-threshold pairs
-// itself, in warp-private chunks of kCandChunk slots; slots a warp leaves
-// unused hold (kCandNone, kCandNone) and are skipped by the consumers.
-constexpr long long kCandChunk = 256;
-constexpr uint32_t kCandNone = 0xFFFFFFFFu;
 
 // Density mode: histogram of the approximate r over [-1, 1) in kHistBins
 // bins (bin = floor((r + 1) * kHistBins / 2)); entry kHistBins counts the
@@ -105,6 +99,8 @@ __device__ __forceinline__ int classify(float r, const Threshold& th) {
 }
 
 // Pointers and sizes shared by the correlation passes.
+constexpr long long kEtabCand = 1LL << 32;
+
 struct CorrArgs {
   const float* z;            // voxel-major [n_pad][ldz], FP32 z-scores (exact recompute source)
   const uint16_t* zhi;       // voxel-major [n_pad][ldb] BF16 hi parts (tensor-core forms)
@@ -121,23 +117,22 @@ struct CorrArgs {
   int32_t* col_idx;          // [nnz]
   float* val;                // [nnz] or null
   long long nnz;             // fill pass: entries of col_idx / val (positions are checked)
-  // near-threshold candidates (count pass appends, recompute resolves)
+  // near-threshold candidates (flagged in the edge lists by the count pass,
+  // listed by collect_candidates_kernel, resolved in place by the recompute)
   uint2* cand;               // (i, j) with i < j
+  long long* cand_pos;       // its edge-list entry
   unsigned long long* cand_count;
   long long cand_cap;
-  // hash of resolved candidates: key (i<<32|j) -> (value, edge flag)
-  unsigned long long* hkeys;
-  float* hval;
-  uint8_t* hedge;
-  unsigned long long hmask;
   // per-tile edge lists written by the count pass, placed by the fill pass:
-  // entry = (il | jl << 7 | candidate << 14, value bits); etab[4*st + q] =
+  // entry = (il | jl << 7 | candidate << 14 | dropped << 15, value bits); etab[4*st + q] =
   // (first entry, count) of part q of 128 x 128 sub-tile st (upper-triangle index)
   uint2* elist;
   unsigned long long* epool;
   long long ecap;
   long long echunk;  // entries per warp chunk (kElistChunkMin .. kElistChunk)
-  long long* wstate; // tensor-core count pass: per epilogue warp (wcur, wend, ccur, cend)
+  long long* wstate; // tensor-core count pass: per epilogue warp (wcur, wend)
+  // (kEtabCand set by the count pass where the part may hold candidates, cleared
+  // by collect_candidates_kernel)
   longlong2* etab;
   // density ties that must not become edges (sorted keys), see FormFullGraph_s
   const unsigned long long* drop_keys;
@@ -146,7 +141,7 @@ struct CorrArgs {
   unsigned long long* stats;  // [0]=band edges [1]=band within 1e-6 [2]=definite listed edges
   unsigned int* hist;         // density histogram pass: kHistBins + 1 counters
   const float* cand_val;      // density: exact values of the candidates (decide pass)
-  float* cand_apx;            // density (tensor-core count pass): r~ of every candidate slot
+  float* cand_apx;            // density, tensor-core forms: r~ of every candidate
 };
 
 // Fill-pass store with a range check (an inconsistent count would otherwise
@@ -164,43 +159,15 @@ __device__ __forceinline__ unsigned long long pair_key(int i, int j) {
   return ((unsigned long long)(uint32_t)i << 32) | (uint32_t)j;
 }
 
-__device__ __forceinline__ unsigned long long hash64(unsigned long long k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdULL;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ULL;
-  k ^= k >> 33;
-  return k;
-}
-
-// Look up a resolved candidate.  Returns false (and flags ERR_HASH_MISS) if absent.
-__device__ __forceinline__ bool hash_lookup(const CorrArgs& a, unsigned long long key, float& v,
-                                            bool& edge) {
-  unsigned long long h = hash64(key) & a.hmask;
-  for (unsigned long long probe = 0; probe <= a.hmask; ++probe) {
-    const unsigned long long k = a.hkeys[h];
-    if (k == key) {
-      v = a.hval[h];
-      edge = a.hedge[h] != 0;
-      return true;
-    }
-    if (k == ~0ull) break;
-    h = (h + 1) & a.hmask;
-  }
-  atomicOr(a.err, ERR_HASH_MISS);
-  v = 0.f;
-  edge = false;
-  return false;
-}
-
-// Append a near-threshold candidate (count pass).
-__device__ __forceinline__ void push_candidate(const CorrArgs& a, int i, int j) {
-  const unsigned long long slot = atomicAdd(a.cand_count, 1ull);
-  if ((long long)slot < a.cand_cap) {
-    a.cand[slot] = make_uint2((unsigned)i, (unsigned)j);
-  } else {
-    atomicOr(a.err, ERR_BAND_OVERFLOW);
-  }
+// Resolve candidate c: its edge-list entry becomes the exact value, an edge or
+// dropped, for the fill pass to read in order (a hash of the resolved pairs,
+// filled here and probed by the fill pass, cost 16 MB to clear per call and a
+// chain of misses per candidate).
+__device__ __forceinline__ void resolve_candidate(const CorrArgs& a, long long c, int i, int j,
+                                                  float r, bool edge) {
+  a.elist[a.cand_pos[c]] =
+      make_uint2((uint32_t)(i & 127) | ((uint32_t)(j & 127) << 7) | (edge ? 0u : 1u << 15),
+                 __float_as_uint(r));
 }
 
 // Upper-triangular 128-block pair (I, J), I <= J -> its row-major index.

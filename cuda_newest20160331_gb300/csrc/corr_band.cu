@@ -32,127 +32,186 @@ __device__ __forceinline__ float exact_r(const CorrArgs& a, int i, int j) {
 __global__ void cand_values_kernel(CorrArgs a, float* vals) {
   const unsigned long long cnt = *a.cand_count;
   const long long n = (long long)cnt < a.cand_cap ? (long long)cnt : a.cand_cap;
-  const int lane = threadIdx.x & 31;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long c = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); c < n;
-       c += nwarps) {
-    const uint2 p = a.cand[c];
-    if (p.x == kCandNone) continue;  // unused slot of a count-pass chunk
-    const float r = exact_r_warp(a, (int)p.x, (int)p.y, lane);
-    if (lane == 0) vals[c] = r;
+  const int lane = threadIdx.x & 31, gl = lane & (kPairLanes - 1);
+  const long long step = (long long)gridDim.x * (blockDim.x / kPairLanes);
+  for (long long c0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * kPairs;
+       c0 < n; c0 += step) {
+    const long long c = c0 + lane / kPairLanes;
+    const uint2 p = c < n ? a.cand[c] : make_uint2(0u, 0u);
+    const float r = post_block(exact_r_pairs_raw(a, c < n, (int)p.x, (int)p.y, lane));
+    if (c < n && gl == 0) vals[c] = r;
   }
 }
 
 // Decide every candidate on its exact value (computed here, or given in
 // a.cand_val), add the edges to the counts and store value + decision in the
-// hash the fill pass reads.
+// edge-list entry the fill pass reads.
 __global__ void recompute_kernel(CorrArgs a) {
   const unsigned long long cnt = *a.cand_count;
   const long long n = (long long)cnt < a.cand_cap ? (long long)cnt : a.cand_cap;
-  const int lane = threadIdx.x & 31;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long n_edge = 0, n_1e6 = 0;  // lane 0's counts, added once per warp
-  for (long long c = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); c < n;
-       c += nwarps) {
-    const uint2 p = a.cand[c];
-    if (p.x == kCandNone) continue;  // unused slot of a count-pass chunk
+  const int lane = threadIdx.x & 31, gl = lane & (kPairLanes - 1);
+  const long long step = (long long)gridDim.x * (blockDim.x / kPairLanes);
+  const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
+  unsigned int n_edge = 0, n_1e6 = 0;  // this lane's counts, added once per warp
+  for (long long c0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * kPairs;
+       c0 < n; c0 += step) {
+    const long long c = c0 + lane / kPairLanes;
+    const uint2 p = c < n ? a.cand[c] : make_uint2(0u, 0u);
     const int i = (int)p.x, j = (int)p.y;
-    const float r = a.cand_val ? a.cand_val[c] : exact_r_rule(a, i, j, lane);
-    if (lane != 0) continue;
-    const unsigned long long key = pair_key(i, j);
+    float r;
+    if (a.cand_val) {
+      r = c < n ? a.cand_val[c] : 0.0f;
+    } else {
+      const float raw = exact_r_pairs_raw(a, c < n, i, j, lane);
+      r = a.th.mode == BNA_THR_R_EPS ? raw : post_block(raw);
+    }
+    if (c >= n || gl != 0) continue;
     bool e = edge_exact(r, a.th);
     if (e && a.th.mode == BNA_THR_DENSITY && r == a.th.tau && a.n_drop > 0 &&
-        in_sorted(a.drop_keys, a.n_drop, key))
+        in_sorted(a.drop_keys, a.n_drop, pair_key(i, j)))
       e = false;
     if (e) {
       atomicAdd(&a.seg[(size_t)(j / kBlk) * a.n_pad + i], 1);
       atomicAdd(&a.seg[(size_t)(i / kBlk) * a.n_pad + j], 1);
       ++n_edge;
     }
-    const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
     if (fabsf((absm ? fabsf(r) : r) - a.th.tau) <= 1e-6f) ++n_1e6;
-    unsigned long long h = hash64(key) & a.hmask;
-    bool stored = false;
-    for (unsigned long long probe = 0; probe <= a.hmask; ++probe) {
-      const unsigned long long prev = atomicCAS(&a.hkeys[h], ~0ull, key);
-      if (prev == ~0ull || prev == key) {
-        a.hval[h] = r;
-        a.hedge[h] = e ? 1 : 0;
-        stored = true;
-        break;
-      }
-      h = (h + 1) & a.hmask;
-    }
-    if (!stored) atomicOr(a.err, ERR_HASH_FULL);
+    resolve_candidate(a, c, i, j, r, e);
   }
-  if (n_edge) atomicAdd(&a.stats[0], n_edge);
-  if (n_1e6) atomicAdd(&a.stats[1], n_1e6);
+  __syncwarp();
+  n_edge = __reduce_add_sync(0xffffffffu, n_edge);
+  n_1e6 = __reduce_add_sync(0xffffffffu, n_1e6);
+  if (lane == 0) {
+    if (n_edge) atomicAdd(&a.stats[0], (unsigned long long)n_edge);
+    if (n_1e6) atomicAdd(&a.stats[1], (unsigned long long)n_1e6);
+  }
 }
 
-// Gather the candidates flagged in the sub-tiles' edge lists into the
-// candidate list (warp per sub-tile, one atomic per warp and round).  Used
-// after the plain FP32 count pass; the tensor-core pass lists its candidates
-// itself.
-__global__ void collect_candidates_kernel(CorrArgs a, long long nst) {
-  const int wpb = blockDim.x >> 5;
+// List the candidates flagged in the sub-tiles' edge lists: their pair, their
+// entry's position and (density) their approximate value; count them and the
+// definite entries.  A warp takes the parts of eight sub-tiles at a time, a lane
+// each for the ranges (sub-tiles a grid apart: the dense ones of networked data
+// lie together), and reads the lists of those that the count pass
+// marked, the next one's first 64 entries in flight; candidates wait in shared
+// memory until 32 are there, so one counter atomic and full lines serve 32.
+// Bound: load latency and issue (45,000 voxels, 9.3 M entries, 44,556
+// candidates: 50 us reading every list a sub-tile at a time, 27 now; 681,935
+// candidates: 78).
+constexpr int kCollectWarps = 8;
+
+__global__ __launch_bounds__(kCollectWarps * 32) void collect_candidates_kernel(CorrArgs a,
+                                                                                long long nst) {
+  __shared__ uint2 bpair[kCollectWarps][64];
+  __shared__ long long bpos[kCollectWarps][64];
+  __shared__ float bapx[kCollectWarps][64];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;
-  for (long long st = (long long)blockIdx.x * wpb + w; st < nst; st += (long long)gridDim.x * wpb) {
-    long long s0 = 0, c0 = 0;
-    if (lane < 4) {
-      const longlong2 e = a.etab[st * 4 + lane];
-      s0 = e.x;
-      c0 = e.y;
-    }
-    long long start[4], cnt[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      start[q] = __shfl_sync(0xffffffffu, s0, q);
-      cnt[q] = __shfl_sync(0xffffffffu, c0, q);
-    }
-    bool inside = true;  // ranges written while the pool overflowed are not read
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      inside &= cnt[q] >= 0 && start[q] >= 0 && start[q] + cnt[q] <= a.ecap;
-    if (!inside) {
-      if (lane == 0) atomicOr(a.err, ERR_ELIST);
-      continue;
-    }
-    const long long E = cnt[0] + cnt[1] + cnt[2] + cnt[3];
-    if (E == 0) continue;
-    int I, J;
-    tile_coords(st, a.nb, I, J);
-    const long long p1 = cnt[0], p2 = p1 + cnt[1], p3 = p2 + cnt[2];
-    for (long long e0 = 0; e0 < E; e0 += 32) {
-      const long long e = e0 + lane;
-      bool flag = false;
-      uint32_t key = 0;
-      if (e < E) {
-        const int q = e < p1 ? 0 : e < p2 ? 1 : e < p3 ? 2 : 3;
-        const long long off = e - (q == 0 ? 0 : q == 1 ? p1 : q == 2 ? p2 : p3);
-        const long long s = q == 0 ? start[0] : q == 1 ? start[1] : q == 2 ? start[2] : start[3];
-        key = a.elist[s + off].x;
-        flag = ((key >> 14) & 1u) != 0u;
-      }
-      const uint32_t bal = __ballot_sync(0xffffffffu, flag);
-      // definite (unflagged) entries of this round, for the density selection
-      const int nvalid = (int)((E - e0) < 32 ? (E - e0) : 32);
-      if (lane == 0 && nvalid - __popc(bal) > 0)
-        atomicAdd(&a.stats[2], (unsigned long long)(nvalid - __popc(bal)));
-      if (!bal) continue;
-      if (lane == 0) atomicAdd(&a.stats[3], (unsigned long long)__popc(bal));
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(a.cand_count, (unsigned long long)__popc(bal));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (flag) {
-        const unsigned long long slot = base + __popc(bal & below);
-        if ((long long)slot < a.cand_cap)
-          a.cand[slot] = make_uint2((unsigned)(I * 128 + (key & 127)),
-                                    (unsigned)(J * 128 + ((key >> 7) & 127)));
-        else
-          atomicOr(a.err, ERR_BAND_OVERFLOW);
+  const long long nw = (long long)gridDim.x * kCollectWarps;
+  long long n_def = 0, n_cand = 0;  // a lane's entries; the warp's candidates
+  int held = 0;
+  auto flush = [&](int m) {  // the first m <= 32 held candidates
+    unsigned long long slot = 0;
+    if (lane == 0) slot = atomicAdd(a.cand_count, (unsigned long long)m);
+    slot = __shfl_sync(0xffffffffu, slot, 0) + lane;
+    if (lane < m) {
+      if ((long long)slot < a.cand_cap) {
+        a.cand[slot] = bpair[w][lane];
+        a.cand_pos[slot] = bpos[w][lane];
+        if (a.cand_apx) a.cand_apx[slot] = bapx[w][lane];
+      } else {
+        atomicOr(a.err, ERR_BAND_OVERFLOW);
       }
     }
+    __syncwarp();
+    held -= m;
+    if (lane < held) {  // the rest moves to the front
+      bpair[w][lane] = bpair[w][m + lane];
+      bpos[w][lane] = bpos[w][m + lane];
+      bapx[w][lane] = bapx[w][m + lane];
+    }
+    __syncwarp();
+  };
+  for (long long st0 = (long long)blockIdx.x * kCollectWarps + w; st0 < nst; st0 += nw * 8) {
+    long long s = 0, c = 0;
+    bool marked = false;
+    const long long mine = st0 + nw * (lane >> 2);
+    if (mine < nst) {
+      const longlong2 r = a.etab[mine * 4 + (lane & 3)];
+      marked = (r.y & kEtabCand) != 0;
+      s = r.x;
+      c = r.y & ~kEtabCand;
+      // ranges written while the pool overflowed are not read
+      if (c < 0 || c > 128 * 128 || s < 0 || s + c > a.ecap) {
+        atomicOr(a.err, ERR_ELIST);
+        c = 0;
+        marked = false;
+      }
+      if (marked) a.etab[mine * 4 + (lane & 3)].y = c;
+    }
+    n_def += c;
+    uint32_t todo = __ballot_sync(0xffffffffu, marked);
+    uint2 nx[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};  // the next part's first entries
+    auto ahead = [&](uint32_t m) {
+      const int l = m ? __ffs(m) - 1 : 0;
+      const long long sl = __shfl_sync(0xffffffffu, s, l);
+      const int cl = m ? (int)__shfl_sync(0xffffffffu, c, l) : 0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        nx[k] = make_uint2(0u, 0u);
+        if (lane + 32 * k < cl) nx[k] = a.elist[sl + lane + 32 * k];
+      }
+    };
+    if (todo) ahead(todo);
+    while (todo) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const long long sl = __shfl_sync(0xffffffffu, s, l);
+      const int cl = (int)__shfl_sync(0xffffffffu, c, l);
+      const uint2 first[2] = {nx[0], nx[1]};
+      if (todo) ahead(todo);
+      int I, J;
+      tile_coords(st0 + nw * (l >> 2), a.nb, I, J);
+      auto take = [&](uint2 en, int e) {  // entry e of this lane
+        const bool flag = ((en.x >> 14) & 1u) != 0u;
+        const uint32_t bal = __ballot_sync(0xffffffffu, flag);
+        if (!bal) return;
+        if (flag) {
+          const int to = held + __popc(bal & below);
+          bpair[w][to] = make_uint2((unsigned)(I * 128 + (en.x & 127)),
+                                    (unsigned)(J * 128 + ((en.x >> 7) & 127)));
+          bpos[w][to] = sl + e;
+          bapx[w][to] = __uint_as_float(en.y);
+        }
+        held += __popc(bal);
+        n_cand += __popc(bal);
+        __syncwarp();
+        if (held >= 32) flush(32);
+      };
+#pragma unroll
+      for (int k = 0; k < 2; ++k) take(first[k], 32 * k + lane);
+      for (int e0 = 64; e0 < cl; e0 += 256) {  // long lists: eight rounds in flight
+        uint2 en[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int e = e0 + 32 * k + lane;
+          en[k] = make_uint2(0u, 0u);
+          if (e < cl) en[k] = a.elist[sl + e];
+        }
+#pragma unroll 1
+        for (int h = 0; h < 256 && e0 + h < cl; h += 32) {
+          take(en[0], e0 + h + lane);
+#pragma unroll
+          for (int k = 0; k < 7; ++k) en[k] = en[k + 1];
+        }
+      }
+    }
+  }
+  if (held > 0) flush(held);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n_def += __shfl_xor_sync(0xffffffffu, n_def, o);
+  if (lane == 0) {
+    if (n_def - n_cand > 0) atomicAdd(&a.stats[2], (unsigned long long)(n_def - n_cand));
+    if (n_cand) atomicAdd(&a.stats[3], (unsigned long long)n_cand);
   }
 }
 
@@ -162,28 +221,32 @@ __global__ void exact_pairs_kernel(CorrArgs a, const uint2* pairs, int n, float*
   if (c < n) out[c] = exact_r(a, (int)pairs[c].x, (int)pairs[c].y);
 }
 
-// seg[b][i] -> exclusive prefix over b; rowlen[i] = row total.  Loads are
-// issued 16 at a time so each thread keeps 16 requests in flight.
+// seg[b][i] -> exclusive prefix over b; rowlen[i] = row total.  A thread per row
+// keeps 16 loads in flight and reads the next 16 while it writes a batch.  Bound:
+// the bytes (180,000 voxels, 1.0 GB of counts: 830 us a batch at a time, 350 now;
+// 45,000, 63 MB: 46, 24 now in blocks of 64; four threads per row with their parts'
+// sums from a first reading: 53).
+constexpr int kSegBatch = 16, kSegRows = 64;
+
 __global__ void seg_scan_rows_kernel(int32_t* seg, int nb, int n_pad, int n, long long* rowlen) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_pad) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // n_pad is a multiple of blockDim.x
+  int32_t* p = seg + i;
+  auto load = [&](int (&c)[kSegBatch], int b) {
+#pragma unroll
+    for (int u = 0; u < kSegBatch; ++u) c[u] = b + u < nb ? p[(size_t)(b + u) * n_pad] : 0;
+  };
   long long acc = 0;
-  int b = 0;
-  for (; b + 16 <= nb; b += 16) {
-    int c[16];
+  int c[kSegBatch];
+  load(c, 0);
+  for (int b = 0; b < nb; b += kSegBatch) {
+    int nx[kSegBatch];
+    load(nx, b + kSegBatch);
 #pragma unroll
-    for (int u = 0; u < 16; ++u) c[u] = seg[(size_t)(b + u) * n_pad + i];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      seg[(size_t)(b + u) * n_pad + i] = (int)acc;
+    for (int u = 0; u < kSegBatch; ++u) {
+      if (b + u < nb) p[(size_t)(b + u) * n_pad] = (int)acc;
       acc += c[u];
+      c[u] = nx[u];
     }
-  }
-  for (; b < nb; ++b) {
-    int32_t* p = seg + (size_t)b * n_pad + i;
-    const int c = *p;
-    *p = (int)acc;
-    acc += c;
   }
   if (i < n) rowlen[i] = acc;
 }
@@ -281,27 +344,22 @@ __global__ void scan_finish_kernel(const long long* pre, const long long* bsum, 
   }
 }
 
-// Candidate slots come in 256-slot chunks filled from the front; a warp count
-// that is a multiple of 256 would give every warp the same offset in each
-// chunk (and the filled offsets to a few warps): the grid is made odd.
-static int odd_grid(int grid) { return grid > 1 ? (grid | 1) - 2 * ((grid & 1) == 0) : 1; }
-
 cudaError_t launch_recompute(const CorrArgs& a, int grid, cudaStream_t stream) {
-  recompute_kernel<<<odd_grid(grid), 256, 0, stream>>>(a);
+  recompute_kernel<<<grid, 256, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cand_values(const CorrArgs& a, float* vals, int grid, cudaStream_t stream) {
-  cand_values_kernel<<<odd_grid(grid), 256, 0, stream>>>(a, vals);
+  cand_values_kernel<<<grid, 256, 0, stream>>>(a, vals);
   return cudaGetLastError();
 }
 
 cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, cudaStream_t stream) {
   const long long nst = (long long)a.nb * (a.nb + 1) / 2;
-  const long long want = (nst + 7) / 8;
+  const long long want = (nst + kCollectWarps - 1) / kCollectWarps;
   const int grid = (int)(want < (long long)sms * 8 ? want : (long long)sms * 8);
   if (grid <= 0) return cudaSuccess;
-  collect_candidates_kernel<<<grid, 256, 0, stream>>>(a, nst);
+  collect_candidates_kernel<<<grid, kCollectWarps * 32, 0, stream>>>(a, nst);
   return cudaGetLastError();
 }
 
@@ -318,7 +376,7 @@ cudaError_t launch_csr_scan(int32_t* seg, int nb, int n_pad, int n, long long* r
                             uint32_t* err, cudaStream_t stream) {
   const int nblk = (n + 4095) / 4096;
   if (nblk > 4096) return cudaErrorInvalidValue;
-  seg_scan_rows_kernel<<<(n_pad + 127) / 128, 128, 0, stream>>>(seg, nb, n_pad, n, rowlen);
+  seg_scan_rows_kernel<<<n_pad / kSegRows, kSegRows, 0, stream>>>(seg, nb, n_pad, n, rowlen);
   scan_block_kernel<<<nblk, 1024, 0, stream>>>(rowlen, n, pre, bsum);
   scan_sums_kernel<<<1, 1024, 0, stream>>>(bsum, nblk, total);
   scan_finish_kernel<<<(n + 1 + 255) / 256, 256, 0, stream>>>(pre, bsum, n, total, row_ptr, err);

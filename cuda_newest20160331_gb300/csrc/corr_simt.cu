@@ -232,7 +232,8 @@ __global__ __launch_bounds__(256, 2) void corr_simt_kernel(CorrArgs a, int nt, i
     const bool fits = !run || (long long)(base + run) <= a.ecap;
     if (!fits) atomicOr(a.err, ERR_ELIST);
     const long long st = subtile_index(I, J, a.nb);
-    a.etab[st * 4 + 0] = fits ? make_longlong2((long long)base, run) : make_longlong2(0, 0);
+    a.etab[st * 4 + 0] = fits && run ? make_longlong2((long long)base, run | kEtabCand)
+                                   : make_longlong2(0, 0);
     a.etab[st * 4 + 1] = make_longlong2(0, 0);
     a.etab[st * 4 + 2] = make_longlong2(0, 0);
     a.etab[st * 4 + 3] = make_longlong2(0, 0);
@@ -249,7 +250,7 @@ __global__ __launch_bounds__(256, 2) void corr_simt_kernel(CorrArgs a, int nt, i
         const int b = i * 8 + j;
         if ((ent >> b) & 1ull) {
           const uint32_t cf = (uint32_t)((cmask >> b) & 1ull);
-          *dst++ = make_uint2(elist_key(il, jl, cf), cf ? 0u : __float_as_uint(acc[i][j]));
+          *dst++ = make_uint2(elist_key(il, jl, cf), __float_as_uint(acc[i][j]));
         }
       }
     }

@@ -169,9 +169,10 @@ __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
 }
 
 // tm_hi / tm_lo: BF16 hi and lo parts (FORM_BF16X3); tm_hi: FP32 z (FORM_TF32).
-// DENS (count pass of the density rule): candidates are listed per 32-column
-// chunk together with their approximate value (a.cand_apx), which the device
-// selection of the k-th largest value needs.
+// Candidates are only flagged in the edge lists, with their approximate value
+// (collect_candidates_kernel lists them after the pass): listing them here cost
+// the density rule's pass 8 % (45,000 x 300, 682,000 candidates: 1.32 ms against
+// 1.21).
 // MULTI: the tiles of several subjects in one persistent launch (count pass).
 // AVG: the average over subjects (W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:418-670):
 // each tile runs through the subjects in order, and a thread keeps the running
@@ -180,7 +181,7 @@ __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
 // through the same epilogue as one subject's values.  No N (N - 1) / 2 matrix
 // is held: adding each subject into one in HBM, 4 bytes per lane in 32
 // different rows, took 4.07 ms per subject at N = 20,000, T = 180-300.
-template <int PASS, bool ABS, int FORM, bool DENS, bool MULTI = false, bool AVG = false>
+template <int PASS, bool ABS, int FORM, bool MULTI = false, bool AVG = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     corr_tc_kernel(const __grid_constant__ CUtensorMap tm_hi,
                    const __grid_constant__ CUtensorMap tm_lo, const TcArgs p) {
@@ -388,12 +389,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     float zlo = 0;  // AVG: an average Fisher z below it is no edge and no candidate
     bool simple = false, zero_int = false;
     uint32_t hphase = 0;
-    // this warp's current edge-list chunk [wcur, wend) and candidate chunk
-    // [ccur, cend), carried from launch to launch of a pass in a.wstate
+    // this warp's current edge-list chunk [wcur, wend), carried from launch to
+    // launch of a pass in a.wstate
     const int wid = (int)blockIdx.x * 8 + (warp - 2);
-    long long wcur = 0, wend = 0, ccur = 0, cend = 0;
+    long long wcur = 0, wend = 0;
     bool wok = true;
-    unsigned long long n_def = 0, n_cand = 0;  // this lane's definite edges and candidates
     int cur_s = -1;
     // the fields the per-value path reads, kept in registers
     int s_n = 0, s_npad = 0, s_nb = 0;
@@ -430,30 +430,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       zero_int = a.th.mode != BNA_THR_R_EPS && ((0.0f >= lo_thr) || (0.0f >= lim));
       if (PASS == 0) {
         long long x = 0;
-        if (lane < 4) x = a.wstate[wid * 4 + lane];
+        if (lane < 2) x = a.wstate[wid * 2 + lane];
         wcur = __shfl_sync(0xffffffffu, x, 0);
         wend = __shfl_sync(0xffffffffu, x, 1);
-        ccur = __shfl_sync(0xffffffffu, x, 2);
-        cend = __shfl_sync(0xffffffffu, x, 3);
       }
       wok = wend <= a.ecap;
     };
-    // leave the current subject: its chunks stay open for the next launch or
-    // visit (seal_candidates_kernel closes the candidate chunks after the
-    // pass); the warp's counts go to its statistics
+    // leave the current subject: its chunk stays open for the next launch or visit
     auto leave = [&]() {
-      if (PASS == 0 && cur_s >= 0) {
-        if (lane < 4)
-          a.wstate[wid * 4 + lane] = lane == 0 ? wcur : lane == 1 ? wend : lane == 2 ? ccur : cend;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          n_def += __shfl_xor_sync(0xffffffffu, n_def, o);
-          n_cand += __shfl_xor_sync(0xffffffffu, n_cand, o);
-        }
-        if (lane == 0 && n_def) atomicAdd(&a.stats[2], n_def);
-        if (lane == 0 && n_cand) atomicAdd(&a.stats[3], n_cand);
-        n_def = n_cand = 0;
-      }
+      if (PASS == 0 && cur_s >= 0 && lane < 2)
+        a.wstate[wid * 2 + lane] = lane == 0 ? wcur : wend;
       __syncwarp();
     };
     auto tile_at = [&](int t, int2& tl, int& ts) {
@@ -524,7 +510,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
       const bool diag = (I == J);
       int rowcount = 0;
-      uint32_t cmk4[4] = {0u, 0u, 0u, 0u};
+      uint32_t cands = 0;  // not 0: this row has a candidate here
       // chunk c of this warp's values: columns c * 32 .. + 31 of the half-tile,
       // v[k] of row il; unc: columns whose pair is recomputed whatever its value
       // (AVG); bad: the half-tile has a voxel with NaN z-scores
@@ -597,8 +583,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
           const int total = __shfl_sync(0xffffffffu, incl, 31);
           uint2* dst = s_elist + wcur + (incl - ne);
-          // classify this lane's few interesting entries; candidates are only
-          // flagged here (collected for the exact recompute after the pass)
+          // classify this lane's few interesting entries
           uint32_t eb = 0;
           uint32_t w2 = it;
           while (w2) {
@@ -610,58 +595,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const float x = ABS ? fabsf(r) : r;
             uint32_t cf = 0;
             if (!((x - tau > delta) && (fabsf(r) < lim)) || (AVG && ((unc >> k) & 1u))) {
-              cf = 1u;  // candidate: collected for the exact recompute after the pass
-              val = 0u;
+              cf = 1u;
             }
             eb |= (cf ^ 1u) << k;
             if (wok) *dst++ = make_uint2(elist_key(il, c * 32 + k, cf), val);
           }
           rowcount += __popc(eb);
-          n_def += __popc(eb);
+          cands |= it & ~eb;
           S.colmask[h][c * 32 + lane][q] = transpose32(eb, lane);
           wcur += total;
-          if (!DENS) {
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4)  // candidates of this chunk (listed after the tile)
-              if (q4 == c) cmk4[q4] = it & ~eb;
-          } else if (__any_sync(0xffffffffu, (it & ~eb) != 0u)) {
-            // candidates with their approximate values, listed now (v[] is live)
-            const uint32_t cmk = it & ~eb;
-            const int nc = __popc(cmk);
-            int cinc = nc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-              const int y = __shfl_up_sync(0xffffffffu, cinc, o);
-              if (lane >= o) cinc += y;
-            }
-            const int ctot = __shfl_sync(0xffffffffu, cinc, 31);
-            if (ccur + ctot > cend) {
-              for (long long sl = ccur + lane; sl < cend && sl < a.cand_cap; sl += 32)
-                a.cand[sl] = make_uint2(kCandNone, kCandNone);
-              const long long need = (ctot + kCandChunk - 1) / kCandChunk * kCandChunk;
-              unsigned long long cb = 0;
-              if (lane == 0) cb = atomicAdd(a.cand_count, (unsigned long long)need);
-              ccur = (long long)__shfl_sync(0xffffffffu, cb, 0);
-              cend = ccur + need;
-            }
-            long long slot = ccur + (cinc - nc);
-            uint32_t w3 = cmk;
-            while (w3) {
-              const int k = __ffs(w3) - 1;
-              w3 &= w3 - 1;
-              const bool badk = (badm >> k) & 1u;
-              const float r = badk ? 0.0f : __uint_as_float(pick32(v, k));
-              if (slot < a.cand_cap) {
-                a.cand[slot] = make_uint2((unsigned)gi, (unsigned)(J * 128 + c * 32 + k));
-                a.cand_apx[slot] = r;
-              } else {
-                atomicOr(a.err, ERR_BAND_OVERFLOW);
-              }
-              ++slot;
-            }
-            ccur += ctot;
-            n_cand += nc;
-          }
       };
       if (AVG) {
         // running sums in registers, rotated so that the loop over the four
@@ -822,47 +764,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         ptx::mbar_arrive(ptx::smem_u32(&S.tempty[acc]));
       }
       if (PASS == 2 || PASS == 3 || PASS == 4) continue;
-      // candidates (rare): warp prefix scan into the warp's candidate chunk
-      if (!DENS && active &&
-          __any_sync(0xffffffffu, (cmk4[0] | cmk4[1] | cmk4[2] | cmk4[3]) != 0u)) {
-        const int nc = __popc(cmk4[0]) + __popc(cmk4[1]) + __popc(cmk4[2]) + __popc(cmk4[3]);
-        int cinc = nc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, cinc, o);
-          if (lane >= o) cinc += y;
-        }
-        const int ctot = __shfl_sync(0xffffffffu, cinc, 31);
-        if (ccur + ctot > cend) {
-          // seal the rest of the chunk, take enough new chunks for this batch
-          for (long long sl = ccur + lane; sl < cend && sl < a.cand_cap; sl += 32)
-            a.cand[sl] = make_uint2(kCandNone, kCandNone);
-          const long long need = (ctot + kCandChunk - 1) / kCandChunk * kCandChunk;
-          unsigned long long cb = 0;
-          if (lane == 0) cb = atomicAdd(a.cand_count, (unsigned long long)need);
-          ccur = (long long)__shfl_sync(0xffffffffu, cb, 0);
-          cend = ccur + need;
-        }
-        long long slot = ccur + (cinc - nc);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t w3 = cmk4[c];
-          while (w3) {
-            const int k = __ffs(w3) - 1;
-            w3 &= w3 - 1;
-            if (slot < a.cand_cap)
-              a.cand[slot] = make_uint2((unsigned)gi, (unsigned)(J * 128 + c * 32 + k));
-            else
-              atomicOr(a.err, ERR_BAND_OVERFLOW);
-            ++slot;
-          }
-        }
-        ccur += ctot;
-        n_cand += nc;
+      if (PASS == 0 && active) {
+        const bool any = __any_sync(0xffffffffu, cands != 0u);
+        if (lane == 0)
+          s_etab[subtile_index(I, J, s_nb) * 4 + q] =
+              wok ? make_longlong2(start, (wcur - start) | (any ? kEtabCand : 0))
+                  : make_longlong2(0, 0);
       }
-      if (active && lane == 0)
-        s_etab[subtile_index(I, J, s_nb) * 4 + q] =
-            wok ? make_longlong2(start, wcur - start) : make_longlong2(0, 0);
       if (!half_sync(S, h, hphase)) {
         atomicOr(a.err, ERR_TIMEOUT);
         S.abort = 1;
@@ -894,18 +802,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (threadIdx.x == 0 && atomicAdd(p.sched + 1, 1u) == gridDim.x - 1) {
     p.sched[0] = 0;
     p.sched[1] = 0;
-  }
-}
-
-// After the last launch of a count pass: mark the unused slots of every
-// warp's open candidate chunk (warp states are (wcur, wend, ccur, cend)).
-__global__ void seal_candidates_kernel(CorrArgs a, int nwarps) {
-  const int lane = threadIdx.x & 31;
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < nwarps;
-       w += gridDim.x * (blockDim.x >> 5)) {
-    const long long ccur = a.wstate[w * 4 + 2], cend = a.wstate[w * 4 + 3];
-    for (long long sl = ccur + lane; sl < cend && sl < a.cand_cap; sl += 32)
-      if (sl >= 0) a.cand[sl] = make_uint2(kCandNone, kCandNone);
   }
 }
 
@@ -1083,26 +979,23 @@ bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad,
 // batch.err receives timeouts of the producer and MMA warps.
 // The multi-subject kernel of a form, with its shared-memory limit set (a
 // call outside any stream capture; the launcher sets it too).
-static void (*tc_multi_kernel(int form, bool dens, bool absm))(CUtensorMap, CUtensorMap, TcArgs) {
+static void (*tc_multi_kernel(int form, bool absm))(CUtensorMap, CUtensorMap, TcArgs) {
   if (form == FORM_BF16X3)
-    return dens ? corr_tc_kernel<0, false, FORM_BF16X3, true, true>
-           : absm ? corr_tc_kernel<0, true, FORM_BF16X3, false, true>
-                  : corr_tc_kernel<0, false, FORM_BF16X3, false, true>;
-  return dens ? corr_tc_kernel<0, false, FORM_TF32, true, true>
-         : absm ? corr_tc_kernel<0, true, FORM_TF32, false, true>
-                : corr_tc_kernel<0, false, FORM_TF32, false, true>;
+    return absm ? corr_tc_kernel<0, true, FORM_BF16X3, true>
+                : corr_tc_kernel<0, false, FORM_BF16X3, true>;
+  return absm ? corr_tc_kernel<0, true, FORM_TF32, true>
+              : corr_tc_kernel<0, false, FORM_TF32, true>;
 }
 
-cudaError_t prepare_corr_tc_multi(int form, bool dens, bool absm) {
-  if (dens && absm) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(tc_multi_kernel(form, dens, absm),
+cudaError_t prepare_corr_tc_multi(int form, bool absm) {
+  return cudaFuncSetAttribute(tc_multi_kernel(form, absm),
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_BYTES);
 }
 
 cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, const int4* tiles4,
-                                 int ntiles, int form, bool dens, bool absm, int grid,
+                                 int ntiles, int form, bool absm, int grid,
                                  unsigned int* sched, cudaStream_t st) {
-  if ((dens && absm) || !sched) return cudaErrorInvalidValue;
+  if (!sched) return cudaErrorInvalidValue;
   TcArgs p{};
   p.a = batch;
   p.sched = sched;
@@ -1112,15 +1005,10 @@ cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, co
   p.nksteps = 0;
   const int g = grid < ntiles ? grid : ntiles;
   if (g <= 0) return cudaSuccess;
-  void (*kern)(CUtensorMap, CUtensorMap, TcArgs) = tc_multi_kernel(form, dens, absm);
+  void (*kern)(CUtensorMap, CUtensorMap, TcArgs) = tc_multi_kernel(form, absm);
   CUtensorMap dummy;
   std::memset(&dummy, 0, sizeof dummy);
   kern<<<g, TC_THREADS, TC_SMEM_BYTES, st>>>(dummy, dummy, p);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_seal_candidates(const CorrArgs& a, int nwarps, cudaStream_t st) {
-  seal_candidates_kernel<<<(nwarps + 7) / 8, 256, 0, st>>>(a, nwarps);
   return cudaGetLastError();
 }
 
@@ -1130,7 +1018,7 @@ cudaError_t launch_seal_candidates(const CorrArgs& a, int nwarps, cudaStream_t s
 cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
                                int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
                                int grid, unsigned int* sched, cudaStream_t st) {
-  if (!sched || nsub < 1 || (pass == 4 && !packed) || a.cand_apx) return cudaErrorInvalidValue;
+  if (!sched || nsub < 1 || (pass == 4 && !packed)) return cudaErrorInvalidValue;
   TcArgs p{};
   p.a = a;
   p.sched = sched;
@@ -1145,15 +1033,15 @@ cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void
   const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
   if (form == FORM_BF16X3)
-    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_BF16X3, false, false, true>
-                               : corr_tc_kernel<0, false, FORM_BF16X3, false, false, true>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false, false, true>
-                       : corr_tc_kernel<4, false, FORM_BF16X3, false, false, true>;
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_BF16X3, false, true>
+                               : corr_tc_kernel<0, false, FORM_BF16X3, false, true>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false, true>
+                       : corr_tc_kernel<4, false, FORM_BF16X3, false, true>;
   else
-    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_TF32, false, false, true>
-                               : corr_tc_kernel<0, false, FORM_TF32, false, false, true>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false, false, true>
-                       : corr_tc_kernel<4, false, FORM_TF32, false, false, true>;
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_TF32, false, true>
+                               : corr_tc_kernel<0, false, FORM_TF32, false, true>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false, true>
+                       : corr_tc_kernel<4, false, FORM_TF32, false, true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)TC_SMEM_BYTES);
   if (e != cudaSuccess) return e;
@@ -1196,21 +1084,15 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
   const int g = grid < ntiles ? grid : ntiles;
   if (g <= 0) return cudaSuccess;
   const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
-  const bool dens = pass == 0 && a.cand_apx != nullptr;
-  if (dens && absm) return cudaErrorInvalidValue;  // the density rule is signed
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
   if (form == FORM_BF16X3)
-    kern = pass == 0   ? (dens   ? corr_tc_kernel<0, false, FORM_BF16X3, true>
-                          : absm ? corr_tc_kernel<0, true, FORM_BF16X3, false>
-                                 : corr_tc_kernel<0, false, FORM_BF16X3, false>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false>
-                       : corr_tc_kernel<2, false, FORM_BF16X3, false>;
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_BF16X3> : corr_tc_kernel<0, false, FORM_BF16X3>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3>
+                       : corr_tc_kernel<2, false, FORM_BF16X3>;
   else
-    kern = pass == 0   ? (dens   ? corr_tc_kernel<0, false, FORM_TF32, true>
-                          : absm ? corr_tc_kernel<0, true, FORM_TF32, false>
-                                 : corr_tc_kernel<0, false, FORM_TF32, false>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false>
-                       : corr_tc_kernel<2, false, FORM_TF32, false>;
+    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_TF32> : corr_tc_kernel<0, false, FORM_TF32>)
+           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32>
+                       : corr_tc_kernel<2, false, FORM_TF32>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)TC_SMEM_BYTES);
   if (e != cudaSuccess) return e;

@@ -4,7 +4,7 @@
 // rows in order, columns ascending, both (i, j) and (j, i) of each pair,
 // V[e] = r of the pair.  Here the count pass has left, per 128 x 128
 // sub-tile (I, J), I <= J, a compact list of its edges (value) and of its
-// near-threshold candidates (resolved by the recompute pass into a hash).
+// near-threshold candidates (resolved in place by the recompute pass).
 // One warp handles one sub-tile for the 128 rows of one row block: the
 // direct entries of sub-tile (I, J), J >= I, or the transposed entries of
 // sub-tile (J, I), J <= I, for the rows of block I:
@@ -60,12 +60,20 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // put_edge for positions in 32 bits (a CSR's row offsets are int32)
 __device__ __forceinline__ void put_edge32(const CorrArgs& a, int pos, int col, float v) {
-  if ((unsigned long long)(unsigned)pos >= (unsigned long long)a.nnz) {
+  if ((unsigned)pos >= (unsigned)a.nnz) {
     atomicOr(a.err, ERR_RANGE);
     return;
   }
   a.col_idx[pos] = col;
   if (a.weighted) a.val[pos] = v;
+}
+
+// Whether an edge-list entry is placed: not a dropped candidate; one that the
+// recompute pass never resolved is flagged.
+__device__ __forceinline__ bool placed(const CorrArgs& a, uint32_t x) {
+  if (x >> 14 == 0) return true;
+  if ((x >> 14) & 1u) atomicOr(a.err, ERR_UNRESOLVED);
+  return false;
 }
 
 // popc_before4 of a 16-byte-aligned row of four mask words, read in one load
@@ -77,44 +85,34 @@ __device__ __forceinline__ int popc_before4v(const uint32_t* m, int pos) {
          (w >= 2 ? __popc(w == 2 ? v.z & low : v.z) : 0) + (w == 3 ? __popc(v.w & low) : 0);
 }
 
-__device__ __forceinline__ int popc_before4(const uint32_t* m, int pos) {
-  const int w = pos >> 5;
-  int c = __popc(m[w] & ((1u << (pos & 31)) - 1u));
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-    if (k < w) c += __popc(m[k]);
-  return c;
-}
-
 // Row-block order: CTA (I, part) handles the rows of 128-row block I and the
 // column blocks of one contiguous range `part`, its warps taking J = j0 + w,
 // j0 + w + 8, ... in turn.  Sub-tile (I, J), J > I, gives the rows of I their
 // entries (direct); sub-tile (J, I), J < I, gives them its column entries
-// (transposed); the diagonal sub-tile both.  Each CSR row is thus written by
-// `parts` CTAs, each filling one contiguous stretch of it segment after
-// segment while it runs, so partial sectors are completed in L2 instead of
-// being read back and written piecemeal.  A lane keeps its first kFillKeep
-// entries, candidates resolved, in registers for the placing pass.
-// Sub-tiles above kFillDenseE entries are queued (once) for
-// csr_fill_dense_kernel.  The block's row starts are read once into shared
-// memory, and each warp's loads run ahead of its work by asynchronous copies
-// into shared memory: while it places a sub-tile's entries, the next
-// sub-tile's segment offsets and first kFillStage entries and the ranges of
-// the one after that are in flight (the entries' load latency was the
-// kernel's main stall).
-constexpr int kFillKeep = 8;
-constexpr int kFillStage = 128;  // entries staged per warp ahead of use
+// (transposed); the diagonal sub-tile both, the transposed ones (columns below
+// the row) first.  Each CSR row is thus written by `parts` CTAs, each filling one
+// contiguous stretch of it segment after segment while it runs, so partial
+// sectors are completed in L2 instead of being read back and written piecemeal.
+// A lane keeps its first kFillStage / 32 entries in registers for the placing
+// pass.  Sub-tiles above kFillDenseE entries are left to csr_fill_dense_kernel.
+// The block's row starts are read once into shared memory, and each warp's loads
+// run ahead of its work by asynchronous copies into shared memory: while it
+// places a sub-tile's entries, the next sub-tile's segment offsets and first
+// kFillStage entries and the ranges of the one after that are in flight.
+// Bound: issue and instruction fetch; one direction's code serves both (45,000
+// voxels, 18.5 M entries: 333 us with a copy of the code per direction and hash
+// probes for the candidates in each, 285 now).
+constexpr int kFillStage = 256;  // entries staged per warp ahead of use
+constexpr int kFillKeep = kFillStage / 32;
 
 __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrArgs a, int I0,
                                                                            int parts) {
-  __shared__ __align__(16) uint32_t rmask[kFillWarps][128][4];  // direct: row il's columns jl
-  __shared__ __align__(16) uint32_t tmask[kFillWarps][128][4];  // transposed: row jl's columns il
-  __shared__ int dbase[kFillWarps][128];
-  __shared__ int tbase[kFillWarps][128];
+  __shared__ __align__(16) uint32_t mask[kFillWarps][128][4];  // row r's columns in block J
+  __shared__ int base[kFillWarps][128];            // row r's first position in block J
   __shared__ int rp_s[128];                        // row_ptr of the block's rows (0 past the end)
   __shared__ int nsg[kFillWarps][128];             // staged: rows' block-J segment offsets
   __shared__ longlong2 netab[kFillWarps][2][4];    // staged: quadrant ranges (two sub-tiles)
-  __shared__ uint2 ent[kFillWarps][kFillStage];    // staged: first entries (raw)
+  __shared__ uint2 ent[kFillWarps][kFillStage];    // staged: first entries
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Ir = blockIdx.x / parts, part = blockIdx.x - Ir * parts;
   const int I = I0 + Ir;
@@ -125,41 +123,39 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
     rp_s[threadIdx.x] = gi < a.n ? a.row_ptr[gi] : 0;
   }
   __syncthreads();
-  uint32_t(*rm)[4] = rmask[w];
-  uint32_t(*tm)[4] = tmask[w];
+  uint32_t(*mk)[4] = mask[w];
   // a sub-tile's four quadrant ranges (lanes 0-3)
   auto fetch_ranges = [&](int J, int slot) {
     const long long st = subtile_index(min(I, J), max(I, J), a.nb);
     if (lane < 4) cp_async16(&netab[w][slot][lane], a.etab + st * 4 + lane);
   };
+  // entry e of quadrant q is elist[b[q] + e] for p[q] <= e < p[q + 1]; the
+  // entries to place here: 0 for the dense pass's sub-tiles, and for ranges
+  // written while the pool overflowed
+  auto ranges = [&](int slot, long long (&b)[4], int (&p)[3]) {
+    int E = 0;
+    bool use = true;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const longlong2 s = netab[w][slot][q];
+      use &= s.y >= 0 && s.y <= kFillDenseE && s.x >= 0 && s.x + s.y <= a.ecap;
+      b[q] = s.x - E;
+      E += (int)s.y;
+      if (q < 3) p[q] = E;
+    }
+    return use && E <= (int)kFillDenseE ? E : 0;
+  };
   // its rows' segment offsets (rows past the last real one read the padding,
-  // never used) and, when the fill places it here, its first entries; its
-  // ranges are in netab[w][slot]
+  // never used) and its first entries; its ranges are in netab[w][slot]
   auto fetch_rest = [&](int J, int slot) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       cp_async4(&nsg[w][lane + 32 * k], a.seg + (size_t)J * a.n_pad + I * 128 + lane + 32 * k);
-    long long s[4], c[4];
-    bool inside = true;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const longlong2 r = netab[w][slot][q];
-      s[q] = r.x;
-      c[q] = r.y;
-      inside &= c[q] >= 0 && s[q] >= 0 && s[q] + c[q] <= a.ecap;
-    }
-    const long long E = c[0] + c[1] + c[2] + c[3];
-    if (!inside || E > kFillDenseE) return;
-    const long long p1 = c[0], p2 = p1 + c[1], p3 = p2 + c[2];
-#pragma unroll
-    for (int k = 0; k < kFillStage / 32; ++k) {
-      const long long e = lane + 32 * k;
-      if (e < E) {
-        const long long at = e < p1 ? s[0] + e : e < p2 ? s[1] + (e - p1)
-                             : e < p3 ? s[2] + (e - p2) : s[3] + (e - p3);
-        cp_async8(&ent[w][e], a.elist + at);
-      }
-    }
+    long long b[4];
+    int p[3];
+    const int E = ranges(slot, b, p);
+    for (int e = lane; e < min(E, kFillStage); e += 32)
+      cp_async8(&ent[w][e], a.elist + (e < p[0] ? b[0] : e < p[1] ? b[1] : e < p[2] ? b[2] : b[3]) + e);
   };
   int v = 0;  // this warp's sub-tile count (range slot v & 1)
   if (j0 + w < j1) {
@@ -173,57 +169,20 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
   }
   for (int J = j0 + w; J < j1; J += kFillWarps, ++v) {
     const int slot = v & 1;
-    const int lo = min(I, J), hi = max(I, J);
     cp_async_wait_all();
     __syncwarp();
-    long long s0 = 0, c0 = 0;
-    if (lane < 4) {
-      s0 = netab[w][slot][lane].x;
-      c0 = netab[w][slot][lane].y;
-    }
-    // rows lane + 32k: start of their block-J segment (the transposed
-    // entries' base; the previous sub-tile's placing is over)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) tbase[w][lane + 32 * k] = rp_s[lane + 32 * k] + nsg[w][lane + 32 * k];
-    // entry e of quadrant q is elist[b[q] + e] for p[q] <= e < p[q + 1]
-    long long b[4], E = 0;
-    int p1 = 0, p2 = 0, p3 = 0;  // a sub-tile placed here has at most kFillDenseE entries
-    bool inside = true;  // ranges written while the pool overflowed are not read
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const long long st = __shfl_sync(0xffffffffu, s0, q);
-      const long long ct = __shfl_sync(0xffffffffu, c0, q);
-      inside &= ct >= 0 && st >= 0 && st + ct <= a.ecap;
-      b[q] = st - E;
-      E += ct;
-      if (q == 0) p1 = (int)E;
-      if (q == 1) p2 = (int)E;
-      if (q == 2) p3 = (int)E;
-    }
-    const bool use = inside && E != 0 && E <= kFillDenseE;  // else flagged / the dense pass's
-    const int Ei = use ? (int)E : 0;
-    auto load = [&](int e) {
-      return a.elist[e + (e < p1 ? b[0] : e < p2 ? b[1] : e < p3 ? b[2] : b[3])];
-    };
-    // candidate bit resolved: bit 15 set = not an edge, .y = the value to store
-    auto resolve = [&](uint2 en) {
-      if ((en.x >> 14) & 1u) {
-        float val = 0.0f;
-        bool edge = false;
-        hash_lookup(a, pair_key(lo * 128 + (en.x & 127), hi * 128 + ((en.x >> 7) & 127)), val,
-                    edge);
-        en.y = __float_as_uint(val);
-        if (!edge) en.x |= 1u << 15;
-      }
-      return en;
-    };
-    const int kmax = min((Ei + 31) / 32, kFillKeep);
+    for (int k = 0; k < 4; ++k) base[w][lane + 32 * k] = rp_s[lane + 32 * k] + nsg[w][lane + 32 * k];
+    long long b[4];
+    int p[3];
+    const int E = ranges(slot, b, p);
+    const int kmax = min((E + 31) / 32, kFillKeep);
     uint2 keep[kFillKeep];
 #pragma unroll
     for (int k = 0; k < kFillKeep; ++k) {
       const int e = lane + 32 * k;
       keep[k] = make_uint2(1u << 15, 0u);
-      if (k < kmax && e < Ei) keep[k] = k < kFillStage / 32 ? ent[w][e] : load(e);
+      if (k < kmax && e < E) keep[k] = ent[w][e];
     }
     __syncwarp();  // the staged data read by every lane before the next copies land
     if (J + kFillWarps < j1) {
@@ -231,59 +190,48 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
       if (J + 2 * kFillWarps < j1) fetch_ranges(J + 2 * kFillWarps, slot);
     }
     cp_async_commit();
-    if (!use) continue;
-#pragma unroll
-    for (int k = 0; k < kFillKeep; ++k)
-      if (k < kmax) keep[k] = resolve(keep[k]);
-    const bool diag = I == J, trans = J < I;
-    // the masks this sub-tile uses: direct (rows of I), transposed (rows of
-    // J as columns of I), both on the diagonal
-    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-    if (!trans)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(rm)[lane + 32 * k] = zero4;
-    if (trans || diag)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(tm)[lane + 32 * k] = zero4;
-    __syncwarp();
-    // 1. masks
-    auto mark = [&](uint2 en) {
-      if ((en.x >> 15) & 1u) return;
-      const int il = en.x & 127, jl = (en.x >> 7) & 127;
-      if (!trans) atomicOr(&rm[il][jl >> 5], 1u << (jl & 31));
-      if (trans || diag) atomicOr(&tm[jl][il >> 5], 1u << (il & 31));
+    if (E == 0) continue;
+    auto load = [&](int e) {
+      return a.elist[e + (e < p[0] ? b[0] : e < p[1] ? b[1] : e < p[2] ? b[2] : b[3])];
     };
+    // row's and column's bits in an entry's key; the diagonal takes both directions
+    int sr = J <= I ? 7 : 0;
+    for (int turn = I == J ? 0 : 1; turn < 2; ++turn) {
+      // 1. masks
+      const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int k = 0; k < kFillKeep; ++k)
-      if (k < kmax) mark(keep[k]);
-    for (int e = lane + 32 * kFillKeep; e < Ei; e += 32) mark(resolve(load(e)));
-    __syncwarp();
-    // 2. segment bases of the block's rows for column block J (on the
-    // diagonal the transposed entries, columns < the row, come first)
+      for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(mk)[lane + 32 * k] = zero4;
+      __syncwarp();
+      auto mark = [&](uint2 en) {
+        const int c = (en.x >> (7 - sr)) & 127;
+        if (placed(a, en.x)) atomicOr(&mk[(en.x >> sr) & 127][c >> 5], 1u << (c & 31));
+      };
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int r = lane + 32 * k;
-      if (diag) {
-        const uint4 c = *reinterpret_cast<const uint4*>(tm[r]);
-        dbase[w][r] = tbase[w][r] + __popc(c.x) + __popc(c.y) + __popc(c.z) + __popc(c.w);
-      } else {
-        dbase[w][r] = tbase[w][r];
+      for (int k = 0; k < kFillKeep; ++k)
+        if (k < kmax) mark(keep[k]);
+      for (int e = lane + kFillStage; e < E; e += 32) mark(load(e));
+      __syncwarp();
+      // 2. place: the entry's rank among its row's columns
+      auto place = [&](uint2 en) {
+        if (en.x >> 15) return;
+        const int r = (en.x >> sr) & 127, c = (en.x >> (7 - sr)) & 127;
+        put_edge32(a, base[w][r] + popc_before4v(mk[r], c), J * 128 + c, __uint_as_float(en.y));
+      };
+#pragma unroll
+      for (int k = 0; k < kFillKeep; ++k)
+        if (k < kmax) place(keep[k]);
+      for (int e = lane + kFillStage; e < E; e += 32) place(load(e));
+      __syncwarp();
+      if (turn == 0) {  // the diagonal's direct entries follow the transposed ones
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint4 m = reinterpret_cast<const uint4*>(mk)[lane + 32 * k];
+          base[w][lane + 32 * k] += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+        }
+        __syncwarp();
+        sr = 0;
       }
     }
-    __syncwarp();
-    // 3. place this block's entries: direct (row il) and transposed (row jl)
-    auto place = [&](uint2 en) {
-      if ((en.x >> 15) & 1u) return;
-      const int il = en.x & 127, jl = (en.x >> 7) & 127;
-      const float val = __uint_as_float(en.y);
-      if (!trans) put_edge32(a, dbase[w][il] + popc_before4v(rm[il], jl), hi * 128 + jl, val);
-      if (trans || diag) put_edge32(a, tbase[w][jl] + popc_before4v(tm[jl], il), lo * 128 + il, val);
-    };
-#pragma unroll
-    for (int k = 0; k < kFillKeep; ++k)
-      if (k < kmax) place(keep[k]);
-    for (int e = lane + 32 * kFillKeep; e < Ei; e += 32) place(resolve(load(e)));
-    __syncwarp();
   }
   cp_async_wait_all();  // nothing in flight into shared memory at exit
 }
@@ -356,10 +304,8 @@ __global__ __launch_bounds__(256) void csr_fill_dense_kernel(CorrArgs a, const i
       for (int u = 0; u < kFillDenseLoads; ++u) {
         if (e0 + 256 * u >= E) break;
         const int il = en[u].x & 127, jl = (en[u].x >> 7) & 127;
-        float v = __uint_as_float(en[u].y);
-        bool edge = true;
-        if ((en[u].x >> 14) & 1u) hash_lookup(a, pair_key(I * 128 + il, J * 128 + jl), v, edge);
-        if (edge) {
+        const float v = __uint_as_float(en[u].y);
+        if (placed(a, en[u].x)) {
           S.val[il][jl] = v;
           atomicOr(&S.rm[il][jl >> 5], 1u << (jl & 31));
           atomicOr(&S.cm[jl][il >> 5], 1u << (il & 31));

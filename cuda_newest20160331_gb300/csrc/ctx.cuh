@@ -122,24 +122,25 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
 cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
                                int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
                                int grid, unsigned int* sched, cudaStream_t st);
-cudaError_t launch_seal_candidates(const CorrArgs& a, int nwarps, cudaStream_t st);
 size_t tc_subj_bytes();
 bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form,
                   float unc_lim = 1.0f);
-cudaError_t prepare_corr_tc_multi(int form, bool dens, bool absm);
+cudaError_t prepare_corr_tc_multi(int form, bool absm);
 cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, const int4* tiles4,
-                                 int ntiles, int form, bool dens, bool absm, int grid,
+                                 int ntiles, int form, bool absm, int grid,
                                  unsigned int* sched, cudaStream_t st);
 cudaError_t launch_rowlen_scan(const long long* rowlen, int n, long long* pre, long long* bsum,
                                long long* total, int32_t* row_ptr, uint32_t* err,
                                cudaStream_t stream);
+size_t rethr_words(int n, long long nnz);
 cudaError_t launch_rethr_count(const CorrArgs& a, const int32_t* rp, const int32_t* ci,
-                               const float* val, const Threshold& th, uint8_t* keep, float* valx,
-                               long long* rowlen, unsigned long long* band, int sms,
-                               cudaStream_t st);
-cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* valx,
-                              const uint8_t* keep, const int32_t* rp2, int32_t* ci2, float* val2,
-                              long long nnz2, uint32_t* err, int sms, cudaStream_t st);
+                               const float* val, const Threshold& th, uint32_t* keep,
+                               uint32_t* exact, float* valx, long long* rowlen,
+                               unsigned long long* band, int sms, cudaStream_t st);
+cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* val,
+                              const float* valx, const uint32_t* keep, const uint32_t* exact,
+                              const int32_t* rp2, int32_t* ci2, float* val2, long long nnz2,
+                              uint32_t* err, int sms, cudaStream_t st);
 cudaError_t launch_avg_exact(const CorrArgs& a, const void* subj, int S, int fisher, float* out,
                              int sms, cudaStream_t st);
 size_t avg_subj_bytes();
@@ -167,7 +168,7 @@ namespace bna {
 
 enum Slot {
   S_BOLD, S_Z, S_ZHI, S_ZLO, S_BAD, S_SEG, S_ROWLEN, S_PRE, S_BSUM, S_ROWPTR, S_COL, S_VAL,
-  S_CAND, S_HKEYS, S_HVAL, S_HEDGE, S_STATUS, S_DROP, S_EC_U, S_EC_PARTS, S_EC_STATE,
+  S_CAND, S_CANDPOS, S_STATUS, S_DROP, S_EC_U, S_EC_PARTS, S_EC_STATE,
   S_EC_R, S_EC_C, S_EC_V, S_EC_VD, S_DUMP, S_TILES, S_BLOCKBAD, S_DUMPTILE, S_ELIST, S_ETAB, S_HIST, S_CANDVAL,
   S_DENSE, S_WSTATE, S_VSTAT,
   S_TILES_SMP, S_DSTATE, S_DHIST, S_DCLS, S_DEIDX, S_DEXACT, S_CANDAPX, S_DTIES,
@@ -313,7 +314,6 @@ int64_t request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t c
                       bool lean);
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 double default_delta(int precision, int T);
-unsigned long long next_pow2(unsigned long long x);
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 // Every entry point starts here: device current, and the call's stream
 // recorded for stream-ordered arena growth.

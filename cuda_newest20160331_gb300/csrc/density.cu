@@ -21,7 +21,7 @@
 //      checked (the window may come from a sample);
 //   4. the pairs of E equal to tau* are sorted by (i, j); the first
 //      k - (pairs above tau*) stay, the rest are dropped;
-//   5. every candidate is decided and stored in the hash the fill pass reads.
+//   5. every candidate is decided and its edge-list entry resolved for the fill pass.
 // The k-th largest is found by a three-digit radix select (11 + 11 + 10 bits
 // of an order-preserving integer key of the float).
 #include "common.cuh"
@@ -94,7 +94,6 @@ __global__ void dens_hist_kernel(CorrArgs a, DensState* ds, const float* exact, 
          i += (long long)gridDim.x * blockDim.x) {
       float v;
       if (which == 0) {
-        if (a.cand[i].x == kCandNone) continue;
         v = a.cand_apx[i];
       } else {
         v = exact[i];
@@ -184,7 +183,7 @@ __global__ void dens_classify_kernel(CorrArgs a, DensState* ds, uint8_t* cls, in
        i0 += stride) {
     const long long i = i0 + lane;
     uint8_t k = 0;
-    if (i < n && a.cand[i].x != kCandNone) {
+    if (i < n) {
       const float r = a.cand_apx[i];
       if (fabsf(r) >= lim || fabsf(r - tq) <= d2) k = 2;
       else k = r > tq ? 1 : 3;
@@ -203,19 +202,20 @@ __global__ void dens_classify_kernel(CorrArgs a, DensState* ds, uint8_t* cls, in
   }
 }
 
-// Exact values of E (warp per item).
+// Exact values of E.
 __global__ void dens_exact_kernel(CorrArgs a, DensState* ds, const int* eidx, float* exact,
                                   float* slot_val) {
   if (ds->err) return;
   const long long n = ds->n_exact;
   const int lane = threadIdx.x & 31;
-  const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long e = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); e < n;
-       e += nw) {
-    const int slot = eidx[e];
+  const long long step = (long long)gridDim.x * (blockDim.x / kPairLanes);
+  for (long long e0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * kPairs;
+       e0 < n; e0 += step) {
+    const long long e = e0 + lane / kPairLanes;
+    const int slot = e < n ? eidx[e] : 0;
     const uint2 p = a.cand[slot];
-    const float r = exact_r_warp(a, (int)p.x, (int)p.y, lane);
-    if (lane == 0) {
+    const float r = post_block(exact_r_pairs_raw(a, e < n, (int)p.x, (int)p.y, lane));
+    if (e < n && (lane & (kPairLanes - 1)) == 0) {
       exact[e] = r;
       slot_val[slot] = r;
     }
@@ -287,7 +287,7 @@ __global__ void dens_drop_kernel(DensState* ds, const unsigned long long* stats,
   }
 }
 
-// Decide every candidate, count the edges into seg, fill the hash.
+// Decide every candidate, count the edges into seg, resolve its edge-list entry.
 __global__ void dens_decide_kernel(CorrArgs a, DensState* ds, const uint8_t* cls,
                                    const float* slot_val, const unsigned long long* drop) {
   if (ds->err) return;
@@ -315,19 +315,7 @@ __global__ void dens_decide_kernel(CorrArgs a, DensState* ds, const uint8_t* cls
       atomicAdd(&a.seg[(size_t)(pi / kBlk) * a.n_pad + pj], 1);
       ++n_edge;
     }
-    unsigned long long h = hash64(key) & a.hmask;
-    bool stored = false;
-    for (unsigned long long probe = 0; probe <= a.hmask; ++probe) {
-      const unsigned long long prev = atomicCAS(&a.hkeys[h], ~0ull, key);
-      if (prev == ~0ull || prev == key) {
-        a.hval[h] = r;
-        a.hedge[h] = e ? 1 : 0;
-        stored = true;
-        break;
-      }
-      h = (h + 1) & a.hmask;
-    }
-    if (!stored) atomicOr(a.err, ERR_HASH_FULL);
+    resolve_candidate(a, i, pi, pj, r, e);
   }
   n_edge = __reduce_add_sync(0xffffffffu, n_edge);
   n_1e6 = __reduce_add_sync(0xffffffffu, n_1e6);

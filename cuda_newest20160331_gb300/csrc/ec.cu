@@ -180,7 +180,7 @@ __device__ __forceinline__ void ec_row_accum(const int32_t* __restrict__ ci,
       x[m] = c[m] < 0 ? make_float2(0.0f, 0.0f) : (l2_only ? __ldcg(uf + c[m]) : uf[c[m]]);
 #pragma unroll
     for (int m = 0; m < 8; ++m)
-      if (32 * m < len) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
+      if (l2_only || 32 * m < len) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
   }
 }
 

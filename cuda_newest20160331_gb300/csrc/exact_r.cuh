@@ -69,13 +69,21 @@ __device__ __forceinline__ bool round_sum_u128(unsigned __int128 acc, unsigned _
   return true;
 }
 
+// Lanes per pair: a warp evaluates four pairs at once, or one when its rows are
+// longer than kPairLongT (the undecided share of pairs grows with the square of
+// the products per lane: 0.6 % at T = 1200 with eight lanes, about 10 % at 5000).
+// With a warp per pair the butterfly outweighed the products: candidates of a
+// TF32 pass (713,000, T = 355) 318 us, 227 with eight lanes each.
+constexpr int kPairLanes = 8, kPairs = 32 / kPairLanes;
+constexpr int kPairLongT = 1600;
+
 // The reference value of a pair is float(sum_t double(float(z_it * z_jt))),
-// the double sum in time order (CorMat.cpp:955-964).  A warp evaluates one
-// pair.  First in float-float: lanes take four time steps at a time, sum their
+// the double sum in time order (CorMat.cpp:955-964).  A group of G
+// lanes evaluates one pair.  First in float-float: lanes take four time steps at a time, sum their
 // products exactly as h + (rounding errors) by TwoSum (Knuth) and the errors c
 // in float, then join by a butterfly of the same.  The rows have unit norm, so
 // sum |p_t| <= 1.01 (Cauchy-Schwarz) bounds every partial sum; with n products
-// per lane c holds n + 5 errors of at most 2^-24 each, added with as many
+// per lane c holds at most n + 5 errors of at most 2^-24 each, added with as many
 // roundings, so |h + c - sum p_t| <= 1.01 (n + 6)^2 2^-48, and the reference's
 // loop lies within 1.01 T 2^-53 of sum p_t.  When no float rounding midpoint
 // lies within both of h + c, the float nearest to h + c is the reference's
@@ -83,6 +91,7 @@ __device__ __forceinline__ bool round_sum_u128(unsigned __int128 acc, unsigned _
 // Padding columns T .. ldz - 1 of the rows are zero and add nothing.
 // Bound: L2 reads of the two rows.  Of the candidates of a TF32 pass (713,000,
 // T = 355) the fixed-point form alone took 1,118 us.
+template <int G>
 __device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
                                             const float* __restrict__ zj, int T, int lane,
                                             float* out) {
@@ -96,8 +105,8 @@ __device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
     c = __fadd_rn(c, __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(p, bb)));
     h = s;
   };
-#pragma unroll 2
-  for (int q = lane; q < nq; q += 32) {
+#pragma unroll(G == 32 ? 2 : 4)
+  for (int q = lane & (G - 1); q < nq; q += G) {
     const float4 a = __ldg(a4 + q), b = __ldg(b4 + q);
     add(__fmul_rn(a.x, b.x));
     add(__fmul_rn(a.y, b.y));
@@ -105,7 +114,7 @@ __device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
     add(__fmul_rn(a.w, b.w));
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = G / 2; o > 0; o >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, h, o);
     const float oc = __shfl_xor_sync(0xffffffffu, c, o);
     c = __fadd_rn(c, oc);
@@ -115,7 +124,7 @@ __device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
   const float q = __fadd_rn(h, c);
   const float bb = __fsub_rn(q, h);
   const float l = __fadd_rn(__fsub_rn(h, __fsub_rn(q, bb)), __fsub_rn(c, bb));
-  const float n6 = (float)(((nq + 31) >> 5) * 4 + 6);
+  const float n6 = (float)(((nq + G - 1) / G) * 4 + 6);
   const float bound = 1.02f * (n6 * n6 * 3.5527137e-15f /* 2^-48 */ +
                                (float)T * 1.1102230e-16f /* 2^-53 */);
   const uint32_t qb = __float_as_uint(q);
@@ -212,7 +221,7 @@ __device__ __forceinline__ float exact_r_warp_raw(const float* z, const uint8_t*
   const float* zi = z + (size_t)i * ldz;
   const float* zj = z + (size_t)j * ldz;
   float r;
-  if (sum_pair_ff(zi, zj, T, lane, &r)) return r;
+  if (sum_pair_ff<32>(zi, zj, T, lane, &r)) return r;
   return exact_r_fixed(zi, zj, T, lane);
 }
 
@@ -221,14 +230,36 @@ __device__ __forceinline__ float exact_r_warp_z(const float* z, const uint8_t* b
   return post_block(exact_r_warp_raw(z, bad, ldz, T, i, j, lane));
 }
 
-__device__ __forceinline__ float exact_r_warp(const CorrArgs& a, int i, int j, int lane) {
-  return exact_r_warp_z(a.z, a.bad, a.ldz, a.T, i, j, lane);
-}
-
-// The value a rule decides on: post_block's, or the raw one for BNA_THR_R_EPS.
-__device__ __forceinline__ float exact_r_rule(const CorrArgs& a, int i, int j, int lane) {
-  const float raw = exact_r_warp_raw(a.z, a.bad, a.ldz, a.T, i, j, lane);
-  return a.th.mode == BNA_THR_R_EPS ? raw : post_block(raw);
+// kPairs pairs by one warp: lane l's group l / kPairLanes evaluates its own
+// (i, j) (on: the group has a pair; all its lanes agree); every lane gets its
+// group's raw value.  Whole warps only.
+__device__ __forceinline__ float exact_r_pairs_raw(const CorrArgs& a, bool on, int i, int j,
+                                                   int lane) {
+  const bool nan = on && (a.bad[i] | a.bad[j]);
+  const bool sum = on && !nan;
+  float r = nan ? __int_as_float(0x7fc00000) : 0.0f;
+  bool done = !sum;
+  if (a.T <= kPairLongT) {
+    // groups without a pair sum nothing but take part in the butterfly
+    float v;
+    const bool ok = sum_pair_ff<kPairLanes>(a.z + (size_t)(sum ? i : 0) * a.ldz,
+                                            a.z + (size_t)(sum ? j : 0) * a.ldz,
+                                            a.T, lane, &v);
+    if (sum && ok) {
+      r = v;
+      done = true;
+    }
+  }
+  for (uint32_t todo = __ballot_sync(0xffffffffu, !done) & 0x01010101u; todo; todo &= todo - 1) {
+    const int l = __ffs(todo) - 1;
+    const float* zi = a.z + (size_t)__shfl_sync(0xffffffffu, i, l) * a.ldz;
+    const float* zj = a.z + (size_t)__shfl_sync(0xffffffffu, j, l) * a.ldz;
+    float v;
+    if (a.T <= kPairLongT || !sum_pair_ff<32>(zi, zj, a.T, lane, &v))
+      v = exact_r_fixed(zi, zj, a.T, lane);
+    if (lane / kPairLanes == l / kPairLanes) r = v;
+  }
+  return r;
 }
 
 // Binary search in ascending keys[0..n).

@@ -23,12 +23,13 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
   const long long nnz_in = in_dev->nnz;
   CorrArgs a = ctx->last;
   Threshold th{mode, (float)tau, ctx->last.th.delta};
-  uint8_t* keep;
+  uint32_t* keep;  // and, behind it, the exact flags
   float* valx;
   long long *rowlen, *pre, *bsum;
   int32_t* rp2;
   DevStatus* ds;
-  ENSURE(S_RT_KEEP, (size_t)std::max(nnz_in, 1LL), keep);
+  const size_t words = rethr_words(N, nnz_in);
+  ENSURE(S_RT_KEEP, 2 * words * sizeof(uint32_t), keep);
   ENSURE(S_RT_VALX, (size_t)std::max(nnz_in, 1LL) * 4, valx);
   ENSURE(S_ROWLEN, (size_t)round_up(N, kBlk) * 8, rowlen);
   ENSURE(S_PRE, (size_t)round_up(N, kBlk) * 8, pre);
@@ -36,8 +37,8 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
   ENSURE(S_RT_ROWPTR, (size_t)(N + 1) * 4, rp2);
   ENSURE(S_STATUS, sizeof(DevStatus), ds);
   CK(cudaMemsetAsync(ds, 0, sizeof(DevStatus), st));
-  CK(launch_rethr_count(a, in_dev->row_ptr, in_dev->col_idx, in_dev->val, th, keep, valx, rowlen,
-                        &ds->stats[1], ctx->sms, st));
+  CK(launch_rethr_count(a, in_dev->row_ptr, in_dev->col_idx, in_dev->val, th, keep, keep + words, valx,
+                        rowlen, &ds->stats[1], ctx->sms, st));
   CK(launch_rowlen_scan(rowlen, N, pre, bsum, &ds->total, rp2, &ds->err, st));
   DevStatus* hs = reinterpret_cast<DevStatus*>(ctx->pinned);
   CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
@@ -47,8 +48,8 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
   float* va2;
   ENSURE(S_RT_COL, (size_t)std::max(nnz, 1LL) * 4, ci2);
   ENSURE(S_RT_VAL, (size_t)std::max(nnz, 1LL) * 4, va2);
-  CK(launch_rethr_fill(N, in_dev->row_ptr, in_dev->col_idx, valx, keep, rp2, ci2, va2, nnz,
-                       &ds->err, ctx->sms, st));
+  CK(launch_rethr_fill(N, in_dev->row_ptr, in_dev->col_idx, in_dev->val, valx, keep, keep + words,
+                       rp2, ci2, va2, nnz, &ds->err, ctx->sms, st));
   CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (hs->err & ERR_RANGE) return fail(ctx, BNA_INTERNAL, "rethreshold: position out of range");

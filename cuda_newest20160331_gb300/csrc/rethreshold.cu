@@ -13,88 +13,172 @@
 
 namespace bna {
 
-// Warp per row: keep flag of every entry, the value to store (exact where it
-// was recomputed), the row's kept count.
-__global__ void rethr_count_kernel(CorrArgs a, const int32_t* __restrict__ rp,
-                                   const int32_t* __restrict__ ci, const float* __restrict__ val,
-                                   Threshold th, uint8_t* keep, float* valx, long long* rowlen,
-                                   unsigned long long* band) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x >> 5);
+// Keep and exact flags, a bit per entry: row i's words start at
+// (rp[i] >> 5) + i, which leaves every row words of its own.
+__host__ __device__ __forceinline__ long long rethr_word(long long b, int i) { return (b >> 5) + i; }
+
+constexpr int kRethrWarps = 8;
+
+// Warp per row: keep flag of every entry, the exact value of those it was
+// recomputed for, the row's kept count.  128 entries in flight at a time; those
+// near a decision wait in shared memory and are recomputed four at a time.
+// Bound: reading the values and, at a wide delta, the recomputed pairs (23,000
+// voxels, TF32, 18.6 M entries: 454, 283 and 204 us for three thresholds with a
+// warp per pair, a byte flag and a copied value per entry; 332, 197 and 139 now.
+// Taking the values below the diagonal from their mirror images, by a search in
+// the other row, cost what it saved: 327, 229 and 179).
+__global__ __launch_bounds__(kRethrWarps * 32) void rethr_count_kernel(
+    CorrArgs a, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+    const float* __restrict__ val, Threshold th, uint32_t* keep, uint32_t* exact, float* valx,
+    long long* rowlen, unsigned long long* band) {
+  __shared__ int list[kRethrWarps][160];  // entries to recompute (offsets in the row)
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t below = (1u << lane) - 1u;
+  const int nw = gridDim.x * kRethrWarps;
   const bool absm = th.mode == BNA_THR_ABS_GT || th.mode == BNA_THR_ABS_GE;
   const float lim = 1.0f - th.delta;
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < a.n; i += nw) {
-    const long long b = rp[i], e = rp[i + 1];
-    long long kept = 0;
-    for (long long e0 = b; e0 < e; e0 += 32) {
-      const long long k = e0 + lane;
-      const bool in = k < e;
-      float v = in ? val[k] : 0.0f;
-      const float x = absm ? fabsf(v) : v;
-      const bool need = in && (fabsf(x - th.tau) <= th.delta || fabsf(v) >= lim);
-      bool kp = in && !need && edge_exact(v, th);
-      uint32_t m = __ballot_sync(0xffffffffu, need);
-      while (m) {  // exact values, one pair per warp pass
-        const int l = __ffs(m) - 1;
-        m &= m - 1;
-        const int j = __shfl_sync(0xffffffffu, in ? ci[k] : 0, l);
-        const float r = exact_r_warp(a, i < j ? i : j, i < j ? j : i, lane);
-        if (lane == l) {
-          v = r;
-          kp = edge_exact(r, th);
-          if (fabsf((absm ? fabsf(r) : r) - th.tau) <= 1e-6f) atomicAdd(band, 1ull);
+  unsigned int n_1e6 = 0;
+  for (int i = blockIdx.x * kRethrWarps + w; i < a.n; i += nw) {
+    const long long b = rp[i];
+    const int len = (int)(rp[i + 1] - b);
+    const long long wb = rethr_word(b, i);
+    int kept = 0, held = 0;
+    auto recompute = [&](int cnt) {  // the first cnt entries of the list
+      __syncwarp();
+      for (int t = 0; t < cnt; t += kPairs) {
+        const int g = t + lane / kPairLanes;
+        const bool on = g < cnt;
+        const int off = on ? list[w][g] : 0;
+        const int j = on ? ci[b + off] : 0;
+        const float r = post_block(exact_r_pairs_raw(a, on, min(i, j), max(i, j), lane));
+        const bool lead = on && (lane & (kPairLanes - 1)) == 0;
+        const bool kp = lead && edge_exact(r, th);
+        if (lead) {
+          valx[b + off] = r;
+          if (fabsf((absm ? fabsf(r) : r) - th.tau) <= 1e-6f) ++n_1e6;
         }
+        if (kp) atomicOr(&keep[wb + (off >> 5)], 1u << (off & 31));
+        kept += __popc(__ballot_sync(0xffffffffu, kp));
       }
-      if (in) {
-        keep[k] = kp ? 1 : 0;
-        valx[k] = v;
+      __syncwarp();
+    };
+    for (int e0 = 0; e0 < len; e0 += 128) {
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = e0 + 32 * u + lane;
+        v[u] = e < len ? __ldg(val + b + e) : 0.0f;
       }
-      kept += __popc(__ballot_sync(0xffffffffu, kp));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = e0 + 32 * u + lane;
+        const bool in = e < len;
+        const float x = absm ? fabsf(v[u]) : v[u];
+        const bool need = in && (fabsf(x - th.tau) <= th.delta || fabsf(v[u]) >= lim);
+        const uint32_t mn = __ballot_sync(0xffffffffu, need);
+        const uint32_t mk = __ballot_sync(0xffffffffu, in && !need && edge_exact(v[u], th));
+        if (lane == 0 && e < len) {
+          keep[wb + (e >> 5)] = mk;
+          exact[wb + (e >> 5)] = mn;
+        }
+        kept += __popc(mk);
+        if (need) list[w][held + __popc(mn & below)] = e;
+        held += __popc(mn);
+      }
+      if (held >= 32) {
+        const int full = held & ~(kPairs - 1);
+        recompute(full);
+        if (lane < held - full) list[w][lane] = list[w][full + lane];
+        held -= full;
+        __syncwarp();
+      }
     }
+    recompute(held);
     if (lane == 0) rowlen[i] = kept;
   }
+  n_1e6 = __reduce_add_sync(0xffffffffu, n_1e6);
+  if (lane == 0 && n_1e6) atomicAdd(band, (unsigned long long)n_1e6);
 }
 
-// Warp per row: copy the kept entries in order.
-__global__ void rethr_fill_kernel(int n, const int32_t* __restrict__ rp,
-                                  const int32_t* __restrict__ ci, const float* __restrict__ valx,
-                                  const uint8_t* __restrict__ keep, const int32_t* __restrict__ rp2,
-                                  int32_t* ci2, float* val2, long long nnz2, uint32_t* err) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
-    const long long b = rp[i], e = rp[i + 1];
+// Warp per row: copy the kept entries in order.  A lane holds one of 32 flag
+// words, whose prefix counts give every word's place, so that the copies of
+// different words are independent.
+__global__ __launch_bounds__(kRethrWarps * 32) void rethr_fill_kernel(
+    int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+    const float* __restrict__ val, const float* __restrict__ valx,
+    const uint32_t* __restrict__ keep, const uint32_t* __restrict__ exact,
+    const int32_t* __restrict__ rp2, int32_t* ci2, float* val2, long long nnz2, uint32_t* err) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t below = (1u << lane) - 1u;
+  const int nw = gridDim.x * kRethrWarps;
+  for (int i = blockIdx.x * kRethrWarps + w; i < n; i += nw) {
+    const long long b = rp[i];
+    const int words = (int)((rp[i + 1] - b + 31) >> 5);
+    const long long wb = rethr_word(b, i);
     long long pos = rp2[i];
-    for (long long e0 = b; e0 < e; e0 += 32) {
-      const long long k = e0 + lane;
-      const bool kp = k < e && keep[k];
-      const uint32_t m = __ballot_sync(0xffffffffu, kp);
-      if (kp) {
-        const long long p = pos + __popc(m & ((1u << lane) - 1u));
-        if (p < nnz2) {
-          ci2[p] = ci[k];
-          if (val2) val2[p] = valx[k];
-        } else {
-          atomicOr(err, ERR_RANGE);
+    for (int w0 = 0; w0 < words; w0 += 32) {
+      const bool in = w0 + lane < words;
+      const uint32_t kw = in ? keep[wb + w0 + lane] : 0u;
+      const uint32_t xw = in ? exact[wb + w0 + lane] : 0u;
+      int incl = __popc(kw);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const int before = incl - __popc(kw);
+      const int nwd = min(32, words - w0);
+      for (int q = 0; q < nwd; q += 4) {
+        int c[4];
+        float v[4];
+        long long to[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t m = __shfl_sync(0xffffffffu, kw, q + u);
+          const uint32_t x = __shfl_sync(0xffffffffu, xw, q + u);
+          to[u] = -1;
+          const int at = __shfl_sync(0xffffffffu, before, q + u) + __popc(m & below);
+          if ((m >> lane) & 1u) {
+            const long long k = b + (long long)(w0 + q + u) * 32 + lane;
+            c[u] = ci[k];
+            v[u] = ((x >> lane) & 1u) ? valx[k] : val[k];
+            to[u] = pos + at;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (to[u] < 0) continue;
+          if (to[u] < nnz2) {
+            ci2[to[u]] = c[u];
+            if (val2) val2[to[u]] = v[u];
+          } else {
+            atomicOr(err, ERR_RANGE);
+          }
         }
       }
-      pos += __popc(m);
+      pos += __shfl_sync(0xffffffffu, incl, 31);
     }
   }
 }
 
+// Words of the flags of one kind.
+size_t rethr_words(int n, long long nnz) { return (size_t)rethr_word(nnz, n) + 1; }
+
 cudaError_t launch_rethr_count(const CorrArgs& a, const int32_t* rp, const int32_t* ci,
-                               const float* val, const Threshold& th, uint8_t* keep, float* valx,
-                               long long* rowlen, unsigned long long* band, int sms,
-                               cudaStream_t st) {
-  rethr_count_kernel<<<sms * 8, 256, 0, st>>>(a, rp, ci, val, th, keep, valx, rowlen, band);
+                               const float* val, const Threshold& th, uint32_t* keep,
+                               uint32_t* exact, float* valx, long long* rowlen,
+                               unsigned long long* band, int sms, cudaStream_t st) {
+  rethr_count_kernel<<<sms * 8, kRethrWarps * 32, 0, st>>>(a, rp, ci, val, th, keep, exact, valx,
+                                                           rowlen, band);
   return cudaGetLastError();
 }
 
-cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* valx,
-                              const uint8_t* keep, const int32_t* rp2, int32_t* ci2, float* val2,
-                              long long nnz2, uint32_t* err, int sms, cudaStream_t st) {
-  rethr_fill_kernel<<<sms * 8, 256, 0, st>>>(n, rp, ci, valx, keep, rp2, ci2, val2, nnz2, err);
+cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* val,
+                              const float* valx, const uint32_t* keep, const uint32_t* exact,
+                              const int32_t* rp2, int32_t* ci2, float* val2, long long nnz2,
+                              uint32_t* err, int sms, cudaStream_t st) {
+  rethr_fill_kernel<<<sms * 8, kRethrWarps * 32, 0, st>>>(n, rp, ci, val, valx, keep, exact, rp2,
+                                                          ci2, val2, nnz2, err);
   return cudaGetLastError();
 }
 
