@@ -12,13 +12,12 @@
 // e1 <= eps or e2 <= eps (no host round trip per iteration); the host replays
 // a captured CUDA graph of 32 iterations and reads the flag between graphs.
 //
-// Normally the whole power iteration is one cooperative, persistent launch
-// (ec_coop_kernel): blocks meet at a grid barrier once per iteration and
-// every block then reduces the block partials in the same fixed order, so no
-// launch, tail or host round trip separates the iterations; graphs with many
-// iterations (a graph that never meets the stop test runs the reference's
-// 10,000) cost microseconds per iteration.  The per-iteration kernel above
-// remains for the no-allocation entry point.
+// Graphs of at most 16,384 vertices run the whole power iteration in one
+// cooperative, persistent launch (ec_coop_kernel): blocks meet at a grid barrier
+// once per iteration and every block then reduces the block partials in the same
+// fixed order, so no launch, tail or host round trip separates the iterations;
+// graphs with many iterations (a graph that never meets the stop test runs the
+// reference's 10,000) cost microseconds per iteration.
 //
 // The SpMV runs in float-float ("double-float") arithmetic instead of FP64,
 // whose rate on this GPU is ~1/70 of FP32: the iterate is kept twice, as
@@ -121,14 +120,13 @@ __global__ __launch_bounds__(kEcThreads) void ec_init_kernel(int n, double* u, f
 // One warp, one row: (sh, sl) += sum over entries [b, e) of val * x[col], eight
 // entries per lane in flight per round, the last round predicated with only the
 // arithmetic that it needs (so a row costs ceil((e - b) / 256) memory round
-// trips).  l2_only: read x through L2 only (the persistent kernel, whose iterate
-// other blocks rewrite in the same launch).
+// trips).
 template <int VK>
 __device__ __forceinline__ void ec_row_accum(const int32_t* __restrict__ ci,
                                              const float* __restrict__ val,
                                              const double* __restrict__ vald,
                                              const float2* uf, long long b, long long e,
-                                             int lane, float& sh, float& sl, bool l2_only) {
+                                             int lane, float& sh, float& sl) {
   if (e <= b) return;
   const int32_t* cp = ci + b + lane;
   const float* vp = VK == 1 ? val + b + lane : nullptr;
@@ -151,7 +149,7 @@ __device__ __forceinline__ void ec_row_accum(const int32_t* __restrict__ ci,
       }
     }
 #pragma unroll
-    for (int m = 0; m < 8; ++m) x[m] = l2_only ? __ldcg(uf + c[m]) : uf[c[m]];
+    for (int m = 0; m < 8; ++m) x[m] = uf[c[m]];
 #pragma unroll
     for (int m = 0; m < 8; ++m) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
     cp += 256;
@@ -177,82 +175,14 @@ __device__ __forceinline__ void ec_row_accum(const int32_t* __restrict__ ci,
     }
 #pragma unroll
     for (int m = 0; m < 8; ++m)
-      x[m] = c[m] < 0 ? make_float2(0.0f, 0.0f) : (l2_only ? __ldcg(uf + c[m]) : uf[c[m]]);
+      x[m] = c[m] < 0 ? make_float2(0.0f, 0.0f) : uf[c[m]];
 #pragma unroll
     for (int m = 0; m < 8; ++m)
-      if (l2_only || 32 * m < len) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
+      if (32 * m < len) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
   }
 }
 
-// Rounds per batch: round k of a block covers rows blockIdx.x * 8 + k * (all
-// warps) .. + 7, one per warp (the interleaving spreads dense row ranges over
-// every block); the batch's float-float row sums wait in shared memory for the
-// thread-per-row FP64 epilogue, one thread per row.
-constexpr int kEcRounds = kEcThreads / (kEcThreads / 32);
-
-// One iteration's work of this block: warp per row for the float-float sums,
-// then one thread per row for the FP64 epilogue (y = sum / lambda, the
-// iterate copies, the partial sums of y^2, (y - u)^2, (y + u)^2).  The FP64
-// pipe of this GPU is narrow and a warp instruction costs it the same with
-// one lane as with 32, so the FP64 work runs on full warps instead of on
-// lane 0 of every row's warp.
-template <int VK>
-__device__ __forceinline__ void ec_block_rows(int n, const int32_t* __restrict__ rp,
-                                              const int32_t* __restrict__ ci,
-                                              const float* __restrict__ val,
-                                              const double* __restrict__ vald, long long nnz_used,
-                                              const double* uc, const float2* ufc, double* un,
-                                              float2* unf, double inv, bool l2_only, double& a0,
-                                              double& a1, double& a2) {
-  constexpr int kW = kEcThreads / 32;
-  __shared__ float2 rs[kEcThreads];
-  __shared__ bool rempty[kEcThreads];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = gridDim.x * kW;
-  for (long long base = (long long)blockIdx.x * kW; base < n; base += (long long)kEcRounds * nw) {
-    for (int k = 0; k < kEcRounds; ++k) {
-      const long long row = base + (long long)k * nw + warp;
-      if (row >= n) break;  // later rounds of this warp are past n too
-      long long b = __ldg(rp + row), e = __ldg(rp + row + 1);
-      if (e > nnz_used) e = nnz_used;
-      float sh = 0.0f, sl = 0.0f;
-      ec_row_accum<VK>(ci, val, vald, ufc, b, e, lane, sh, sl, l2_only);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
-        const float ol = __shfl_xor_sync(0xffffffffu, sl, o);
-        float s2, e2;
-        two_sum(sh, oh, s2, e2);
-        sh = s2;
-        sl = __fadd_rn(sl, __fadd_rn(ol, e2));
-      }
-      if (lane == 0) {
-        rs[k * kW + warp] = make_float2(sh, sl);
-        rempty[k * kW + warp] = e <= b;
-      }
-    }
-    __syncthreads();
-    {
-      const int k = threadIdx.x / kW, w = threadIdx.x % kW;
-      const long long row = base + (long long)k * nw + w;
-      if (row < n) {
-        // y = A (u / lambda) as the reference orders it (weighted-net.cu:160-167):
-        // a row without entries gives 0 even when 1 / lambda is infinite (an
-        // all-zero iterate), where sum * (1 / lambda) would give 0 * inf = NaN
-        const float2 sm = rs[threadIdx.x];
-        const double y = rempty[threadIdx.x] ? 0.0 : ((double)sm.x + (double)sm.y) * inv;
-        const double old = l2_only ? __ldcg(uc + row) : uc[row];
-        un[row] = y;
-        unf[row] = split_df(y);
-        a0 += y * y;
-        const double d = y - old, p = y + old;
-        a1 += d * d;
-        a2 += p * p;
-      }
-    }
-    __syncthreads();
-  }
-}
+constexpr int kEcRounds = kEcThreads / (kEcThreads / 32);  // rows of a block per batch and warp
 
 // The same iteration's work for a sparse graph (average degree <= 2, the
 // graphs whose centrality converges slowly or never): one thread per row
@@ -303,7 +233,7 @@ __device__ __forceinline__ void ec_block_rows_sparse(int n, const int32_t* __res
       const int src = __ffs(m) - 1;
       const long long wb = __shfl_sync(0xffffffffu, b, src), we = __shfl_sync(0xffffffffu, e, src);
       float wh = 0.0f, wl = 0.0f;
-      ec_row_accum<VK>(ci, val, vald, ufc, wb, we, lane, wh, wl, false);
+      ec_row_accum<VK>(ci, val, vald, ufc, wb, we, lane, wh, wl);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const float oh = __shfl_xor_sync(0xffffffffu, wh, o);
@@ -319,7 +249,7 @@ __device__ __forceinline__ void ec_block_rows_sparse(int n, const int32_t* __res
       }
     }
     if (row < n) {
-      // as ec_block_rows: a row without entries gives 0 (weighted-net.cu:160-167)
+      // as the persistent kernel: a row without entries gives 0 (weighted-net.cu:160-167)
       const double y = e <= b ? 0.0 : ((double)sh + (double)sl) * inv;
       const double old = uc[row];
       un[row] = y;
@@ -464,7 +394,7 @@ __global__ __launch_bounds__(kRangeThreads, 4 * kEcThreads / kRangeThreads) void
     claim();
     if (e > nnz_used) e = nnz_used;
     float sh = 0.0f, sl = 0.0f;
-    ec_row_accum<VK>(ci, val, vald, uf, b, e, lane, sh, sl, false);
+    ec_row_accum<VK>(ci, val, vald, uf, b, e, lane, sh, sl);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float oh = __shfl_xor_sync(0xffffffffu, sh, o);
@@ -529,32 +459,109 @@ cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const f
 }
 
 // ---- persistent form ----------------------------------------------------------
+//
+// The whole iteration in one cooperative launch of at most one block per SM.  An
+// iteration of a small graph is a chain of latencies, so: a warp sums four rows
+// side by side (their column and value loads hit L1 from the second iteration
+// on; the iterate, which other blocks rewrite, is read through L2); blocks meet at
+// one counter barrier; and the totals of the previous iteration (lambda, the stop
+// test) are taken from the block partials by three more warps of every block
+// while the row warps already gather, since only the epilogue needs them.  The
+// rows of an iteration that turns out to be past the stop are dropped.
+// Graphs of kCoopStageDeg entries per row copy the iterate into shared memory
+// each iteration (128 KB at most) and gather there instead of a sector of L2 per
+// entry (2,000, 12,000 and 16,000 vertices, 60 entries: 7.3, 10.1 and 10.6 us per
+// iteration against 7.6, 11.1 and 11.6; 20 entries: 6.7, 9.0 and 9.3 against 6.0,
+// 7.9 and 8.1).  Rows one at a time, with the last block to arrive reducing the
+// partials and publishing the totals, took 14.9 us on 2,000 vertices, 17.8, 20.2
+// and 29.7 on 12,000 of 20, 130 and 300 entries per row; 6.0, 7.9, 11.7 and 15.2
+// now.  Eight row warps: 15.0 us on 16,000 x 130, sixteen 12.2.
+constexpr int kCoopWarps = 16;                          // row warps
+constexpr int kCoopThreads = (kCoopWarps + 3) * 32;     // and one per total
+constexpr int kCoopRows = 4;                            // rows side by side
+constexpr int kCoopSlots = 32;                          // most rows per warp
+constexpr long long kCoopStageDeg = 50;                 // entries per row from which to stage
 
-// Grid barrier for a cooperative launch (all blocks co-resident).  Bounded:
-// a wait longer than limit_ns gives up and returns false.
-__device__ __forceinline__ bool grid_barrier(EcState* st, uint64_t limit_ns) {
+// (sh, sl)[r] = sum of val * x over the len[r] entries from b[r]; STAGE: x in
+// shared memory.
+template <int VK, bool STAGE>
+__device__ __forceinline__ void coop_rows(const int32_t* __restrict__ ci,
+                                          const float* __restrict__ val,
+                                          const double* __restrict__ vald, const float2* uf,
+                                          const int (&b)[kCoopRows], const int (&len)[kCoopRows],
+                                          int lane, float (&sh)[kCoopRows], float (&sl)[kCoopRows]) {
+  int most = 0;
+#pragma unroll
+  for (int r = 0; r < kCoopRows; ++r) {
+    sh[r] = sl[r] = 0.0f;
+    most = max(most, len[r]);
+  }
+  for (int k0 = 0; k0 < most; k0 += 64) {
+    int c[kCoopRows][2];
+    float vh[kCoopRows][2], vl[kCoopRows][2];
+    float2 x[kCoopRows][2];
+#pragma unroll
+    for (int r = 0; r < kCoopRows; ++r)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int k = k0 + 32 * m + lane;
+        const bool ok = k < len[r];
+        c[r][m] = ok ? __ldg(ci + b[r] + k) : -1;
+        vh[r][m] = 1.0f;
+        vl[r][m] = 0.0f;
+        if (VK == 1) vh[r][m] = ok ? __ldg(val + b[r] + k) : 0.0f;
+        if (VK == 2) {
+          const float2 d = split_df(ok ? __ldg(vald + b[r] + k) : 0.0);
+          vh[r][m] = d.x;
+          vl[r][m] = d.y;
+        }
+      }
+#pragma unroll
+    for (int r = 0; r < kCoopRows; ++r)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        x[r][m] = c[r][m] < 0 ? make_float2(0.0f, 0.0f)
+                              : STAGE ? uf[c[r][m]] : __ldcg(uf + c[r][m]);
+#pragma unroll
+    for (int r = 0; r < kCoopRows; ++r)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) df_accum<VK>(sh[r], sl[r], vh[r][m], vl[r][m], x[r][m]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int r = 0; r < kCoopRows; ++r) {
+      const float oh = __shfl_xor_sync(0xffffffffu, sh[r], o);
+      const float ol = __shfl_xor_sync(0xffffffffu, sl[r], o);
+      float s2, e2;
+      two_sum(sh[r], oh, s2, e2);
+      sh[r] = s2;
+      sl[r] = __fadd_rn(sl[r], __fadd_rn(ol, e2));
+    }
+  }
+}
+
+// Barrier of the cooperative grid: `round` barriers have gone before since the
+// counter was zeroed.  Bounded: a wait longer than limit_ns gives up, flags the
+// state and returns false (every block's wait then runs out).
+__device__ __forceinline__ bool grid_barrier(EcState* st, unsigned int round, uint64_t limit_ns) {
   __shared__ int ok_s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned int* gen = &st->bar_gen;
-    const unsigned int g = *gen;  // the generation cannot advance before this block arrives
+    const unsigned int target = (round + 1) * gridDim.x;
+    volatile unsigned int* count = &st->bar_count;
     __threadfence();
+    atomicAdd(&st->bar_count, 1u);
     int ok = 1;
-    if (atomicAdd(&st->bar_count, 1u) == gridDim.x - 1) {
-      st->bar_count = 0;
-      __threadfence();
-      atomicAdd(&st->bar_gen, 1u);
-    } else {
-      uint64_t t0;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-      while (*gen == g) {
-        uint64_t t1;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-        if (t1 - t0 > limit_ns) {
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
+    uint64_t t0;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    while ((int)(*count - target) < 0) {
+      uint64_t t1;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+      if (t1 - t0 > limit_ns) {
+        ok = 0;
+        atomicOr(&st->err, 1);
+        break;
       }
     }
     __threadfence();
@@ -564,114 +571,114 @@ __device__ __forceinline__ bool grid_barrier(EcState* st, uint64_t limit_ns) {
   return ok_s != 0;
 }
 
-// Grid barrier of the persistent kernel that also reduces the iteration's
-// block partials pp (grid x 3): the last block to arrive sums them in a fixed
-// order (thread-strided sums, then a shared-memory tree: the order of the
-// per-iteration kernel's reduce_partials), publishes lam2, e1, e2 and the next
-// iteration's lambda and 1/lambda in st->tot, and releases the others — each
-// partial is read once, not once per block.  Bounded like grid_barrier.
-__device__ __forceinline__ bool grid_sync_reduce(EcState* st, const double* pp,
-                                                 uint64_t limit_ns) {
-  __shared__ int last_s, ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned int* gen = &st->bar_gen;
-    const unsigned int g = *gen;  // the generation cannot advance before this block arrives
-    __threadfence();
-    const bool last = atomicAdd(&st->bar_count, 1u) == gridDim.x - 1;
-    last_s = last ? 1 : 0;
-    ok_s = 1;
-    if (!last) {
-      uint64_t t0;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-      while (*gen == g) {
-        uint64_t t1;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-        if (t1 - t0 > limit_ns) {
-          ok_s = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  if (last_s) {
-    __shared__ double red[kEcThreads][3];
-    double s0 = 0, s1 = 0, s2 = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-      s0 += __ldcg(pp + b * 3 + 0);
-      s1 += __ldcg(pp + b * 3 + 1);
-      s2 += __ldcg(pp + b * 3 + 2);
-    }
-    red[threadIdx.x][0] = s0;
-    red[threadIdx.x][1] = s1;
-    red[threadIdx.x][2] = s2;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) {
-        red[threadIdx.x][0] += red[threadIdx.x + w][0];
-        red[threadIdx.x][1] += red[threadIdx.x + w][1];
-        red[threadIdx.x][2] += red[threadIdx.x + w][2];
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const double r0 = red[0][0], inv = rsqrt(r0);
-      st->tot[0] = r0;
-      st->tot[1] = sqrt(red[0][1]);
-      st->tot[2] = sqrt(red[0][2]);
-      st->tot[3] = r0 == 0.0 ? 0.0 : r0 * inv;
-      st->tot[4] = inv;
-      st->bar_count = 0;
-      __threadfence();
-      atomicAdd(&st->bar_gen, 1u);
-    }
-    __syncthreads();
-    return true;
-  }
-  if (!ok_s && threadIdx.x == 0) atomicOr(&st->err, 1);
-  return ok_s != 0;
-}
-
-template <int VK>
-__global__ __launch_bounds__(kEcThreads, 4) void ec_coop_kernel(
+template <int VK, bool STAGE>
+__global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
     int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, const double* __restrict__ vald, long long nnz_used,
     double* u, float2* uf, double* parts, EcState* st, int it_end, int max_iter, double eps) {
+  extern __shared__ float2 xs[];  // STAGE: the iterate
+  __shared__ float2 rs[kCoopSlots * kCoopWarps];
+  __shared__ bool rempty[kCoopSlots * kCoopWarps];
+  __shared__ double tot_s[5];  // lam2, e1, e2, lambda, 1 / lambda
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = gridDim.x * kCoopWarps;
+  // slot s of warp w: row blockIdx * kCoopWarps + w + s nw (dense row ranges
+  // spread over the blocks); lane s keeps its entries' start and number
+  const int first = blockIdx.x * kCoopWarps + warp;
+  const int slots = (n + nw - 1) / nw;  // at most kCoopSlots (ec_coop_grid)
+  int rb = 0, rl = 0;
+  if (warp < kCoopWarps && lane < slots && first + lane * nw < n) {
+    rb = rp[first + lane * nw];
+    rl = max(0, (int)(min((long long)rp[first + lane * nw + 1], nnz_used) - rb));
+  }
   // resume from the state block (ec_init_kernel's, or the previous segment's)
   double lam2 = st->lam2, lam_used = st->lambda_used, e1 = st->e1, e2 = st->e2;
-  int it = st->iter;
+  const int it0 = st->iter;
+  int it = it0;
   if (st->done) it_end = it;
   if (it_end > max_iter) it_end = max_iter;
-  // lambda and its reciprocal for the first iteration (FP64 sqrt and division
-  // are long instruction sequences on this GPU: one thread computes them)
-  __shared__ double lam_s[2];
-  if (threadIdx.x == 0) {
-    lam_s[1] = rsqrt(lam2);
-    lam_s[0] = lam2 == 0.0 ? 0.0 : lam2 * lam_s[1];
+  if (threadIdx.x == 0) {  // FP64 roots are long instruction sequences: one thread's
+    const double inv = rsqrt(lam2);
+    tot_s[0] = lam2;
+    tot_s[1] = e1;
+    tot_s[2] = e2;
+    tot_s[3] = lam2 == 0.0 ? 0.0 : lam2 * inv;
+    tot_s[4] = inv;
   }
-  __syncthreads();
-  double lam = lam_s[0], inv = lam_s[1];
-  while (it < it_end) {
+  double lam = 0.0;
+  for (;; ++it) {
     const size_t cur = (size_t)(it & 1) * n, nxt = (size_t)((it + 1) & 1) * n;
-    // the iterate was written by other blocks: read it from L2 (__ldcg), not L1
+    if (STAGE && it < it_end) {
+#pragma unroll 8
+      for (int k = threadIdx.x; k < n; k += kCoopThreads) xs[k] = __ldcg(uf + cur + k);
+      __syncthreads();
+    }
+    if (warp < kCoopWarps) {
+      if (it < it_end) {
+        for (int s = 0; s < slots; s += kCoopRows) {
+          int b[kCoopRows], len[kCoopRows];
+          float sh[kCoopRows], sl[kCoopRows];
+#pragma unroll
+          for (int r = 0; r < kCoopRows; ++r) {
+            b[r] = __shfl_sync(0xffffffffu, rb, (s + r) & 31);
+            len[r] = s + r < slots ? __shfl_sync(0xffffffffu, rl, (s + r) & 31) : 0;
+          }
+          coop_rows<VK, STAGE>(ci, val, vald, STAGE ? xs : uf + cur, b, len, lane, sh, sl);
+#pragma unroll
+          for (int r = 0; r < kCoopRows; ++r)
+            if (lane == r && s + r < slots) {
+              rs[(s + r) * kCoopWarps + warp] = make_float2(sh[r], sl[r]);
+              rempty[(s + r) * kCoopWarps + warp] = len[r] == 0;
+            }
+        }
+      }
+    } else if (it > it0) {
+      // total k of the previous iteration, in a fixed order
+      const int k = warp - kCoopWarps;
+      const double* pp = parts + (size_t)((it - 1) & 1) * gridDim.x * 3;
+      double t = 0.0;
+      for (int q = lane; q < (int)gridDim.x; q += 32) t += __ldcg(pp + q * 3 + k);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) {
+        if (k == 0) {
+          const double inv = rsqrt(t);
+          tot_s[0] = t;
+          tot_s[3] = t == 0.0 ? 0.0 : t * inv;  // sqrt(0) = 0, 1 / 0 = inf
+          tot_s[4] = inv;
+        } else {
+          tot_s[k] = sqrt(t);
+        }
+      }
+    }
+    __syncthreads();
+    lam_used = it > it0 ? lam : lam_used;
+    lam2 = tot_s[0];
+    e1 = tot_s[1];
+    e2 = tot_s[2];
+    lam = tot_s[3];
+    const double inv = tot_s[4];
+    if (it >= it_end || (it > it0 && (e1 <= eps || e2 <= eps))) break;
     double a0 = 0, a1 = 0, a2 = 0;
-    ec_block_rows<VK>(n, rp, ci, val, vald, nnz_used, u + cur, uf + cur, u + nxt, uf + nxt, inv,
-                      true, a0, a1, a2);
-    double* pp = parts + (size_t)(it & 1) * gridDim.x * 3;
-    ec_block_partials(a0, a1, a2, kEcThreads / 32, pp);
-    if (!grid_sync_reduce(st, pp, 2000000000ull)) return;
-    // the totals: published by the last block (L2 reads; the same bits everywhere)
-    lam_used = lam;
-    lam2 = __ldcg(&st->tot[0]);
-    e1 = __ldcg(&st->tot[1]);
-    e2 = __ldcg(&st->tot[2]);
-    lam = __ldcg(&st->tot[3]);
-    inv = __ldcg(&st->tot[4]);
-    ++it;
-    if (e1 <= eps || e2 <= eps) break;
+    const int row = blockIdx.x * kCoopWarps + (int)threadIdx.x % kCoopWarps +
+                    (int)threadIdx.x / kCoopWarps * nw;
+    if ((int)threadIdx.x < slots * kCoopWarps && row < n) {
+      // y = A (u / lambda) as the reference orders it (weighted-net.cu:160-167):
+      // a row without entries gives 0 even when 1 / lambda is infinite (an
+      // all-zero iterate), where sum * (1 / lambda) would give 0 * inf = NaN
+      const float2 sm = rs[threadIdx.x];
+      const double y = rempty[threadIdx.x] ? 0.0 : ((double)sm.x + (double)sm.y) * inv;
+      const double old = __ldcg(u + cur + row);
+      u[nxt + row] = y;
+      uf[nxt + row] = split_df(y);
+      a0 = y * y;
+      const double d = y - old, p = y + old;
+      a1 = d * d;
+      a2 = p * p;
+    }
+    ec_block_partials(a0, a1, a2, (slots * kCoopWarps + 31) / 32,
+                      parts + (size_t)(it & 1) * gridDim.x * 3);
+    if (!grid_barrier(st, (unsigned int)it, 2000000000ull)) return;
   }
   // every block has read the state above before the first grid barrier; with
   // no iteration run, block 0 writes back what it read
@@ -693,14 +700,18 @@ __global__ __launch_bounds__(kEcThreads, 4) void ec_coop_kernel(
 int ec_coop_grid(int n, int sms) {
   if (n > kEcCoopMaxN) return 0;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ec_coop_kernel<1>, kEcThreads, 0) !=
+  if (cudaFuncSetAttribute(ec_coop_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kEcCoopMaxN * sizeof(float2)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ec_coop_kernel<2, true>, kCoopThreads,
+                                                    kEcCoopMaxN * sizeof(float2)) !=
           cudaSuccess ||
       per_sm < 1) {
     cudaGetLastError();
     return 0;
   }
-  const int want = (n + 8 * (kEcThreads / 32) - 1) / (8 * (kEcThreads / 32));
-  return want < sms ? (want < 1 ? 1 : want) : sms;
+  const int want = (n + 63) / 64;
+  const int grid = want < sms ? want : sms;
+  return (long long)grid * kCoopWarps * kCoopSlots >= n ? grid : 0;
 }
 
 // The power iteration from the state block's iteration up to it_end (the
@@ -712,10 +723,20 @@ cudaError_t launch_ec_coop(int n, const int32_t* rp, const int32_t* ci, const fl
   EcState* s = (EcState*)st;
   void* args[] = {&n,     &rp, &ci, &val, &vald,   &nnz_used, &u,
                   &uf,    &parts, &s, &it_end, &max_iter, &eps};
-  const void* fn = val    ? (const void*)ec_coop_kernel<1>
-                   : vald ? (const void*)ec_coop_kernel<2>
-                          : (const void*)ec_coop_kernel<0>;
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kEcThreads), args, 0, stream);
+  const bool stage = nnz_used >= kCoopStageDeg * (long long)n;
+  const void* fn = val    ? (stage ? (const void*)ec_coop_kernel<1, true>
+                                   : (const void*)ec_coop_kernel<1, false>)
+                   : vald ? (stage ? (const void*)ec_coop_kernel<2, true>
+                                   : (const void*)ec_coop_kernel<2, false>)
+                          : (stage ? (const void*)ec_coop_kernel<0, true>
+                                   : (const void*)ec_coop_kernel<0, false>);
+  const size_t smem = stage ? (size_t)n * sizeof(float2) : 0;
+  if (stage) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kEcCoopMaxN * sizeof(float2)));
+    if (e != cudaSuccess) return e;
+  }
+  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kCoopThreads), args, smem, stream);
 }
 
 size_t ec_state_bytes() { return sizeof(EcState); }

@@ -13,9 +13,7 @@ struct EcState {
   int done;
   unsigned int counter;
   int err;                // bounded grid barrier expired (persistent kernel)
-  unsigned int bar_count, bar_gen;  // grid barrier of the persistent kernel
-  double tot[5];          // persistent kernel: lam2, e1, e2, lambda, 1/lambda published by
-                          // the last block to reach the barrier
+  unsigned int bar_count;  // arrivals at the persistent kernel's barrier, all iterations
 };
 
 // (hi, lo) float pair of a double: hi = RN(x), lo = RN(x - hi).

@@ -88,3 +88,42 @@ def test_centrality_of_sparse_rows(builder, n, deg):
     ec, lam, it, conv = builder.ec(csr, max_iter=60)
     assert it == it_o and conv == conv_o
     assert np.max(np.abs(ec.cpu().numpy() - want)) <= 1e-9 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n,deg", [(2, 1), (65, 20), (65, 60), (2433, 49), (2433, 51), (9729, 70),
+                                   (16384, 30), (16384, 60)])
+def test_persistent_kernel(builder, n, deg):
+    """Either side of the row length from which the iterate is staged in shared
+    memory, one block and all of them, rows that do not fill a group of four; a
+    run cut into segments of 7 iterations gives the same bits."""
+    import torch
+    rng = np.random.default_rng(n + deg)
+    offs = rng.choice(n, deg, replace=False)
+    C = np.sort((np.arange(n)[:, None] + offs[None, :]) % n, axis=1).astype(np.int32)
+    keep = rng.random(n) > 0.05  # some rows are empty
+    keep[0] = True
+    lens = np.where(keep, deg, 0)
+    R = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    C = np.ascontiguousarray(C[keep].ravel())
+    V = rng.uniform(0.05, 1.0, len(C)).astype(np.float32)
+    d = lambda a: torch.from_numpy(a).cuda()
+    for vals in (V, None):
+        want, lam_o, it_o, conv_o = oracle.ec(R, C, None if vals is None else vals.astype(np.float64),
+                                              max_iter=40)
+        csr = bna.CsrResult(n, len(C), d(R), d(C), None if vals is None else d(vals), {})
+        ec, lam, it, conv = builder.ec(csr, max_iter=40)
+        ec = ec.cpu().numpy()
+        assert it == it_o and conv == conv_o
+        assert np.max(np.abs(ec - want)) <= 1e-9 * np.max(np.abs(want))
+        assert abs(lam - lam_o) <= 1e-9 * abs(lam_o)
+        builder.set_option("ec_iters_per_launch", 7)
+        try:
+            cut = builder.ec(csr, max_iter=40)
+        finally:
+            builder.set_option("ec_iters_per_launch", 0)
+        assert np.array_equal(cut[0].cpu().numpy(), ec) and cut[1:] == (lam, it, conv)
+    Vd = V.astype(np.float64) * (1.0 + 2.0 ** -30)
+    want, lam_o, it_o, conv_o = oracle.ec(R, C, Vd)
+    ec, lam, it, conv = builder.lead_vector(R, C, Vd)
+    assert abs(it - it_o) <= 1 and conv == conv_o
+    assert np.max(np.abs(ec - want)) <= 1e-5 * np.max(np.abs(want))
