@@ -12,7 +12,7 @@
 // e1 <= eps or e2 <= eps (no host round trip per iteration); the host replays
 // a captured CUDA graph of 32 iterations and reads the flag between graphs.
 //
-// Graphs of at most 16,384 vertices run the whole power iteration in one
+// Graphs of at most 24,576 vertices run the whole power iteration in one
 // cooperative, persistent launch (ec_coop_kernel): blocks meet at a grid barrier
 // once per iteration and every block then reduces the block partials in the same
 // fixed order, so no launch, tail or host round trip separates the iterations;
@@ -469,7 +469,7 @@ cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const f
 // while the row warps already gather, since only the epilogue needs them.  The
 // rows of an iteration that turns out to be past the stop are dropped.
 // Graphs of kCoopStageDeg entries per row copy the iterate into shared memory
-// each iteration (128 KB at most) and gather there instead of a sector of L2 per
+// each iteration (192 KB at most) and gather there instead of a sector of L2 per
 // entry (2,000, 12,000 and 16,000 vertices, 60 entries: 7.3, 10.1 and 10.6 us per
 // iteration against 7.6, 11.1 and 11.6; 20 entries: 6.7, 9.0 and 9.3 against 6.0,
 // 7.9 and 8.1).  Rows one at a time, with the last block to arrive reducing the
@@ -695,8 +695,9 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
 // The persistent kernel serves small graphs only (n <= kEcCoopMaxN), with at
 // most one block per SM, so a long iteration (a graph that never meets the
 // stop test runs 10,000 of them) occupies a small share of the GPU.  Larger
-// graphs use per-iteration launches: their gathers then hit in L1, which the
-// persistent kernel must bypass.  Returns 0 for "use per-iteration launches".
+// graphs use per-iteration launches: their iterate does not fit beside the block.
+// 20,000 vertices of 4, 60 and 300 entries per row: 17.6, 19.7 and 23.0 us per
+// iteration in launches, 9.0, 12.6 and 20.3 here.  Returns 0 for "use per-iteration launches".
 int ec_coop_grid(int n, int sms) {
   if (n > kEcCoopMaxN) return 0;
   int per_sm = 0;

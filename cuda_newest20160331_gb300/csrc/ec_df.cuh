@@ -48,7 +48,7 @@ __device__ __forceinline__ void df_accum(float& sh, float& sl, float vh, float v
   sl = __fadd_rn(sl, __fadd_rn(e, pe));
 }
 
-constexpr int kEcCoopMaxN = 16384;  // largest graph of the persistent kernel (ec.cu)
+constexpr int kEcCoopMaxN = 24576;  // largest graph of the persistent kernel (ec.cu): 192 KB
 
 // Entries a row costs beside its own where rows are dealt out by entries
 // (ec_range_kernel: 120,000 vertices in contiguous networks, 645 entries per

@@ -68,9 +68,9 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
 // iterations' traffic, so it takes calls of at least kFlowMinIters allowed
 // iterations, on graphs whose rows have ascending columns, of up to
 // kFlowChunkMax chunks with at least kFlowMinDeg entries per row and chunk on
-// average (a block stages every chunk and walks every row in it: one chunk,
-// 20,000 vertices, 60 and 100 entries per row: 19.6 and 20.0 us against 19.4 and
-// 22.4 ranged; two, 45,000, 100 and 150: 37.2 and 38.5 against 31.7 and 40.8;
+// average (a block stages every chunk and walks every row in it: two chunks,
+// 45,000 vertices, 100 and 150 entries per row: 37.2 and 38.5 us against 31.7 and 40.8
+// ranged;
 // four, 90,000, 200 and 300: 99 and 104 against 85 and 113), whose gathers fall in a sector of their own for at
 // least kFlowFresh of the entries (45,000 vertices, 98 % such entries: 93 us
 // per iteration with a warp per row, 56 streamed; 120,000 in contiguous

@@ -1,5 +1,5 @@
-"""Centrality of graphs above the persistent kernel's size against the FP64
-oracle, at the sizes where the per-iteration kernels change: the streamed form
+"""Centrality against the FP64 oracle at the sizes where the kernels change: the
+persistent kernel takes up to 24,576 vertices; the streamed form
 holds the iterate 24,576 columns at a time (up to four times) and gives every
 warp a range of rows; the ranged form gives every block one.  Empty rows, rows
 joined to everything, an odd number of entries and unsorted columns are in it."""
@@ -91,7 +91,7 @@ def test_centrality_of_sparse_rows(builder, n, deg):
 
 
 @pytest.mark.parametrize("n,deg", [(2, 1), (65, 20), (65, 60), (2433, 49), (2433, 51), (9729, 70),
-                                   (16384, 30), (16384, 60)])
+                                   (16384, 30), (16384, 60), (24576, 49), (24576, 51)])
 def test_persistent_kernel(builder, n, deg):
     """Either side of the row length from which the iterate is staged in shared
     memory, one block and all of them, rows that do not fill a group of four; a
