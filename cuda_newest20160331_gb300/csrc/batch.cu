@@ -14,6 +14,7 @@ struct BatchSubj {
   double delta = 0, winA = 0, winB = 0;
   long long k_dens = 0;
   bool sampled = false;
+  float cut = -2.0f;  // density histogram: lowest value with a bin
   bool fallback = false;
   DevStatus* ds = nullptr;
   long long *rowlen = nullptr, *pre = nullptr, *bsum = nullptr;
@@ -27,6 +28,28 @@ struct BatchSubj {
   unsigned long long* dties = nullptr;
   long long nnz = 0;
 };
+
+// Density histogram pass of one subject (hist_all: a bin for every value).
+int32_t batch_hist(bna_ctx* ctx, BatchSubj& b, int prec, bool hist_all, unsigned int* hist_host,
+                   cudaStream_t st) {
+  CorrArgs& a = b.a;
+  unsigned int* hist;
+  ENSURE(S_HIST, (kHistBins + 1) * sizeof(unsigned int), hist);
+  CK(cudaMemsetAsync(hist, 0, (kHistBins + 1) * sizeof(unsigned int), st));
+  a.hist = hist;
+  a.th.mode = BNA_THR_R_GE;
+  a.th.delta = (float)b.delta;
+  b.sampled = ctx->ntiles >= 4 * kSampleTiles;
+  b.cut = hist_all ? -2.0f
+                   : hist_cut_for(b.k_dens, b.sampled, b.N,
+                                  b.sampled ? ctx->ntiles_smp : ctx->ntiles, b.T);
+  a.th.tau = b.cut;
+  int32_t s = corr_pass(ctx, a, prec, 3, st, b.sampled);
+  if (s) return s;
+  CK(cudaMemcpyAsync(hist_host, hist, (kHistBins + 1) * sizeof(unsigned int),
+                     cudaMemcpyDeviceToHost, st));
+  return BNA_OK;
+}
 
 // z-scores, buffers and (density) the histogram pass of one subject.
 int32_t batch_prep(bna_ctx* ctx, BatchSubj& b, const float* bold, const bna_corr_opts* opts,
@@ -66,18 +89,7 @@ int32_t batch_prep(bna_ctx* ctx, BatchSubj& b, const float* bold, const bna_corr
     a.th.tau = 2.0f;
     a.th.delta = (float)b.delta;
   } else {
-    unsigned int* hist;
-    ENSURE(S_HIST, (kHistBins + 1) * sizeof(unsigned int), hist);
-    CK(cudaMemsetAsync(hist, 0, (kHistBins + 1) * sizeof(unsigned int), st));
-    a.hist = hist;
-    a.th.mode = BNA_THR_R_GE;
-    a.th.tau = 0.0f;
-    a.th.delta = (float)b.delta;
-    b.sampled = ctx->ntiles >= 4 * kSampleTiles;
-    s = corr_pass(ctx, a, prec, 3, st, b.sampled);
-    if (s) return s;
-    CK(cudaMemcpyAsync(hist_host, hist, (kHistBins + 1) * sizeof(unsigned int),
-                       cudaMemcpyDeviceToHost, st));
+    return batch_hist(ctx, b, prec, false, hist_host, st);
   }
   return BNA_OK;
 }
@@ -219,10 +231,17 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
     if (s) return fail(ctx, s, "subject %d: %s", k, ctx->kids[k]->last_error.c_str());
   }
   CK(cudaStreamSynchronize(st));
-  for (int k = 0; k < nsub; ++k)
-    if (density && bs[k].k_dens > 0)
-      window_from_hist(ctx->hist_host + hbins * k, bs[k].k_dens, bs[k].sampled, N[k],
-                       bs[k].delta, &bs[k].winA, &bs[k].winB, &bs[k].a.th);
+  for (int k = 0; k < nsub; ++k) {
+    BatchSubj& b = bs[k];
+    if (!density || b.k_dens == 0) continue;
+    unsigned int* hh = ctx->hist_host + hbins * k;
+    while (!window_from_hist(hh, b.k_dens, b.sampled, N[k], b.delta, b.cut, &b.winA, &b.winB,
+                             &b.a.th)) {  // below the cut: again with every value
+      s = batch_hist(ctx->kids[k], b, prec, true, hh, st);
+      if (s) return fail(ctx, s, "subject %d: %s", k, ctx->kids[k]->last_error.c_str());
+      CK(cudaStreamSynchronize(st));
+    }
+  }
   // ---- one persistent count pass over the tiles of every subject
   const bool dev_sel = density;
   std::vector<char> table((size_t)nsub * tc_subj_bytes());

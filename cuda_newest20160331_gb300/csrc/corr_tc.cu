@@ -77,7 +77,7 @@ struct TcSmem {
   uint32_t tmem_base;
   volatile uint32_t abort;
   uint32_t colmask[2][128][4];
-  unsigned int hist[kHistBins + 1];  // density histogram pass
+  unsigned int hist[kHistBins + 1 + 32];  // density histogram pass; what is left out, by lane
   CorrArgs eargs[8];                 // each epilogue warp's current subject's arguments
 };
 
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     ptx::fence_mbar_init();
   }
   if (PASS == 3)
-    for (int b = threadIdx.x; b <= kHistBins; b += blockDim.x) S.hist[b] = 0u;
+    for (int b = threadIdx.x; b <= kHistBins + 32; b += blockDim.x) S.hist[b] = 0u;
   if (warp == 1) {
     ptx::tmem_alloc(ptx::smem_u32(&S.tmem_base), TC_TMEM_COLS);
     ptx::tmem_relinquish();
@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     float tau = 0, delta = 0, lim = 0, lo_thr = 0;
     float zlo = 0;  // AVG: an average Fisher z below it is no edge and no candidate
     bool simple = false, zero_int = false;
+    unsigned int hist_n = 0;  // density histogram: this lane's values
     uint32_t hphase = 0;
     // this warp's current edge-list chunk [wcur, wend), carried from launch to
     // launch of a pass in a.wstate
@@ -533,18 +534,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             return;
           }
           if (PASS == 3) {
-            // density histogram of the approximate values (exact 0 for NaN voxels)
-            uint32_t badm3 = 0;
-            if (slow)
-              for (int k = 0; k < 32; ++k)
-                if (rowbad || (jb + k < s_npad && s_bad[jb + k])) badm3 |= 1u << k;
+            // density histogram of the approximate values (exact 0 for NaN voxels);
+            // values below tau are left out, bin 0 then holds the number of all
+            // (hist_cut).  What is left out goes to a counter of the lane's own:
+            // no branch per value, and no conflict (an atomic into the crowded
+            // bins for every value took three times a tile's products, a branch
+            // around it five times).
+            hist_n += __popc(valid);
+            if (valid != 0xffffffffu || slow) {
+#pragma unroll
+              for (int k = 0; k < 32; ++k) {
+                if (slow && (rowbad || (jb + k < s_npad && s_bad[jb + k]))) v[k] = 0u;
+                if (!((valid >> k) & 1u)) v[k] = __float_as_uint(-3.0f);
+              }
+            }
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
-              if ((valid >> k) & 1u) {
-                const bool badk = (badm3 >> k) & 1u;
-                const float r = badk ? 0.0f : __uint_as_float(v[k]);
-                atomicAdd(&S.hist[(!badk && !(fabsf(r) < lim)) ? kHistBins : hist_bin(r)], 1u);
-              }
+              const float r = __uint_as_float(v[k]);
+              // floor((r + 1) kHistBins / 2), from the low bits of a float sum
+              const int b = (int)(__float_as_uint(__fmaf_rd(r, 0.5f * kHistBins,
+                                                            0.5f * kHistBins + 8388608.0f)) &
+                                  0x7FFFFFu);
+              const int at = fabsf(r) < lim ? b : kHistBins;
+              atomicAdd(&S.hist[r < tau ? kHistBins + 1 + lane : at], 1u);
             }
             return;
           }
@@ -788,6 +800,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
     }
     leave();
+    if (PASS == 3 && p.a.th.tau > -1.0f && hist_n) atomicAdd(&S.hist[0], hist_n);
   }
   ptx::tc_fence_before();
   __syncthreads();

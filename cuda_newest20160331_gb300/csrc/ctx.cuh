@@ -326,8 +326,9 @@ int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st);
 // The tile list alone, for nb blocks (kept until nb or the band changes).
 int32_t tc_tiles(bna_ctx* ctx, int nb, cudaStream_t st);
 long long elist_chunk(const bna_ctx* ctx, const CorrArgs& a);
-void window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, int N,
-                      double delta, double* winA, double* winB, Threshold* th);
+float hist_cut_for(long long k_dens, bool sampled, int N, int nt, int T);
+bool window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, int N, double delta,
+                      float cut, double* winA, double* winB, Threshold* th);
 // The caller's launch gate (bna_ctx_set_gate), if any.
 inline void gate(bna_ctx* ctx, cudaStream_t st, int phase, long long done) {
   if (ctx->gate) ctx->gate(ctx->gate_user, st, phase, done);
