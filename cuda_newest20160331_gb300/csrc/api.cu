@@ -164,8 +164,10 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
     e2 = static_cast<float*>(ctx->ptr[S_E2]);
     a.eblk = static_cast<float*>(ctx->ptr[S_EBLK]);
   }
-  CK(launch_zscore(bold, N, T, a.n_pad, z, a.ldz, zhi, zlo, a.ldb, bad, vstat, st, zq, a.ldq,
-                   e2));
+  uint8_t* bb;  // with the screen's operands launch_block_bad fills it (tc_prepare)
+  ENSURE(S_BLOCKBAD, (size_t)a.nb, bb);
+  CK(launch_zscore(bold, N, T, a.n_pad, z, a.ldz, zhi, zlo, a.ldb, bad, vstat, st, zq, a.ldq, e2,
+                   zq ? nullptr : bb));
   ctx->klaunch += 2;
   a.zq = zq;
   a.z = z;
@@ -175,14 +177,13 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
   return BNA_OK;
 }
 
-// Tensor-core preparation: per-block NaN flags and the upper-triangle tile list.
+// Tensor-core preparation: the screen's block bounds and the tile list.
 int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st) {
-  uint8_t* bb;
-  ENSURE(S_BLOCKBAD, (size_t)a.nb, bb);
-  CK(launch_block_bad(a.bad, a.nb, bb, st,
-                      a.zq ? static_cast<const float*>(ctx->ptr[S_E2]) : nullptr,
-                      const_cast<float*>(a.eblk)));
-  ctx->klaunch += 1;
+  if (a.zq) {
+    CK(launch_block_bad(a.bad, a.nb, static_cast<uint8_t*>(ctx->ptr[S_BLOCKBAD]), st,
+                        static_cast<const float*>(ctx->ptr[S_E2]), const_cast<float*>(a.eblk)));
+    ctx->klaunch += 1;
+  }
   return tc_tiles(ctx, a.nb, st);
 }
 
@@ -352,8 +353,9 @@ static int32_t screened_pass(bna_ctx* ctx, const CorrArgs& a, int precision, flo
 // sampled tile list, tensor-core forms)
 
 
+// sched: the launches' tile counters where the caller has zeroed them.
 int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cudaStream_t st,
-                  bool sampled) {
+                  bool sampled, unsigned int* sched) {
   switch (precision) {
     case BNA_PREC_FP32:
       CK(launch_corr_simt(a, pass, st));
@@ -364,9 +366,10 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
       const int2* tiles = reinterpret_cast<const int2*>(ctx->ptr[sampled ? S_TILES_SMP : S_TILES]);
       const int nt = sampled ? ctx->ntiles_smp : ctx->ntiles;
       const int per = ctx->tiles_per_launch > 0 ? ctx->tiles_per_launch : nt;
-      unsigned int* sched;
-      ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
-      CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
+      if (!sched) {
+        ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
+        CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
+      }
       if (pass == 0 && a.zq) {
         const float limit = screen_limit(a.th, default_delta(precision, a.T));
         if (screen_pays(ctx, a.nb, a.T, limit))
@@ -688,8 +691,12 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   ENSURE(S_BSUM, (size_t)4096 * 8, bsum);
   int32_t* row_ptr;
   ENSURE(S_ROWPTR, (size_t)(N + 1) * 4, row_ptr);
-  DevStatus* ds;
-  ENSURE(S_STATUS, sizeof(DevStatus), ds);
+  const int nwarps = ctx->sms * 8;  // epilogue warps of the tensor-core pass
+  const size_t state_bytes = kCountStateBytes + (size_t)nwarps * 2 * sizeof(long long);
+  CountState* cs;
+  ENSURE(S_STATUS, state_bytes, cs);
+  DevStatus* ds = &cs->ds;
+  a.wstate = reinterpret_cast<long long*>(reinterpret_cast<char*>(cs) + kCountStateBytes);
   a.err = &ds->err;
   a.cand_count = &ds->cand_count;
   a.stats = ds->stats;
@@ -699,6 +706,8 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   DevStatus* hs = reinterpret_cast<DevStatus*>(ctx->pinned);
   const long long nst = (long long)a.nb * (a.nb + 1) / 2;
   ENSURE(S_ETAB, (size_t)nst * 4 * sizeof(longlong2), a.etab);
+  int* dense_list;
+  ENSURE(S_DENSE, (size_t)nst * sizeof(int), dense_list);
   a.epool = &ds->epool;
 
   // ---- threshold of the count pass
@@ -766,16 +775,13 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
         ENSURE(S_CANDVAL, (size_t)a.cand_cap * sizeof(float), cvals);
       a.cand_apx = nullptr;
       if (dev_sel) ENSURE(S_CANDAPX, (size_t)a.cand_cap * sizeof(float), a.cand_apx);
-      CK(cudaMemsetAsync(ds, 0, sizeof(DevStatus), st));
-      const int nwarps = ctx->sms * 8;  // epilogue warps of the tensor-core pass
-      ENSURE(S_WSTATE, (size_t)nwarps * 2 * sizeof(long long), a.wstate);
-      CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 2 * sizeof(long long), st));
+      CK(cudaMemsetAsync(cs, 0, state_bytes, st));
       a.th = count_th;
-      s = corr_pass(ctx, a, prec, 0, st);
+      s = corr_pass(ctx, a, prec, 0, st, false, cs->sched);
       if (s) return s;
       ++passes;
       CK(cudaEventRecord(ctx->ev[2], st));
-      CK(launch_collect_candidates(a, ctx->sms, st));
+      CK(launch_collect_candidates(a, ctx->sms, dense_list, &ds->dense, st));
       ctx->klaunch += 1;
       if (dev_sel) {
         void* dstate;
@@ -794,7 +800,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
         CK(cudaMemsetAsync(dhist, 0, 2048 * sizeof(unsigned int), st));
         CK(launch_density_select(a, dstate, dhist, dcls, deidx, dexact, cvals, dties,
                                  dties + dens_ties_cap(), ctx->sms, st));
-        ctx->klaunch += 18 + 4;  // selection and decision, scan
+        ctx->klaunch += 18 + csr_scan_launches(N);  // selection and decision, scan
         CK(cudaEventRecord(ctx->ev[3], st));
         CK(launch_csr_scan(a.seg, a.nb, a.n_pad, N, rowlen, pre, bsum, &ds->total, row_ptr,
                            a.err, st));
@@ -815,7 +821,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
           ctx->klaunch += 1;
         }
         CK(launch_recompute(a, band_grid(ctx), st));
-        ctx->klaunch += 1 + 4;  // recompute, scan
+        ctx->klaunch += 1 + csr_scan_launches(N);  // recompute, scan
         CK(cudaEventRecord(ctx->ev[3], st));
         CK(launch_csr_scan(a.seg, a.nb, a.n_pad, N, rowlen, pre, bsum, &ds->total, row_ptr,
                            a.err, st));
@@ -912,7 +918,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     a.th.tau = tau_star;
     a.cand_val = cvals;
     CK(launch_recompute(a, band_grid(ctx), st));
-    ctx->klaunch += 1 + 4;  // decide, scan
+    ctx->klaunch += 1 + csr_scan_launches(N);  // decide, scan
     CK(cudaEventRecord(ctx->ev[3], st));
     CK(launch_csr_scan(a.seg, a.nb, a.n_pad, N, rowlen, pre, bsum, &ds->total, row_ptr, a.err,
                        st));
@@ -948,9 +954,8 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   a.col_idx = col;
   a.val = val;
   a.nnz = nnz;
-  int* dense_list;
-  ENSURE(S_DENSE, (size_t)nst * sizeof(int), dense_list);
-  int fill_launches = 3;
+  const unsigned int n_dense = hs->dense;
+  int fill_launches = n_dense ? 2 : 1;
   bna_ctx::Sink* sink = ctx->sink;
   if (sink && nnz <= sink->cap && (nnz == 0 || sink->col) && sink->row_ptr[N] == nnz) {
     // chunked fill, each chunk's entries copied out while the next fills
@@ -958,7 +963,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
       CK(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
       for (auto& e : ctx->chunk_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
-    CK(launch_csr_fill_dense(a, ctx->sms, dense_list, &ds->dense, st));
+    CK(launch_csr_fill_dense(a, ctx->sms, dense_list, n_dense, st));
     const int nch = std::min(kFillChunks, a.nb);
     for (int c = 0; c < nch; ++c) {
       const int I0 = (int)((long long)c * a.nb / nch), I1 = (int)((long long)(c + 1) * a.nb / nch);
@@ -978,19 +983,19 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     CK(cudaEventRecord(ctx->chunk_ev[nch], ctx->copy_stream));
     CK(cudaStreamWaitEvent(st, ctx->chunk_ev[nch], 0));
     sink->done = true;
-    fill_launches = 2 + nch;
+    fill_launches = (n_dense ? 1 : 0) + nch;
   } else if (ctx->gate) {
     // row-block chunks with the gate between them
-    CK(launch_csr_fill_dense(a, ctx->sms, dense_list, &ds->dense, st));
+    CK(launch_csr_fill_dense(a, ctx->sms, dense_list, n_dense, st));
     const int nch = std::min(kFillChunks, a.nb);
     for (int c = 0; c < nch; ++c) {
       if (c > 0) gate(ctx, st, BNA_PHASE_FILL, (long long)c * a.nb / nch);
       CK(launch_csr_fill_rows(a, ctx->sms, (int)((long long)c * a.nb / nch),
                               (int)((long long)(c + 1) * a.nb / nch), st));
     }
-    fill_launches = 2 + nch;
+    fill_launches = (n_dense ? 1 : 0) + nch;
   } else {
-    CK(launch_csr_fill(a, ctx->sms, dense_list, &ds->dense, st));
+    CK(launch_csr_fill(a, ctx->sms, dense_list, n_dense, st));
   }
   CK(cudaEventRecord(ctx->ev[5], st));
   CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
@@ -1129,9 +1134,7 @@ int32_t bna_corr_tile_values(bna_ctx* ctx, const float* bold_dev, int32_t N, int
     case BNA_PREC_FP32: CK(launch_corr_simt_dump(a, I, J, out_dev, st)); break;
     case BNA_PREC_BF16X3:
     case BNA_PREC_TF32: {
-      uint8_t* bb;
-      ENSURE(S_BLOCKBAD, (size_t)a.nb, bb);
-      CK(launch_block_bad(a.bad, a.nb, bb, st));
+      const uint8_t* bb = static_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]);
       int2* d;
       ENSURE(S_DUMPTILE, sizeof(int2), d);
       const int2 t = make_int2(I, J / 2);

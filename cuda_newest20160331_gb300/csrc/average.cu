@@ -50,9 +50,8 @@ static int32_t avg_subjects(bna_ctx* ctx, int32_t nsub, const float* const* bold
     uint8_t* bb = bballs + (size_t)k * nb;
     CK(launch_zscore(bold_dev[k], N, T[k], n_pad, const_cast<float*>(as.z), as.ldz,
                      const_cast<uint16_t*>(as.zhi), const_cast<uint16_t*>(as.zlo), as.ldb,
-                     const_cast<uint8_t*>(as.bad), vstat, st));
-    CK(launch_block_bad(as.bad, nb, bb, st));
-    ctx->klaunch += 3;
+                     const_cast<uint8_t*>(as.bad), vstat, st, nullptr, 0, nullptr, bb));
+    ctx->klaunch += 2;
     const double dk = delta_opt > 0 ? delta_opt : default_delta(prec, T[k]);
     *dsum += dk;
     avg_subj_fill(subj_host.data(), k, as.z, as.bad, as.ldz, T[k]);

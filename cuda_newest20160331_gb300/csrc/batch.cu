@@ -14,6 +14,8 @@ struct BatchSubj {
   double delta = 0, winA = 0, winB = 0;
   long long k_dens = 0;
   bool sampled = false;
+  int* dense_list = nullptr;
+  unsigned int n_dense = 0;
   float cut = -2.0f;  // density histogram: lowest value with a bin
   bool fallback = false;
   DevStatus* ds = nullptr;
@@ -28,6 +30,10 @@ struct BatchSubj {
   unsigned long long* dties = nullptr;
   long long nnz = 0;
 };
+
+size_t batch_state_bytes(const bna_ctx* ctx) {
+  return kCountStateBytes + (size_t)ctx->sms * 8 * 2 * sizeof(long long);
+}
 
 // Density histogram pass of one subject (hist_all: a bin for every value).
 int32_t batch_hist(bna_ctx* ctx, BatchSubj& b, int prec, bool hist_all, unsigned int* hist_host,
@@ -71,13 +77,15 @@ int32_t batch_prep(bna_ctx* ctx, BatchSubj& b, const float* bold, const bna_corr
   ENSURE(S_PRE, (size_t)a.n_pad * 8, b.pre);
   ENSURE(S_BSUM, (size_t)4096 * 8, b.bsum);
   ENSURE(S_ROWPTR, (size_t)(b.N + 1) * 4, b.row_ptr);
-  ENSURE(S_STATUS, sizeof(DevStatus), b.ds);
+  ENSURE(S_STATUS, batch_state_bytes(ctx), b.ds);  // CountState's first member
+  a.wstate = reinterpret_cast<long long*>(reinterpret_cast<char*>(b.ds) + kCountStateBytes);
   a.err = &b.ds->err;
   a.cand_count = &b.ds->cand_count;
   a.stats = b.ds->stats;
   a.epool = &b.ds->epool;
   const long long nst = (long long)a.nb * (a.nb + 1) / 2;
   ENSURE(S_ETAB, (size_t)nst * 4 * sizeof(longlong2), a.etab);
+  ENSURE(S_DENSE, (size_t)nst * sizeof(int), b.dense_list);
   const bool density = opts->mode == BNA_THR_DENSITY;
   b.k_dens = density ? bna_density_nnz(b.N, opts->value) / 2 : 0;
   if (!density) {
@@ -116,17 +124,14 @@ int32_t batch_buffers(bna_ctx* ctx, BatchSubj& b, bool dev_sel, cudaStream_t st)
     ENSURE(S_DEXACT, (size_t)a.cand_cap * sizeof(float), b.dexact);
     ENSURE(S_DTIES, 2 * dens_ties_cap() * sizeof(unsigned long long), b.dties);
   }
-  const int nwarps = ctx->sms * 8;
-  ENSURE(S_WSTATE, (size_t)nwarps * 2 * sizeof(long long), a.wstate);
-  CK(cudaMemsetAsync(b.ds, 0, sizeof(DevStatus), st));
-  CK(cudaMemsetAsync(a.wstate, 0, (size_t)nwarps * 2 * sizeof(long long), st));
+  CK(cudaMemsetAsync(b.ds, 0, batch_state_bytes(ctx), st));
   return BNA_OK;
 }
 
 // After the count pass: candidates, density selection or recompute, scan.
 int32_t batch_after(bna_ctx* ctx, BatchSubj& b, bool dev_sel, cudaStream_t st) {
   CorrArgs& a = b.a;
-  CK(launch_collect_candidates(a, ctx->sms, st));
+  CK(launch_collect_candidates(a, ctx->sms, b.dense_list, &b.ds->dense, st));
   if (dev_sel) {
     CK(dens_set(b.dstate, b.k_dens, (float)b.delta, b.winA, b.winB, st));
     CK(cudaMemsetAsync(b.dhist, 0, 2048 * sizeof(unsigned int), st));
@@ -154,10 +159,7 @@ int32_t batch_fill(bna_ctx* ctx, BatchSubj& b, cudaStream_t st) {
   a.col_idx = col;
   a.val = val;
   a.nnz = b.nnz;
-  const long long nst = (long long)a.nb * (a.nb + 1) / 2;
-  int* dense_list;
-  ENSURE(S_DENSE, (size_t)nst * sizeof(int), dense_list);
-  CK(launch_csr_fill(a, ctx->sms, dense_list, &b.ds->dense, st));
+  CK(launch_csr_fill(a, ctx->sms, b.dense_list, b.n_dense, st));
   CK(cudaMemcpyAsync(ctx->pinned, b.ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
   return BNA_OK;
 }
@@ -354,6 +356,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
     if (!bad && kid->max_nnz > 0 && hs->total > kid->max_nnz) bad = true;
     b.fallback = bad;
     b.nnz = hs->total;
+    b.n_dense = hs->dense;
     if (stats && !bad) {
       bna_corr_stats& o = stats[k];
       std::memset(&o, 0, sizeof o);
@@ -398,7 +401,7 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
       stats[k].ms_total = ms_total;  // the whole batch
       stats[k].ms_count = ms_count;
       stats[k].kernel_launches = ctx->kids[k]->klaunch + (k == 0 ? launches : 0) +
-                                 (dev_sel ? 1 + 18 + 4 : 1 + 1 + 4) + 2;
+                                 (dev_sel ? 18 : 1) + 1 + csr_scan_launches(N[k]) + (b.n_dense ? 2 : 1);
     }
   }
   return BNA_OK;

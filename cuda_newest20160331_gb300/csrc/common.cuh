@@ -100,6 +100,7 @@ __device__ __forceinline__ int classify(float r, const Threshold& th) {
 
 // Pointers and sizes shared by the correlation passes.
 constexpr long long kEtabCand = 1LL << 32;
+constexpr long long kFillDenseE = 1024;  // entries above which a sub-tile takes the dense fill
 
 struct CorrArgs {
   const float* z;            // voxel-major [n_pad][ldz], FP32 z-scores (exact recompute source)

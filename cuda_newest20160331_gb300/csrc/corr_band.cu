@@ -89,7 +89,7 @@ __global__ void recompute_kernel(CorrArgs a) {
 
 // List the candidates flagged in the sub-tiles' edge lists: their pair, their
 // entry's position and (density) their approximate value; count them and the
-// definite entries.  A warp takes the parts of eight sub-tiles at a time, a lane
+// definite entries; list the sub-tiles that the fill pass takes as dense.  A warp takes the parts of eight sub-tiles at a time, a lane
 // each for the ranges (sub-tiles a grid apart: the dense ones of networked data
 // lie together), and reads the lists of those that the count pass
 // marked, the next one's first 64 entries in flight; candidates wait in shared
@@ -99,8 +99,8 @@ __global__ void recompute_kernel(CorrArgs a) {
 // candidates: 78).
 constexpr int kCollectWarps = 8;
 
-__global__ __launch_bounds__(kCollectWarps * 32) void collect_candidates_kernel(CorrArgs a,
-                                                                                long long nst) {
+__global__ __launch_bounds__(kCollectWarps * 32) void collect_candidates_kernel(
+    CorrArgs a, long long nst, int* __restrict__ dense_list, unsigned int* dense_count) {
   __shared__ uint2 bpair[kCollectWarps][64];
   __shared__ long long bpos[kCollectWarps][64];
   __shared__ float bapx[kCollectWarps][64];
@@ -149,6 +149,9 @@ __global__ __launch_bounds__(kCollectWarps * 32) void collect_candidates_kernel(
       if (marked) a.etab[mine * 4 + (lane & 3)].y = c;
     }
     n_def += c;
+    long long E = c + __shfl_xor_sync(0xffffffffu, c, 1);  // of the sub-tile's four parts
+    E += __shfl_xor_sync(0xffffffffu, E, 2);
+    if ((lane & 3) == 0 && E > kFillDenseE) dense_list[atomicAdd(dense_count, 1u)] = (int)mine;
     uint32_t todo = __ballot_sync(0xffffffffu, marked);
     uint2 nx[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};  // the next part's first entries
     auto ahead = [&](uint32_t m) {
@@ -354,12 +357,14 @@ cudaError_t launch_cand_values(const CorrArgs& a, float* vals, int grid, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, cudaStream_t stream) {
+cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, int* dense_list,
+                                      unsigned int* dense_count, cudaStream_t stream) {
   const long long nst = (long long)a.nb * (a.nb + 1) / 2;
   const long long want = (nst + kCollectWarps - 1) / kCollectWarps;
   const int grid = (int)(want < (long long)sms * 8 ? want : (long long)sms * 8);
   if (grid <= 0) return cudaSuccess;
-  collect_candidates_kernel<<<grid, kCollectWarps * 32, 0, stream>>>(a, nst);
+  collect_candidates_kernel<<<grid, kCollectWarps * 32, 0, stream>>>(a, nst, dense_list,
+                                                                     dense_count);
   return cudaGetLastError();
 }
 
@@ -371,16 +376,61 @@ cudaError_t launch_exact_pairs(const CorrArgs& a, const uint2* pairs, int n, flo
 }
 
 // rowlen/pre: n int64; bsum: ceil(n/4096) int64 (<= 4096 blocks); total: 1 int64.
-cudaError_t launch_csr_scan(int32_t* seg, int nb, int n_pad, int n, long long* rowlen,
-                            long long* pre, long long* bsum, long long* total, int32_t* row_ptr,
-                            uint32_t* err, cudaStream_t stream) {
-  const int nblk = (n + 4095) / 4096;
-  if (nblk > 4096) return cudaErrorInvalidValue;
-  seg_scan_rows_kernel<<<n_pad / kSegRows, kSegRows, 0, stream>>>(seg, nb, n_pad, n, rowlen);
-  scan_block_kernel<<<nblk, 1024, 0, stream>>>(rowlen, n, pre, bsum);
-  scan_sums_kernel<<<1, 1024, 0, stream>>>(bsum, nblk, total);
-  scan_finish_kernel<<<(n + 1 + 255) / 256, 256, 0, stream>>>(pre, bsum, n, total, row_ptr, err);
-  return cudaGetLastError();
+// Exclusive prefix of up to kScanOne * 4096 row lengths -> row_ptr, total, in one
+// launch: a block of 4,096 rows sums the lengths before it for itself (three
+// launches, 11 us at 45,000 rows, @@@ so).
+constexpr int kScanOne = 64;
+
+__device__ __forceinline__ long long block_scan_1024(long long s, long long* wsum, long long& all) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long x = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) wsum[warp] = x;
+  __syncthreads();
+  long long before = 0;
+  all = 0;
+#pragma unroll
+  for (int w = 0; w < 32; ++w) {
+    const long long y = wsum[w];
+    before += w < warp ? y : 0;
+    all += y;
+  }
+  return before + x - s;
+}
+
+__global__ __launch_bounds__(1024) void scan_rows_kernel(const long long* __restrict__ in, int n,
+                                                         long long* total, int32_t* row_ptr,
+                                                         uint32_t* err) {
+  __shared__ long long wsum[32];
+  const int start = blockIdx.x * 4096;
+  long long s = 0, base = 0, own = 0;
+#pragma unroll 8
+  for (int k = threadIdx.x; k < start; k += 1024) s += __ldg(in + k);
+  block_scan_1024(s, wsum, base);
+  const int b = start + threadIdx.x * 4;
+  long long v[4];
+  s = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[k] = b + k < n ? in[b + k] : 0;
+    s += v[k];
+  }
+  long long run = base + block_scan_1024(s, wsum, own);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (b + k < n) row_ptr[b + k] = (int32_t)run;
+    run += v[k];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    *total = base + own;
+    row_ptr[n] = (int32_t)(base + own);
+    if (base + own > 0x7fffffffLL) atomicOr(err, ERR_NNZ_INT32);
+  }
 }
 
 // Exclusive prefix of given row lengths -> row_ptr (no seg step).
@@ -389,10 +439,24 @@ cudaError_t launch_rowlen_scan(const long long* rowlen, int n, long long* pre, l
                                cudaStream_t stream) {
   const int nblk = (n + 4095) / 4096;
   if (nblk > 4096) return cudaErrorInvalidValue;
+  if (nblk <= kScanOne) {
+    scan_rows_kernel<<<nblk, 1024, 0, stream>>>(rowlen, n, total, row_ptr, err);
+    return cudaGetLastError();
+  }
   scan_block_kernel<<<nblk, 1024, 0, stream>>>(rowlen, n, pre, bsum);
   scan_sums_kernel<<<1, 1024, 0, stream>>>(bsum, nblk, total);
   scan_finish_kernel<<<(n + 1 + 255) / 256, 256, 0, stream>>>(pre, bsum, n, total, row_ptr, err);
   return cudaGetLastError();
 }
+
+cudaError_t launch_csr_scan(int32_t* seg, int nb, int n_pad, int n, long long* rowlen,
+                            long long* pre, long long* bsum, long long* total, int32_t* row_ptr,
+                            uint32_t* err, cudaStream_t stream) {
+  seg_scan_rows_kernel<<<n_pad / kSegRows, kSegRows, 0, stream>>>(seg, nb, n_pad, n, rowlen);
+  return launch_rowlen_scan(rowlen, n, pre, bsum, total, row_ptr, err, stream);
+}
+
+// Kernels of a scan of n rows.
+int csr_scan_launches(int n) { return (n + 4095) / 4096 <= kScanOne ? 2 : 4; }
 
 }  // namespace bna

@@ -16,7 +16,7 @@
 // Each sub-tile is read twice (once per direction) so that each CTA writes
 // contiguous stretches of the CSR rows.
 // Sub-tiles with more than kFillDenseE edge-list entries (the dense blocks of
-// networked data) are listed first (csr_dense_list_kernel, which also checks
+// networked data) are listed first (collect_candidates_kernel, which also checks
 // every sub-tile's ranges) and placed by csr_fill_dense_kernel, one block per
 // sub-tile, before the row-block pass, which skips them: the entries' values are staged in a 128 x 128 shared-
 // memory matrix, and each row run and each column run of the sub-tile is then
@@ -29,7 +29,6 @@
 namespace bna {
 
 constexpr int kFillWarps = 8;
-constexpr long long kFillDenseE = 1024;  // entries above which a sub-tile takes the dense path
 constexpr int kFillDenseLoads = 8;       // edge-list loads in flight per thread (dense path)
 
 // Asynchronous global -> shared copies (no registers held while in flight).
@@ -236,27 +235,6 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
   cp_async_wait_all();  // nothing in flight into shared memory at exit
 }
 
-// The dense sub-tiles' list (and the check of every sub-tile's ranges),
-// one thread per sub-tile.
-__global__ __launch_bounds__(256) void csr_dense_list_kernel(CorrArgs a, long long nst,
-                                                             int* dense_list,
-                                                             unsigned int* dense_count) {
-  const long long st = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (st >= nst) return;
-  long long E = 0;
-  bool inside = true;  // ranges written while the pool overflowed are not read
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const longlong2 e = a.etab[st * 4 + q];
-    inside &= e.y >= 0 && e.x >= 0 && e.x + e.y <= a.ecap;
-    E += e.y;
-  }
-  if (!inside)
-    atomicOr(a.err, ERR_ELIST);
-  else if (E > kFillDenseE)
-    dense_list[atomicAdd(dense_count, 1u)] = (int)st;
-}
-
 // Dense sub-tiles, one block (8 warps) per sub-tile.
 struct DenseSmem {
   float val[128][129];  // val[il][jl] of the listed edges (padded: column reads conflict-free)
@@ -266,12 +244,11 @@ struct DenseSmem {
 };
 
 __global__ __launch_bounds__(256) void csr_fill_dense_kernel(CorrArgs a, const int* dense_list,
-                                                             const unsigned int* dense_count) {
+                                                             unsigned int n) {
   extern __shared__ __align__(16) uint8_t fill_smem[];
   DenseSmem& S = *reinterpret_cast<DenseSmem*>(fill_smem);
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const uint32_t below = (1u << lane) - 1u;
-  const unsigned int n = *dense_count;
   for (unsigned int idx = blockIdx.x; idx < n; idx += gridDim.x) {
     const long long st = dense_list[idx];
     if (tid < 4) {
@@ -287,7 +264,7 @@ __global__ __launch_bounds__(256) void csr_fill_dense_kernel(CorrArgs a, const i
     int I, J;
     tile_coords(st, a.nb, I, J);
     const bool diag = (I == J);
-    // 1. bitmasks and values (ranges were checked by csr_dense_list_kernel)
+    // 1. bitmasks and values (ranges were checked by collect_candidates_kernel)
     const long long p1 = S.cnt[0], p2 = p1 + S.cnt[1], p3 = p2 + S.cnt[2], E = p3 + S.cnt[3];
     const long long s0 = S.start[0], s1 = S.start[1] - p1, s2 = S.start[2] - p2,
                     s3 = S.start[3] - p3;  // entry e of quadrant q is elist[s_q + e]
@@ -350,18 +327,17 @@ __global__ __launch_bounds__(256) void csr_fill_dense_kernel(CorrArgs a, const i
   }
 }
 
-cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, int* dense_list,
-                                  unsigned int* dense_count, cudaStream_t stream) {
-  if (a.nb <= 0) return cudaSuccess;
-  const long long nst = (long long)a.nb * (a.nb + 1) / 2;
-  cudaError_t e = cudaMemsetAsync(dense_count, 0, sizeof(unsigned int), stream);
+// The n_dense sub-tiles of dense_list (collect_candidates_kernel's).
+cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, const int* dense_list,
+                                  unsigned int n_dense, cudaStream_t stream) {
+  if (a.nb <= 0 || n_dense == 0) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(csr_fill_dense_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(DenseSmem));
   if (e != cudaSuccess) return e;
-  csr_dense_list_kernel<<<(unsigned)((nst + 255) / 256), 256, 0, stream>>>(a, nst, dense_list,
-                                                                         dense_count);
-  e = cudaFuncSetAttribute(csr_fill_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(DenseSmem));
-  if (e != cudaSuccess) return e;
-  csr_fill_dense_kernel<<<sms * 3, 256, sizeof(DenseSmem), stream>>>(a, dense_list, dense_count);
+  const unsigned int most = (unsigned int)sms * 3;
+  csr_fill_dense_kernel<<<n_dense < most ? n_dense : most, 256, sizeof(DenseSmem), stream>>>(
+      a, dense_list, n_dense);
   return cudaGetLastError();
 }
 
@@ -377,9 +353,9 @@ cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1,
   return cudaGetLastError();
 }
 
-cudaError_t launch_csr_fill(const CorrArgs& a, int sms, int* dense_list, unsigned int* dense_count,
-                            cudaStream_t stream) {
-  cudaError_t e = launch_csr_fill_dense(a, sms, dense_list, dense_count, stream);
+cudaError_t launch_csr_fill(const CorrArgs& a, int sms, const int* dense_list,
+                            unsigned int n_dense, cudaStream_t stream) {
+  cudaError_t e = launch_csr_fill_dense(a, sms, dense_list, n_dense, stream);
   if (e != cudaSuccess) return e;
   return launch_csr_fill_rows(a, sms, 0, a.nb, stream);
 }

@@ -29,7 +29,7 @@ size_t zscore_scratch_bytes(int n_pad);
 cudaError_t launch_zscore(const float* bold, int N, int T, int n_pad, float* z, int ldz,
                           uint16_t* zhi, uint16_t* zlo, int ldb, uint8_t* bad, void* scratch,
                           cudaStream_t stream, uint8_t* zq = nullptr, int ldq = 0,
-                          float* e2 = nullptr);
+                          float* e2 = nullptr, uint8_t* blockbad = nullptr);
 cudaError_t launch_corr_simt(const CorrArgs& a, int pass, cudaStream_t stream);
 cudaError_t launch_corr_simt_dump(const CorrArgs& a, int I, int J, float* out,
                                   cudaStream_t stream);
@@ -154,12 +154,14 @@ cudaError_t launch_density_select(const CorrArgs& a, void* state, unsigned int* 
                                   uint8_t* cls, int* eidx, float* exact, float* slot_val,
                                   unsigned long long* ties, unsigned long long* drop, int sms,
                                   cudaStream_t st);
-cudaError_t launch_csr_fill(const CorrArgs& a, int sms, int* dense_list, unsigned int* dense_count,
-                            cudaStream_t stream);
-cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, int* dense_list,
-                                  unsigned int* dense_count, cudaStream_t stream);
+cudaError_t launch_csr_fill(const CorrArgs& a, int sms, const int* dense_list,
+                            unsigned int n_dense, cudaStream_t stream);
+cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, const int* dense_list,
+                                  unsigned int n_dense, cudaStream_t stream);
+int csr_scan_launches(int n);
 cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1, cudaStream_t stream);
-cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, cudaStream_t stream);
+cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, int* dense_list,
+                                      unsigned int* dense_count, cudaStream_t stream);
 cudaError_t launch_cand_values(const CorrArgs& a, float* vals, int grid, cudaStream_t stream);
 }  // namespace bna
 
@@ -170,7 +172,7 @@ enum Slot {
   S_BOLD, S_Z, S_ZHI, S_ZLO, S_BAD, S_SEG, S_ROWLEN, S_PRE, S_BSUM, S_ROWPTR, S_COL, S_VAL,
   S_CAND, S_CANDPOS, S_STATUS, S_DROP, S_EC_U, S_EC_PARTS, S_EC_STATE,
   S_EC_R, S_EC_C, S_EC_V, S_EC_VD, S_DUMP, S_TILES, S_BLOCKBAD, S_DUMPTILE, S_ELIST, S_ETAB, S_HIST, S_CANDVAL,
-  S_DENSE, S_WSTATE, S_VSTAT,
+  S_DENSE, S_VSTAT,
   S_TILES_SMP, S_DSTATE, S_DHIST, S_DCLS, S_DEIDX, S_DEXACT, S_CANDAPX, S_DTIES,
   S_RT_KEEP, S_RT_VALX, S_RT_ROWPTR, S_RT_COL, S_RT_VAL,
   S_AVG_Z, S_AVG_ZHI, S_AVG_ZLO, S_AVG_BAD, S_AVG_BADZ, S_AVG_SUBJ, S_AVG_TC,
@@ -186,11 +188,19 @@ enum Slot {
 struct DevStatus {
   unsigned long long cand_count;
   uint32_t err;
-  uint32_t dense;  // dense sub-tiles queued by the fill pass
+  uint32_t dense;  // dense sub-tiles listed for the fill pass
   unsigned long long stats[4];
   long long total;
   unsigned long long epool;  // edge-list entries handed out by the count pass
 };
+
+// The status, the tile counters and the warps' chunk states of a count pass lie in
+// one slot (S_STATUS), which one fill zeroes.
+struct CountState {
+  DevStatus ds;
+  unsigned int sched[2];
+};
+constexpr size_t kCountStateBytes = (sizeof(CountState) + 255) / 256 * 256;
 
 struct EcGraph {
   cudaGraphExec_t exec = nullptr;
@@ -343,7 +353,7 @@ inline int band_grid(const bna_ctx* ctx) {
 // pass 0: count (+ edge lists); pass 3: density histogram (sampled: on the
 // sampled tile list, tensor-core forms)
 int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cudaStream_t st,
-                  bool sampled = false);
+                  bool sampled = false, unsigned int* sched = nullptr);
 // Free the arena on `st` (to_driver: the pool's cached memory too).
 void arena_release(bna_ctx* ctx, cudaStream_t st, bool to_driver);
 // Everything after the z-scores of a single build.

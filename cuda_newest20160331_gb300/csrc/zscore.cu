@@ -52,7 +52,8 @@
 //                        voxels, computes z, and writes the voxel-major rows
 //                        (z FP32, BF16 hi = bf16(z), lo = bf16(z - hi)) through
 //                        a shared-memory transpose, two steps per lane and
-//                        store.  bad[i] = 1 when z has a NaN.
+//                        store.  bad[i] = 1 when z has a NaN, and (blockbad
+//                        given) its block of 128 voxels.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -183,7 +184,7 @@ static __device__ __noinline__ double zs_centred_sum(const float* bold, int N, i
 
 __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
     const float* __restrict__ bold, int N, int T, VoxStat* __restrict__ vs,
-    uint8_t* __restrict__ bad, float* __restrict__ e2) {
+    uint8_t* __restrict__ bad, float* __restrict__ e2, uint8_t* __restrict__ blockbad) {
   __shared__ uint32_t pmax[kZStatWarps][32], pmin[kZStatWarps][32];
   __shared__ long long pacc[kZStatWarps][32], pmag[kZStatWarps][32];
   __shared__ ulonglong2 pq[kZStatWarps][32];
@@ -320,6 +321,7 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
       vs[gv] = o;
     }
     bad[gv] = 0;
+    if (blockbad && (gv & (kBlk - 1)) == 0) blockbad[gv / kBlk] = 0;
     if (e2) e2[gv] = 0.0f;  // the emit kernel adds to it
   }
   __syncthreads();
@@ -403,7 +405,7 @@ __global__ __launch_bounds__(256) void zscore_emit_kernel(
     const float* __restrict__ bold, int N, int T, const VoxStat* __restrict__ vs,
     float* __restrict__ z, int ldz, uint16_t* __restrict__ zhi, uint16_t* __restrict__ zlo,
     int ldb, uint8_t* __restrict__ bad, uint8_t* __restrict__ zq, int ldq,
-    float* __restrict__ e2) {
+    float* __restrict__ e2, uint8_t* __restrict__ blockbad) {
   // z_near's relative bound: 2^-44, and half of s2's relative distance from S
   // (twice the (T + 16) 2^-53 above, for the conversions and the split)
   const float rel = 5.6843419e-14f + (float)(T + 16) * 1.1102230e-16f;
@@ -477,7 +479,10 @@ __global__ __launch_bounds__(256) void zscore_emit_kernel(
       if (lane == 0) atomicAdd(e2 + v0 + warp + 8 * k, err[k]);
     }
   }
-  if (nan_seen) bad[gv] = 1;
+  if (nan_seen) {
+    bad[gv] = 1;
+    if (blockbad) blockbad[gv / kBlk] = 1;
+  }
 }
 
 size_t zscore_scratch_bytes(int n_pad) { return (size_t)n_pad * sizeof(VoxStat); }
@@ -485,21 +490,23 @@ size_t zscore_scratch_bytes(int n_pad) { return (size_t)n_pad * sizeof(VoxStat);
 // scratch: zscore_scratch_bytes(n_pad) bytes of device memory.
 cudaError_t launch_zscore(const float* bold, int N, int T, int n_pad, float* z, int ldz,
                           uint16_t* zhi, uint16_t* zlo, int ldb, uint8_t* bad, void* scratch,
-                          cudaStream_t stream, uint8_t* zq, int ldq, float* e2) {
+                          cudaStream_t stream, uint8_t* zq, int ldq, float* e2,
+                          uint8_t* blockbad) {
   if (n_pad % 128 != 0 || ldz % 32 != 0 || (zhi && ldb % 64 != 0) || !scratch ||
       (zq && (ldq % 128 != 0 || !e2)))
     return cudaErrorInvalidValue;
   VoxStat* vs = static_cast<VoxStat*>(scratch);
-  zscore_stats_kernel<<<n_pad / 32, kZStatWarps * 32, 0, stream>>>(bold, N, T, vs, bad, e2);
+  zscore_stats_kernel<<<n_pad / 32, kZStatWarps * 32, 0, stream>>>(bold, N, T, vs, bad, e2,
+                                                                  blockbad);
   const int ldbv = zhi ? ldb : 0;
   const int tmax = max(max(ldz, ldbv), zq ? ldq : 0);
   const dim3 grid(n_pad / 32, (tmax + kZEmitT - 1) / kZEmitT);
   if (zq)
     zscore_emit_kernel<true><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
-                                                       bad, zq, ldq, e2);
+                                                       bad, zq, ldq, e2, blockbad);
   else
     zscore_emit_kernel<false><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
-                                                        bad, nullptr, 0, nullptr);
+                                                        bad, nullptr, 0, nullptr, blockbad);
   return cudaGetLastError();
 }
 

@@ -66,3 +66,19 @@ def test_rethreshold_and_degree(builder, N, T, K, delta):
         want = [np.add.accumulate(g.val[R[k]:R[k + 1]], dtype=np.float32)[-1] if R[k + 1] > R[k]
                 else 0.0 for k in range(N)]
         assert np.array_equal(deg, np.array(want, np.float32))
+
+
+@pytest.mark.parametrize("N", [4095, 4096, 4097, 8193])
+def test_row_offsets_over_blocks_of_rows(builder, N):
+    """Row offsets where the rows fill the scan's blocks of 4,096, or spill one
+    over; a dense corner gives some sub-tiles the dense fill."""
+    import torch
+    rng = np.random.default_rng(N)
+    b = rng.integers(400, 600, (24, N)).astype(np.float32)
+    b[:, -200:] = b[:, -1:] + rng.integers(-9, 10, (24, 200))
+    P = oracle.cormat_packed(oracle.zscore(b))
+    R, C, V = oracle.threshold_csr(P, N, "r_gt", 0.7)
+    res = builder.corr_csr(torch.from_numpy(b).cuda(), mode="r_gt", value=0.7, precision="bf16x3")
+    g = res.numpy()
+    assert np.array_equal(g.row_ptr, R) and np.array_equal(g.col_idx, C)
+    assert np.max(np.abs(g.val - V)) <= res.stats["delta"]
