@@ -800,7 +800,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
         CK(cudaMemsetAsync(dhist, 0, 2048 * sizeof(unsigned int), st));
         CK(launch_density_select(a, dstate, dhist, dcls, deidx, dexact, cvals, dties,
                                  dties + dens_ties_cap(), ctx->sms, st));
-        ctx->klaunch += 18 + csr_scan_launches(N);  // selection and decision, scan
+        ctx->klaunch += 12 + csr_scan_launches(N);  // selection and decision, scan
         CK(cudaEventRecord(ctx->ev[3], st));
         CK(launch_csr_scan(a.seg, a.nb, a.n_pad, N, rowlen, pre, bsum, &ds->total, row_ptr,
                            a.err, st));

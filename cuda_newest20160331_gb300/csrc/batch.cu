@@ -401,7 +401,8 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
       stats[k].ms_total = ms_total;  // the whole batch
       stats[k].ms_count = ms_count;
       stats[k].kernel_launches = ctx->kids[k]->klaunch + (k == 0 ? launches : 0) +
-                                 (dev_sel ? 18 : 1) + 1 + csr_scan_launches(N[k]) + (b.n_dense ? 2 : 1);
+                                 (dev_sel ? 12 : 1) + 1 + csr_scan_launches(N[k]) +
+                                 (b.n_dense ? 2 : 1);
     }
   }
   return BNA_OK;

@@ -378,7 +378,7 @@ cudaError_t launch_exact_pairs(const CorrArgs& a, const uint2* pairs, int n, flo
 // rowlen/pre: n int64; bsum: ceil(n/4096) int64 (<= 4096 blocks); total: 1 int64.
 // Exclusive prefix of up to kScanOne * 4096 row lengths -> row_ptr, total, in one
 // launch: a block of 4,096 rows sums the lengths before it for itself (three
-// launches, 11 us at 45,000 rows, @@@ so).
+// launches, 11 us and the gaps between them at 45,000 rows; 8.5 us so).
 constexpr int kScanOne = 64;
 
 __device__ __forceinline__ long long block_scan_1024(long long s, long long* wsum, long long& all) {

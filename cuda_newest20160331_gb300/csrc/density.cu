@@ -47,6 +47,7 @@ struct DensState {
   long long n_ties;
   long long greater;    // pairs above tau*
   int n_drop;
+  unsigned int arrived; // blocks of the current digit's launch
 };
 
 enum : int {
@@ -74,15 +75,27 @@ __global__ void dens_init_kernel(DensState* ds, const unsigned long long* stats)
 }
 
 // Histogram of one key digit over the selected items whose key matches the
-// prefix so far.  which = 0: candidate slots (r~); 1: the E list (exact).
-__global__ void dens_hist_kernel(CorrArgs a, DensState* ds, const float* exact, int which,
-                                 int shift, int nbits, unsigned int* hist) {
-  __shared__ unsigned int h[2048];
+// prefix so far (which = 0: candidate slots (r~); 1: the E list (exact)); the last
+// block to finish picks the digit value that holds the kk-th largest item and
+// leaves the bins zero (a launch of its own took 4.5 us, six times).  first: set
+// kk from the rank wanted; last: store the selected value.
+constexpr int kDigitThreads = 256, kDigitBins = 2048;
+
+__global__ __launch_bounds__(kDigitThreads) void dens_digit_kernel(CorrArgs a, DensState* ds,
+                                                                   const float* exact, int which,
+                                                                   int shift, int nbits, int first,
+                                                                   int last, unsigned int* hist) {
+  __shared__ unsigned int h[kDigitBins];
+  __shared__ long long part[kDigitThreads / 32];
+  __shared__ bool last_block;
+  __shared__ int found;
   const int nb = 1 << nbits;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) h[b] = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = threadIdx.x; b < nb; b += kDigitThreads) h[b] = 0;
   __syncthreads();
-  if (ds->err == 0) {
-    const uint32_t prefix = ds->prefix, mask = ds->mask;
+  const bool bad = ds->err != 0;
+  const uint32_t prefix = first ? 0u : ds->prefix, mask = first ? 0u : ds->mask;
+  if (!bad) {
     long long n;
     if (which == 0) {
       const long long c = (long long)*a.cand_count;
@@ -90,116 +103,125 @@ __global__ void dens_hist_kernel(CorrArgs a, DensState* ds, const float* exact, 
     } else {
       n = ds->n_exact;
     }
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-      float v;
-      if (which == 0) {
-        v = a.cand_apx[i];
-      } else {
-        v = exact[i];
-      }
-      const uint32_t key = okey(v);
+    const float* v = which == 0 ? a.cand_apx : exact;
+    for (long long i = blockIdx.x * (long long)kDigitThreads + threadIdx.x; i < n;
+         i += (long long)gridDim.x * kDigitThreads) {
+      const uint32_t key = okey(v[i]);
       if ((key & mask) == prefix) atomicAdd(&h[(key >> shift) & (uint32_t)(nb - 1)], 1u);
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
+  for (int b = threadIdx.x; b < nb; b += kDigitThreads)
     if (h[b]) atomicAdd(&hist[b], h[b]);
-}
-
-// One block: pick the digit value that holds the kk-th largest item.
-// first: set kk from the rank wanted; last: store the selected value.
-__global__ void dens_pick_kernel(DensState* ds, unsigned int* hist, int which, int shift,
-                                 int nbits, int first, int last) {
-  __shared__ long long part[1024];
-  __shared__ int found;
-  const int nb = 1 << nbits;
-  const int per = nb / 1024 > 0 ? nb / 1024 : 1;  // bins per thread (1 or 2)
-  if (ds->err) return;
-  if (first && threadIdx.x == 0) {
-    ds->kk = which == 0 ? ds->need : ds->need - ds->n_above;
-    ds->prefix = 0;
-    ds->mask = 0;
-  }
-  __syncthreads();
-  const long long kk = ds->kk;
-  // thread t owns bins [nb - per*(t+1), nb - per*t): descending order
-  long long mine = 0;
-  const int hi = nb - per * (int)threadIdx.x;
-  for (int q = 1; q <= per; ++q)
-    if (hi - q >= 0) mine += hist[hi - q];
-  part[threadIdx.x] = mine;
-  if (threadIdx.x == 0) found = -1;
-  __syncthreads();
-  // inclusive scan over threads (descending bins)
-  for (int o = 1; o < 1024; o <<= 1) {
-    const long long y = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += y;
-    __syncthreads();
-  }
-  const long long before = threadIdx.x ? part[threadIdx.x - 1] : 0;
-  if (kk >= 1 && before < kk && part[threadIdx.x] >= kk && hi > 0) {
-    long long c = before;
-    for (int q = 1; q <= per; ++q) {
-      const int b = hi - q;
-      if (b < 0) break;
-      if (c + hist[b] >= kk) {
-        ds->kk = kk - c;
-        ds->prefix |= (uint32_t)b << shift;
-        ds->mask |= (uint32_t)(nb - 1) << shift;
-        found = 1;
-        break;
-      }
-      c += hist[b];
-    }
-  }
+  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (found < 0) {
-      ds->err = which == 0 ? DENS_ERR_WINDOW : DENS_ERR_RANK;
-    } else if (last) {
-      const float v = okey_inv(ds->prefix);
-      if (which == 0) ds->tau_apx = v;
-      else ds->tau = v;
-      ds->prefix = 0;  // the next selection's first histogram starts unfiltered
-      ds->mask = 0;
+    last_block = atomicAdd(&ds->arrived, 1u) == gridDim.x - 1;
+    found = -1;
+  }
+  __syncthreads();
+  if (!last_block) return;
+  __threadfence();
+  if (threadIdx.x == 0) ds->arrived = 0;
+  if (!bad) {
+    const long long kk = first ? (which == 0 ? ds->need : ds->need - ds->n_above) : ds->kk;
+    // thread t owns bins [nb - per (t + 1), nb - per t): descending order
+    const int per = nb / kDigitThreads;
+    const int hi = nb - per * (int)threadIdx.x;
+    unsigned int c[kDigitBins / kDigitThreads];
+    long long mine = 0;
+#pragma unroll
+    for (int q = 0; q < kDigitBins / kDigitThreads; ++q) {
+      c[q] = q < per ? __ldcg(hist + hi - 1 - q) : 0u;
+      mine += c[q];
+    }
+    long long x = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) part[warp] = x;
+    __syncthreads();
+    long long before = x - mine;
+    for (int w = 0; w < warp; ++w) before += part[w];
+    if (kk >= 1 && before < kk && before + mine >= kk) {
+      long long s = before;
+#pragma unroll
+      for (int q = 0; q < kDigitBins / kDigitThreads; ++q) {
+        if (found < 0 && q < per && s + c[q] >= kk) {
+          ds->kk = kk - s;
+          ds->prefix = prefix | ((uint32_t)(hi - 1 - q) << shift);
+          ds->mask = mask | ((uint32_t)(nb - 1) << shift);
+          found = 1;
+        }
+        s += c[q];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (found < 0) {
+        ds->err = which == 0 ? DENS_ERR_WINDOW : DENS_ERR_RANK;
+      } else if (last) {
+        const float v = okey_inv(ds->prefix);
+        if (which == 0) ds->tau_apx = v;
+        else ds->tau = v;
+      }
     }
   }
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) hist[b] = 0;  // ready for the next digit
+  for (int b = threadIdx.x; b < nb; b += kDigitThreads) hist[b] = 0;  // ready for the next digit
 }
 
 // Classify the candidates against tau~: 1 surely above, 3 surely below,
-// 2 exact value needed (listed in eidx).
+// 2 exact value needed (listed in eidx).  A warp takes 256 candidates at a time,
+// so that one atomic serves them (an atomic per 32 on one counter, and one on the
+// other, took 47 us for 682,000 candidates; 7.8 now).
 __global__ void dens_classify_kernel(CorrArgs a, DensState* ds, uint8_t* cls, int* eidx) {
+  constexpr int kR = 8;
   const long long c = (long long)*a.cand_count;
   const long long n = c < a.cand_cap ? c : a.cand_cap;
   const int lane = threadIdx.x & 31;
   if (ds->err) return;
   const float tq = ds->tau_apx, d2 = 2.0f * ds->delta * 1.0001f, lim = 1.0f - ds->delta;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  // whole warps iterate together (warp-aggregated appends)
-  for (long long i0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); i0 < n;
+  const long long stride = (long long)gridDim.x * blockDim.x * kR;
+  unsigned int above = 0;  // the warp's
+  // whole warps iterate together
+  for (long long i0 = (blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31)) * kR; i0 < n;
        i0 += stride) {
-    const long long i = i0 + lane;
-    uint8_t k = 0;
-    if (i < n) {
-      const float r = a.cand_apx[i];
-      if (fabsf(r) >= lim || fabsf(r - tq) <= d2) k = 2;
-      else k = r > tq ? 1 : 3;
+    float r[kR];
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+      const long long i = i0 + 32 * u + lane;
+      r[u] = i < n ? a.cand_apx[i] : 0.0f;
     }
-    if (i < n) cls[i] = k;
-    const uint32_t m2 = __ballot_sync(0xffffffffu, k == 2);
-    const uint32_t m1 = __ballot_sync(0xffffffffu, k == 1);
+    uint32_t m2[kR];
+    unsigned int need = 0;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+      const long long i = i0 + 32 * u + lane;
+      uint8_t k = 0;
+      if (i < n) {
+        if (fabsf(r[u]) >= lim || fabsf(r[u] - tq) <= d2) k = 2;
+        else k = r[u] > tq ? 1 : 3;
+        cls[i] = k;
+      }
+      m2[u] = __ballot_sync(0xffffffffu, k == 2);
+      above += __popc(__ballot_sync(0xffffffffu, k == 1));
+      need += __popc(m2[u]);
+    }
+    if (!need) continue;
     long long base = 0;
-    if (lane == 0) {
-      if (m1) atomicAdd((unsigned long long*)&ds->n_above, (unsigned long long)__popc(m1));
-      if (m2) base = (long long)atomicAdd((unsigned long long*)&ds->n_exact,
-                                          (unsigned long long)__popc(m2));
-    }
+    if (lane == 0)
+      base = (long long)atomicAdd((unsigned long long*)&ds->n_exact, (unsigned long long)need);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (k == 2) eidx[base + __popc(m2 & ((1u << lane) - 1u))] = (int)i;
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+      if ((m2[u] >> lane) & 1u)
+        eidx[base + __popc(m2[u] & ((1u << lane) - 1u))] = (int)(i0 + 32 * u + lane);
+      base += __popc(m2[u]);
+    }
   }
+  if (lane == 0 && above) atomicAdd((unsigned long long*)&ds->n_above, (unsigned long long)above);
 }
 
 // Exact values of E.
@@ -339,7 +361,7 @@ void dens_state_read(const void* host, int* err, float* tau, long long* n_exact,
   *n_drop = d->n_drop;
 }
 
-// The whole selection and decision (15 kernels, no host synchronisation).
+// The whole selection and decision (12 kernels, no host synchronisation).
 // Buffers: state (dens_state_bytes, k/delta/A/B filled by dens_set), hist
 // (2048 uint, zero), cls (cand_cap bytes), eidx (cand_cap int), exact
 // (cand_cap float), slot_val (cand_cap float), ties (kMaxTies u64), drop
@@ -357,10 +379,8 @@ cudaError_t launch_density_select(const CorrArgs& a, void* state, unsigned int* 
       dens_exact_kernel<<<sms * 8, 256, 0, st>>>(a, ds, eidx, exact, slot_val);
     }
     for (int d = 0; d < 3; ++d) {
-      dens_hist_kernel<<<sms * 2, 256, 0, st>>>(a, ds, exact, which, digits[d][0], digits[d][1],
-                                                hist);
-      dens_pick_kernel<<<1, 1024, 0, st>>>(ds, hist, which, digits[d][0], digits[d][1], d == 0,
-                                           d == 2);
+      dens_digit_kernel<<<sms * 2, kDigitThreads, 0, st>>>(a, ds, exact, which, digits[d][0],
+                                                           digits[d][1], d == 0, d == 2, hist);
     }
   }
   dens_ties_kernel<<<sms * 2, 256, 0, st>>>(a, ds, eidx, exact, ties);
