@@ -967,7 +967,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     const int nch = std::min(kFillChunks, a.nb);
     for (int c = 0; c < nch; ++c) {
       const int I0 = (int)((long long)c * a.nb / nch), I1 = (int)((long long)(c + 1) * a.nb / nch);
-      CK(launch_csr_fill_rows(a, ctx->sms, I0, I1, st));
+      CK(launch_csr_fill_rows(a, ctx->sms, I0, I1, n_dense, st));
       CK(cudaEventRecord(ctx->chunk_ev[c], st));
       CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->chunk_ev[c], 0));
       const long long e0 = sink->row_ptr[std::min(I0 * kBlk, N)];
@@ -991,7 +991,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     for (int c = 0; c < nch; ++c) {
       if (c > 0) gate(ctx, st, BNA_PHASE_FILL, (long long)c * a.nb / nch);
       CK(launch_csr_fill_rows(a, ctx->sms, (int)((long long)c * a.nb / nch),
-                              (int)((long long)(c + 1) * a.nb / nch), st));
+                              (int)((long long)(c + 1) * a.nb / nch), n_dense, st));
     }
     fill_launches = (n_dense ? 1 : 0) + nch;
   } else {

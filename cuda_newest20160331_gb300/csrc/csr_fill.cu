@@ -98,12 +98,24 @@ __device__ __forceinline__ int popc_before4v(const uint32_t* m, int pos) {
 // run ahead of its work by asynchronous copies into shared memory: while it
 // places a sub-tile's entries, the next sub-tile's segment offsets and first
 // kFillStage entries and the ranges of the one after that are in flight.
-// Bound: issue and instruction fetch; one direction's code serves both (45,000
-// voxels, 18.5 M entries: 333 us with a copy of the code per direction and hash
-// probes for the candidates in each, 285 now).
-constexpr int kFillStage = 256;  // entries staged per warp ahead of use
+// ORDERED: the block's eight sub-tiles, side by side in the rows, go through a
+// buffer in row order, so that a warp's stores fall in a few lines instead of one
+// each (groups with a dense or the diagonal sub-tile, or more entries than the
+// buffer holds, are placed directly; taking fewer sub-tiles at a time instead was
+// slower, 236 us below and 346 against 284 on 23,000 voxels of 18.6 M entries).  Networked graphs, with more than
+// one sub-tile in kFillDenseShare dense and most others empty, gain nothing from
+// it and pay for the block's barriers (180,000 voxels, 1.7 % dense: 0.73 ms
+// without, 1.00 with).
+// Bound: shared memory and issue.  45,000 voxels, 18.5 M entries: 333 us with a
+// copy of the code per direction and hash probes for the candidates in each, 285
+// with one copy and resolved candidates, 206 in row order.
+constexpr int kFillStage = 224;  // entries staged per warp ahead of use
+constexpr int kFillOut = 1792;   // entries of eight sub-tiles put in row order (with the rest:
+                                 // four blocks' shared memory per SM)
 constexpr int kFillKeep = kFillStage / 32;
+constexpr long long kFillDenseShare = 128;
 
+template <bool ORDERED>
 __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrArgs a, int I0,
                                                                            int parts) {
   __shared__ __align__(16) uint32_t mask[kFillWarps][128][4];  // row r's columns in block J
@@ -112,6 +124,9 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
   __shared__ int nsg[kFillWarps][128];             // staged: rows' block-J segment offsets
   __shared__ longlong2 netab[kFillWarps][2][4];    // staged: quadrant ranges (two sub-tiles)
   __shared__ uint2 ent[kFillWarps][kFillStage];    // staged: first entries
+  __shared__ uint2 out[ORDERED ? kFillOut : 1];                  // (column in the group | row << 16, value)
+  __shared__ int shift_s[128];                     // row's CSR position less its place in out
+  __shared__ int cnt_s[2][kFillWarps];             // the sub-tiles' entries, -1: no row order
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Ir = blockIdx.x / parts, part = blockIdx.x - Ir * parts;
   const int I = I0 + Ir;
@@ -131,7 +146,7 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
   // entry e of quadrant q is elist[b[q] + e] for p[q] <= e < p[q + 1]; the
   // entries to place here: 0 for the dense pass's sub-tiles, and for ranges
   // written while the pool overflowed
-  auto ranges = [&](int slot, long long (&b)[4], int (&p)[3]) {
+  auto ranges = [&](int slot, long long (&b)[4], int (&p)[3], bool& dense) {
     int E = 0;
     bool use = true;
 #pragma unroll
@@ -142,7 +157,8 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
       E += (int)s.y;
       if (q < 3) p[q] = E;
     }
-    return use && E <= (int)kFillDenseE ? E : 0;
+    dense = !(use && E <= (int)kFillDenseE);
+    return dense ? 0 : E;
   };
   // its rows' segment offsets (rows past the last real one read the padding,
   // never used) and its first entries; its ranges are in netab[w][slot]
@@ -152,7 +168,8 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
       cp_async4(&nsg[w][lane + 32 * k], a.seg + (size_t)J * a.n_pad + I * 128 + lane + 32 * k);
     long long b[4];
     int p[3];
-    const int E = ranges(slot, b, p);
+    bool dense;
+    const int E = ranges(slot, b, p, dense);
     for (int e = lane; e < min(E, kFillStage); e += 32)
       cp_async8(&ent[w][e], a.elist + (e < p[0] ? b[0] : e < p[1] ? b[1] : e < p[2] ? b[2] : b[3]) + e);
   };
@@ -166,15 +183,18 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
     if (j0 + w + kFillWarps < j1) fetch_ranges(j0 + w + kFillWarps, 1);
     cp_async_commit();
   }
-  for (int J = j0 + w; J < j1; J += kFillWarps, ++v) {
-    const int slot = v & 1;
+  for (int Jg = j0; Jg < j1; Jg += kFillWarps, ++v) {
+    const int J = Jg + w, slot = v & 1;
+    const bool on = J < j1;
     cp_async_wait_all();
     __syncwarp();
+    if (on)
 #pragma unroll
     for (int k = 0; k < 4; ++k) base[w][lane + 32 * k] = rp_s[lane + 32 * k] + nsg[w][lane + 32 * k];
     long long b[4];
     int p[3];
-    const int E = ranges(slot, b, p);
+    bool dense = false;
+    const int E = on ? ranges(slot, b, p, dense) : 0;
     const int kmax = min((E + 31) / 32, kFillKeep);
     uint2 keep[kFillKeep];
 #pragma unroll
@@ -189,14 +209,13 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
       if (J + 2 * kFillWarps < j1) fetch_ranges(J + 2 * kFillWarps, slot);
     }
     cp_async_commit();
-    if (E == 0) continue;
     auto load = [&](int e) {
       return a.elist[e + (e < p[0] ? b[0] : e < p[1] ? b[1] : e < p[2] ? b[2] : b[3])];
     };
     // row's and column's bits in an entry's key; the diagonal takes both directions
+    const bool diag = I == J;
     int sr = J <= I ? 7 : 0;
-    for (int turn = I == J ? 0 : 1; turn < 2; ++turn) {
-      // 1. masks
+    auto mark_all = [&]() {
       const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
       for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(mk)[lane + 32 * k] = zero4;
@@ -210,18 +229,83 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
         if (k < kmax) mark(keep[k]);
       for (int e = lane + kFillStage; e < E; e += 32) mark(load(e));
       __syncwarp();
-      // 2. place: the entry's rank among its row's columns
+    };
+    // an entry's position: its rank among its row's columns
+    auto place_all = [&](auto put) {
       auto place = [&](uint2 en) {
         if (en.x >> 15) return;
         const int r = (en.x >> sr) & 127, c = (en.x >> (7 - sr)) & 127;
-        put_edge32(a, base[w][r] + popc_before4v(mk[r], c), J * 128 + c, __uint_as_float(en.y));
+        put(r, c, base[w][r] + popc_before4v(mk[r], c), en.y);
       };
 #pragma unroll
       for (int k = 0; k < kFillKeep; ++k)
         if (k < kmax) place(keep[k]);
       for (int e = lane + kFillStage; e < E; e += 32) place(load(e));
       __syncwarp();
-      if (turn == 0) {  // the diagonal's direct entries follow the transposed ones
+    };
+    auto direct = [&](int r, int c, int pos, uint32_t v32) {
+      put_edge32(a, pos, J * 128 + c, __uint_as_float(v32));
+    };
+    if (ORDERED) {
+      if (on && !diag) mark_all();
+      if (lane == 0) cnt_s[slot][w] = dense || (on && diag) ? -1 : E;
+      __syncthreads();
+      int total = 0;
+      bool ordered = true;
+#pragma unroll
+      for (int q = 0; q < kFillWarps; ++q) {
+        total += cnt_s[slot][q];
+        ordered &= cnt_s[slot][q] >= 0;
+      }
+      if (total == 0 && ordered) continue;
+      if (ordered && total <= kFillOut) {
+        // every warp finds the rows' places in out for itself: a row's entries of
+        // the group's sub-tiles follow each other in the CSR
+        const int last = min(kFillWarps, j1 - Jg) - 1;
+        int len[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int r = 4 * lane + k;
+          const uint4 m = *reinterpret_cast<const uint4*>(mask[last][r]);
+          len[k] = base[last][r] - base[0][r] + __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+          sum += len[k];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        int at = incl - sum;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          shift_s[4 * lane + k] = base[0][4 * lane + k] - at;  // the same from every warp
+          at += len[k];
+        }
+        const int n_out = __shfl_sync(0xffffffffu, incl, 31);
+        __syncwarp();
+        place_all([&](int r, int c, int pos, uint32_t v32) {
+          const int to = pos - shift_s[r];
+          if ((unsigned)to < (unsigned)kFillOut)
+            out[to] = make_uint2((uint32_t)(w * 128 + c) | ((uint32_t)r << 16), v32);
+          else
+            atomicOr(a.err, ERR_RANGE);
+        });
+        __syncthreads();
+        for (int k = threadIdx.x; k < min(n_out, kFillOut); k += kFillWarps * 32) {
+          const uint2 o = out[k];
+          put_edge32(a, k + shift_s[(o.x >> 16) & 127], Jg * 128 + (int)(o.x & 0xFFFFu),
+                     __uint_as_float(o.y));
+        }
+        continue;
+      }
+    } else if (E > 0 && !diag) {
+      mark_all();
+    }
+    if (E > 0) {
+      if (diag) {  // the transposed entries, then the direct ones behind them
+        mark_all();
+        place_all(direct);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint4 m = reinterpret_cast<const uint4*>(mk)[lane + 32 * k];
@@ -229,7 +313,9 @@ __global__ __launch_bounds__(kFillWarps * 32, 4) void csr_fill_rows_kernel(CorrA
         }
         __syncwarp();
         sr = 0;
+        mark_all();
       }
+      place_all(direct);
     }
   }
   cp_async_wait_all();  // nothing in flight into shared memory at exit
@@ -341,7 +427,8 @@ cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, const int* dense_l
   return cudaGetLastError();
 }
 
-cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1,
+// n_dense: the sub-tiles left to the dense fill.
+cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1, unsigned int n_dense,
                                  cudaStream_t stream) {
   if (I1 <= I0) return cudaSuccess;
   const int rows = I1 - I0;
@@ -349,7 +436,10 @@ cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1,
   int parts = (sms * 8 + rows - 1) / rows;
   if (parts > (a.nb + 7) / 8) parts = (a.nb + 7) / 8;
   if (parts < 1) parts = 1;
-  csr_fill_rows_kernel<<<rows * parts, kFillWarps * 32, 0, stream>>>(a, I0, parts);
+  const long long nst = (long long)a.nb * (a.nb + 1) / 2;
+  auto fn = (long long)n_dense * kFillDenseShare <= nst ? csr_fill_rows_kernel<true>
+                                                        : csr_fill_rows_kernel<false>;
+  fn<<<rows * parts, kFillWarps * 32, 0, stream>>>(a, I0, parts);
   return cudaGetLastError();
 }
 
@@ -357,7 +447,7 @@ cudaError_t launch_csr_fill(const CorrArgs& a, int sms, const int* dense_list,
                             unsigned int n_dense, cudaStream_t stream) {
   cudaError_t e = launch_csr_fill_dense(a, sms, dense_list, n_dense, stream);
   if (e != cudaSuccess) return e;
-  return launch_csr_fill_rows(a, sms, 0, a.nb, stream);
+  return launch_csr_fill_rows(a, sms, 0, a.nb, n_dense, stream);
 }
 
 }  // namespace bna

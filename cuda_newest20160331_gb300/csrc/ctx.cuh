@@ -159,7 +159,8 @@ cudaError_t launch_csr_fill(const CorrArgs& a, int sms, const int* dense_list,
 cudaError_t launch_csr_fill_dense(const CorrArgs& a, int sms, const int* dense_list,
                                   unsigned int n_dense, cudaStream_t stream);
 int csr_scan_launches(int n);
-cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1, cudaStream_t stream);
+cudaError_t launch_csr_fill_rows(const CorrArgs& a, int sms, int I0, int I1, unsigned int n_dense,
+                                 cudaStream_t stream);
 cudaError_t launch_collect_candidates(const CorrArgs& a, int sms, int* dense_list,
                                       unsigned int* dense_count, cudaStream_t stream);
 cudaError_t launch_cand_values(const CorrArgs& a, float* vals, int grid, cudaStream_t stream);
