@@ -99,7 +99,6 @@ struct TcArgs {
   // multi-subject average (AVG): every tile adds up the values of subj[0 ..
   // nsub); pass 4 writes the averages to packed[idx(i, j)]
   int nsub;
-  int fisher;
   float* packed;
   // multi-subject count pass: tiles4 = (I, J-pair, subject), subj the table
   const int4* tiles4;
@@ -174,14 +173,14 @@ __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
 // the density rule's pass 8 % (45,000 x 300, 682,000 candidates: 1.32 ms against
 // 1.21).
 // MULTI: the tiles of several subjects in one persistent launch (count pass).
-// AVG: the average over subjects (W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:418-670):
+// AVG: 1 the average over subjects, 2 of their Fisher z (W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:418-670):
 // each tile runs through the subjects in order, and a thread keeps the running
 // sums of its 128 pairs in registers (post_block's accumulation, :847-883: r~
 // or its Fisher z, values outside [-1, 1] skipped), then takes the average
 // through the same epilogue as one subject's values.  No N (N - 1) / 2 matrix
 // is held: adding each subject into one in HBM, 4 bytes per lane in 32
 // different rows, took 4.07 ms per subject at N = 20,000, T = 180-300.
-template <int PASS, bool ABS, int FORM, bool MULTI = false, bool AVG = false>
+template <int PASS, bool ABS, int FORM, bool MULTI = false, int AVG = 0>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     corr_tc_kernel(const __grid_constant__ CUtensorMap tm_hi,
                    const __grid_constant__ CUtensorMap tm_lo, const TcArgs p) {
@@ -619,7 +618,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       };
       if (AVG) {
         // running sums in registers, rotated so that the loop over the four
-        // chunks keeps one copy of its code: after four turns chunk 0 leads again
+        // chunks keeps one copy of its code: after four turns chunk 0 leads again.
+        // Bound: the eight epilogue warps' issue and instruction fetch (20,000
+        // voxels, four subjects of 180 to 300 samples: 2.24 ms with the Fisher
+        // switch at run time, a range mask per value and a division for every
+        // pair, 1.89 now; unrolling the chunks by two or four, without the
+        // rotation, 3.3 and 4.3)
         uint32_t sm[128], un[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 128; ++k) sm[k] = 0u;
@@ -639,7 +643,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const bool rowbad = slow && e.a.bad[gi];
             const float unc_lim = e.unc_lim;
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c0 = 0; c0 < 4; c0 += 1) {
+#pragma unroll
+              for (int cc = 0; cc < 1; ++cc) {
+                const int c = c0 + cc;
               uint32_t um = 0;
 #pragma unroll
               for (int g = 0; g < 32; g += 16) {  // 16 values at a time fit the registers
@@ -653,12 +660,28 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
                 // |r| >= 1/2 (and NaN) are rare: the logarithm's form, and
                 // post_block's range, for the columns where some lane has one
+                uint32_t mx = 0;  // the largest square's bits (a NaN's are larger)
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                  const float r = __uint_as_float(v[k]);
+                  mx = max(mx, __float_as_uint(__fmul_rn(r, r)));
+                }
+                if (!__any_sync(0xffffffffu, mx >= 0x3E800000u /* 1/4 */)) {
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) {
+                    float r = __uint_as_float(v[k]);
+                    if (AVG == 2) r = fisher_z_half(r);
+                    sm[cc * 32 + g + k] = __float_as_uint(__fadd_rn(__uint_as_float(sm[cc * 32 + g + k]), r));
+                  }
+                  continue;
+                }
                 uint32_t big = 0;
 #pragma unroll
                 for (int k = 0; k < 16; ++k)
                   big |= fabsf(__uint_as_float(v[k])) < 0.5f ? 0u : 1u << k;
                 // (one copy of that code in a loop: sixteen in line made the
                 // kernel wait for instructions, 6.3 ms instead of 2.3)
+#pragma unroll 1
                 for (uint32_t w = __reduce_or_sync(0xffffffffu, big); w; w &= w - 1) {
                   const int kk = __ffs(w) - 1;
                   uint32_t x = 0u;
@@ -667,13 +690,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                   if ((big >> kk) & 1u) {
                     const float r = __uint_as_float(x);
                     um |= !(fabsf(r) < unc_lim) ? 1u << (g + kk) : 0u;
-                    const float add = p.fisher ? fisher_z(r) : r;
+                    const float add = AVG == 2 ? fisher_z(r) : r;
                     x = r >= -1.0f && r <= 1.0f ? __float_as_uint(add) : 0u;
                   }
 #pragma unroll
                   for (int k = 0; k < 16; ++k) v[k] = k == kk ? x : v[k];
                 }
-                if (p.fisher) {
+                if (AVG == 2) {
 #pragma unroll
                   for (int k = 0; k < 16; ++k) {
                     const float z = fisher_z_half(__uint_as_float(v[k]));
@@ -682,10 +705,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
 #pragma unroll
                 for (int k = 0; k < 16; ++k)
-                  sm[g + k] = __float_as_uint(
-                      __fadd_rn(__uint_as_float(sm[g + k]), __uint_as_float(v[k])));
+                  sm[cc * 32 + g + k] = __float_as_uint(
+                      __fadd_rn(__uint_as_float(sm[cc * 32 + g + k]), __uint_as_float(v[k])));
               }
-              const uint32_t u0 = un[0] | um;
+              un[cc] |= um;
+              }
               uint32_t lead[32];
 #pragma unroll
               for (int k = 0; k < 32; ++k) lead[k] = sm[k];
@@ -693,10 +717,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
               for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
 #pragma unroll
               for (int k = 0; k < 32; ++k) sm[96 + k] = lead[k];
-              un[0] = un[1];
-              un[1] = un[2];
-              un[2] = un[3];
-              un[3] = u0;
+              uint32_t ul[1];
+#pragma unroll
+              for (int k = 0; k < 1; ++k) ul[k] = un[k];
+#pragma unroll
+              for (int k = 0; k < 3; ++k) un[k] = un[k + 1];
+#pragma unroll
+              for (int k = 0; k < 1; ++k) un[3 + k] = ul[k];
             }
           }
           ptx::tc_fence_before();
@@ -712,28 +739,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t v[32];  // takes sm[0 .. 31]'s place
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              v[k] = __float_as_uint(__fdiv_rn(__uint_as_float(sm[k]), fs));
-            }
-            if (p.fisher) {  // back from z, in the columns where some lane's average counts
+            if (AVG == 2) {  // back from z, where a lane's average counts; 0: below lo_thr
               uint32_t need = un[0];
 #pragma unroll
               for (int k = 0; k < 32; ++k) {
-                const float z = __uint_as_float(v[k]);
-                need |= (ABS ? fabsf(z) : z) < zlo ? 0u : 1u << k;
+                const float z = __uint_as_float(sm[k]);  // zlo's margin covers the division
+                need |= (ABS ? fabsf(z) : z) < zlo * fs ? 0u : 1u << k;
               }
-              const uint32_t cols = __reduce_or_sync(0xffffffffu, need);
-              for (uint32_t w = cols; w; w &= w - 1) {
+#pragma unroll
+              for (int k = 0; k < 32; ++k) v[k] = (need >> k) & 1u ? sm[k] : 0u;
+#pragma unroll 1
+              for (uint32_t w = need; w; w &= w - 1) {
                 const int kk = __ffs(w) - 1;
-                const uint32_t x =
-                    __float_as_uint(fisher_r(__uint_as_float(pick32(v, kk))));
+                const uint32_t x = __float_as_uint(
+                    fisher_r(__fdiv_rn(__uint_as_float(pick32(v, kk)), fs)));
 #pragma unroll
                 for (int k = 0; k < 32; ++k) v[k] = k == kk ? x : v[k];
               }
+            } else {
 #pragma unroll
-              for (int k = 0; k < 32; ++k)  // 0: below lo_thr
-                if (!((cols >> k) & 1u)) v[k] = 0u;
+              for (int k = 0; k < 32; ++k)
+                v[k] = __float_as_uint(__fdiv_rn(__uint_as_float(sm[k]), fs));
             }
             chunk(v, c, un[0], false, false);
 #pragma unroll
@@ -1025,6 +1051,14 @@ cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, co
   return cudaGetLastError();
 }
 
+template <int FORM, int AVG>
+static void (*tc_avg_kernel(int pass, bool absm))(CUtensorMap, CUtensorMap, TcArgs) {
+  return pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM, false, AVG>
+                             : corr_tc_kernel<0, false, FORM, false, AVG>)
+         : pass == 3 ? corr_tc_kernel<3, false, FORM, false, AVG>
+                     : corr_tc_kernel<4, false, FORM, false, AVG>;
+}
+
 // The average over the subjects of a table (tc_subj_fill): pass 0 count (+ edge
 // lists), 3 density histogram, 4 the packed averages.  a: the average's own
 // sizes, rule and lists.
@@ -1039,22 +1073,17 @@ cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void
   p.ntiles = ntiles;
   p.subj = static_cast<const TcSubj*>(subj_dev);
   p.nsub = nsub;
-  p.fisher = fisher;
   p.packed = packed;
   const int g = grid < ntiles ? grid : ntiles;
   if (g <= 0) return cudaSuccess;
   const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
   if (form == FORM_BF16X3)
-    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_BF16X3, false, true>
-                               : corr_tc_kernel<0, false, FORM_BF16X3, false, true>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_BF16X3, false, true>
-                       : corr_tc_kernel<4, false, FORM_BF16X3, false, true>;
+    kern = fisher ? tc_avg_kernel<FORM_BF16X3, 2>(pass, absm)
+                  : tc_avg_kernel<FORM_BF16X3, 1>(pass, absm);
   else
-    kern = pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM_TF32, false, true>
-                               : corr_tc_kernel<0, false, FORM_TF32, false, true>)
-           : pass == 3 ? corr_tc_kernel<3, false, FORM_TF32, false, true>
-                       : corr_tc_kernel<4, false, FORM_TF32, false, true>;
+    kern = fisher ? tc_avg_kernel<FORM_TF32, 2>(pass, absm)
+                  : tc_avg_kernel<FORM_TF32, 1>(pass, absm);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)TC_SMEM_BYTES);
   if (e != cudaSuccess) return e;
