@@ -470,15 +470,16 @@ cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const f
 // rows of an iteration that turns out to be past the stop are dropped.
 // Graphs of kCoopStageDeg entries per row copy the iterate into shared memory
 // each iteration (192 KB at most) and gather there instead of a sector of L2 per
-// entry (2,000, 12,000 and 16,000 vertices, 60 entries: 7.3, 10.1 and 10.6 us per
-// iteration against 7.6, 11.1 and 11.6; 20 entries: 6.7, 9.0 and 9.3 against 6.0,
+// entry (2,000, 12,000 and 16,000 vertices, 60 entries: 6.9, 9.4 and 10.2 us per
+// iteration against 7.6, 11.1 and 11.6; 20 entries: 6.2, 8.3 and 8.9 against 6.0,
 // 7.9 and 8.1).  Rows one at a time, with the last block to arrive reducing the
 // partials and publishing the totals, took 14.9 us on 2,000 vertices, 17.8, 20.2
-// and 29.7 on 12,000 of 20, 130 and 300 entries per row; 6.0, 7.9, 11.7 and 15.2
-// now.  Eight row warps: 15.0 us on 16,000 x 130, sixteen 12.2.
+// and 29.7 on 12,000 of 20, 130 and 300 entries per row; 6.0, 7.9, 11.0 and 14.5
+// now.  Eight row warps: 15.0 us on 16,000 x 130 where sixteen took 12.2.
 constexpr int kCoopWarps = 16;                          // row warps
 constexpr int kCoopThreads = (kCoopWarps + 3) * 32;     // and one per total
 constexpr int kCoopRows = 4;                            // rows side by side
+constexpr int kCoopStageBytes = (kEcCoopMaxN + 1) * (int)sizeof(float2);  // most shared memory
 constexpr int kCoopSlots = 32;                          // most rows per warp
 constexpr long long kCoopStageDeg = 50;                 // entries per row from which to stage
 
@@ -576,7 +577,7 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
     int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, const double* __restrict__ vald, long long nnz_used,
     double* u, float2* uf, double* parts, EcState* st, int it_end, int max_iter, double eps) {
-  extern __shared__ float2 xs[];  // STAGE: the iterate
+  extern __shared__ __align__(16) float2 xs[];  // STAGE: the iterate
   __shared__ float2 rs[kCoopSlots * kCoopWarps];
   __shared__ bool rempty[kCoopSlots * kCoopWarps];
   __shared__ double tot_s[5];  // lam2, e1, e2, lambda, 1 / lambda
@@ -608,9 +609,27 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
   double lam = 0.0;
   for (;; ++it) {
     const size_t cur = (size_t)(it & 1) * n, nxt = (size_t)((it + 1) & 1) * n;
+    // 16 bytes at a time, five loads of a thread in flight; an iterate on an odd
+    // 8-byte boundary is staged with the element before it, which keeps both sides
+    // aligned (8 bytes at a time, 12,000 vertices of 60 and 300 entries per row: 10.1
+    // and 15.2 us per iteration, 9.4 and 14.5 so)
+    const int odd = STAGE && (reinterpret_cast<uintptr_t>(uf + cur) & 8u) ? 1 : 0;
     if (STAGE && it < it_end) {
-#pragma unroll 8
-      for (int k = threadIdx.x; k < n; k += kCoopThreads) xs[k] = __ldcg(uf + cur + k);
+      const float4* src = reinterpret_cast<const float4*>(uf + cur - odd);
+      float4* dst = reinterpret_cast<float4*>(xs);
+      const int n4 = (n + odd) / 2;
+      constexpr int kU = 5;
+      for (int k0 = threadIdx.x; k0 < n4; k0 += kU * kCoopThreads) {
+        float4 v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+          if (k0 + u * kCoopThreads < n4) v[u] = __ldcg(src + k0 + u * kCoopThreads);
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+          if (k0 + u * kCoopThreads < n4) dst[k0 + u * kCoopThreads] = v[u];
+      }
+      if (((n + odd) & 1) && threadIdx.x == kCoopThreads - 1)
+        xs[n + odd - 1] = __ldcg(uf + cur + n - 1);
       __syncthreads();
     }
     if (warp < kCoopWarps) {
@@ -623,7 +642,7 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
             b[r] = __shfl_sync(0xffffffffu, rb, (s + r) & 31);
             len[r] = s + r < slots ? __shfl_sync(0xffffffffu, rl, (s + r) & 31) : 0;
           }
-          coop_rows<VK, STAGE>(ci, val, vald, STAGE ? xs : uf + cur, b, len, lane, sh, sl);
+          coop_rows<VK, STAGE>(ci, val, vald, STAGE ? xs + odd : uf + cur, b, len, lane, sh, sl);
 #pragma unroll
           for (int r = 0; r < kCoopRows; ++r)
             if (lane == r && s + r < slots) {
@@ -702,9 +721,9 @@ int ec_coop_grid(int n, int sms) {
   if (n > kEcCoopMaxN) return 0;
   int per_sm = 0;
   if (cudaFuncSetAttribute(ec_coop_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kEcCoopMaxN * sizeof(float2)) != cudaSuccess ||
+                           kCoopStageBytes) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ec_coop_kernel<2, true>, kCoopThreads,
-                                                    kEcCoopMaxN * sizeof(float2)) !=
+                                                    kCoopStageBytes) !=
           cudaSuccess ||
       per_sm < 1) {
     cudaGetLastError();
@@ -731,10 +750,10 @@ cudaError_t launch_ec_coop(int n, const int32_t* rp, const int32_t* ci, const fl
                                    : (const void*)ec_coop_kernel<2, false>)
                           : (stage ? (const void*)ec_coop_kernel<0, true>
                                    : (const void*)ec_coop_kernel<0, false>);
-  const size_t smem = stage ? (size_t)n * sizeof(float2) : 0;
+  const size_t smem = stage ? (size_t)(n + 1) * sizeof(float2) : 0;
   if (stage) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(kEcCoopMaxN * sizeof(float2)));
+                                               kCoopStageBytes);
     if (e != cudaSuccess) return e;
   }
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kCoopThreads), args, smem, stream);
