@@ -63,7 +63,9 @@
 namespace bna {
 
 constexpr int kZStatWarps = 8;  // time slices per block of 32 voxels
-constexpr int kZEmitT = 256;  // time steps per emit block (8 chunks of 32)
+// Time steps per emit block: kZEmitT, fewer (in chunks of 64) where that leaves
+// less than kZEmitBlocks blocks: 4,096 x 240 took 13.0 us in 128 blocks, 9.3 in 512.
+constexpr int kZEmitT = 256, kZEmitBlocks = 608;
 
 // Per-voxel statistics handed from the stats kernel to the emit kernel.
 struct VoxStat {
@@ -405,7 +407,7 @@ __global__ __launch_bounds__(256) void zscore_emit_kernel(
     const float* __restrict__ bold, int N, int T, const VoxStat* __restrict__ vs,
     float* __restrict__ z, int ldz, uint16_t* __restrict__ zhi, uint16_t* __restrict__ zlo,
     int ldb, uint8_t* __restrict__ bad, uint8_t* __restrict__ zq, int ldq,
-    float* __restrict__ e2, uint8_t* __restrict__ blockbad) {
+    float* __restrict__ e2, uint8_t* __restrict__ blockbad, int slice) {
   // z_near's relative bound: 2^-44, and half of s2's relative distance from S
   // (twice the (T + 16) 2^-53 above, for the conversions and the split)
   const float rel = 5.6843419e-14f + (float)(T + 16) * 1.1102230e-16f;
@@ -416,10 +418,10 @@ __global__ __launch_bounds__(256) void zscore_emit_kernel(
   const bool live = gv < N;
   const VoxStat st = vs[gv];  // gv < n_pad: the grid covers n_pad / 32 groups
   const int tmax = max(max(ldz, ldb), Q8 ? ldq : 0);
-  const int tb = blockIdx.y * kZEmitT;
+  const int tb = blockIdx.y * slice;
   bool nan_seen = false;
   float err[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  for (int t0 = tb; t0 < tb + kZEmitT && t0 < tmax; t0 += 64) {
+  for (int t0 = tb; t0 < tb + slice && t0 < tmax; t0 += 64) {
     float xs[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -500,13 +502,15 @@ cudaError_t launch_zscore(const float* bold, int N, int T, int n_pad, float* z, 
                                                                   blockbad);
   const int ldbv = zhi ? ldb : 0;
   const int tmax = max(max(ldz, ldbv), zq ? ldq : 0);
-  const dim3 grid(n_pad / 32, (tmax + kZEmitT - 1) / kZEmitT);
+  int slice = kZEmitT;
+  while (slice > 64 && n_pad / 32 * ((tmax + slice - 1) / slice) < kZEmitBlocks) slice -= 64;
+  const dim3 grid(n_pad / 32, (tmax + slice - 1) / slice);
   if (zq)
     zscore_emit_kernel<true><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
-                                                       bad, zq, ldq, e2, blockbad);
+                                                       bad, zq, ldq, e2, blockbad, slice);
   else
     zscore_emit_kernel<false><<<grid, 256, 0, stream>>>(bold, N, T, vs, z, ldz, zhi, zlo, ldbv,
-                                                        bad, nullptr, 0, nullptr, blockbad);
+                                                        bad, nullptr, 0, nullptr, blockbad, slice);
   return cudaGetLastError();
 }
 
