@@ -136,7 +136,8 @@ size_t rethr_words(int n, long long nnz);
 cudaError_t launch_rethr_count(const CorrArgs& a, const int32_t* rp, const int32_t* ci,
                                const float* val, const Threshold& th, uint32_t* keep,
                                uint32_t* exact, float* valx, long long* rowlen,
-                               unsigned long long* band, int sms, cudaStream_t st);
+                               unsigned long long* band, unsigned long long* next, int sms,
+                               cudaStream_t st);
 cudaError_t launch_rethr_fill(int n, const int32_t* rp, const int32_t* ci, const float* val,
                               const float* valx, const uint32_t* keep, const uint32_t* exact,
                               const int32_t* rp2, int32_t* ci2, float* val2, long long nnz2,

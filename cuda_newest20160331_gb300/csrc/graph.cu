@@ -36,9 +36,10 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
   ENSURE(S_BSUM, (size_t)4096 * 8, bsum);
   ENSURE(S_RT_ROWPTR, (size_t)(N + 1) * 4, rp2);
   ENSURE(S_STATUS, sizeof(DevStatus), ds);
+  // epool serves as the count's row counter
   CK(cudaMemsetAsync(ds, 0, sizeof(DevStatus), st));
   CK(launch_rethr_count(a, in_dev->row_ptr, in_dev->col_idx, in_dev->val, th, keep, keep + words, valx,
-                        rowlen, &ds->stats[1], ctx->sms, st));
+                        rowlen, &ds->stats[1], &ds->epool, ctx->sms, st));
   CK(launch_rowlen_scan(rowlen, N, pre, bsum, &ds->total, rp2, &ds->err, st));
   DevStatus* hs = reinterpret_cast<DevStatus*>(ctx->pinned);
   CK(cudaMemcpyAsync(hs, ds, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));

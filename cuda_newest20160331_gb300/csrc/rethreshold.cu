@@ -24,21 +24,25 @@ constexpr int kRethrWarps = 8;
 // near a decision wait in shared memory and are recomputed four at a time.
 // Bound: reading the values and, at a wide delta, the recomputed pairs (23,000
 // voxels, TF32, 18.6 M entries: 454, 283 and 204 us for three thresholds with a
-// warp per pair, a byte flag and a copied value per entry; 332, 197 and 139 now.
+// warp per pair, a byte flag and a copied value per entry; 332, 197 and 139 with
+// rows dealt out in turn, 276, 162 and 112 from a counter.
 // Taking the values below the diagonal from their mirror images, by a search in
 // the other row, cost what it saved: 327, 229 and 179).
 __global__ __launch_bounds__(kRethrWarps * 32) void rethr_count_kernel(
     CorrArgs a, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
     const float* __restrict__ val, Threshold th, uint32_t* keep, uint32_t* exact, float* valx,
-    long long* rowlen, unsigned long long* band) {
+    long long* rowlen, unsigned long long* band, unsigned long long* next) {
   __shared__ int list[kRethrWarps][160];  // entries to recompute (offsets in the row)
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;
-  const int nw = gridDim.x * kRethrWarps;
   const bool absm = th.mode == BNA_THR_ABS_GT || th.mode == BNA_THR_ABS_GE;
   const float lim = 1.0f - th.delta;
   unsigned int n_1e6 = 0;
-  for (int i = blockIdx.x * kRethrWarps + w; i < a.n; i += nw) {
+  for (;;) {  // rows from a counter: their lengths and recomputed pairs vary
+    int i = 0;
+    if (lane == 0) i = (int)min(atomicAdd(next, 1ull), (unsigned long long)a.n);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= a.n) break;
     const long long b = rp[i];
     const int len = (int)(rp[i + 1] - b);
     const long long wb = rethr_word(b, i);
@@ -167,9 +171,10 @@ size_t rethr_words(int n, long long nnz) { return (size_t)rethr_word(nnz, n) + 1
 cudaError_t launch_rethr_count(const CorrArgs& a, const int32_t* rp, const int32_t* ci,
                                const float* val, const Threshold& th, uint32_t* keep,
                                uint32_t* exact, float* valx, long long* rowlen,
-                               unsigned long long* band, int sms, cudaStream_t st) {
-  rethr_count_kernel<<<sms * 8, kRethrWarps * 32, 0, st>>>(a, rp, ci, val, th, keep, exact, valx,
-                                                           rowlen, band);
+                               unsigned long long* band, unsigned long long* next, int sms,
+                               cudaStream_t st) {
+  rethr_count_kernel<<<sms * 4, kRethrWarps * 32, 0, st>>>(a, rp, ci, val, th, keep, exact, valx,
+                                                           rowlen, band, next);
   return cudaGetLastError();
 }
 
