@@ -52,22 +52,30 @@ cudaMemPool_t lib_pool(int device) {
 
 namespace bna {
 
+// Free a slot on `st`.  What a context keeps in it from call to call goes with
+// it: the tile lists are built again for the buffer that takes its place.
+static cudaError_t slot_free(bna_ctx* ctx, int s, cudaStream_t st) {
+  if (s == S_TILES || s == S_TILES_SMP) ctx->tiles_nb = -1;
+  if (s == S_SC_TILES) ctx->sc_nb = -1;
+  if (s == S_BATCH_TILES) ctx->batch_nb.clear();
+  const cudaError_t e = ctx->ptr[s] ? cudaFreeAsync(ctx->ptr[s], st) : cudaSuccess;
+  ctx->ptr[s] = nullptr;
+  ctx->cap[s] = 0;
+  return e;
+}
+
 int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
   if (bytes == 0) bytes = 16;
   if (ctx->cap[s] < bytes) {
     // stream-ordered on the call's stream: growing one context's arena does
     // not wait for the work other contexts have on the device
-    if (ctx->ptr[s]) {
-      cudaError_t e = cudaFreeAsync(ctx->ptr[s], ctx->cur);
-      ctx->ptr[s] = nullptr;
-      ctx->cap[s] = 0;
-      if (e != cudaSuccess)
-        return fail(ctx, BNA_CUDA_ERROR, "cudaFreeAsync: %s", cudaGetErrorString(e));
-    }
+    cudaError_t e = slot_free(ctx, s, ctx->cur);
+    if (e != cudaSuccess)
+      return fail(ctx, BNA_CUDA_ERROR, "cudaFreeAsync: %s", cudaGetErrorString(e));
     const size_t want = bytes + bytes / 8;  // headroom so small growth does not reallocate
     cudaMemPool_t pool = lib_pool(ctx->device);
     if (!pool) return fail(ctx, BNA_CUDA_ERROR, "no device memory pool");
-    cudaError_t e = cudaMallocFromPoolAsync(&ctx->ptr[s], want, pool, ctx->cur);
+    e = cudaMallocFromPoolAsync(&ctx->ptr[s], want, pool, ctx->cur);
     if (e != cudaSuccess) {
       cudaGetLastError();
       cudaStreamSynchronize(ctx->cur);
@@ -100,12 +108,7 @@ bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want) {
     ok = ok && ensure(ctx, w.slot, w.bytes, &p) == BNA_OK;
   }
   if (ok) return true;
-  for (const SlotSize& w : want) {
-    if (ctx->ptr[w.slot]) cudaFreeAsync(ctx->ptr[w.slot], ctx->cur);
-    ctx->ptr[w.slot] = nullptr;
-    ctx->cap[w.slot] = 0;
-  }
-  ctx->sc_nb = -1;  // the screen's tile list may have been among them
+  for (const SlotSize& w : want) slot_free(ctx, w.slot, ctx->cur);
   return false;
 }
 
@@ -526,16 +529,10 @@ int32_t bna_ctx_set_option(bna_ctx* ctx, int32_t option, int64_t value) {
 // pool's cached memory then goes back to the driver); the caller guarantees
 // that no work using the arena is pending on any other stream.
 void bna::arena_release(bna_ctx* ctx, cudaStream_t st, bool to_driver) {
-  for (int s = 0; s < S_COUNT; ++s) {
-    if (ctx->ptr[s]) cudaFreeAsync(ctx->ptr[s], st);
-    ctx->ptr[s] = nullptr;
-    ctx->cap[s] = 0;
-  }
+  for (int s = 0; s < S_COUNT; ++s) slot_free(ctx, s, st);
   cudaStreamSynchronize(st);
   if (to_driver)
     if (cudaMemPool_t pool = lib_pool(ctx->device)) cudaMemPoolTrimTo(pool, 0);
-  ctx->tiles_nb = -1;  // the tile lists lived in the arena
-  ctx->sc_nb = -1;
   ctx->last_ok = false;
   if (ctx->ecg.exec) cudaGraphExecDestroy(ctx->ecg.exec);
   ctx->ecg = EcGraph();
