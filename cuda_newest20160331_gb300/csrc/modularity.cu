@@ -591,6 +591,9 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
       for (int q = threadIdx.x; q < nr; q += kModThreads) stage[q] = __ldcg(ypc + q);
       __syncthreads();
     }
+    // set in the previous step; read before the barrier behind the gathers, since the
+    // thread that keeps the factor may set it in this one right after it
+    const bool go_deep = !deep && deep_s != 0;
     auto spmv = [&](auto fast) {
       constexpr bool kFast = decltype(fast)::value;
       const float2* st = staged ? stage : nullptr;
@@ -615,7 +618,6 @@ __device__ bool lead_vector(const ModArgs& a, ModGroup* g, int r, int b0, int nb
     // + (sumBG - beta) x_{s-1}) (:344)
     float2 pe[4] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f),
                     make_float2(0.0f, 0.0f)};
-    const bool go_deep = !deep && deep_s != 0;  // set in the previous step, the same in all threads
     for (int p = p0 + (int)threadIdx.x; p < p1; p += kModThreads) {
       if (!one) own = node(p);
       if (own.k == 0.0f) {
