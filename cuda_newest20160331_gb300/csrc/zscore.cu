@@ -379,8 +379,12 @@ __device__ __forceinline__ float z_near(float x, const VoxStat& v, float rel, bo
   // |mean|), times inv
   const uint32_t qb = __float_as_uint(qh);
   const uint32_t e8 = (qb >> 23) & 0xFFu;
-  if (e8 >= 25u && e8 <= 253u && (qb & 0x7FFFFFu) != 0u) {
-    const float half_ulp = __uint_as_float((e8 - 24u) << 23);
+  // half the spacing to the neighbouring floats, half of that below a power of two
+  // (a two-level series of 4^k samples has z = +-2^-k throughout; sent to the exact
+  // path, 45,000 x 256 of them took 39 ms instead of 0.13)
+  const uint32_t sp = (qb & 0x7FFFFFu) ? 24u : 25u;
+  if (e8 > sp && e8 <= 253u) {
+    const float half_ulp = __uint_as_float((e8 - sp) << 23);
     const float bound = fabsf(qh) * rel + (fabsf(x) + fabsf(v.m0)) * fabsf(v.ih) *
                                               1.3552527e-20f /* 2^-66 */;
     ok = half_ulp - fabsf(ql) > bound;
