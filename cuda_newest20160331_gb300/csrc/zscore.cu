@@ -33,7 +33,10 @@
 //     midpoint (or in the float subnormal range), where the IEEE division is
 //     redone; the float rounding is done on the bits.
 // Voxels outside the fixed-point form (more than 2^53 units, subnormal or
-// non-finite samples, extreme scales) take sequential double sums throughout.
+// non-finite samples, extreme scales) take sequential double sums throughout;
+// so do the squares of every voxel of a series longer than kZNearT, since the share
+// of elements that fail the test grows with T and so does the sum that each of
+// them adds (30,000 steps: 39 ms for 10,000 voxels where the sums up front take 7).
 //
 // Two kernels:
 //   zscore_stats_kernel  32 voxels per block, the time steps dealt out to its
@@ -66,6 +69,12 @@ constexpr int kZStatWarps = 8;  // time slices per block of 32 voxels
 // Time steps per emit block: kZEmitT, fewer (in chunks of 64) where that leaves
 // less than kZEmitBlocks blocks: 4,096 x 240 took 13.0 us in 128 blocks, 9.3 in 512.
 constexpr int kZEmitT = 256, kZEmitBlocks = 608;
+// Longest series whose norms come from the integer sums (45,000 x 5,000: 3.4 ms, 4.6
+// with exact sums up front; 4,000 x 10,000: 2.6 against 1.4).
+constexpr int kZNearT = 8192;
+// Voxels of a block outside the integer form from which one warp adds all their
+// sums, a lane each (fewer: a warp each).
+constexpr int kZSlowLanes = 8;
 
 // Per-voxel statistics handed from the stats kernel to the emit kernel.
 struct VoxStat {
@@ -184,13 +193,64 @@ static __device__ __noinline__ double zs_centred_sum(const float* bold, int N, i
   return s;
 }
 
-__global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
+// The reference's sequential sums of the block's 32 voxels (samples, or the squares
+// of the centred ones): warp 0 adds, a lane per voxel, in 64 cycles per step, while
+// the others form the next 32 steps' terms.  Every thread gives its lane's mean;
+// warp 0 gets the sums.  Bound: the FP64 pipe (30,000 voxels x 10,000 integer samples
+// 4.6 ms, 20,000 x 15,000 floats 7.5; a warp per voxel 9.0 and 16.2).  A block whose
+// every voxel spans more binades than the integer form (no scanner's do) takes the
+// two chains after a sweep for nothing: 45,000 x 240 0.30 ms, 0.26 without the sweep.
+constexpr int kZTerms = 32;
+
+static __device__ __noinline__ double zs_block_sums(const float* bold, int N, int T, int gv,
+                                                    bool centred, double mean,
+                                                    double (*terms)[kZTerms][32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kW = kZStatWarps - 1, kPer = (kZTerms + kW - 1) / kW;
+  const int chunks = (T + kZTerms - 1) / kZTerms;
+  auto form = [&](int c) {  // warps 1 and up; steps past the end add 0
+    float xs[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int t = c * kZTerms + warp - 1 + k * kW;
+      xs[k] = gv < N && t < T ? __ldg(bold + (size_t)t * N + gv) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int q = warp - 1 + k * kW;
+      if (q >= kZTerms) break;
+      double p = f2d_exact(xs[k]);
+      if (centred) {
+        p = __dsub_rn(p, mean);
+        p = __dmul_rn(p, p);
+      }
+      terms[c & 1][q][lane] = c * kZTerms + q < T ? p : 0.0;
+    }
+  };
+  double s = 0.0;
+  if (warp > 0) form(0);
+  __syncthreads();
+  for (int c = 0; c < chunks; ++c) {
+    if (warp > 0) {
+      if (c + 1 < chunks) form(c + 1);
+    } else {
+#pragma unroll 8
+      for (int k = 0; k < kZTerms; ++k) s = __dadd_rn(s, terms[c & 1][k][lane]);
+    }
+    __syncthreads();
+  }
+  return s;
+}
+
+__global__ __launch_bounds__(kZStatWarps * 32, 5) void zscore_stats_kernel(
     const float* __restrict__ bold, int N, int T, VoxStat* __restrict__ vs,
     uint8_t* __restrict__ bad, float* __restrict__ e2, uint8_t* __restrict__ blockbad) {
   __shared__ uint32_t pmax[kZStatWarps][32], pmin[kZStatWarps][32];
   __shared__ long long pacc[kZStatWarps][32], pmag[kZStatWarps][32];
   __shared__ ulonglong2 pq[kZStatWarps][32];
-  __shared__ int nslow, slow_v[32], slow_finite[32];
+  __shared__ int nslow, slow_v[kZSlowLanes], slow_finite[kZSlowLanes];
+  __shared__ uint32_t lane_sums, lane_means;  // voxels whose sums are added a lane each
+  __shared__ double mean_s[32], terms[2][kZTerms][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gv = blockIdx.x * 32 + lane;  // the grid covers n_pad / 32 blocks
   const bool live = gv < N;
@@ -218,7 +278,6 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
   });
   pmax[warp][lane] = mx;
   pmin[warp][lane] = mn;
-  if (threadIdx.x == 0) nslow = 0;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kZStatWarps; ++w) {
@@ -232,20 +291,41 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
   const int eb = (int)(mx >> 23) - head;  // biased exponent whose ulp is the unit
   const int emin = (int)((mn + 1u) >> 23);
   bool exact = mx == 0u || (mx < 0x7F800000u && mn + 1u >= 0x800000u && emin >= eb);
+  // a long series takes the integer sum alone, for the mean, if sum |x| < T 2^24
+  // of the largest ulps is surely within 2^53 of the smallest for the whole block
+  const bool longT = T > kZNearT;
+  if (longT && !__all_sync(0xffffffffu, mx == 0u || (exact && (int)(mx >> 23) - emin + 24 + 32 -
+                                                                  __clz(T) <= 53)))
+    exact = false;
   const int e0 = eb - 150;
   unsigned long long mag = 0, neg = 0, qlo = 0, qhi = 0;
-  if (__any_sync(0xffffffffu, exact))
-    each([&](uint32_t b) {
-      const uint32_t m24 = (b << 1) ? (b & 0x7FFFFFu) | 0x800000u : 0u;
-      const int sh = max((int)((b >> 23) & 0xFFu) - eb, 0) & 31;
+  if (__any_sync(0xffffffffu, exact)) {
+    auto units = [&](uint32_t b, int& sh) {  // |x| in units of the unit's ulp, less the shift
+      sh = max((int)((b >> 23) & 0xFFu) - eb, 0) & 31;
+      return (b << 1) ? (b & 0x7FFFFFu) | 0x800000u : 0u;
+    };
+    auto add = [&](uint32_t b, uint32_t m24, int sh) {
       const unsigned long long m = (unsigned long long)m24 << sh;
       mag += m;
       neg += (b >> 31) ? m : 0ull;
-      const unsigned long long sq = (unsigned long long)m24 * m24;  // < 2^48
-      const unsigned long long lo = sq << (2 * sh), hi = (sq >> 1) >> (63 - 2 * sh);
-      qlo += lo;
-      qhi += hi + (qlo < lo ? 1u : 0u);
-    });
+    };
+    if (longT)
+      each([&](uint32_t b) {
+        int sh;
+        const uint32_t m24 = units(b, sh);
+        add(b, m24, sh);
+      });
+    else
+      each([&](uint32_t b) {
+        int sh;
+        const uint32_t m24 = units(b, sh);
+        add(b, m24, sh);
+        const unsigned long long sq = (unsigned long long)m24 * m24;  // < 2^48
+        const unsigned long long lo = sq << (2 * sh), hi = (sq >> 1) >> (63 - 2 * sh);
+        qlo += lo;
+        qhi += hi + (qlo < lo ? 1u : 0u);
+      });
+  }
   pacc[warp][lane] = (long long)(mag - 2 * neg);
   pmag[warp][lane] = (long long)mag;
   pq[warp][lane] = make_ulonglong2(qlo, qhi);
@@ -278,6 +358,7 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
     const float aih = fabsf(o.ih);
     return o.nrm > 0.0 && isfinite(o.nrm) && aih >= 1.0e-30f && aih <= 1.0e30f;
   };
+  bool split = false;  // set_mean's verdict (warp 0)
   if (warp == 0) {
     // one thread per voxel joins the slices
     long long acc = 0, sum = 0;
@@ -295,11 +376,11 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
     bool slow = false;
     if (live) {
       slow = !exact;
-      if (!slow) {
+      if (exact) {
         // exact integer -> double (at most 53 significant bits), then the
         // exact power-of-two scale
         const double unit = ldexp(1.0, e0);
-        const bool split = set_mean(__ddiv_rn(__dmul_rn(__ll2double_rn(acc), unit), (double)T));
+        split = set_mean(__ddiv_rn(__dmul_rn(__ll2double_rn(acc), unit), (double)T));
         // T q - acc^2 is 0 for a constant voxel, whose centred samples are
         // exactly 0 in the reference too
         const long long m = acc < 0 ? -acc : acc;
@@ -312,21 +393,45 @@ __global__ __launch_bounds__(kZStatWarps * 32) void zscore_stats_kernel(
             set_norm(__ddiv_rn(__dmul_rn(__dmul_rn(nd, unit), unit), (double)T));
         o.fast = split && scale;
         o.near = num != 0 ? 1 : 0;
-        slow = o.near && !o.fast;
+        slow = longT || (o.near && !o.fast);
       }
     }
-    if (slow) {
-      const int k = atomicAdd(&nslow, 1);
+    const uint32_t todo = __ballot_sync(0xffffffffu, slow);
+    const bool lanes = longT || __popc(todo) > kZSlowLanes;
+    const bool exact_all = __all_sync(0xffffffffu, exact || !live);
+    if (slow && !lanes) {
+      const int k = __popc(todo & ((1u << lane) - 1u));
       slow_v[k] = gv;
       slow_finite[k] = mx < 0x7F800000u ? 1 : 0;
-    } else {
-      vs[gv] = o;
     }
+    if (lane == 0) {
+      nslow = lanes ? 0 : __popc(todo);
+      lane_sums = lanes ? todo : 0u;
+      lane_means = lanes && !(longT && exact_all) ? todo : 0u;
+    }
+    if (!slow) vs[gv] = o;
     bad[gv] = 0;
     if (blockbad && (gv & (kBlk - 1)) == 0) blockbad[gv / kBlk] = 0;
     if (e2) e2[gv] = 0.0f;  // the emit kernel adds to it
   }
   __syncthreads();
+  // many voxels outside the integer form, or a long series: a lane per voxel
+  if (lane_sums) {
+    const bool slow = (lane_sums >> lane) & 1u;
+    if (lane_means) {
+      const double s1 = zs_block_sums(bold, N, T, gv, false, 0.0, terms);
+      if (warp == 0 && slow) split = set_mean(__ddiv_rn(s1, (double)T));
+    }
+    if (warp == 0) mean_s[lane] = o.mean;
+    __syncthreads();
+    const double s2 = zs_block_sums(bold, N, T, gv, true, mean_s[lane], terms);
+    if (warp == 0 && slow) {
+      o.near = 0;
+      o.fast = set_norm(s2) && split;
+      vs[gv] = o;
+    }
+    return;
+  }
   // voxels outside the integer form: the reference's sums, a warp per voxel
   for (int k = warp; k < nslow; k += kZStatWarps) {
     const int v = slow_v[k];
