@@ -374,7 +374,7 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
         CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
       }
       if (pass == 0 && a.zq) {
-        const float limit = screen_limit(a.th, default_delta(precision, a.T));
+        const float limit = screen_limit(a.th, default_delta(precision, a.T), a.T);
         if (screen_pays(ctx, a.nb, a.T, limit))
           return screened_pass(ctx, a, precision, limit, sched, st);
       }
@@ -658,7 +658,7 @@ int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
   if (prec != BNA_PREC_FP32) {
     const Threshold th{opts->mode, rule_tau(opts), (float)delta};
     q8 = screen_pays(ctx, round_up(N, kBlk) / kBlk, T,
-                     density ? 1.0f : screen_limit(th, default_delta(prec, T)));
+                     density ? 1.0f : screen_limit(th, default_delta(prec, T), T));
   }
   s = run_zscore(ctx, bold_dev, N, T, prec == BNA_PREC_BF16X3, a, st, q8);
   if (s) return s;

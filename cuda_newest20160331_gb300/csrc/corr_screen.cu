@@ -9,7 +9,7 @@
 // kernel; rows z have unit norm),
 //   |z_i . z_j - q_i . q_j| <= e_i + e_j + e_i e_j,
 // so a tile whose largest q_i . q_j stays below the count pass's lower limit by
-// that, by the form's own error and by kAccSlack holds nothing.  The tiles that
+// that, by the form's own error and by acc_slack holds nothing.  The tiles that
 // remain go to the count kernel, which computes them as ever: graph, values and
 // candidates do not depend on the screen.
 //
@@ -32,6 +32,8 @@
 // the probe hit (1 of 64 tiles is then screened).
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -48,10 +50,18 @@ constexpr uint64_t kScWaitNs = 4000000000ull;
 constexpr int kScQ = 8;          // queue of claimed tiles
 constexpr int kScRun = 16;       // tiles claimed at a time
 constexpr int kScRunRich = 64;   // the same where the last probes hit
-// Largest |sum of the tensor core's rounding errors| allowed for: 38 steps of
-// K = 32 at T = 1,200 with an accumulator of 13 fraction bits (the least any
-// generation has been seen to keep for 8-bit operands) stay below 0.005.
+// Allowance for the tensor core's rounding of sum q_i q_j.  Measured on GB300 (sums
+// of powers of two that cancel): a step of K = 32 keeps its products and the
+// accumulator down to 2^-25 of the largest's power of two and leaves 24 bits of the
+// sum, both truncated.  Products and sums stay below 2 (rows of unit norm, e_i <
+// 0.1), so a step loses less than 33 x 2^-25 + 2^-23; unit-norm rows of 10,240 steps
+// were off by 6.4e-6 at most, where that allows 3.5e-4.  Twice the bound, and no
+// less than kAccSlack.
 constexpr float kAccSlack = 0.01f;
+static double acc_slack(int T) {
+  const double steps = (T + 31) / 32;
+  return std::max((double)kAccSlack, 2.0 * 37.0 * std::ldexp(1.0, -25) * steps);
+}
 
 struct ScSmem {
   uint64_t full[kScStages], empty[kScStages], tfull, tempty[2], done, ebar;
@@ -438,13 +448,13 @@ cudaError_t launch_screen_list(int nb, int band, int2* out, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The lower limit the screen works to for a rule's count pass (th) and a form
-// whose values lie within form_delta of the exact ones; 0 where it does not
-// apply: rules that a pair below the limit, or with a NaN voxel, can satisfy.
-float screen_limit(const Threshold& th, double form_delta) {
+// The lower limit the screen works to for a rule's count pass (th) on series of T
+// steps and a form whose values lie within form_delta of the exact ones; 0 where it
+// does not apply: rules that a pair below the limit, or with a NaN voxel, can satisfy.
+float screen_limit(const Threshold& th, double form_delta, int T) {
   const float lo = th.tau - th.delta;
   if (!(th.tau < 1.0f - th.delta) || !(lo > 0.0f)) return 0.0f;
-  const float lim = lo - (float)form_delta - kAccSlack - 1e-5f;
+  const float lim = lo - (float)form_delta - (float)acc_slack(T) - 1e-5f;
   return lim > 0.0f ? lim : 0.0f;
 }
 

@@ -108,7 +108,7 @@ cudaError_t launch_block_bad(const uint8_t* bad, int nb, uint8_t* blockbad, cuda
                              const float* e2 = nullptr, float* eblk = nullptr);
 long long sc_tile_count(int nb);
 cudaError_t launch_screen_list(int nb, int band, int2* out, cudaStream_t st);
-float screen_limit(const Threshold& th, double form_delta);
+float screen_limit(const Threshold& th, double form_delta, int T);
 cudaError_t launch_corr_screen(const CorrArgs& a, float limit, const int2* sup, int nsup,
                                uint8_t* keep, bool ends, int grid, unsigned int* sched,
                                cudaStream_t st);
