@@ -211,7 +211,7 @@ int32_t tc_tiles(bna_ctx* ctx, int nb, cudaStream_t st) {
     // built on the device in stream order: no host wait for the work ahead
     const long long nt = tc_tile_count(nb);
     // every s-th tile: the sample the density histogram may be taken on
-    const int s = (int)std::max<long long>(kSampleStep, nt / kSampleTiles);
+    const int s = (int)std::max<long long>(1, nt / kSampleTiles);
     const long long nsmp = (nt + s - 1) / s;
     int2 *d, *ds;
     ENSURE(S_TILES, (size_t)nt * sizeof(int2), d);
@@ -714,7 +714,7 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
   // density with a tensor-core form: the k-th value is selected on the device;
   // its window comes first from a histogram of sampled tiles, and from the
   // full histogram if the sample's window missed
-  bool sampled = density && k_dens > 0 && tc && !ctx->avg && ctx->ntiles >= kSampleTiles;
+  bool sampled = density && k_dens > 0 && tc && !ctx->avg && ctx->ntiles >= 4 * kSampleTiles;
   bool dev_sel = density && k_dens > 0 && tc && !ctx->avg;
   bool hist_all = !dev_sel;  // bins for every value
   double winA = 0, winB = 0;

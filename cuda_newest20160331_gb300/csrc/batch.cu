@@ -45,7 +45,7 @@ int32_t batch_hist(bna_ctx* ctx, BatchSubj& b, int prec, bool hist_all, unsigned
   a.hist = hist;
   a.th.mode = BNA_THR_R_GE;
   a.th.delta = (float)b.delta;
-  b.sampled = ctx->ntiles >= kSampleTiles;
+  b.sampled = ctx->ntiles >= 4 * kSampleTiles;
   b.cut = hist_all ? -2.0f
                    : hist_cut_for(b.k_dens, b.sampled, b.N,
                                   b.sampled ? ctx->ntiles_smp : ctx->ntiles, b.T);

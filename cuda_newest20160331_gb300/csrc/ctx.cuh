@@ -216,12 +216,14 @@ struct EcGraph {
 };
 
 constexpr int kGraphIters = 32;
-// Density rule: problems of at least kSampleTiles tiles take the histogram that
-// locates the k-th value on every s-th tile, s = kSampleStep or more, so that about
-// kSampleTiles or fewer are taken (12,289 x 600 at 0.5 %, 2,401 tiles: 168 us on
-// all of them, 57 on every fourth; the request 2.10 -> 2.07 ms).
+// Density rule: the histogram that locates the k-th value runs on about this
+// many tiles (every s-th tile) when the problem has at least 4x as many.  The
+// margin of a sample is that of single pairs, but tiles are sampled, and in a
+// network whose correlated voxels lie together few of them hold the edges: every
+// fourth of 2,048 to 8,191 tiles missed the window on most such networks, and the
+// second histogram and count pass took 12,289 x 1,000 from 1.44 to 1.93 ms (one on
+// every tile costs unrelated series 0.1 ms there).
 constexpr int kSampleTiles = 2048;
-constexpr int kSampleStep = 4;
 // Row blocks per band of the tensor-core tile list (BNA_OPT_TILE_BAND): 64
 // keeps a band's row operands (T = 1200: 64 x 0.6 MB) and the column pairs in
 // flight in L2 and reads every column pair from DRAM once per band (measured
