@@ -195,11 +195,17 @@ int32_t tc_prepare(bna_ctx* ctx, const CorrArgs& a, cudaStream_t st) {
 // ordinary series) by kScreenSigma standard deviations of a chance correlation
 // of T samples - below that nearly every tile of 32,768 unrelated pairs
 // reaches it - and the pass has to be long against the screen's own launches:
-// series from kScreenMinT steps on, kScreenTiles tiles per SM.  Measured (rule,
-// count pass without -> with): 180,000 x 1,200 in 60 networks, r >= 0.4,
-// 60.4 -> 15.7 ms; every tile with edges (unrelated loadings), 60,000 x 1,000,
-// 5.50 -> 5.60 ms, 15,000 x 600, 0.245 -> 0.271 ms.
-constexpr int kScreenMinT = 512, kScreenTiles = 16;
+// series from kScreenMinT steps on, kScreenTiles tiles per SM.  Measured (r >= 0.45,
+// the whole build without -> with the screen and its operands), 60 contiguous
+// networks, then unrelated loadings, where nearly every tile holds edges:
+//   12,500 x 520   0.43 -> 0.36 ms   0.35 -> 0.40   (below the line)
+//   16,000 x 520   0.54 -> 0.42      0.46 -> 0.51   (below the line)
+//   20,000 x 520   0.70 -> 0.50      0.62 -> 0.66
+//   28,000 x 1,200 2.02 -> 1.05      2.01 -> 2.08
+//   45,000 x 1,200 4.49 -> 1.84      4.50 -> 4.63
+//   100,000 x 520 10.41 -> 4.14     10.21 -> 10.29
+// and 180,000 x 1,200, r >= 0.4, count pass 60.4 -> 15.7 ms.
+constexpr int kScreenMinT = 512, kScreenTiles = 40;
 constexpr double kScreenErr = 0.06, kScreenSigma = 4.5;
 static bool screen_pays(const bna_ctx* ctx, int nb, int T, float limit) {
   return T >= kScreenMinT && tc_tile_count(nb) >= (long long)kScreenTiles * ctx->sms &&
