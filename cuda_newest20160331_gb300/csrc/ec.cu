@@ -483,19 +483,82 @@ constexpr int kCoopStageBytes = (kEcCoopMaxN + 1) * (int)sizeof(float2);  // mos
 constexpr int kCoopSlots = 32;                          // most rows per warp
 constexpr long long kCoopStageDeg = 50;                 // entries per row from which to stage
 
+// Rows of more than kCoopWide entries and more than four times the mean are shared
+// out to their block's warps (the first kCoopWideMax of a block): a warp that sums the longest row of a graph with
+// hubs by itself is what an iteration waits for (24,000 vertices, 10 entries per row
+// and hubs of up to 24,000: 110 us per iteration, 40 as launches with a warp per row,
+// 12 so).
+constexpr int kCoopWide = 1024;
+constexpr int kCoopWideMax = 64;
+
+// (sh, sl) += this lane's share of val * x over len entries from b, eight of a lane
+// in flight; STAGE: x in shared memory.
+template <int VK, bool STAGE>
+__device__ __forceinline__ void coop_long(const int32_t* __restrict__ ci,
+                                          const float* __restrict__ val,
+                                          const double* __restrict__ vald, const float2* uf, int b,
+                                          int len, int lane, float& sh, float& sl) {
+  for (int k0 = 0; k0 < len; k0 += 256) {
+    int c[8];
+    float vh[8], vl[8];
+    float2 x[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int k = k0 + 32 * m + lane;
+      const bool ok = k < len;
+      c[m] = ok ? __ldg(ci + b + k) : -1;
+      vh[m] = 1.0f;
+      vl[m] = 0.0f;
+      if (VK == 1) vh[m] = ok ? __ldg(val + b + k) : 0.0f;
+      if (VK == 2) {
+        const float2 d = split_df(ok ? __ldg(vald + b + k) : 0.0);
+        vh[m] = d.x;
+        vl[m] = d.y;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+      x[m] = c[m] < 0 ? make_float2(0.0f, 0.0f) : STAGE ? uf[c[m]] : __ldcg(uf + c[m]);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) df_accum<VK>(sh, sl, vh[m], vl[m], x[m]);
+  }
+}
+
 // (sh, sl)[r] = sum of val * x over the len[r] entries from b[r]; STAGE: x in
-// shared memory.
+// shared memory.  Rows of unlike lengths one after another, where that takes fewer
+// rounds of loads.
 template <int VK, bool STAGE>
 __device__ __forceinline__ void coop_rows(const int32_t* __restrict__ ci,
                                           const float* __restrict__ val,
                                           const double* __restrict__ vald, const float2* uf,
                                           const int (&b)[kCoopRows], const int (&len)[kCoopRows],
                                           int lane, float (&sh)[kCoopRows], float (&sl)[kCoopRows]) {
-  int most = 0;
+  int most = 0, rounds = 0;
 #pragma unroll
   for (int r = 0; r < kCoopRows; ++r) {
     sh[r] = sl[r] = 0.0f;
     most = max(most, len[r]);
+    rounds += (len[r] + 255) >> 8;
+  }
+  if (rounds < (most + 63) >> 6) {
+#pragma unroll 1
+    for (int r = 0; r < kCoopRows; ++r) {
+      int br = b[0], lr = len[0];
+#pragma unroll
+      for (int q = 1; q < kCoopRows; ++q) {
+        br = r == q ? b[q] : br;
+        lr = r == q ? len[q] : lr;
+      }
+      float h = 0.0f, l = 0.0f;
+      coop_long<VK, STAGE>(ci, val, vald, uf, br, lr, lane, h, l);
+#pragma unroll
+      for (int q = 0; q < kCoopRows; ++q)
+        if (r == q) {
+          sh[q] = h;
+          sl[q] = l;
+        }
+    }
+    most = 0;
   }
   for (int k0 = 0; k0 < most; k0 += 64) {
     int c[kCoopRows][2];
@@ -580,6 +643,10 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
   extern __shared__ __align__(16) float2 xs[];  // STAGE: the iterate
   __shared__ float2 rs[kCoopSlots * kCoopWarps];
   __shared__ bool rempty[kCoopSlots * kCoopWarps];
+  __shared__ int2 wide_row[kCoopWideMax];                  // start and length
+  __shared__ float2 wide_part[kCoopWideMax][kCoopWarps];   // the warps' sums
+  __shared__ short wide_of[kCoopSlots * kCoopWarps];       // a row's place in the list, or -1
+  __shared__ int wide_n[kCoopWarps];                       // the warps' numbers of wide rows
   __shared__ double tot_s[5];  // lam2, e1, e2, lambda, 1 / lambda
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nw = gridDim.x * kCoopWarps;
@@ -592,6 +659,27 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
     rb = rp[first + lane * nw];
     rl = max(0, (int)(min((long long)rp[first + lane * nw + 1], nnz_used) - rb));
   }
+  // the wide rows, in the order of warps and slots; their own warps leave them out
+  const int wide_len = (int)max((long long)kCoopWide, 4 * nnz_used / n);
+  const uint32_t wide = __ballot_sync(0xffffffffu, rl > wide_len);
+  if (warp < kCoopWarps && lane == 0) wide_n[warp] = __popc(wide);
+  __syncthreads();
+  int nwide = 0, wq = __popc(wide & ((1u << lane) - 1u));
+  for (int w = 0; w < kCoopWarps; ++w) {
+    wq += w < warp ? wide_n[w] : 0;
+    nwide += wide_n[w];
+  }
+  nwide = min(nwide, kCoopWideMax);
+  if (warp < kCoopWarps) {
+    const bool listed = rl > wide_len && wq < kCoopWideMax;
+    rempty[lane * kCoopWarps + warp] = rl == 0;
+    wide_of[lane * kCoopWarps + warp] = listed ? (short)wq : (short)-1;
+    if (listed) {
+      wide_row[wq] = make_int2(rb, rl);
+      rl = 0;
+    }
+  }
+  __syncthreads();
   // resume from the state block (ec_init_kernel's, or the previous segment's)
   double lam2 = st->lam2, lam_used = st->lambda_used, e1 = st->e1, e2 = st->e2;
   const int it0 = st->iter;
@@ -634,6 +722,24 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
     }
     if (warp < kCoopWarps) {
       if (it < it_end) {
+        for (int q = 0; q < nwide; ++q) {  // this warp's part of every wide row
+          const int2 wr = wide_row[q];
+          const int k0 = (int)((long long)wr.y * warp / kCoopWarps);
+          const int k1 = (int)((long long)wr.y * (warp + 1) / kCoopWarps);
+          float h = 0.0f, l = 0.0f;
+          coop_long<VK, STAGE>(ci, val, vald, STAGE ? xs + odd : uf + cur, wr.x + k0, k1 - k0, lane,
+                               h, l);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const float oh = __shfl_xor_sync(0xffffffffu, h, o);
+            const float ol = __shfl_xor_sync(0xffffffffu, l, o);
+            float s2, e2;
+            two_sum(h, oh, s2, e2);
+            h = s2;
+            l = __fadd_rn(l, __fadd_rn(ol, e2));
+          }
+          if (lane == 0) wide_part[q][warp] = make_float2(h, l);
+        }
         for (int s = 0; s < slots; s += kCoopRows) {
           int b[kCoopRows], len[kCoopRows];
           float sh[kCoopRows], sl[kCoopRows];
@@ -645,10 +751,8 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
           coop_rows<VK, STAGE>(ci, val, vald, STAGE ? xs + odd : uf + cur, b, len, lane, sh, sl);
 #pragma unroll
           for (int r = 0; r < kCoopRows; ++r)
-            if (lane == r && s + r < slots) {
+            if (lane == r && s + r < slots)
               rs[(s + r) * kCoopWarps + warp] = make_float2(sh[r], sl[r]);
-              rempty[(s + r) * kCoopWarps + warp] = len[r] == 0;
-            }
         }
       }
     } else if (it > it0) {
@@ -685,7 +789,13 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
       // y = A (u / lambda) as the reference orders it (weighted-net.cu:160-167):
       // a row without entries gives 0 even when 1 / lambda is infinite (an
       // all-zero iterate), where sum * (1 / lambda) would give 0 * inf = NaN
-      const float2 sm = rs[threadIdx.x];
+      float2 sm = rs[threadIdx.x];
+      if (const int q = wide_of[threadIdx.x]; q >= 0)
+        for (int w = 0; w < kCoopWarps; ++w) {  // in the warps' order
+          float s2, e2;
+          two_sum(sm.x, wide_part[q][w].x, s2, e2);
+          sm = make_float2(s2, __fadd_rn(sm.y, __fadd_rn(wide_part[q][w].y, e2)));
+        }
       const double y = rempty[threadIdx.x] ? 0.0 : ((double)sm.x + (double)sm.y) * inv;
       const double old = __ldcg(u + cur + row);
       u[nxt + row] = y;
