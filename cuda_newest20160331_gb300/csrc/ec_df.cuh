@@ -49,6 +49,16 @@ __device__ __forceinline__ void df_accum(float& sh, float& sl, float vh, float v
 }
 
 constexpr int kEcCoopMaxN = 24576;  // largest graph of the persistent kernel (ec.cu): 192 KB
+// Above kEcCoopDenseN vertices it takes graphs of up to kEcCoopDeg entries per row: an
+// iteration of denser ones streams more than the launches between iterations cost
+// (200 iterations, persistent against the forms of larger graphs: 20,000 x 600 4.9 and
+// 5.7 ms, 24,000 x 500 5.0 and 5.8, 24,000 x 800 8.8 and 7.7, 24,000 x 1,500 16.8 and
+// 12.3, 17,000 x 1,500 9.9 and 9.8).
+constexpr int kEcCoopDenseN = 16384;
+constexpr long long kEcCoopDeg = 700;
+inline bool ec_coop_sized(int n, long long nnz_used) {
+  return n <= kEcCoopMaxN && (n <= kEcCoopDenseN || nnz_used <= kEcCoopDeg * n);
+}
 
 // Entries a row costs beside its own where rows are dealt out by entries
 // (ec_range_kernel: 120,000 vertices in contiguous networks, 645 entries per

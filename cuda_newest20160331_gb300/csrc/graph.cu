@@ -85,7 +85,7 @@ constexpr long long kEcSparseDeg = 2;
 
 // Whether a graph of this size may take the streamed form, and its workspace.
 static bool flow_sized(int n, long long nnz_used) {
-  return n > kEcCoopMaxN && flow_chunks(n) <= kFlowChunkMax &&
+  return !ec_coop_sized(n, nnz_used) && flow_chunks(n) <= kFlowChunkMax &&
          nnz_used >= kFlowMinDeg * flow_chunks(n) * (long long)n &&
          nnz_used + flow_pad() < 0x7fffffffLL;
 }
@@ -109,7 +109,7 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
   CK(cudaMemsetAsync(state, 0, ec_state_bytes(), st));
   CK(launch_ec_init(n, u, uf, parts, state, grid, max_iter, st));
   // the whole iteration as one cooperative persistent launch
-  const int cgrid = ec_coop_grid(n, ctx->sms);
+  const int cgrid = ec_coop_grid(n, nnz_used, ctx->sms);
   if (cgrid > 0) {
     // one launch; with a launch gate, segments of about a millisecond of
     // iterations (each resumes from the state block) with the gate between
