@@ -147,11 +147,13 @@ __device__ __forceinline__ bool sum_pair_ff(const float* __restrict__ zi,
 // 128-bit fixed point and its float is the reference's unless a rounding
 // midpoint lies within the loop's rounding bound (round_sum_u128).  (3) Only
 // then, or with subnormal or non-finite products, does lane 0 run the
-// sequential double adds.
-static __device__ __noinline__ float exact_r_fixed(const float* zi, const float* zj, int T, int lane) {
+// sequential double adds.  (In line: as a function of its own it took 2.5 times as
+// long, and pairs of 30,000 steps, 40 % of which come here, 22.6 ms where the fixed
+// point alone took 17.2; 12.9 in line.)
+__device__ __forceinline__ float exact_r_fixed(const float* zi, const float* zj, int T, int lane) {
   int emin = 1 << 20, emax = -(1 << 20);
   bool special = false;
-#pragma unroll 4
+#pragma unroll 8
   for (int t = lane; t < T; t += 32) {
     const uint32_t b = __float_as_uint(__fmul_rn(__ldg(zi + t), __ldg(zj + t)));
     const int e8 = (int)((b >> 23) & 0xFFu);
@@ -170,11 +172,12 @@ static __device__ __noinline__ float exact_r_fixed(const float* zi, const float*
     done = true;
   } else if (!special && (emax - emin) + 24 + (32 - __clz(T)) <= 62) {  // no int64 overflow
     long long acc = 0, mag = 0;
-    for (int t = lane; t < T; t += 32) {
+#pragma unroll 8
+    for (int t = lane; t < T; t += 32) {  // without a branch: eight rounds of loads in flight
       const uint32_t b = __float_as_uint(__fmul_rn(__ldg(zi + t), __ldg(zj + t)));
       const int e8 = (int)((b >> 23) & 0xFFu);
-      if (e8 == 0) continue;
-      const long long m = (long long)((b & 0x7FFFFFu) | 0x800000u) << (e8 - 150 - emin);
+      const long long m24 = e8 ? (b & 0x7FFFFFu) | 0x800000u : 0u;
+      const long long m = m24 << max(e8 - 150 - emin, 0);  // a product of zero adds nothing
       mag += m;
       acc += (b >> 31) ? -m : m;
     }
