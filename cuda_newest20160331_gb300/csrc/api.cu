@@ -64,6 +64,37 @@ static cudaError_t slot_free(bna_ctx* ctx, int s, cudaStream_t st) {
   return e;
 }
 
+// Slots that only save time: a call that finds no room takes their memory.
+constexpr Slot kOptionalSlots[] = {S_ZQ,       S_E2,         S_EBLK,    S_SC_TILES, S_SC_KEEP,
+                                   S_SC_OUT,   S_SC_COUNT,   S_EC_VAL,  S_EC_C16,   S_EC_SPLIT,
+                                   S_EC_REND,  S_EC_WST};
+
+// Free them in the context and its batch contexts; whether there were any.
+bool release_optional(bna_ctx* ctx) {
+  bool any = false;
+  for (Slot s : kOptionalSlots) {
+    any = any || ctx->ptr[s];
+    slot_free(ctx, s, ctx->cur);
+  }
+  for (bna_ctx* k : ctx->kids) {
+    k->cur = ctx->cur;
+    any = release_optional(k) || any;
+  }
+  return any;
+}
+
+static cudaError_t slot_alloc(bna_ctx* ctx, Slot s, size_t bytes, cudaMemPool_t pool) {
+  if (ctx->arena_limit > 0 &&
+      (size_t)bna_ctx_arena_bytes(ctx) + bytes > ctx->arena_limit)  // as the driver's refusal
+    return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMallocFromPoolAsync(&ctx->ptr[s], bytes, pool, ctx->cur);
+  if (e == cudaSuccess)
+    ctx->cap[s] = bytes;
+  else
+    ctx->ptr[s] = nullptr;
+  return e;
+}
+
 int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
   if (bytes == 0) bytes = 16;
   if (ctx->cap[s] < bytes) {
@@ -75,20 +106,19 @@ int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
     const size_t want = bytes + bytes / 8;  // headroom so small growth does not reallocate
     cudaMemPool_t pool = lib_pool(ctx->device);
     if (!pool) return fail(ctx, BNA_CUDA_ERROR, "no device memory pool");
-    e = cudaMallocFromPoolAsync(&ctx->ptr[s], want, pool, ctx->cur);
+    e = slot_alloc(ctx, s, want, pool);
+    // cached blocks of other sizes go back first, then what earlier calls left of the
+    // workspaces that only save time (those of the call in progress: its entry point)
+    for (int tries = 0; e != cudaSuccess && tries < 2; ++tries) {
+      cudaGetLastError();
+      if (tries == 1 && (ctx->opt_used || !release_optional(ctx))) break;
+      cudaStreamSynchronize(ctx->cur);
+      cudaMemPoolTrimTo(pool, 0);
+      e = slot_alloc(ctx, s, bytes, pool);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
-      cudaStreamSynchronize(ctx->cur);
-      cudaMemPoolTrimTo(pool, 0);  // cached blocks of other sizes go back first
-      e = cudaMallocFromPoolAsync(&ctx->ptr[s], bytes, pool, ctx->cur);
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        ctx->ptr[s] = nullptr;
-        return fail(ctx, BNA_OOM, "cudaMalloc(%zu bytes) failed", bytes);
-      }
-      ctx->cap[s] = bytes;
-    } else {
-      ctx->cap[s] = want;
+      return fail(ctx, BNA_OOM, "cudaMalloc(%zu bytes) failed", bytes);
     }
   }
   *out = ctx->ptr[s];
@@ -102,12 +132,15 @@ int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
 // reach or the context is to keep to the smaller forms.
 bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want) {
   if (ctx->lean) return false;
+  const bool used = ctx->opt_used;
+  ctx->opt_used = true;  // none of them gives way to the next
   bool ok = true;
   for (const SlotSize& w : want) {
     void* p;
     ok = ok && ensure(ctx, w.slot, w.bytes, &p) == BNA_OK;
   }
   if (ok) return true;
+  ctx->opt_used = used;
   for (const SlotSize& w : want) slot_free(ctx, w.slot, ctx->cur);
   return false;
 }
@@ -128,6 +161,7 @@ double default_delta(int precision, int T) {
 int32_t set_device(bna_ctx* ctx, cudaStream_t st) {
   CK(cudaSetDevice(ctx->device));
   ctx->cur = st;
+  ctx->opt_used = false;
   return BNA_OK;
 }
 
@@ -565,6 +599,11 @@ int32_t bna_ctx_trim(bna_ctx* ctx) {
   return BNA_OK;
 }
 
+// A ceiling on the arena, as if the device had no more memory (no part of the ABI).
+extern "C" void bna_ctx_limit_arena(bna_ctx* ctx, int64_t bytes) {
+  ctx->arena_limit = bytes > 0 ? (size_t)bytes : 0;
+}
+
 int64_t bna_ctx_arena_bytes(const bna_ctx* ctx) {
   if (!ctx) return 0;
   int64_t t = 0;
@@ -637,9 +676,9 @@ float bna::rule_tau(const bna_corr_opts* o) {
 }
 
 
-int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
-                     const bna_corr_opts* opts, bna_csr* out_dev, bna_corr_stats* stats,
-                     void* stream) {
+static int32_t corr_csr_once(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
+                             const bna_corr_opts* opts, bna_csr* out_dev, bna_corr_stats* stats,
+                             void* stream) {
   if (!ctx || !bold_dev || !opts || !out_dev || N < 1 || T < 1)
     return fail(ctx, BNA_BAD_ARG, "bna_corr_csr: bad arguments");
   if (!mode_known(opts->mode))
@@ -674,6 +713,19 @@ int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
   }
   CK(cudaEventRecord(ctx->ev[1], st));
   return corr_csr_core(ctx, a, N, T, opts, prec, delta, out_dev, stats, st);
+}
+
+int32_t bna_corr_csr(bna_ctx* ctx, const float* bold_dev, int32_t N, int32_t T,
+                     const bna_corr_opts* opts, bna_csr* out_dev, bna_corr_stats* stats,
+                     void* stream) {
+  int32_t s = corr_csr_once(ctx, bold_dev, N, T, opts, out_dev, stats, stream);
+  if (s == BNA_OOM && ctx->opt_used) {  // the tile screen's workspaces stood in the way
+    release_optional(ctx);
+    ctx->lean = true;
+    s = corr_csr_once(ctx, bold_dev, N, T, opts, out_dev, stats, stream);
+    ctx->lean = false;
+  }
+  return s;
 }
 
 // Everything after the z-scores: count pass(es), candidates, density rule,

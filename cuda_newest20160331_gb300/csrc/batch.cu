@@ -166,9 +166,9 @@ int32_t batch_fill(bna_ctx* ctx, BatchSubj& b, cudaStream_t st) {
 
 }  // namespace
 
-int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev,
-                           const int32_t* N, const int32_t* T, const bna_corr_opts* opts,
-                           bna_csr* out_dev, bna_corr_stats* stats, void* stream) {
+static int32_t batch_once(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev,
+                          const int32_t* N, const int32_t* T, const bna_corr_opts* opts,
+                          bna_csr* out_dev, bna_corr_stats* stats, void* stream) {
   if (!ctx || nsub < 1 || !bold_dev || !N || !T || !opts || !out_dev)
     return fail(ctx, BNA_BAD_ARG, "bna_corr_csr_batch: bad arguments");
   for (int k = 0; k < nsub; ++k)
@@ -408,3 +408,12 @@ int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_
   return BNA_OK;
 }
 
+int32_t bna_corr_csr_batch(bna_ctx* ctx, int32_t nsub, const float* const* bold_dev,
+                           const int32_t* N, const int32_t* T, const bna_corr_opts* opts,
+                           bna_csr* out_dev, bna_corr_stats* stats, void* stream) {
+  int32_t s = batch_once(ctx, nsub, bold_dev, N, T, opts, out_dev, stats, stream);
+  // a subject's context cannot take back what the others hold; this one can
+  if (s == BNA_OOM && release_optional(ctx))
+    s = batch_once(ctx, nsub, bold_dev, N, T, opts, out_dev, stats, stream);
+  return s;
+}

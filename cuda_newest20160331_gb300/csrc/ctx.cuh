@@ -265,6 +265,8 @@ struct bna_ctx {
   int band = kDefaultBand;  // BNA_OPT_TILE_BAND
   int band_now = kDefaultBand;  // the band of the current call (the autotuner's for AUTO)
   bool lean = false;  // leave out the workspaces that only save time (ensure_optional)
+  bool opt_used = false;   // the call in progress uses such workspaces
+  size_t arena_limit = 0;  // bytes the arena may hold (0: what the device gives; tests)
   int sc_nb = -1;     // the screen's tile list: block count and band it was built for
   int sc_band = 0;
   int ntiles = 0;
@@ -325,6 +327,7 @@ struct SlotSize {
   size_t bytes;
 };
 bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want);
+bool release_optional(bna_ctx* ctx);
 void ctx_set_lean(bna_ctx* ctx, bool lean);
 int64_t ec_optional_bytes(int n, long long nnz);
 int64_t request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int64_t cap, bool with_ec,

@@ -169,14 +169,15 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
     fl.nch = flow_chunks(n);
     fl.W = ctx->sms * flow_warps_per_block();
     const size_t ne = (size_t)nnz_used + flow_pad();
+    // what every form needs comes first
+    ENSURE(S_EC_PART, (size_t)n * sizeof(float2), fl.part);
+    ENSURE(S_EC_ROWS, (size_t)(fl.W + 1) * sizeof(int), fl.wrow);
     flow = flow && ensure_optional(ctx, {{S_EC_VAL, ne * 4 * (size_t)fl.vk},
                                          {S_EC_C16, ne * sizeof(uint16_t)},
                                          {S_EC_SPLIT, (size_t)std::max(fl.nch - 1, 1) * n * 4},
                                          {S_EC_REND, (size_t)fl.nch * n * sizeof(int)},
                                          {S_EC_WST, (size_t)fl.nch * fl.W * sizeof(int)}});
     if (flow) {
-      ENSURE(S_EC_PART, (size_t)n * sizeof(float2), fl.part);
-      ENSURE(S_EC_ROWS, (size_t)(fl.W + 1) * sizeof(int), fl.wrow);
       fl.csplit = static_cast<int*>(ctx->ptr[S_EC_SPLIT]);
       fl.c16 = static_cast<uint16_t*>(ctx->ptr[S_EC_C16]);
       fl.val = ctx->ptr[S_EC_VAL];
