@@ -103,7 +103,8 @@ int32_t ensure(bna_ctx* ctx, Slot s, size_t bytes, void** out) {
     cudaError_t e = slot_free(ctx, s, ctx->cur);
     if (e != cudaSuccess)
       return fail(ctx, BNA_CUDA_ERROR, "cudaFreeAsync: %s", cudaGetErrorString(e));
-    const size_t want = bytes + bytes / 8;  // headroom so small growth does not reallocate
+    // headroom so small growth does not reallocate
+    const size_t want = ctx->lean ? bytes : bytes + bytes / 8;
     cudaMemPool_t pool = lib_pool(ctx->device);
     if (!pool) return fail(ctx, BNA_CUDA_ERROR, "no device memory pool");
     e = slot_alloc(ctx, s, want, pool);
@@ -145,7 +146,12 @@ bool ensure_optional(bna_ctx* ctx, std::initializer_list<SlotSize> want) {
   return false;
 }
 
-void ctx_set_lean(bna_ctx* ctx, bool lean) { ctx->lean = lean; }
+// From the next call on, without those workspaces, what the context still holds of
+// them included, and without headroom.
+void ctx_set_lean(bna_ctx* ctx, bool lean) {
+  if (lean) release_optional(ctx);
+  ctx->lean = lean;
+}
 
 double default_delta(int precision, int T) {
   const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23);

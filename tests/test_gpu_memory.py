@@ -90,3 +90,26 @@ def test_build_after_a_streamed_centrality():
     for e in (e1, e2, e3):
         assert e[2] == e0[2] and abs(e[1] - e0[1]) <= 1e-9 * e0[1]
         assert torch.max(torch.abs(e[0] - e0[0])) <= 1e-9 * torch.max(torch.abs(e0[0]))
+
+
+def test_lean_request_after_one_that_was_not():
+    """One slot: a screened request with a streamed centrality, then one that the
+    budget holds only without those workspaces.  The slot gives back what it still
+    has of them, so it stays within the budget."""
+    a, t = 25600, 520  # (from 25,100 voxels on the edge lists come in long chunks)
+    b, need = 31000, {}
+    for n in (a, b):
+        need[n] = bna.request_bytes(n, t, mode="density", value=0.6, cap=bna.density_nnz(n, 0.6))
+    x = {n: bna.synth_bold(n, t, 12, n) for n in (a, b)}
+    with bna.Server(0, slots=1, hbm_budget=2 * need[b]) as s:
+        want = {n: s.wait(s.submit(x[n], mode="density", value=0.6, precision="bf16x3"))
+                for n in (a, b)}
+    budget = need[b] - 1
+    assert need[a] < budget
+    with bna.Server(0, slots=1, hbm_budget=budget) as s:
+        for n in (a, b):
+            r = s.wait(s.submit(x[n], mode="density", value=0.6, precision="bf16x3"))
+            assert r.status == 0 and r.nnz == want[n].nnz
+            assert np.array_equal(r.row_ptr, want[n].row_ptr)
+            assert np.array_equal(r.col_idx, want[n].col_idx)
+        assert s.device_bytes <= budget
