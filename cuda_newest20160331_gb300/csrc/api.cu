@@ -535,7 +535,9 @@ int64_t bna::request_bytes(int32_t N, int32_t T, const bna_corr_opts* opts, int6
     b += n_pad * round_up(T, 128) + n_pad * 4 + ntiles * 13;
   b += nst * 64 + nst * 4 + ntiles * 8 + nb;                   // etab, dense list, tiles, flags
   b += elist * 8;                                              // edge lists
-  b += cand * 16 + (density ? cand * 4 : 0);                   // candidates, values
+  b += cand * 16;                                              // candidates, positions
+  if (density)                                                 // values, selection
+    b += cand * (opts->precision == BNA_PREC_FP32 ? 4 : 17);
   b += (long long)(N + 1) * 4 + nnz * (opts->weighted ? 8 : 4);  // CSR
   if (with_ec) b += (long long)N * (2 * 16 + 8) + 64 * 1024;     // iterates, output, partials
   if (with_ec && !lean) b += ec_optional_bytes(N, nnz);          // the streamed form
