@@ -643,10 +643,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const bool rowbad = slow && e.a.bad[gi];
             const float unc_lim = e.unc_lim;
 #pragma unroll 1
-            for (int c0 = 0; c0 < 4; c0 += 1) {
-#pragma unroll
-              for (int cc = 0; cc < 1; ++cc) {
-                const int c = c0 + cc;
+            for (int c = 0; c < 4; ++c) {  // chunk c's sums lead, in sm[0 .. 31] and un[0]
               uint32_t um = 0;
 #pragma unroll
               for (int g = 0; g < 32; g += 16) {  // 16 values at a time fit the registers
@@ -671,7 +668,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                   for (int k = 0; k < 16; ++k) {
                     float r = __uint_as_float(v[k]);
                     if (AVG == 2) r = fisher_z_half(r);
-                    sm[cc * 32 + g + k] = __float_as_uint(__fadd_rn(__uint_as_float(sm[cc * 32 + g + k]), r));
+                    sm[g + k] = __float_as_uint(__fadd_rn(__uint_as_float(sm[g + k]), r));
                   }
                   continue;
                 }
@@ -705,25 +702,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
 #pragma unroll
                 for (int k = 0; k < 16; ++k)
-                  sm[cc * 32 + g + k] = __float_as_uint(
-                      __fadd_rn(__uint_as_float(sm[cc * 32 + g + k]), __uint_as_float(v[k])));
+                  sm[g + k] = __float_as_uint(
+                      __fadd_rn(__uint_as_float(sm[g + k]), __uint_as_float(v[k])));
               }
-              un[cc] |= um;
-              }
-              uint32_t lead[32];
+              un[0] |= um;
+              uint32_t lead[32];  // the next chunk leads
 #pragma unroll
               for (int k = 0; k < 32; ++k) lead[k] = sm[k];
 #pragma unroll
               for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
 #pragma unroll
               for (int k = 0; k < 32; ++k) sm[96 + k] = lead[k];
-              uint32_t ul[1];
-#pragma unroll
-              for (int k = 0; k < 1; ++k) ul[k] = un[k];
-#pragma unroll
-              for (int k = 0; k < 3; ++k) un[k] = un[k + 1];
-#pragma unroll
-              for (int k = 0; k < 1; ++k) un[3 + k] = ul[k];
+              const uint32_t ul = un[0];
+              un[0] = un[1];
+              un[1] = un[2];
+              un[2] = un[3];
+              un[3] = ul;
             }
           }
           ptx::tc_fence_before();
