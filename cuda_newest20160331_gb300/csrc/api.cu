@@ -67,7 +67,8 @@ static cudaError_t slot_free(bna_ctx* ctx, int s, cudaStream_t st) {
 // Slots that only save time: a call that finds no room takes their memory.
 constexpr Slot kOptionalSlots[] = {S_ZQ,       S_E2,         S_EBLK,    S_SC_TILES, S_SC_KEEP,
                                    S_SC_OUT,   S_SC_COUNT,   S_EC_VAL,  S_EC_C16,   S_EC_SPLIT,
-                                   S_EC_REND,  S_EC_WST};
+                                   S_EC_REND,  S_EC_WST,     S_AVG_ZHI, S_AVG_ZLO,  S_AVG_SUMS,
+                                   S_AVG_UNC};
 
 // Free them in the context and its batch contexts; whether there were any.
 bool release_optional(bna_ctx* ctx) {
@@ -428,8 +429,9 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
         if (t0 > 0) gate(ctx, st, BNA_PHASE_CORR, t0);
         if (ctx->avg)
           CK(launch_corr_tc_avg(a, pass, precision == BNA_PREC_BF16X3 ? 0 : 1, ctx->avg->tc,
-                                ctx->avg->S, ctx->avg->fisher, tiles + t0, std::min(per, nt - t0),
-                                nullptr, ctx->sms, sched, st));
+                                ctx->avg->sums.sums ? 0 : ctx->avg->S, ctx->avg->fisher,
+                                tiles + t0, std::min(per, nt - t0), nullptr, ctx->sms, sched, st,
+                                ctx->avg->sums.sums ? &ctx->avg->sums : nullptr));
         else
           CK(launch_corr_tc(a, pass, precision == BNA_PREC_BF16X3 ? 0 : 1, tiles + t0,
                             std::min(per, nt - t0),

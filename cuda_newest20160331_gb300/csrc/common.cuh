@@ -145,6 +145,18 @@ struct CorrArgs {
   float* cand_apx;            // density, tensor-core forms: r~ of every candidate
 };
 
+// Sums of a multi-subject average between its launches (corr_tc.cu): N (N - 1) / 2
+// floats, the flags of pairs that are recomputed (or null; avg_unc_words words),
+// whether a launch starts from them and whether it leaves them, and the number of
+// subjects of all launches.
+struct AvgSums {
+  float* sums;
+  uint32_t* unc;
+  bool in, out;
+  int nsub_all;
+};
+inline size_t avg_unc_words(int nb) { return (size_t)nb * (nb + 1) / 2 * 128 * 4; }
+
 // Fill-pass store with a range check (an inconsistent count would otherwise
 // write outside the CSR).
 __device__ __forceinline__ void put_edge(const CorrArgs& a, long long pos, int col, float v) {

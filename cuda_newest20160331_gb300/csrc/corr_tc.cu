@@ -94,12 +94,21 @@ struct TcSubj {  // 64-byte aligned through its CUtensorMap members
 constexpr size_t TC_SMEM_BYTES = 1024 + (size_t)TC_RING_BYTES + sizeof(TcSmem);
 static_assert(TC_SMEM_BYTES <= 232448, "shared memory per CTA");
 
+constexpr int kSumsIn = 1, kSumsOut = 2;
+
 struct TcArgs {
   CorrArgs a;
   // multi-subject average (AVG): every tile adds up the values of subj[0 ..
   // nsub); pass 4 writes the averages to packed[idx(i, j)]
   int nsub;
   float* packed;
+  // subjects in several launches: the tiles' sums so far, laid out like packed, and
+  // (or null) the pairs met so far that are recomputed whatever their average, a bit
+  // each: read before the subjects of this launch (kSumsIn), left behind them without
+  // an average being taken (kSumsOut); nsub_all: all launches' subjects
+  float* sums;
+  uint32_t* unc;
+  int sums_mode, nsub_all;
   // multi-subject count pass: tiles4 = (I, J-pair, subject), subj the table
   const int4* tiles4;
   const TcSubj* subj;
@@ -180,7 +189,7 @@ __device__ __forceinline__ bool half_sync(TcSmem& S, int h, uint32_t& phase) {
 // through the same epilogue as one subject's values.  No N (N - 1) / 2 matrix
 // is held: adding each subject into one in HBM, 4 bytes per lane in 32
 // different rows, took 4.07 ms per subject at N = 20,000, T = 180-300.
-template <int PASS, bool ABS, int FORM, bool MULTI = false, int AVG = 0>
+template <int PASS, bool ABS, int FORM, bool MULTI = false, int AVG = 0, bool SUMS = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     corr_tc_kernel(const __grid_constant__ CUtensorMap tm_hi,
                    const __grid_constant__ CUtensorMap tm_lo, const TcArgs p) {
@@ -514,7 +523,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       // chunk c of this warp's values: columns c * 32 .. + 31 of the half-tile,
       // v[k] of row il; unc: columns whose pair is recomputed whatever its value
       // (AVG); bad: the half-tile has a voxel with NaN z-scores
-      auto chunk = [&](uint32_t(&v)[32], int c, uint32_t unc, bool slow, bool rowbad) {
+      auto valid_of = [&](int c) {  // columns of chunk c that are pairs of row il
           const int jb = J * 128 + c * 32;
           uint32_t valid = (jb + 32 <= s_n) ? 0xffffffffu
                                             : (jb >= s_n ? 0u : ((1u << (s_n - jb)) - 1u));
@@ -522,10 +531,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const int lo = il - c * 32 + 1;  // first column index k with jl > il
             valid &= (lo <= 0) ? 0xffffffffu : (lo >= 32 ? 0u : (0xffffffffu << lo));
           }
+          return valid;
+      };
+      // packed upper-triangle index of (gi, j): gi (2n - gi - 1) / 2 + j - gi - 1
+      auto packed_row = [&]() { return (long long)gi * (2LL * s_n - gi - 1) / 2 - gi - 1; };
+      auto chunk = [&](uint32_t(&v)[32], int c, uint32_t unc, bool slow, bool rowbad) {
+          const int jb = J * 128 + c * 32;
+          const uint32_t valid = valid_of(c);
           if (PASS == 4) {
             if (gi < s_n) {
-              // packed upper-triangle index of (gi, j): gi (2n - gi - 1) / 2 + j - gi - 1
-              const long long rowbase = (long long)gi * (2LL * s_n - gi - 1) / 2 - gi - 1;
+              const long long rowbase = packed_row();
 #pragma unroll
               for (int k = 0; k < 32; ++k)
                 if ((valid >> k) & 1u) p.packed[rowbase + jb + k] = __uint_as_float(v[k]);
@@ -627,6 +642,25 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         uint32_t sm[128], un[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 128; ++k) sm[k] = 0u;
+        uint32_t* const uw = SUMS && p.unc && active
+                                 ? p.unc + (subtile_index(I, J, s_nb) * 128 + il) * 4
+                                 : nullptr;
+        if (SUMS && active && (p.sums_mode & kSumsIn)) {
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t valid = gi < s_n ? valid_of(c) : 0u;
+            const float* at = p.sums + packed_row() + J * 128 + c * 32;
+#pragma unroll
+            for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+              sm[96 + k] = (valid >> k) & 1u ? __float_as_uint(at[k]) : 0u;
+            un[0] = un[1];
+            un[1] = un[2];
+            un[2] = un[3];
+            un[3] = uw ? uw[c] : 0u;
+          }
+        }
         bool expired = false;
         for (int sub = 0; sub < nsub; ++sub, ++u) {
           const int acc = u & 1;
@@ -728,8 +762,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           S.abort = 1;
           break;
         }
-        if (active) {
-          const float fs = (float)nsub;
+        if (SUMS && active && (p.sums_mode & kSumsOut)) {
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t valid = gi < s_n ? valid_of(c) : 0u;
+            float* at = p.sums + packed_row() + J * 128 + c * 32;
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+              if ((valid >> k) & 1u) at[k] = __uint_as_float(sm[k]);
+#pragma unroll
+            for (int k = 0; k < 96; ++k) sm[k] = sm[k + 32];
+            if (uw) uw[c] = un[0];
+            un[0] = un[1];
+            un[1] = un[2];
+            un[2] = un[3];
+          }
+        } else if (active) {
+          const float fs = (float)(SUMS ? p.nsub_all : nsub);
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t v[32];  // takes sm[0 .. 31]'s place
@@ -1045,21 +1094,26 @@ cudaError_t launch_corr_tc_multi(const CorrArgs& batch, const void* subj_dev, co
   return cudaGetLastError();
 }
 
-template <int FORM, int AVG>
+template <int FORM, int AVG, bool SUMS = false>
 static void (*tc_avg_kernel(int pass, bool absm))(CUtensorMap, CUtensorMap, TcArgs) {
-  return pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM, false, AVG>
-                             : corr_tc_kernel<0, false, FORM, false, AVG>)
-         : pass == 3 ? corr_tc_kernel<3, false, FORM, false, AVG>
-                     : corr_tc_kernel<4, false, FORM, false, AVG>;
+  return pass == 0   ? (absm ? corr_tc_kernel<0, true, FORM, false, AVG, SUMS>
+                             : corr_tc_kernel<0, false, FORM, false, AVG, SUMS>)
+         : pass == 3 ? corr_tc_kernel<3, false, FORM, false, AVG, SUMS>
+                     : corr_tc_kernel<4, false, FORM, false, AVG, SUMS>;
 }
 
 // The average over the subjects of a table (tc_subj_fill): pass 0 count (+ edge
 // lists), 3 density histogram, 4 the packed averages.  a: the average's own
-// sizes, rule and lists.
+// sizes, rule and lists.  sums: where the subjects take several launches (split
+// form; as kernels of their own: with both in one, four subjects of 20,000 voxels
+// took 2.70 ms instead of 2.58).
 cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
                                int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
-                               int grid, unsigned int* sched, cudaStream_t st) {
-  if (!sched || nsub < 1 || (pass == 4 && !packed)) return cudaErrorInvalidValue;
+                               int grid, unsigned int* sched, cudaStream_t st,
+                               const AvgSums* sums) {
+  if (!sched || nsub < 0 || (pass == 4 && !packed && !sums) || (nsub == 0 && !sums) ||
+      (sums && form != FORM_BF16X3))
+    return cudaErrorInvalidValue;
   TcArgs p{};
   p.a = a;
   p.sched = sched;
@@ -1068,11 +1122,20 @@ cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void
   p.subj = static_cast<const TcSubj*>(subj_dev);
   p.nsub = nsub;
   p.packed = packed;
+  if (sums) {
+    p.sums = sums->sums;
+    p.unc = sums->unc;
+    p.sums_mode = (sums->in ? kSumsIn : 0) | (sums->out ? kSumsOut : 0);
+    p.nsub_all = sums->nsub_all;
+  }
   const int g = grid < ntiles ? grid : ntiles;
   if (g <= 0) return cudaSuccess;
   const bool absm = (a.th.mode == BNA_THR_ABS_GT || a.th.mode == BNA_THR_ABS_GE);
   void (*kern)(CUtensorMap, CUtensorMap, TcArgs);
-  if (form == FORM_BF16X3)
+  if (sums)
+    kern = fisher ? tc_avg_kernel<FORM_BF16X3, 2, true>(pass, absm)
+                  : tc_avg_kernel<FORM_BF16X3, 1, true>(pass, absm);
+  else if (form == FORM_BF16X3)
     kern = fisher ? tc_avg_kernel<FORM_BF16X3, 2>(pass, absm)
                   : tc_avg_kernel<FORM_BF16X3, 1>(pass, absm);
   else

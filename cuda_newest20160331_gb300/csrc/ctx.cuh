@@ -121,7 +121,8 @@ cudaError_t launch_corr_tc(const CorrArgs& a, int pass, int form, const int2* ti
                            const unsigned int* ntiles_dev = nullptr);
 cudaError_t launch_corr_tc_avg(const CorrArgs& a, int pass, int form, const void* subj_dev,
                                int nsub, int fisher, const int2* tiles, int ntiles, float* packed,
-                               int grid, unsigned int* sched, cudaStream_t st);
+                               int grid, unsigned int* sched, cudaStream_t st,
+                               const AvgSums* sums = nullptr);
 size_t tc_subj_bytes();
 bool tc_subj_fill(void* host, int s, const CorrArgs& a, const uint8_t* blockbad, int form,
                   float unc_lim = 1.0f);
@@ -177,7 +178,7 @@ enum Slot {
   S_DENSE, S_VSTAT,
   S_TILES_SMP, S_DSTATE, S_DHIST, S_DCLS, S_DEIDX, S_DEXACT, S_CANDAPX, S_DTIES,
   S_RT_KEEP, S_RT_VALX, S_RT_ROWPTR, S_RT_COL, S_RT_VAL,
-  S_AVG_Z, S_AVG_ZHI, S_AVG_ZLO, S_AVG_BAD, S_AVG_BADZ, S_AVG_SUBJ, S_AVG_TC,
+  S_AVG_Z, S_AVG_ZHI, S_AVG_ZLO, S_AVG_BAD, S_AVG_BADZ, S_AVG_SUBJ, S_AVG_TC, S_AVG_SUMS, S_AVG_UNC,
   S_BATCH_SUBJ, S_BATCH_TILES,
   S_MOD_LABEL, S_MOD_ROWS, S_MOD_LOC, S_MOD_CNT, S_MOD_LRP, S_MOD_LCI, S_MOD_VD, S_MOD_VF,
   S_MOD_RS, S_MOD_Y, S_MOD_PARTS, S_MOD_GROUPS, S_MOD_BLKGRP, S_MOD_ASSIGN, S_MOD_KMOD,
@@ -284,6 +285,7 @@ struct bna_ctx {
     const void* tc;
     int S;
     int fisher;
+    AvgSums sums;  // sums.sums: the subjects have been added up, the passes read the sums
   };
   const Avg* avg = nullptr;
   // batches: one context per subject (their arenas), the host staging of the
