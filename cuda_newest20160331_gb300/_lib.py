@@ -46,7 +46,8 @@ class CorrStats(C.Structure):
                 ("ms_scan", C.c_float), ("ms_fill", C.c_float), ("ms_total", C.c_float),
                 ("passes", C.c_int32), ("kernel_launches", C.c_int32),
                 ("precision", C.c_int32), ("tile_band", C.c_int32),
-                ("reserved", C.c_int32 * 4)]
+                ("count_tiles", C.c_int32), ("screen_tiles", C.c_int32),
+                ("reserved", C.c_int32 * 2)]
 
     def as_dict(self) -> dict:
         return {k: getattr(self, k) for k, _ in self._fields_ if k != "reserved"}

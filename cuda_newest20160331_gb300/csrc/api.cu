@@ -66,9 +66,8 @@ static cudaError_t slot_free(bna_ctx* ctx, int s, cudaStream_t st) {
 
 // Slots that only save time: a call that finds no room takes their memory.
 constexpr Slot kOptionalSlots[] = {S_ZQ,       S_E2,         S_EBLK,    S_SC_TILES, S_SC_KEEP,
-                                   S_SC_OUT,   S_SC_COUNT,   S_EC_VAL,  S_EC_C16,   S_EC_SPLIT,
-                                   S_EC_REND,  S_EC_WST,     S_AVG_ZHI, S_AVG_ZLO,  S_AVG_SUMS,
-                                   S_AVG_UNC};
+                                   S_SC_OUT,   S_EC_VAL,     S_EC_C16,  S_EC_SPLIT, S_EC_REND,
+                                   S_EC_WST,   S_AVG_ZHI,    S_AVG_ZLO, S_AVG_SUMS, S_AVG_UNC};
 
 // Free them in the context and its batch contexts; whether there were any.
 bool release_optional(bna_ctx* ctx) {
@@ -201,9 +200,8 @@ int32_t run_zscore(bna_ctx* ctx, const float* bold, int N, int T, bool need_bf16
                             {S_E2, (size_t)a.n_pad * sizeof(float)},
                             {S_EBLK, (size_t)a.nb * sizeof(float)},
                             {S_SC_TILES, nsup * sizeof(int2)},
-                            {S_SC_KEEP, (nsup + 15) / 16 * 16},
-                            {S_SC_OUT, (size_t)tc_tile_count(a.nb) * sizeof(int2)},
-                            {S_SC_COUNT, sizeof(unsigned int)}})) {
+                            {S_SC_KEEP, (nsup + 15) / 16 * 16 + 16},
+                            {S_SC_OUT, (size_t)tc_tile_count(a.nb) * sizeof(int2)}})) {
     zq = static_cast<uint8_t*>(ctx->ptr[S_ZQ]);
     e2 = static_cast<float*>(ctx->ptr[S_E2]);
     a.eblk = static_cast<float*>(ctx->ptr[S_EBLK]);
@@ -352,6 +350,8 @@ bool window_from_hist(const unsigned int* hh, long long k_dens, bool sampled, in
   return true;
 }
 
+constexpr size_t kScreenHost = 4000;  // its two counts in the pinned buffer
+
 // The count pass behind the tile screen: the tiles that the screen leaves, in
 // one launch that reads their number on the device, or - where launches are
 // bounded (BNA_OPT_TILES_PER_LAUNCH) - in several; a screen launch of half as
@@ -362,15 +362,16 @@ static int32_t screened_pass(bna_ctx* ctx, const CorrArgs& a, int precision, flo
   int2* sup = static_cast<int2*>(ctx->ptr[S_SC_TILES]);  // all by run_zscore
   int2* out = static_cast<int2*>(ctx->ptr[S_SC_OUT]);
   uint8_t* keep = static_cast<uint8_t*>(ctx->ptr[S_SC_KEEP]);
-  unsigned int* n_out = static_cast<unsigned int*>(ctx->ptr[S_SC_COUNT]);
   const size_t nkeep = ((size_t)nsup + 15) / 16 * 16;
+  // behind the flags: the tiles that remain, and those that the screen multiplied
+  unsigned int* n_out = reinterpret_cast<unsigned int*>(keep + nkeep);
   if (ctx->sc_nb != a.nb || ctx->sc_band != ctx->band_now) {
     CK(launch_screen_list(a.nb, ctx->band_now, sup, st));
     ctx->klaunch += 1;
     ctx->sc_nb = a.nb;
     ctx->sc_band = ctx->band_now;
   }
-  CK(cudaMemsetAsync(keep, 0, nkeep, st));
+  CK(cudaMemsetAsync(keep, 0, nkeep + 16, st));
   const int form = precision == BNA_PREC_BF16X3 ? 0 : 1;
   const uint8_t* bb = reinterpret_cast<const uint8_t*>(ctx->ptr[S_BLOCKBAD]);
   const long long per = ctx->tiles_per_launch;
@@ -378,21 +379,22 @@ static int32_t screened_pass(bna_ctx* ctx, const CorrArgs& a, int precision, flo
   for (long long t0 = 0; t0 < nsup; t0 += per_sup, ++ctx->klaunch) {
     if (t0 > 0) gate(ctx, st, BNA_PHASE_CORR, t0);
     CK(launch_corr_screen(a, limit, sup + t0, (int)std::min(per_sup, nsup - t0), keep + t0,
-                          t0 + per_sup >= nsup, ctx->sms, sched, st));
+                          t0 + per_sup >= nsup, ctx->sms, sched, n_out + 1, st));
   }
   CK(launch_screen_compact(keep, sup, (int)nsup, out, n_out, ctx->sms, st));
   ctx->klaunch += 1;
+  unsigned int* left = reinterpret_cast<unsigned int*>(static_cast<char*>(ctx->pinned) + kScreenHost);
+  CK(cudaMemcpyAsync(left, n_out, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+  ctx->screened = true;
   if (per == 0) {
     CK(launch_corr_tc(a, 0, form, out, ctx->ntiles, bb, nullptr, 0, ctx->sms, sched, st, n_out));
     ctx->klaunch += 1;
     return BNA_OK;
   }
-  unsigned int* left = reinterpret_cast<unsigned int*>(static_cast<char*>(ctx->pinned) + 4000);
-  CK(cudaMemcpyAsync(left, n_out, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   const long long n = *left;
   for (long long t0 = 0; t0 < n; t0 += per, ++ctx->klaunch) {
-    gate(ctx, st, BNA_PHASE_CORR, t0);
+    gate(ctx, st, BNA_PHASE_CORR, nsup + t0);  // behind the screen's own tiles
     CK(launch_corr_tc(a, 0, form, out + t0, (int)std::min(per, n - t0), bb, nullptr, 0, ctx->sms,
                       sched, st));
   }
@@ -420,6 +422,7 @@ int32_t corr_pass(bna_ctx* ctx, const CorrArgs& a, int precision, int pass, cuda
         ENSURE(S_TCSCHED, 2 * sizeof(unsigned int), sched);
         CK(cudaMemsetAsync(sched, 0, 2 * sizeof(unsigned int), st));
       }
+      if (pass == 0) ctx->screened = false;
       if (pass == 0 && a.zq) {
         const float limit = screen_limit(a.th, default_delta(precision, a.T), a.T);
         if (screen_pays(ctx, a.nb, a.T, limit))
@@ -1088,6 +1091,12 @@ int32_t bna::corr_csr_core(bna_ctx* ctx, CorrArgs& a, int32_t N, int32_t T,
     stats->kernel_launches = ctx->klaunch + fill_launches;
     stats->precision = prec;
     stats->tile_band = prec != BNA_PREC_FP32 ? ctx->band_now : 0;
+    if (prec != BNA_PREC_FP32) {
+      const unsigned int* sc = reinterpret_cast<const unsigned int*>(
+          static_cast<const char*>(ctx->pinned) + kScreenHost);
+      stats->count_tiles = ctx->screened ? (int32_t)sc[0] : ctx->ntiles;
+      stats->screen_tiles = ctx->screened ? (int32_t)sc[1] : 0;
+    }
     cudaEventElapsedTime(&stats->ms_zscore, ctx->ev[0], ctx->ev[1]);
     cudaEventElapsedTime(&stats->ms_count, ctx->ev[1], ctx->ev[2]);
     cudaEventElapsedTime(&stats->ms_recompute, ctx->ev[2], ctx->ev[3]);

@@ -91,6 +91,7 @@ struct ScArgs {
   uint8_t* keep;        // [nsup] bits: row blocks 2 I2, 2 I2 + 1 remain
   uint8_t last;         // the bits of the list's last tile when it is kept whole
   unsigned int* sched;  // [0]: next tile to claim, [1]: CTAs finished
+  unsigned int* n_screened;  // += tiles multiplied
   uint32_t* err;
 };
 
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(kScThreads, 1)
           }
         }
       }
+      atomicAdd(p.n_screened, m);
       publish(-1);
       for (int s = 0; s < kScStages; ++s)
         if (last_round[s] >= 0)
@@ -466,7 +468,7 @@ float screen_limit(const Threshold& th, double form_delta, int T) {
 
 cudaError_t launch_corr_screen(const CorrArgs& a, float limit, const int2* sup, int nsup,
                                uint8_t* keep, bool ends, int grid, unsigned int* sched,
-                               cudaStream_t st) {
+                               unsigned int* n_screened, cudaStream_t st) {
   CUtensorMap m;
   if (!a.zq || !a.eblk || a.ldq % 128 != 0 || !(limit > 0.0f) || !sched ||
       !tc_map_bytes(&m, a.zq, a.ldq, a.n_pad))
@@ -485,6 +487,7 @@ cudaError_t launch_corr_screen(const CorrArgs& a, float limit, const int2* sup, 
   p.keep = keep;
   p.last = ends && (a.nb & 1) ? 1 : 3;
   p.sched = sched;
+  p.n_screened = n_screened;
   p.err = a.err;
   const int g = grid < nsup ? grid : nsup;
   if (g <= 0) return cudaSuccess;

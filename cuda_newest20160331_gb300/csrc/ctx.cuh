@@ -111,7 +111,7 @@ cudaError_t launch_screen_list(int nb, int band, int2* out, cudaStream_t st);
 float screen_limit(const Threshold& th, double form_delta, int T);
 cudaError_t launch_corr_screen(const CorrArgs& a, float limit, const int2* sup, int nsup,
                                uint8_t* keep, bool ends, int grid, unsigned int* sched,
-                               cudaStream_t st);
+                               unsigned int* n_screened, cudaStream_t st);
 cudaError_t launch_screen_compact(const uint8_t* keep, const int2* sup, int nsup, int2* out,
                                   unsigned int* n_out, int sms, cudaStream_t st);
 // sched: the launch's tile counters (two, zero; the launch leaves them zero)
@@ -184,7 +184,7 @@ enum Slot {
   S_MOD_RS, S_MOD_Y, S_MOD_PARTS, S_MOD_GROUPS, S_MOD_BLKGRP, S_MOD_ASSIGN, S_MOD_KMOD,
   S_MOD_ADJ, S_EC_SPLIT, S_EC_PART, S_EC_ROWS, S_EC_FLAG, S_EC_C16, S_EC_VAL,
   S_EC_REND, S_EC_WST, S_TCSCHED,
-  S_ZQ, S_E2, S_EBLK, S_SC_TILES, S_SC_KEEP, S_SC_OUT, S_SC_COUNT, S_COUNT
+  S_ZQ, S_E2, S_EBLK, S_SC_TILES, S_SC_KEEP, S_SC_OUT, S_COUNT
 };
 
 // Small device block the host reads once per pass.
@@ -268,6 +268,7 @@ struct bna_ctx {
   bool lean = false;  // leave out the workspaces that only save time (ensure_optional)
   bool opt_used = false;   // the call in progress uses such workspaces
   size_t arena_limit = 0;  // bytes the arena may hold (0: what the device gives; tests)
+  bool screened = false;  // the last count pass ran behind the screen
   int sc_nb = -1;     // the screen's tile list: block count and band it was built for
   int sc_band = 0;
   int ntiles = 0;

@@ -114,7 +114,10 @@ typedef struct bna_corr_stats {
   int32_t kernel_launches; /* kernels this call launched */
   int32_t precision;       /* the form that ran (BNA_PREC_AUTO resolved) */
   int32_t tile_band;       /* tensor-core forms: row blocks per band of the tile order */
-  int32_t reserved[4];
+  int32_t count_tiles;     /* single builds, tensor-core forms: 128 x 256 tiles multiplied by
+                              the count pass, */
+  int32_t screen_tiles;    /* and 256 x 256 tiles by its 8-bit tile screen (0: no screen) */
+  int32_t reserved[2];
 } bna_corr_stats;
 
 typedef struct bna_ctx bna_ctx;
@@ -161,7 +164,7 @@ int32_t bna_ctx_set_option(bna_ctx* ctx, int32_t option, int64_t value);
 /* Launch gate (no reference counterpart).  Long passes call gate(user,
  * stream, phase, done) on the calling thread between their launches: before
  * each correlation launch after the first (BNA_PHASE_CORR, done = tiles
- * launched), before each fill chunk after the first (BNA_PHASE_FILL, done =
+ * launched, a tile screen's before the count pass's), before each fill chunk after the first (BNA_PHASE_FILL, done =
  * row blocks filled) and before each centrality launch or graph replay after
  * the first (BNA_PHASE_EC, done = iterations completed).  With a gate set,
  * the fill runs in row-block chunks and a centrality launch or replay holds

@@ -49,8 +49,15 @@ def test_screened_graph_is_the_plain_forms(kind, n, precision, mode, value):
     d = _case(kind, n)
     with bna.Builder(0) as b:
         want = b.corr_csr(d, mode=mode, value=value, precision="fp32").numpy()
-        got = [b.corr_csr(d, mode=mode, value=value, precision=precision).numpy()]
+        one = b.corr_csr(d, mode=mode, value=value, precision=precision)
+        got = [one.numpy()]
         b.set_option("tiles_per_launch", 700)
         got.append(b.corr_csr(d, mode=mode, value=value, precision=precision).numpy())
+    nb = (n + 127) // 128
+    tiles = sum((nb + 1) // 2 - i // 2 for i in range(nb))
+    assert one.stats["screen_tiles"] > 0 or mode == "density"  # a density's limit may be too low
+    assert 0 < one.stats["count_tiles"] <= tiles
+    if kind != "everywhere" and one.stats["screen_tiles"]:
+        assert one.stats["count_tiles"] < tiles // 2
     for g in got:
         assert np.array_equal(g.row_ptr, want.row_ptr) and np.array_equal(g.col_idx, want.col_idx)
