@@ -5,8 +5,8 @@
 // (W/CorMat/CUCorMat/CUCorMat/CorMat.cpp:955-964): float products of the
 // float z-scores, accumulated in double in time order, rounded to float;
 // then post_block's clamp (CorMat.cpp:883; not for the 2mm tools' rule,
-// BNA_THR_R_EPS) and the exact threshold rule.
-// Sequential per pair, so the value is bit-identical to the reference's.
+// BNA_THR_R_EPS) and the exact threshold rule.  The value is bit-identical to the
+// reference's sequential loop (exact_r.cuh).
 //
 // Scan: seg[b][i] (edges of row i in column block b) becomes the exclusive
 // prefix along b, and row_ptr = exclusive prefix of the row totals

@@ -7,8 +7,8 @@
 // never exists.
 //
 // The tile epilogue (count pass) counts edges per row (seg[J][i]) and per
-// column (seg[I][j]), sends near-threshold pairs to the candidate list, and
-// appends the tile's edges with their values to its edge list (one pool
+// column (seg[I][j]) and appends the tile's edges with their values, and its
+// near-threshold pairs flagged as candidates, to its edge list (one pool
 // allocation per tile, slots by a block prefix scan).  The fill pass
 // (csr_fill.cu) places every listed edge at row_ptr[row] + seg[block][row] +
 // its rank in the tile's row (or column) bitmask, writing (i, j) and (j, i).

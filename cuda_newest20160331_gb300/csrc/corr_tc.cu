@@ -18,11 +18,11 @@
 //               one compare per value marks the "interesting" entries (edge or
 //               near-threshold candidate); a warp prefix scan gives their slots
 //               in the sub-tile's compact edge list (warp-private bump
-//               allocator), candidates only flagged; row counts from register
+//               allocator), candidates only flagged there
+//               (collect_candidates_kernel lists them); row counts from register
 //               bitmasks, column counts from a 32 x 32 bit transpose across the
-//               warp; the rare candidates also go to the candidate list
-//               (warp-private chunks).  The fill pass (csr_fill.cu) places the
-//               listed edges; the GEMM runs once.
+//               warp.  The fill pass (csr_fill.cu) places the listed edges; the
+//               GEMM runs once.
 //
 // Every wait is bounded (4 s of wall time); on expiry the kernel raises
 // ERR_TIMEOUT, drains its own copies and MMAs, frees TMEM and returns.

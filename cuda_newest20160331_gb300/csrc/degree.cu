@@ -20,6 +20,7 @@ namespace {
 constexpr int kDegWarps = 4;
 constexpr int kDegWide = 256;   // shortest row taken by itself
 constexpr int kDegChunk = 512;  // its values at a time
+
 __global__ __launch_bounds__(kDegWarps * 32) void degree_kernel(int n,
                                                                 const int32_t* __restrict__ rp,
                                                                 const float* __restrict__ val,

@@ -17,8 +17,8 @@
 //
 // Limits and sharing rules:
 //   - N <= kNoAllocMaxN (262,144 vertices); larger graphs get
-//     BNA_SCRATCH_LIMIT.  The array holds 4 * kNoAllocMaxN doubles plus block
-//     partials and state (about 8 MB); every GPU that loads the library keeps
+//     BNA_SCRATCH_LIMIT.  The array holds 5 * kNoAllocMaxN doubles plus block
+//     partials, row ranges and state (10.5 MB); every GPU that loads the library keeps
 //     it until the process exits.
 //   - Every call shares the array.  Calls that overlap on a GPU (two host
 //     threads, or two streams running at once) race on it; serialise them.

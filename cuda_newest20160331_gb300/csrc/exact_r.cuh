@@ -71,7 +71,8 @@ __device__ __forceinline__ bool round_sum_u128(unsigned __int128 acc, unsigned _
 
 // Lanes per pair: a warp evaluates four pairs at once, or one when its rows are
 // longer than kPairLongT (the undecided share of pairs grows with the square of
-// the products per lane: 0.6 % at T = 1200 with eight lanes, about 10 % at 5000).
+// the products per lane: of pairs near 0.4, 0.6 % at T = 1200 with eight lanes, about
+// 10 % at 5000).
 // With a warp per pair the butterfly outweighed the products: candidates of a
 // TF32 pass (713,000, T = 355) 318 us, 227 with eight lanes each.
 constexpr int kPairLanes = 8, kPairs = 32 / kPairLanes;
@@ -86,8 +87,8 @@ constexpr int kPairLongT = 1600;
 // per lane c holds at most n + 5 errors of at most 2^-24 each, added with as many
 // roundings, so |h + c - sum p_t| <= 1.01 (n + 6)^2 2^-48, and the reference's
 // loop lies within 1.01 T 2^-53 of sum p_t.  When no float rounding midpoint
-// lies within both of h + c, the float nearest to h + c is the reference's
-// (all but about 2^-15 of the pairs at T = 240, 2^-11 at T = 1200).
+// lies within both of h + c, the float nearest to h + c is the reference's (of
+// pairs near 0.4, all but 0.04 % at T = 240 and 0.6 % at 1,200 with eight lanes).
 // Padding columns T .. ldz - 1 of the rows are zero and add nothing.
 // Bound: L2 reads of the two rows.  Of the candidates of a TF32 pass (713,000,
 // T = 355) the fixed-point form alone took 1,118 us.
