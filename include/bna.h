@@ -324,7 +324,7 @@ int32_t bna_ec(bna_ctx* ctx, const bna_csr* csr_dev, int32_t max_iter, double ep
  * the result (a process whose device memory is held by its own pool, an
  * embedder that forbids allocation after load).  Same kernels and results as
  * bna_ec, but the working vectors and iteration state live in a fixed
- * __device__ array of the library (about 8 MB, kept by every GPU that loads
+ * __device__ array of the library (10.5 MB, kept by every GPU that loads
  * the library until exit), so the call allocates nothing; no context is
  * needed.  Call it from ordinary host code, not from a stream callback or a
  * cudaLaunchHostFunc function: it issues CUDA calls (launches, copies, a

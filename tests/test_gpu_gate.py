@@ -9,7 +9,7 @@ import cuda_newest20160331_gb300 as bna
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,T,screened", [(25001, 240, False), (19700, 520, True)])
+@pytest.mark.parametrize("N,T,screened", [(25001, 240, False), (19800, 520, True)])
 def test_gate_of_screened_passes_and_replays(N, T, screened):
     import torch
     x = torch.from_numpy(bna.synth_bold(N, T, 20, 508)).cuda()
@@ -31,6 +31,7 @@ def test_gate_of_screened_passes_and_replays(N, T, screened):
     for phase in (0, 1):
         done = [d for p, d in calls[:n_corr] if p == phase]
         assert len(done) >= 3 and done == sorted(set(done))
+    assert (whole.stats["screen_tiles"] > 0) == screened
     if screened:  # the screen's launches of 750 super-tiles, then the kept tiles'
         nsup = ((N + 127) // 128 + 1) // 2
         assert max(d for p, d in calls[:n_corr] if p == 0) >= nsup * (nsup + 1) // 2

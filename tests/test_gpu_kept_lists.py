@@ -31,6 +31,8 @@ def test_screened_build_after_a_larger_unscreened_one(precision):
         first = b.corr_csr(ds, mode="r_ge", value=0.45, precision=precision)
         mid = b.corr_csr(dl, mode="density", value=20.0, precision=precision)
         again = b.corr_csr(ds, mode="r_ge", value=0.45, precision=precision)
+    assert first.stats["screen_tiles"] == again.stats["screen_tiles"] > 0
+    assert mid.stats["screen_tiles"] == 0
     assert mid.nnz == bna.density_nnz(m, 20.0) and want.nnz > n
     for g in (first.numpy(), again.numpy()):
         assert np.array_equal(g.row_ptr, want.row_ptr) and np.array_equal(g.col_idx, want.col_idx)

@@ -49,6 +49,7 @@ def test_build_without_room_for_the_screen(mode, value):
     with bna.Builder(0) as b:
         want = b.corr_csr(x, **kw)
         most = b.arena_bytes
+    assert want.stats["screen_tiles"] > 0 or mode == "density"
     with bna.Builder(0) as b:
         _lean(b, True)  # without the screen's buffers, and without headroom
         _same(want, b.corr_csr(x, **kw))
