@@ -75,7 +75,7 @@ cudaError_t launch_ec_sparse(int n, const int32_t* rp, const int32_t* ci, const 
 void ec_state_read(const void* host_copy, double* lam2, double* lambda_used, double* e1,
                    double* e2, int* iter, int* done);
 int ec_state_err(const void* host_copy);
-int ec_coop_grid(int n, long long nnz_used, int sms);
+int ec_coop_grid(int n, long long nnz_used, int max_iter, int sms);
 constexpr int kFlowChunkMax = 4;  // column chunks of the streamed centrality (graph.cu)
 int flow_chunks(int n);
 int flow_warps_per_block();

@@ -827,8 +827,8 @@ __global__ __launch_bounds__(kCoopThreads, 1) void ec_coop_kernel(
 // graphs use per-iteration launches: their iterate does not fit beside the block.
 // 20,000 vertices of 4, 60 and 300 entries per row: 17.6, 19.7 and 23.0 us per
 // iteration in launches, 9.0, 12.6 and 20.3 here.  Returns 0 for "use per-iteration launches".
-int ec_coop_grid(int n, long long nnz_used, int sms) {
-  if (!ec_coop_sized(n, nnz_used)) return 0;
+int ec_coop_grid(int n, long long nnz_used, int max_iter, int sms) {
+  if (!ec_coop_sized(n, nnz_used, max_iter)) return 0;
   int per_sm = 0;
   if (cudaFuncSetAttribute(ec_coop_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kCoopStageBytes) != cudaSuccess ||

@@ -53,11 +53,14 @@ constexpr int kEcCoopMaxN = 24576;  // largest graph of the persistent kernel (e
 // iteration of denser ones streams more than the launches between iterations cost
 // (200 iterations, persistent against the forms of larger graphs: 20,000 x 600 4.9 and
 // 5.7 ms, 24,000 x 500 5.0 and 5.8, 24,000 x 800 8.8 and 7.7, 24,000 x 1,500 16.8 and
-// 12.3, 17,000 x 1,500 9.9 and 9.8).
+// 12.3, 17,000 x 1,500 9.9 and 9.8) - in calls of kEcFewIters allowed iterations or
+// more (five: 24,000 x 800 0.29 and 0.42 ms).
 constexpr int kEcCoopDenseN = 16384;
 constexpr long long kEcCoopDeg = 700;
-inline bool ec_coop_sized(int n, long long nnz_used) {
-  return n <= kEcCoopMaxN && (n <= kEcCoopDenseN || nnz_used <= kEcCoopDeg * n);
+constexpr int kEcFewIters = 16;
+inline bool ec_coop_sized(int n, long long nnz_used, int max_iter) {
+  return n <= kEcCoopMaxN &&
+         (n <= kEcCoopDenseN || nnz_used <= kEcCoopDeg * n || max_iter < kEcFewIters);
 }
 
 // Entries a row costs beside its own where rows are dealt out by entries

@@ -50,7 +50,7 @@ cudaError_t launch_ec_range(int n, const int32_t* rp, const int32_t* ci, const f
 void ec_state_read(const void* host_copy, double* lam2, double* lambda_used, double* e1,
                    double* e2, int* iter, int* done);
 int ec_state_err(const void* host_copy);
-int ec_coop_grid(int n, long long nnz_used, int sms);
+int ec_coop_grid(int n, long long nnz_used, int max_iter, int sms);
 cudaError_t launch_ec_coop(int n, const int32_t* rp, const int32_t* ci, const float* val,
                            const double* vald, long long nnz_used, double* u, float2* uf,
                            double* parts, void* st, int grid, int it_end, int max_iter,
@@ -162,7 +162,7 @@ extern "C" int32_t bna_ec_noalloc(const bna_csr* csr_dev, int32_t max_iter, doub
   int it = 0, done = 0;
   // the same choice as bna_ec: small graphs run as one persistent launch
   // (its 2 x grid x 3 partials fit the partials region: grid <= SM count)
-  const int cgrid = std::min(ec_coop_grid(n, nnz_used, sms), kNoAllocMaxGrid / 2);
+  const int cgrid = std::min(ec_coop_grid(n, nnz_used, max_iter, sms), kNoAllocMaxGrid / 2);
   if (cgrid > 0) {
     e = launch_ec_coop(n, csr_dev->row_ptr, csr_dev->col_idx, csr_dev->val, nullptr, nnz_used, u,
                        uf, parts, state, cgrid, max_iter, max_iter, eps, st);

@@ -66,7 +66,7 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
 // ---------------------------------------------------------------- centrality
 
 // The streamed form (ec_flow.cu) copies the graph once per call, about two
-// iterations' traffic, so it takes calls of at least kFlowMinIters allowed
+// iterations' traffic, so it takes calls of at least kEcFewIters allowed
 // iterations, on graphs whose rows have ascending columns, of up to
 // kFlowChunkMax chunks with at least kFlowMinDeg entries per row and chunk on
 // average (a block stages every chunk and walks every row in it: two chunks,
@@ -76,7 +76,6 @@ int32_t bna_csr_rethreshold(bna_ctx* ctx, const bna_csr* in_dev, int32_t mode, d
 // least kFlowFresh of the entries (45,000 vertices, 98 % such entries: 93 us
 // per iteration with a warp per row, 56 streamed; 120,000 in contiguous
 // networks, 43 %: 121 us ranged, 334 in streams, L1 serves the gathers).
-constexpr int kFlowMinIters = 16;
 constexpr double kFlowFresh = 0.6;
 constexpr long long kFlowMinDeg = 65;
 // Graphs of at most this many entries per row on average (those whose
@@ -85,7 +84,7 @@ constexpr long long kEcSparseDeg = 2;
 
 // Whether a graph of this size may take the streamed form, and its workspace.
 static bool flow_sized(int n, long long nnz_used) {
-  return !ec_coop_sized(n, nnz_used) && flow_chunks(n) <= kFlowChunkMax &&
+  return !ec_coop_sized(n, nnz_used, kEcFewIters) && flow_chunks(n) <= kFlowChunkMax &&
          nnz_used >= kFlowMinDeg * flow_chunks(n) * (long long)n &&
          nnz_used + flow_pad() < 0x7fffffffLL;
 }
@@ -109,7 +108,7 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
   CK(cudaMemsetAsync(state, 0, ec_state_bytes(), st));
   CK(launch_ec_init(n, u, uf, parts, state, grid, max_iter, st));
   // the whole iteration as one cooperative persistent launch
-  const int cgrid = ec_coop_grid(n, nnz_used, ctx->sms);
+  const int cgrid = ec_coop_grid(n, nnz_used, max_iter, ctx->sms);
   if (cgrid > 0) {
     // one launch; with a launch gate, segments of about a millisecond of
     // iterations (each resumes from the state block) with the gate between
@@ -155,7 +154,7 @@ static int32_t ec_run(bna_ctx* ctx, int n, const int32_t* rp, const int32_t* ci,
   }
   const bool sparse = nnz_used <= kEcSparseDeg * (long long)n;
   EcFlow fl{};
-  bool flow = max_iter >= kFlowMinIters && flow_sized(n, nnz_used) && !ctx->lean;
+  bool flow = max_iter >= kEcFewIters && flow_sized(n, nnz_used) && !ctx->lean;
   if (flow) {
     unsigned long long* info;
     ENSURE(S_EC_FLAG, 2 * sizeof(unsigned long long), info);

@@ -91,4 +91,5 @@ def test_dense_graphs_above_16384_vertices(n, deg, near):
     rng = np.random.default_rng(n + deg)
     lens = np.full(n, deg) + rng.integers(-3, 4, n)
     lens[:2] = lens[n // 2] = 0
-    _check(*_graph(lens, n, deg, near), iters=12, to_the_end=not near)
+    _check(*_graph(lens, n, deg, near), iters=16, to_the_end=not near)
+    _check(*_graph(lens, n, deg, near), iters=3, to_the_end=False)  # the persistent kernel
